@@ -68,7 +68,7 @@ typedef struct rcmvs_options {
     uint32_t tile_h;         /* stereo tile height in pixels; 0 = default (8) */
     uint32_t flags;          /* RCMVS_FLAG_* bits; 0 = defaults */
     uint32_t threads_per_pixel; /* Jacobi passes: 0 or 1 = one thread per pixel
-                                (default: streamed, see
+                                (default: staged, see
                                 RCMVS_FLAG_LOCKSTEP_PASSES); 5 = five lanes per
                                 pixel, one per window column (tiles of at most
                                 128 pixels).  Same results bit for bit. */
@@ -149,15 +149,19 @@ typedef struct rcmvs_options {
 
 /* The Jacobi passes run one thread per pixel in lockstep (tiles of
  * tile_w x tile_h): a warp runs each candidate slot for as long as its
- * slowest lane needs.  By default (threads_per_pixel 0 or 1) a pass
- * streams the pixels of 16x16 tiles through blocks of 64 threads: each
- * lane evaluates its pixel's candidates one window row at a time, starts
- * the next candidate as soon as one ends and claims the tile's next pixel
- * as soon as its pixel ends.  The streamed passes run as persistent
- * launches and keep each block's random candidates in a device scratch of
- * the scene (48 bytes per tile pixel per resident block, about 29 MB on a
- * 148-SM GPU).  Same results bit for bit (and the same work counters);
- * tile_w/tile_h and the autotuner's shapes then apply to the init only. */
+ * slowest lane needs.  By default (threads_per_pixel 0 or 1) a pass is
+ * staged: the candidates of a 16x16 tile go through the support views
+ * together, one view per stage, and the survivors are packed before the
+ * next; a window term whose pixel a bounded projection is certain of skips
+ * the reference's divide chain.  With RCMVS_COUNT set or
+ * RCMVS_FLAG_NO_SKIP_DUPLICATES the default is the streamed pass instead
+ * (each lane evaluates its pixel's candidates one window row at a time and
+ * claims the tile's next pixel as soon as its pixel ends), whose work counts
+ * are the reference sequence's.  Both run as persistent launches and keep
+ * their candidates in a device scratch of the scene (40 KB per resident
+ * block of the staged pass, about 48 MB on a 148-SM GPU).  Same results bit
+ * for bit; tile_w/tile_h and the autotuner's shapes then apply to the init
+ * only. */
 #define RCMVS_FLAG_LOCKSTEP_PASSES 512u
 
 #define RCMVS_MAX_PASSES 4096u

@@ -189,9 +189,10 @@ struct StereoBatch {
     std::vector<int32_t> start;  // n_jobs + 1
     std::vector<int> order;      // launch position -> caller's job index
     LaunchGeom geom{};
-    // streamed passes (pass_stream_kernel, the default): the jobs' tile starts
-    // in that kernel's tiling (n_jobs + 1) and its launch geometry
-    bool stream = false;
+    // tiled passes (pass_staged_kernel, the default, and pass_stream_kernel):
+    // the kernel (TILED_*), the jobs' tile starts in its tiling (n_jobs + 1)
+    // and its launch geometry
+    int tiled = TILED_NONE;
     std::vector<int32_t> sstart;
     LaunchGeom sgeom{};
 };

@@ -95,16 +95,25 @@ int assemble(rcmvs_ctx* ctx, rcmvs_scene* sc, const rcmvs_job* jobs, int n_jobs,
     if (tiles > INT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "too many tiles in one batch");
     b.start[n_jobs] = (int32_t)tiles;
     b.geom = LaunchGeom{nthr, smem, (int)tiles, nullptr};
-    // the streamed passes' own tiling of the same jobs, in launch order
-    b.sstart.resize(n_jobs + 1);
-    int64_t stiles = 0;
-    for (int p = 0; p < n_jobs; ++p) {
-        b.sstart[p] = (int32_t)stiles;
-        stiles += stream_tiles(b.jobs[p].w, b.jobs[p].h);
+    for (const DevJob& J : b.jobs)
+        for (int q = 0; q < J.nsrc; ++q) b.geom.radial = b.geom.radial || J.src[q].k != 0.0f;
+    for (int j = 0; j < n_jobs; ++j) b.geom.radial = b.geom.radial || sc->cams[jobs[j].ref_idx].k != 0.0;
+    return RCMVS_OK;
+}
+
+// The tiled passes' own tiling of b's jobs, in launch order.
+int assemble_tiled(rcmvs_ctx* ctx, int kind, StereoBatch& b) {
+    b.tiled = kind;
+    b.sstart.resize(b.jobs.size() + 1);
+    int64_t tiles = 0;
+    for (size_t p = 0; p < b.jobs.size(); ++p) {
+        b.sstart[p] = (int32_t)tiles;
+        tiles += tiled_tiles(kind, b.jobs[p].w, b.jobs[p].h);
+        if (tiles > INT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "too many tiles in one batch");
     }
-    if (stiles > INT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "too many tiles in one batch");
-    b.sstart[n_jobs] = (int32_t)stiles;
-    b.sgeom = stream_geom((int)stiles);
+    b.sstart.back() = (int32_t)tiles;
+    b.sgeom = tiled_geom(kind, (int)tiles);
+    b.sgeom.radial = b.geom.radial;
     return RCMVS_OK;
 }
 
@@ -314,7 +323,13 @@ int build_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const rcmvs_job* jobs, int n_jo
     }
     int rc = assemble(ctx, sc, jobs, n_jobs, shp, true, b);
     b.geom.tpp = tpp;
-    b.stream = tpp == 1 && !(opts->flags & RCMVS_FLAG_LOCKSTEP_PASSES);
+    // The staged passes evaluate candidates ahead of the reference's sequence;
+    // work counts and its own call sequence come from the streamed ones.
+    if (rc == RCMVS_OK && tpp == 1 && !(opts->flags & RCMVS_FLAG_LOCKSTEP_PASSES))
+        rc = assemble_tiled(ctx,
+                            ctx->count_work || (opts->flags & RCMVS_FLAG_NO_SKIP_DUPLICATES) ? TILED_STREAM
+                                                                                             : TILED_STAGED,
+                            b);
     return rc;
 }
 
@@ -332,25 +347,25 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
     SCK(sc->arena.get(kSlotJobs, sizeof(DevJob) * n_jobs, &pj));
     SCK(sc->arena.get(kSlotJobStart, sizeof(int32_t) * (n_jobs + 1), &ps));
     const int n_launch = 1 + (int)s.n_passes;
-    // the streamed passes are always persistent (each block owns a slice of
-    // the scratch), so their launches take queue counters too
-    if (s.persistent || b.stream) SCK(sc->arena.get(kSlotQueue, sizeof(unsigned int) * n_launch, &pq));
+    // the tiled passes are always persistent (each block owns a slice of the
+    // scratch), so their launches take queue counters too
+    if (s.persistent || b.tiled) SCK(sc->arena.get(kSlotQueue, sizeof(unsigned int) * n_launch, &pq));
     // pageable -> device copies return once the host data has been staged
     SCK(cudaMemcpyAsync(pj, b.jobs.data(), sizeof(DevJob) * n_jobs, cudaMemcpyHostToDevice, st));
     SCK(cudaMemcpyAsync(ps, b.start.data(), sizeof(int32_t) * (n_jobs + 1), cudaMemcpyHostToDevice, st));
     void *pss = nullptr, *pscr = nullptr;
     LaunchGeom sgeom = b.sgeom;
-    if (b.stream) {
+    if (b.tiled) {
         SCK(sc->arena.get(kSlotStreamStart, sizeof(int32_t) * (n_jobs + 1), &pss));
         SCK(cudaMemcpyAsync(pss, b.sstart.data(), sizeof(int32_t) * (n_jobs + 1), cudaMemcpyHostToDevice, st));
-        sgeom.scratch_blocks = std::min(stream_grid(sgeom), sgeom.tiles);
-        SCK(sc->arena.get(kSlotStreamScratch, stream_scratch_bytes(sgeom.scratch_blocks), &pscr));
-        sgeom.scratch = (float4*)pscr;
+        sgeom.scratch_blocks = std::min(tiled_grid(sgeom), sgeom.tiles);
+        SCK(sc->arena.get(kSlotStreamScratch, tiled_scratch_bytes(b.tiled, sgeom.scratch_blocks), &pscr));
+        sgeom.scratch = (unsigned char*)pscr;
     }
     const DevJob* dj = (const DevJob*)pj;
     const int32_t* dst = (const int32_t*)ps;
-    // the passes' tile starts and geometry (the streamed tiling by default)
-    const int32_t* pst = b.stream ? (const int32_t*)pss : dst;
+    // the passes' tile starts and geometry (the kernel's own tiling by default)
+    const int32_t* pst = b.tiled ? (const int32_t*)pss : dst;
     unsigned int* queue = (unsigned int*)pq;
     // pass flags (the repeat skip) only with the duplicate skip: both off is
     // the reference's own call sequence
@@ -384,7 +399,7 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
                             s.init == Schedule::ONE_CANDIDATE ? 1 : (s.init == Schedule::TABLE ? 2 : 0));
         hk.end(s.init == Schedule::LEARNED ? "learned_init" : "stereo_init");
         if (e) return e;
-        LaunchGeom gp = b.stream ? sgeom : b.geom;
+        LaunchGeom gp = b.tiled ? sgeom : b.geom;
         for (uint64_t pass = 0; pass < s.n_passes; ++pass) {
             gp.queue = queue ? queue + 1 + pass : nullptr;
             hk.begin("stereo_pass");
@@ -414,8 +429,9 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
     append(key, b.geom.nthr);
     append(key, b.geom.smem);
     append(key, b.geom.tpp);
-    append(key, b.stream);
-    append(key, b.sstart.data(), sizeof(int32_t) * (n_jobs + 1));
+    append(key, b.tiled);
+    append(key, b.geom.radial);
+    append(key, b.sstart.data(), sizeof(int32_t) * b.sstart.size());
     append(key, sgeom.scratch_blocks);
     append(key, (int)s.init);
     append(key, s.nh);

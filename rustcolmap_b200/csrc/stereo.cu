@@ -3,7 +3,8 @@
 // Restates mvs/src/stereo.rs:
 //   plane_cost      stereo.rs:158-228   (device function plane_cost)
 //   init sweep      stereo.rs:247-269   (init_kernel)
-//   Jacobi passes   stereo.rs:271-371   (pass_kernel, one launch per pass)
+//   Jacobi passes   stereo.rs:271-371   (pass_staged_kernel by default, one
+//                   launch per pass; pass_kernel is the plain form)
 //   texture gate    stereo.rs:373-393   (gate_kernel)
 //   pixel RNG       stereo.rs:47-78
 //
@@ -280,6 +281,199 @@ __device__ __forceinline__ float cost_row(const Smem& sm, int row, const SrcRegs
     return sum;
 }
 
+// ---------------------------------------------------------------- bounded projection
+// A window term's value depends only on the integer pixel (u, v) its point
+// falls on (and on whether that is inside the source), so the reference's
+// exact f32 chain -- three IEEE divides and separate multiplies and adds,
+// about 85 instructions -- is needed only where a cheaper evaluation cannot
+// tell which pixel it is.  With a plane n.X = d and a source pose (R, t) the
+// projected direction is M r, M = d R + t n^T, for the cell's ray r = (rx,
+// ry, 1): z = d / (n.r) and zs * (n.r) = (M r)_z, so xs / zs = (M r)_x /
+// (M r)_z.  That is 6 fused multiply-adds, one reciprocal and two more, with
+// M made once per (plane, source).  Both this value and the reference's are
+// within a first-order rounding bound of the exact one (u = 2^-24; the
+// bound's terms are counted rounding by rounding):
+//   reference    f u / zs' [d (3 |R0| RX + 3 |R1| RY + |R2|) + (|tx| + |xn| |tz|) (2 a + 3 N)
+//                + |xn| (the same of row z)] + 6 f |xn| u + u |x|
+//   here         f u / zs' [d (2 |R0| RX + 3 |R1| RY + 3 |R2|) + 4 N (|tx| + |xn| |tz|)
+//                + |xn| d (|R6| RX + 2 |R7| RY + 2 |R8|)] + 4 f |xn| u + u |x| + u |cx|
+// with zs' = (M r)_z, a = n.r <= N = |nx| RX + |ny| RY + |nz|, R0..2 the
+// pose's row of x (y alike), RX / RY the tile's largest ray components, and
+// |xn|, 1 / zs' bounded over the candidate's own window.  E is their sum with
+// 10% slack for second-order terms; a term whose coordinate lies within E of
+// an integer (image borders are integers) is "near" and is evaluated by the
+// reference's chain, every other has the reference's pixel.  Typical E at
+// f = 2208: 0.001 px in x, 0.0005 px in y, so about 0.3% of the terms are
+// near (one bound for both axes and the whole image made it 1%, and the near
+// terms 39% of the pass).  Planes and sources that leave no bound (window
+// cells whose n.ray or depth in the source is close to the reference's gates)
+// take the reference's chain for every term.
+// RADIAL: some camera has k != 0; the distortion multiplies the bound of both
+// axes by 1 + 3.5 |k| r^2 and adds 8 f |xn| u.
+struct RayBox {
+    float rx, ry, step;  // largest |ray.x|, |ray.y| of the tile; largest change from a window's centre to a cell
+};
+
+__device__ __forceinline__ float rcp_approx(float x) {  // relative error at most 2^-23
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// What of the bound a plane does not change, per source: with ax = f |xn|,
+// E_x = (d wx + N tx + ax (d wz + N tz)) / zs' + c ax + bx.
+struct ProjConst {
+    float wx, wy, wz, tx, ty, tz, bx, by;
+};
+
+// wx = +inf leaves no bound.
+template <bool RADIAL>
+__device__ __forceinline__ ProjConst proj_const(const DevSrc& s, const RayBox& rb) {
+    constexpr float u = 6.6e-8f;  // 1.1 * 2^-24
+    const float uf = u * s.f;
+    const bool ok = s.f > 0.0f && (float)s.w * (float)s.h < 2147483000.0f;
+    ProjConst c;
+    c.wx = ok ? uf * (5.0f * fabsf(s.rs[0]) * rb.rx + 6.0f * fabsf(s.rs[1]) * rb.ry + 4.0f * fabsf(s.rs[2])) : INFINITY;
+    c.wy = uf * (5.0f * fabsf(s.rs[3]) * rb.rx + 6.0f * fabsf(s.rs[4]) * rb.ry + 4.0f * fabsf(s.rs[5]));
+    c.wz = u * (4.0f * fabsf(s.rs[6]) * rb.rx + 5.0f * fabsf(s.rs[7]) * rb.ry + 3.0f * fabsf(s.rs[8]));
+    c.tx = 9.0f * uf * fabsf(s.ts[0]);
+    c.ty = 9.0f * uf * fabsf(s.ts[1]);
+    c.tz = 9.0f * u * fabsf(s.ts[2]);
+    c.bx = u * (3.0f * fabsf(s.cx) + 1.0f);
+    c.by = u * (3.0f * fabsf(s.cy) + 1.0f);
+    return c;
+}
+
+// Two f32 in a 64-bit register pair: the packed instructions run at the FP32
+// rate in half the issue slots.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+struct Proj {
+    f32x2 m0, m1, m2;      // columns of M, rows x and y (scaled by f unless RADIAL)
+    float z0, z1, z2;      // row z
+    f32x2 ch;              // cx - 0.5, cy - 0.5
+    float lu, lv;          // 0.5 - E: a fraction within them of 0.5 is certain
+    float f, k;            // RADIAL
+    unsigned sw, sh;
+};
+
+// The projection of plane (n, d) into source s for window cells around the
+// ray rc; false when no bound holds.
+template <bool RADIAL>
+__device__ __forceinline__ bool make_proj(const SrcRegs& s, const ProjConst& c, float nx, float ny, float nz, float d,
+                                          float2 rc, const RayBox& rb, Proj& P) {
+    const float fs = RADIAL ? 1.0f : s.f;
+    const float fd = fs * d, t0 = fs * s.ts0, t1 = fs * s.ts1;
+    P.m0 = pack2(__fmaf_rn(fd, s.rs0, t0 * nx), __fmaf_rn(fd, s.rs3, t1 * nx));
+    P.m1 = pack2(__fmaf_rn(fd, s.rs1, t0 * ny), __fmaf_rn(fd, s.rs4, t1 * ny));
+    P.m2 = pack2(__fmaf_rn(fd, s.rs2, t0 * nz), __fmaf_rn(fd, s.rs5, t1 * nz));
+    P.z0 = __fmaf_rn(d, s.rs6, s.ts2 * nx);
+    P.z1 = __fmaf_rn(d, s.rs7, s.ts2 * ny);
+    P.z2 = __fmaf_rn(d, s.rs8, s.ts2 * nz);
+    P.ch = pack2(s.cx - 0.5f, s.cy - 0.5f);
+    P.sw = (unsigned)s.sw;
+    P.sh = (unsigned)s.sh;
+    if (RADIAL) {
+        P.f = s.f;
+        P.k = s.k;
+    }
+    const float n = __fmaf_rn(fabsf(nx), rb.rx, __fmaf_rn(fabsf(ny), rb.ry, fabsf(nz)));
+    const float amin = __fmaf_rn(nx, rc.x, __fmaf_rn(ny, rc.y, nz)) - (fabsf(nx) + fabsf(ny)) * rb.step;
+    const float zmin = __fmaf_rn(P.z0, rc.x, __fmaf_rn(P.z1, rc.y, P.z2)) - (fabsf(P.z0) + fabsf(P.z1)) * rb.step;
+    const float iz = rcp_approx(zmin);
+    // largest f |xn|, f |yn| of the window's cells
+    float cx, cy, ax, ay, bx, by;
+    unpack2(fma2(P.m0, pack2(rc.x, rc.x), fma2(P.m1, pack2(rc.y, rc.y), P.m2)), cx, cy);
+    unpack2(P.m0, ax, ay);
+    unpack2(P.m1, bx, by);
+    const float fz = RADIAL ? s.f * iz : iz;
+    ax = __fmaf_rn(fabsf(ax) + fabsf(bx), rb.step, fabsf(cx)) * fz;
+    ay = __fmaf_rn(fabsf(ay) + fabsf(by), rb.step, fabsf(cy)) * fz;
+    const float ez = __fmaf_rn(d, c.wz, n * c.tz) * iz + (RADIAL ? 1.32e-6f : 7.92e-7f);  // 20 u, 12 u with slack
+    float ex = __fmaf_rn(ax, ez, __fmaf_rn(__fmaf_rn(d, c.wx, n * c.tx), iz, c.bx));
+    float ey = __fmaf_rn(ay, ez, __fmaf_rn(__fmaf_rn(d, c.wy, n * c.ty), iz, c.by));
+    if (RADIAL) {
+        const float fi = rcp_approx(s.f), xn = ax * fi, yn = ay * fi;
+        ex = ey = fmaxf(ex, ey) * __fmaf_rn(3.6f * fabsf(s.k), __fmaf_rn(xn, xn, yn * yn), 1.0f);
+    }
+    P.lu = 0.5f - ex;
+    P.lv = 0.5f - ey;
+    return d > 0.0f && amin > 0.0501f && n < 10.0f && zmin > 0.002f * n && ex < 0.25f && ey < 0.25f;
+}
+
+// Where (M r)_xy = xy, (M r)_z = z lands: inside the source, and then at
+// census index off - (sw + 1).  Returns the coordinates' fractions - 0.5
+// (past P.lu / P.lv the reference's chain must decide).
+template <bool RADIAL>
+__device__ __forceinline__ f32x2 proj_pixel(const Proj& P, f32x2 xy, float z, bool& in, unsigned& off) {
+    constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23: x + MAGIC holds round(x) in its low mantissa bits
+    const float q = rcp_approx(z);
+    f32x2 uv;  // coordinates - 0.5: their nearest integer is the pixel
+    if (RADIAL) {
+        float xs, ys;
+        unpack2(xy, xs, ys);
+        const float xn = xs * q, yn = ys * q;
+        const float g = P.f * __fmaf_rn(P.k, __fmaf_rn(xn, xn, yn * yn), 1.0f);
+        uv = fma2(pack2(xn, yn), pack2(g, g), P.ch);
+    } else {
+        uv = fma2(xy, pack2(q, q), P.ch);
+    }
+    const f32x2 fl = add2(uv, pack2(MAGIC, MAGIC));
+    float fu, fv;
+    unpack2(fl, fu, fv);
+    // floor + 1, at least 1: inside when floor is in [-1, n) (trunc(-1 < x < 0) = 0)
+    const unsigned tu = max((unsigned)__float_as_int(fu) - 0x4B3FFFFFu, 1u);
+    const unsigned tv = max((unsigned)__float_as_int(fv) - 0x4B3FFFFFu, 1u);
+    in = tu <= P.sw && tv <= P.sh;
+    off = in ? tv * P.sw + tu : P.sw + 1u;
+    return fma2(add2(fl, pack2(-MAGIC, -MAGIC)), pack2(-1.0f, -1.0f), uv);
+}
+
+// The reference's chain for one term (stereo.rs:185-213): census index or -1.
+__device__ __forceinline__ int exact_index(const SrcRegs& s, float2 r, float nx, float ny, float nz, float d) {
+    const float denom = nx * r.x + ny * r.y + nz;
+    const float z = d / denom;
+    const float xr = z * r.x;
+    const float yr = z * r.y;
+    const float xs = s.rs0 * xr + s.rs1 * yr + s.rs2 * z + s.ts0;
+    const float ys = s.rs3 * xr + s.rs4 * yr + s.rs5 * z + s.ts1;
+    const float zs = s.rs6 * xr + s.rs7 * yr + s.rs8 * z + s.ts2;
+    const float xn = xs / zs;
+    const float yn = ys / zs;
+    const float dist = 1.0f + s.k * (xn * xn + yn * yn);
+    int u, v;
+    const bool in_u = trunc_index(s.f * xn * dist + s.cx, s.swf, u);
+    const bool in_v = trunc_index(s.f * yn * dist + s.cy, s.shf, v);
+    return !(denom < 0.05f) && !(zs < 1e-3f) && in_u && in_v ? v * s.sw + u : -1;
+}
+
+// sum / den > thr without the divide unless the two sides agree to 1e-6
+// (thr > 0): then the rounded quotient is on the same side of thr.
+__device__ __forceinline__ bool mean_above(float sum, float den, float thr) {
+    const float p = thr * den;
+    if (sum > p * 1.000001f) return true;
+    if (sum < p * 0.999999f) return false;
+    return sum / den > thr;
+}
+
 // stereo.rs:158-228, one candidate at a time.  (lx, ly): the pixel's
 // position in the tile; window cell (dx, dy) of the pixel is shared cell
 // (ly+dy)*stw + lx+dx (dx, dy in 0..4), which holds the clamped pixel
@@ -547,7 +741,9 @@ __global__ void __maxnreg__(72)
 }
 
 // ---------------------------------------------------------------- streamed passes
-// The same pass with the tile's pixels streamed through the block's lanes.
+// The same pass with the tile's pixels streamed through the block's lanes
+// (work counting and RCMVS_FLAG_NO_SKIP_DUPLICATES: it meets the candidates
+// one by one, as the reference does).
 // In pass_kernel a warp holds every candidate slot for as long as its
 // slowest lane needs: most evaluations abort after a window row or two while
 // a good candidate runs all 5*K rows, so most lanes wait.  Here a block of
@@ -595,7 +791,7 @@ constexpr int STREAM_PX = STREAM_TW * STREAM_TH;
 constexpr int STREAM_THREADS = RCMVS_STREAM_THREADS;
 static_assert(STREAM_THREADS % 32 == 0 && STREAM_TW <= 256 && STREAM_TH <= 256, "stream tile");
 constexpr int STREAM_CELLS = (STREAM_TW + 2 * HALO) * (STREAM_TH + 2 * HALO);
-constexpr int SF_N = 19;  // rs[9], ts[3], f, cx, cy, k, (float)w, (float)h, w (int bits)
+constexpr int SF_N = 20;  // rs[9], ts[3], f, cx, cy, k, (float)w, (float)h, w, h (int bits)
 
 struct StreamSmem {
     uint64_t* cen;      // halo tile
@@ -627,8 +823,10 @@ __device__ __forceinline__ StreamSmem carve_stream(unsigned char* base) {
     return s;
 }
 
-__device__ __forceinline__ SrcRegs load_src_fm(const StreamSmem& sm, int si) {
-    const float* b = sm.sf + si;
+// One source from the field-major table sf (field f of source si at
+// f * RCMVS_MAX_SOURCES + si); sc: its census.
+__device__ __forceinline__ SrcRegs load_src_fields(const float* sf, const uint64_t* sc, int si) {
+    const float* b = sf + si;
     constexpr int S = RCMVS_MAX_SOURCES;
     SrcRegs r;
     r.rs0 = b[0 * S];
@@ -650,9 +848,18 @@ __device__ __forceinline__ SrcRegs load_src_fm(const StreamSmem& sm, int si) {
     r.swf = b[16 * S];
     r.shf = b[17 * S];
     r.sw = __float_as_int(b[18 * S]);
-    r.sh = 0;  // not read by cost_row
-    r.sc = sm.scp[si];
+    r.sh = __float_as_int(b[19 * S]);
+    r.sc = sc;
     return r;
+}
+__device__ __forceinline__ float src_field(const DevSrc& S, int f) {
+    if (f < 16) return reinterpret_cast<const float*>(&S)[f];  // rs[9], ts[3], f, cx, cy, k
+    if (f == 16) return (float)S.w;
+    if (f == 17) return (float)S.h;
+    return __int_as_float(f == 18 ? S.w : S.h);
+}
+__device__ __forceinline__ SrcRegs load_src_fm(const StreamSmem& sm, int si) {
+    return load_src_fields(sm.sf, sm.scp[si], si);
 }
 
 template <bool COUNT, bool PERSIST>
@@ -691,17 +898,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, RCMVS_STREAM_MINB)
         // ---- staging: support views (field-major), h/48 table, halo tile
         for (int i = threadIdx.x; i < nsrc * SF_N; i += STREAM_THREADS) {
             const int s = i / SF_N, f = i - s * SF_N;
-            const DevSrc& S = J->src[s];
-            float v;
-            if (f < 16)
-                v = reinterpret_cast<const float*>(&S)[f];  // rs[9], ts[3], f, cx, cy, k
-            else if (f == 16)
-                v = (float)S.w;
-            else if (f == 17)
-                v = (float)S.h;
-            else
-                v = __int_as_float(S.w);
-            sm.sf[f * RCMVS_MAX_SOURCES + s] = v;
+            sm.sf[f * RCMVS_MAX_SOURCES + s] = src_field(J->src[s], f);
         }
         for (int s = threadIdx.x; s < nsrc; s += STREAM_THREADS) sm.scp[s] = census + J->src[s].off;
         for (int i = threadIdx.x; i < 49; i += STREAM_THREADS) sm.tab[i] = (float)i / 48.0f;
@@ -904,6 +1101,409 @@ __global__ void __launch_bounds__(STREAM_THREADS, RCMVS_STREAM_MINB)
     }
     if (COUNT) flush_work(wc, d_work);
 }
+
+// ---------------------------------------------------------------- staged passes
+// The default pass.  The streamed kernel above spends its time on lanes at
+// different support views and rows (each iteration pays for the slowest of
+// claim, candidate switch and row code, and a tile ends with a few long
+// evaluations on two warps).  Here a tile's candidates go through the
+// sources together, one source per stage, and the survivors are packed
+// before the next:
+//   1. preparation, one thread per pixel (as in the streamed kernel): every
+//      candidate that passes the gates and skip rules becomes a list entry;
+//   2. stage si = 0, 1, ...: each thread takes a list entry and evaluates
+//      source si's 25 terms (make_proj / proj_index; near terms by the
+//      reference's chain); entries whose evaluation ends -- abort, early
+//      rejection -- leave the list, the others are appended to the next
+//      stage's list with their sum.  All lanes read the same source, and a
+//      warp whose lanes have all ended leaves the stage early;
+//   3. resolution, one thread per pixel: the completed candidates in the
+//      reference's order.
+// Every candidate is evaluated under the limits of the pixel's stored cost,
+// the loosest the reference's sequence can have.  Exact: an evaluation that
+// ends under them ends under any tighter ones too, so it is no candidate
+// for either; one that completes has the reference's cost C, and is kept if
+// C is below the best cost so far, unless -- after an earlier candidate of
+// the pixel improved it -- the tighter limits would have ended it.  The
+// rejection bound ends it only if C is not below the best cost; the abort
+// ends it when some row's mean exceeds best + 0.14, which the stage's
+// running maximum of the means decides (to 2e-6; the rare closer call is
+// evaluated again row by row).
+//
+// What bounds it: instruction issue (78% of the slots, 24 of 32 lanes) and,
+// behind it, the census gathers.  12 passes over 16 views 960x720, K = 8:
+// 69.0 ms streamed, 37.4 staged; 4 passes after the learned init over 16 views
+// 1920x1080, K = 10: 164 -> 90 ms; 12 passes over 8 views 384x288, K = 4:
+// 11.3 -> 4.4 ms.  Of the 37.4 ms, 7.1 are the preparation, 19 source 0.
+// Tiles of 16x16 in blocks of 128 threads at 64 registers (8 blocks = 32
+// warps an SM): 16x16 / 64 threads 43.9, 32x16 / 128 42.2, 32x32 / 256 42.3,
+// 16x16 / 256 40.8, 16x8 / 128 39.6, 16x8 / 64 39.7, at 80 registers 40.5 (each
+// against 40.1 or 38.9 for this choice in the same build).  Unrolling the
+// rows: 48.0 (spills).
+#ifndef RCMVS_STAGED_TW
+#define RCMVS_STAGED_TW 16
+#define RCMVS_STAGED_TH 16
+#define RCMVS_STAGED_THREADS 128
+#define RCMVS_STAGED_MINB 8
+#endif
+template <int TW_, int TH_, int THREADS_, int MINB_>
+struct StagedCfg {
+    static constexpr int TW = TW_, TH = TH_, THREADS = THREADS_, MINB = MINB_;
+    static constexpr int PX = TW * TH, STW = TW + 2 * HALO, CELLS = STW * (TH + 2 * HALO);
+    static constexpr int CAP = 7 * PX;  // list entries: at most 4 neighbours and 3 perturbations a pixel
+    static_assert(PX <= 1024 && THREADS % 32 == 0, "staged tile");
+};
+
+template <class C>
+struct StagedSmem {
+    uint64_t cen[C::CELLS];
+    float2 ray[C::CELLS];
+    const uint64_t* scp[RCMVS_MAX_SOURCES];
+    float sf[SF_N * RCMVS_MAX_SOURCES];
+    ProjConst pc[RCMVS_MAX_SOURCES];
+    f32x2 colx[C::STW + 1];  // without distortion: the halo columns' ray.x, twice (ray.y depends on the row alone)
+    float tab[64];
+    float pcost[C::PX];
+    uint32_t done[C::PX];    // completed candidates, one bit each
+    uint16_t list[C::CAP];   // tile pixel | candidate << 10
+    int box[4];              // float bits (non-negative): RayBox's maxima, horizontal and vertical ray steps
+    int n, next, tile;
+};
+
+// Bytes of a resident block's scratch: the random candidates' planes, the
+// list's (sum, largest mean), the completed candidates' (cost, largest mean).
+template <class C>
+__host__ __device__ constexpr size_t staged_block_bytes() {
+    return C::PX * 3 * sizeof(float4) + C::CAP * 2 * sizeof(float2);
+}
+
+// Candidate q of the tile pixel whose window starts at `cell`.
+template <class C>
+__device__ __forceinline__ float4 staged_plane(const StagedSmem<C>& sm, const float4* __restrict__ prev_nz, size_t tb,
+                                               int w, int lx, int ly, int q, const float4* __restrict__ rnd, int p) {
+    if (q >= 4) return rnd[p * 3 + q - 4];
+    const int ddx = q == 0 ? -1 : (q == 1 ? 1 : 0);
+    const int ddy = q == 2 ? -1 : (q == 3 ? 1 : 0);
+    float4 nb = prev_nz[(ptrdiff_t)tb + (ptrdiff_t)(ly + ddy) * w + lx + ddx];
+    const float2 rj = sm.ray[(ly + HALO + ddy) * C::STW + lx + HALO + ddx];
+    nb.w = nb.w * (nb.x * rj.x + nb.y * rj.y + nb.z);
+    return nb;
+}
+
+// The evaluation of one candidate row by row under `thr` and `rej`, as
+// pass_kernel's (the close calls of the resolution).
+template <class C>
+__device__ __noinline__ bool staged_completes(const StagedSmem<C>& sm, int cell, int nsrc, float4 pl, float thr,
+                                              float rej) {
+    const Smem rs{nullptr, const_cast<float*>(sm.tab), const_cast<float2*>(sm.ray), const_cast<uint64_t*>(sm.cen)};
+    float sum = 0.f;
+    int32_t hs = 0;
+    for (int si = 0; si < nsrc; ++si) {
+        const SrcRegs s = load_src_fields(sm.sf, sm.scp[si], si);
+        for (int dy = 0; dy < 5; ++dy) {
+            sum = cost_row<false, false>(rs, cell + dy * C::STW, s, pl.x, pl.y, pl.z, pl.w, sum, hs);
+            if (sum / abort_den(dy, si, nsrc, true) > thr || sum >= rej) return false;
+        }
+    }
+    return true;
+}
+
+template <class C, bool RADIAL>
+__global__ void __launch_bounds__(C::THREADS, C::MINB)
+    pass_staged_kernel(const DevJob* __restrict__ jobs, const int32_t* __restrict__ stile_start, int n_jobs, int tiles,
+                       unsigned int* queue, uint64_t pass, float sig_inv, float sig_n,
+                       const uint64_t* __restrict__ census, const float2* __restrict__ rays, PlaneBuf prev,
+                       PlaneBuf next, unsigned char* __restrict__ scratch) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    StagedSmem<C>& sm = *reinterpret_cast<StagedSmem<C>*>(smem_raw);
+    unsigned char* const blk = scratch + (size_t)blockIdx.x * staged_block_bytes<C>();
+    float4* const rnd = reinterpret_cast<float4*>(blk);
+    float2* const lsum = reinterpret_cast<float2*>(rnd + C::PX * 3);
+    float2* const res = lsum + C::CAP;
+    const uint8_t* __restrict__ pflag = prev.flag;
+    const int tid = threadIdx.x, lane = tid & 31;
+    constexpr int stw = C::STW;
+    for (int i = tid; i < 49; i += C::THREADS) sm.tab[i] = (float)i / 48.0f;
+    for (int it = 0;; ++it) {
+        const int tile = next_tile(queue, tiles, it, &sm.tile);
+        if (tile < 0) break;
+        const int j = find_item(stile_start, n_jobs, tile);
+        const DevJob* J = jobs + j;
+        const int w = J->w, h = J->h, nsrc = J->nsrc;
+        const int t = tile - stile_start[j];
+        const int stx = (w + C::TW - 1) / C::TW;
+        const int x0 = (t % stx) * C::TW, y0 = (t / stx) * C::TH;
+        const int vw = min(C::TW, w - x0), vh = min(C::TH, h - y0);
+        const size_t base = (size_t)J->off;
+        const size_t tb = base + (size_t)y0 * w + x0;  // the tile's first pixel
+
+        // ---- staging: support views (field-major), halo tile, ray box
+        for (int i = tid; i < nsrc * SF_N; i += C::THREADS) {
+            const int s = i / SF_N, f = i - s * SF_N;
+            sm.sf[f * RCMVS_MAX_SOURCES + s] = src_field(J->src[s], f);
+        }
+        for (int s = tid; s < nsrc; s += C::THREADS) sm.scp[s] = census + J->src[s].off;
+        for (int i = tid; i < C::CELLS; i += C::THREADS) {
+            const int sx = i % stw, sy = i / stw;
+            const int gx = min(max(x0 - HALO + sx, 0), w - 1);
+            const int gy = min(max(y0 - HALO + sy, 0), h - 1);
+            const size_t g = base + (size_t)gy * w + gx;
+            sm.ray[i] = __ldg(rays + g);
+            sm.cen[i] = __ldg(census + g);
+        }
+        if (tid < 4) sm.box[tid] = 0;
+        if (tid == 0) sm.n = 0;
+        __syncthreads();
+        {
+            float bx = 0.f, by = 0.f, sh = 0.f, sv = 0.f;
+            for (int i = tid; i < C::CELLS; i += C::THREADS) {
+                const float2 r = sm.ray[i];
+                bx = fmaxf(bx, fabsf(r.x));
+                by = fmaxf(by, fabsf(r.y));
+                if (i % stw != stw - 1) {
+                    const float2 e = sm.ray[i + 1];
+                    sh = fmaxf(sh, fmaxf(fabsf(e.x - r.x), fabsf(e.y - r.y)));
+                }
+                if (i + stw < C::CELLS) {
+                    const float2 e = sm.ray[i + stw];
+                    sv = fmaxf(sv, fmaxf(fabsf(e.x - r.x), fabsf(e.y - r.y)));
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                bx = fmaxf(bx, __shfl_xor_sync(0xffffffffu, bx, o));
+                by = fmaxf(by, __shfl_xor_sync(0xffffffffu, by, o));
+                sh = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, o));
+                sv = fmaxf(sv, __shfl_xor_sync(0xffffffffu, sv, o));
+            }
+            if (lane == 0) {
+                atomicMax(&sm.box[0], __float_as_int(bx));
+                atomicMax(&sm.box[1], __float_as_int(by));
+                atomicMax(&sm.box[2], __float_as_int(sh));
+                atomicMax(&sm.box[3], __float_as_int(sv));
+            }
+        }
+        __syncthreads();
+        const RayBox rb{__int_as_float(sm.box[0]), __int_as_float(sm.box[1]),
+                        2.001f * (__int_as_float(sm.box[2]) + __int_as_float(sm.box[3]))};
+        for (int s = tid; s < nsrc; s += C::THREADS) sm.pc[s] = proj_const<RADIAL>(J->src[s], rb);
+        if (!RADIAL)
+            for (int c = tid; c < stw; c += C::THREADS) sm.colx[c] = pack2(sm.ray[c].x, sm.ray[c].x);
+
+        const float total = 5.0f * 5.0f * (float)nsrc;
+        const float inv_min = J->inv_min, inv_max = J->inv_max;
+        const float zlo = J->zmin * 0.5f, zhi = J->zmax * 2.0f;
+
+        // ---- 1. preparation: pixel (lx, ly) of the tile is p = ly * TW + lx
+        for (int p = tid; p < C::PX; p += C::THREADS) {
+            const int lx = p % C::TW, ly = p / C::TW;
+            if (lx >= vw || ly >= vh) continue;
+            const int x = x0 + lx, y = y0 + ly;
+            const size_t i = base + (size_t)y * w + x;
+            const float2 ri = sm.ray[(ly + HALO) * stw + lx + HALO];
+            uint64_t seed = pixel_rng(x, y, pass + 7);
+            const float4 cur = prev.nz[i];
+            const float cur_cost = prev.cost[i];
+            const float cur_d = prev.d[i];
+            const bool repeat = pflag != nullptr && !(pflag[i] & 2);
+            unsigned mask = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // the gates of pass_kernel's neighbour()
+                const int ddx = q == 0 ? -1 : (q == 1 ? 1 : 0);
+                const int ddy = q == 2 ? -1 : (q == 3 ? 1 : 0);
+                const int xx = x + ddx, yy = y + ddy;
+                if (xx < 0 || yy < 0 || xx >= w || yy >= h) continue;
+                const size_t ni = base + (size_t)yy * w + xx;
+                if (repeat && !(pflag[ni] & 1)) continue;
+                const float4 nb = prev.nz[ni];
+                const float2 rj = sm.ray[(ly + HALO + ddy) * stw + lx + HALO + ddx];
+                const float a_nb = nb.x * rj.x + nb.y * rj.y + nb.z;
+                if (a_nb < 0.1f) continue;
+                const float d_plane = nb.w * a_nb;
+                const float a_here = nb.x * ri.x + nb.y * ri.y + nb.z;
+                if (a_here < 0.1f) continue;
+                const float zcand = d_plane / a_here;
+                if (!(zlo <= zcand && zcand <= zhi)) continue;
+                if (__float_as_uint(d_plane) == __float_as_uint(cur_d) &&
+                    __float_as_uint(nb.x) == __float_as_uint(cur.x) && __float_as_uint(nb.y) == __float_as_uint(cur.y) &&
+                    __float_as_uint(nb.z) == __float_as_uint(cur.z))
+                    continue;
+                mask |= 1u << q;
+            }
+#pragma unroll 1
+            for (int r = 0; r < 3; ++r) {  // stereo.rs:323-353, as pass_kernel
+                const float inv = 1.0f / fmaxf(cur.w, 1e-6f);
+                const float inv_new = inv + sig_inv * (inv_max - inv_min) * gauss3(seed);
+                if (inv_new <= 0.0f) continue;
+                const float zcand = 1.0f / inv_new;
+                if (!(zlo <= zcand && zcand <= zhi)) continue;
+                float nnx = cur.x + sig_n * gauss3(seed);
+                float nny = cur.y + sig_n * gauss3(seed);
+                float nnz = cur.z + sig_n * gauss3(seed);
+                const float len = sqrtf(nnx * nnx + nny * nny + nnz * nnz);
+                if (len < 1e-6f) continue;
+                nnx = nnx / len;
+                nny = nny / len;
+                nnz = nnz / len;
+                const float a_here = nnx * ri.x + nny * ri.y + nnz;
+                if (a_here < 0.1f) continue;
+                rnd[p * 3 + r] = make_float4(nnx, nny, nnz, zcand * a_here);
+                mask |= 16u << r;
+            }
+            next.nz[i] = cur;  // nothing accepted (stereo.rs:278)
+            next.cost[i] = cur_cost;
+            next.d[i] = cur_d;
+            if (next.flag) next.flag[i] = 0;
+            sm.pcost[p] = cur_cost;
+            sm.done[p] = 0;
+            if (mask) {
+                int at = atomicAdd(&sm.n, __popc(mask));
+                for (unsigned m = mask; m; m &= m - 1) sm.list[at++] = (uint16_t)(p | (__ffs(m) - 1) << 10);
+            }
+        }
+
+        // ---- 2. one source after the other
+        for (int si = 0; si < nsrc; ++si) {
+            __syncthreads();  // the list, the sums and (si = 0) the staging are complete
+            const int n = sm.n;
+            if (n == 0) break;
+            if (tid == 0) sm.next = 0;
+            const uint64_t* __restrict__ sc = sm.scp[si];
+            for (int b = 0; b < n; b += C::THREADS) {
+                const bool have = b + tid < n;
+                uint32_t e = 0;
+                float2 sv = make_float2(0.f, 0.f);
+                if (have) {
+                    e = sm.list[b + tid];
+                    if (si > 0) sv = lsum[b + tid];
+                }
+                __syncthreads();  // read before the survivors are appended over them
+                bool alive = have;
+                const int p = e & 1023, q = e >> 10;
+                const int lx = p % C::TW, ly = p / C::TW;
+                const int cell = ly * stw + lx;
+                float sum = sv.x, top = sv.y;
+                if (have) {
+                    const float4 pl = staged_plane(sm, prev.nz, tb, w, lx, ly, q, rnd, p);
+                    const float best_c = sm.pcost[p];
+                    const float thr = (best_c + 0.02f) + 0.12f;
+                    const float rej = reject_bound(best_c, total);
+                    Proj P;
+                    const bool bound = make_proj<RADIAL>(load_src_fields(sm.sf, sc, si), sm.pc[si], pl.x, pl.y, pl.z,
+                                                         pl.w, sm.ray[cell + HALO * stw + HALO], rb, P);
+                    if (!bound) P.lu = -1.0f;
+                    const uint64_t* __restrict__ sc1 = sc - (P.sw + 1u);
+#pragma unroll 1
+                    for (int dy = 0; dy < 5; ++dy) {
+                        const int row = cell + dy * stw;
+                        f32x2 by = 0;
+                        float bz = 0.0f;
+                        if (!RADIAL) {
+                            const float ry = sm.ray[row].y;
+                            by = fma2(P.m1, pack2(ry, ry), P.m2);
+                            bz = __fmaf_rn(P.z1, ry, P.z2);
+                        }
+                        unsigned near = 0;
+                        int hc[5];
+#pragma unroll
+                        for (int dx = 0; dx < 5; ++dx) {
+                            f32x2 xy;
+                            float z;
+                            if (RADIAL) {
+                                const float2 r = sm.ray[row + dx];
+                                xy = fma2(P.m0, pack2(r.x, r.x), fma2(P.m1, pack2(r.y, r.y), P.m2));
+                                z = __fmaf_rn(P.z0, r.x, __fmaf_rn(P.z1, r.y, P.z2));
+                            } else {
+                                const f32x2 rr = sm.colx[lx + dx];
+                                float rx, rx2;
+                                unpack2(rr, rx, rx2);
+                                xy = fma2(P.m0, rr, by);
+                                z = __fmaf_rn(P.z0, rx, bz);
+                            }
+                            bool in;
+                            unsigned off;
+                            float du, dv;
+                            unpack2(proj_pixel<RADIAL>(P, xy, z, in, off), du, dv);
+                            if (!(fabsf(du) <= P.lu && fabsf(dv) <= P.lv)) near |= 1u << dx;
+                            const int hv = __popcll(sm.cen[row + dx] ^ __ldg(sc1 + off));
+                            hc[dx] = in ? hv : 48;
+                        }
+                        while (near) {
+                            const int c = __ffs(near) - 1;
+                            near &= near - 1;
+                            const int v = exact_index(load_src_fields(sm.sf, sc, si), sm.ray[row + c], pl.x, pl.y,
+                                                      pl.z, pl.w);
+                            const int hv = v < 0 ? 48 : __popcll(sm.cen[row + c] ^ __ldg(sc + max(v, 0)));
+#pragma unroll
+                            for (int dx = 0; dx < 5; ++dx) hc[dx] = c == dx ? hv : hc[dx];
+                        }
+#pragma unroll
+                        for (int dx = 0; dx < 5; ++dx) sum += sm.tab[hc[dx]];
+                        const float den = abort_den(dy, si, nsrc, true);
+                        if (mean_above(sum, den, thr) || sum >= rej) {
+                            alive = false;
+                            break;
+                        }
+                        top = fmaxf(top, sum * rcp_approx(den));
+                    }
+                }
+                if (alive) {
+                    if (si == nsrc - 1) {
+                        res[p * 7 + q] = make_float2(sum / total, top);
+                        atomicOr(&sm.done[p], 1u << q);
+                    } else {
+                        const int at = atomicAdd(&sm.next, 1);
+                        sm.list[at] = (uint16_t)e;
+                        lsum[at] = make_float2(sum, top);
+                    }
+                }
+            }
+            __syncthreads();
+            if (tid == 0) sm.n = sm.next;
+        }
+        __syncthreads();
+
+        // ---- 3. the completed candidates in order (stereo.rs:355-367)
+        for (int p = tid; p < C::PX; p += C::THREADS) {
+            const int lx = p % C::TW, ly = p / C::TW;
+            if (lx >= vw || ly >= vh) continue;
+            unsigned m = sm.done[p];
+            if (!m) continue;
+            const float cost0 = sm.pcost[p];
+            float best_c = cost0;
+            int best = -1;
+            for (; m; m &= m - 1) {
+                const int q = __ffs(m) - 1;
+                const float2 r = res[p * 7 + q];
+                if (!(r.x < best_c)) continue;
+                if (best >= 0) {
+                    const float thr = (best_c + 0.02f) + 0.12f;
+                    if (r.y > thr * 1.000002f) continue;  // the tighter limit ends it
+                    if (!(r.y < thr * 0.999998f) &&
+                        !staged_completes(sm, ly * stw + lx, nsrc, staged_plane(sm, prev.nz, tb, w, lx, ly, q, rnd, p),
+                                          thr, reject_bound(best_c, total)))
+                        continue;
+                }
+                best_c = r.x;
+                best = q;
+            }
+            if (best < 0) continue;
+            const float4 pl = staged_plane(sm, prev.nz, tb, w, lx, ly, best, rnd, p);
+            const float2 ri = sm.ray[(ly + HALO) * stw + lx + HALO];
+            const float a_here = pl.x * ri.x + pl.y * ri.y + pl.z;
+            const size_t i = tb + (size_t)ly * w + lx;
+            if (a_here > 0.05f) {
+                next.nz[i] = make_float4(pl.x, pl.y, pl.z, pl.w / a_here);
+                next.cost[i] = fminf(best_c, 1.0f);
+                next.d[i] = pl.w;
+                if (next.flag) next.flag[i] = 1;
+            } else if (next.flag) {
+                next.flag[i] = 2;
+            }
+        }
+    }
+}
+
+using StagedDefault = StagedCfg<RCMVS_STAGED_TW, RCMVS_STAGED_TH, RCMVS_STAGED_THREADS, RCMVS_STAGED_MINB>;
 
 // ---------------------------------------------------------------- split passes
 // The same pass with five lanes per pixel (threads per pixel = 5, an
@@ -1660,16 +2260,26 @@ size_t stereo_smem_bytes(TileShape ts) { return smem_bytes(ts.tw, ts.th); }
 // Threads of a split-pass block for tiles of up to `px` pixels.
 int split_threads(int px) { return 32 * ((px + SPLIT_PX - 1) / SPLIT_PX); }
 
-int stream_tiles(int w, int h) { return ((w + STREAM_TW - 1) / STREAM_TW) * ((h + STREAM_TH - 1) / STREAM_TH); }
+int tiled_tiles(int kind, int w, int h) {
+    const int tw = kind == TILED_STREAM ? STREAM_TW : StagedDefault::TW;
+    const int th = kind == TILED_STREAM ? STREAM_TH : StagedDefault::TH;
+    return ((w + tw - 1) / tw) * ((h + th - 1) / th);
+}
 
-LaunchGeom stream_geom(int tiles) {
+LaunchGeom tiled_geom(int kind, int tiles) {
     LaunchGeom g{STREAM_THREADS, stream_smem_bytes(), tiles, nullptr};
-    g.stream = true;
+    if (kind == TILED_STAGED) {
+        g.nthr = StagedDefault::THREADS;
+        g.smem = sizeof(StagedSmem<StagedDefault>);
+    }
+    g.tiled = kind;
     return g;
 }
 
-
-size_t stream_scratch_bytes(int blocks) { return sizeof(float4) * STREAM_PX * 3 * (size_t)blocks; }
+size_t tiled_scratch_bytes(int kind, int blocks) {
+    return (kind == TILED_STREAM ? sizeof(float4) * STREAM_PX * 3 : staged_block_bytes<StagedDefault>()) *
+           (size_t)blocks;
+}
 
 namespace {
 // Blocks of a persistent launch: as many as stay resident on all SMs at
@@ -1690,11 +2300,18 @@ int launch_grid(K kernel, const LaunchGeom& g) {
 }  // namespace
 
 int stereo_resident_grid(const LaunchGeom& g) { return launch_grid(pass_kernel<false, 3, true>, g); }
-int stream_grid(const LaunchGeom& g) {
+int tiled_grid(const LaunchGeom& g) {
     LaunchGeom q = g;
     unsigned int dummy = 0;
     q.queue = &dummy;  // any non-null queue: the resident grid
-    return std::max(launch_grid(pass_stream_kernel<false, true>, q), 1);
+    int n = 0;
+    if (g.tiled == TILED_STREAM)
+        n = launch_grid(pass_stream_kernel<false, true>, q);
+    else if (g.radial)
+        n = launch_grid(pass_staged_kernel<StagedDefault, true>, q);
+    else
+        n = launch_grid(pass_staged_kernel<StagedDefault, false>, q);
+    return std::max(n, 1);
 }
 
 namespace {
@@ -1717,12 +2334,24 @@ template <bool COUNT, bool PERSIST>
 void pass_as(const DevJob* d_jobs, const int32_t* d_job_start, int n_jobs, const LaunchGeom& g, uint64_t pass,
              float sig_inv, float sig_n, const uint64_t* census, const float2* rays, PlaneBuf prev, PlaneBuf next,
              unsigned long long* d_work, cudaStream_t st) {
-    if (g.stream) {  // always persistent: block b owns slice b of the scratch
+    if (g.tiled) {  // always persistent: block b owns slice b of the scratch
         if (!PERSIST) return;
-        const int grid = std::min(launch_grid(pass_stream_kernel<COUNT, true>, g), g.scratch_blocks);
-        pass_stream_kernel<COUNT, true><<<grid, STREAM_THREADS, stream_smem_bytes(), st>>>(
-            d_jobs, d_job_start, n_jobs, g.tiles, g.queue, pass, sig_inv, sig_n, census, rays, prev, next, g.scratch,
-            d_work);
+        if (g.tiled == TILED_STREAM) {
+            const int grid = std::min(launch_grid(pass_stream_kernel<COUNT, true>, g), g.scratch_blocks);
+            pass_stream_kernel<COUNT, true><<<grid, STREAM_THREADS, stream_smem_bytes(), st>>>(
+                d_jobs, d_job_start, n_jobs, g.tiles, g.queue, pass, sig_inv, sig_n, census, rays, prev, next,
+                reinterpret_cast<float4*>(g.scratch), d_work);
+            return;
+        }
+        auto run = [&](auto kernel) {
+            const int grid = std::min(launch_grid(kernel, g), g.scratch_blocks);
+            kernel<<<grid, g.nthr, g.smem, st>>>(d_jobs, d_job_start, n_jobs, g.tiles, g.queue, pass, sig_inv, sig_n,
+                                                 census, rays, prev, next, g.scratch);
+        };
+        if (g.radial)
+            run(pass_staged_kernel<StagedDefault, true>);
+        else
+            run(pass_staged_kernel<StagedDefault, false>);
         return;
     }
     if (g.tpp == SPLIT) {
@@ -1760,7 +2389,8 @@ cudaError_t launch_pass(const DevJob* d_jobs, const int32_t* d_job_start, int n_
                         uint64_t pass, float sig_inv, float sig_n, const uint64_t* census, const float2* rays,
                         PlaneBuf prev, PlaneBuf next, unsigned long long* d_work, cudaStream_t st) {
     if (g.tiles <= 0) return cudaSuccess;
-    if (g.stream && (!g.queue || !g.scratch || g.scratch_blocks <= 0)) return cudaErrorInvalidValue;
+    if (g.tiled && (!g.queue || !g.scratch || g.scratch_blocks <= 0)) return cudaErrorInvalidValue;
+    if (g.tiled == TILED_STAGED && (d_work || !prev.d || !next.d)) return cudaErrorInvalidValue;
     if (d_work) {
         if (g.queue)
             pass_as<true, true>(d_jobs, d_job_start, n_jobs, g, pass, sig_inv, sig_n, census, rays, prev, next, d_work,
