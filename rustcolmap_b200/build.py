@@ -33,7 +33,8 @@ LIBS = {
 }
 LINK = {"librcmvs.so": ["-lz"]}  # zlib: the grey PNG writer
 HEADERS = [os.path.join(CSRC, "rcmvs_internal.cuh"), os.path.join(CSRC, "ctx_internal.cuh"),
-           os.path.join(CSRC, "learned.cuh"), os.path.join(ROOT, "include", "rcmvs.h"),
+           os.path.join(CSRC, "learned.cuh"),
+           os.path.join(CSRC, "tc.cuh"), os.path.join(ROOT, "include", "rcmvs.h"),
            os.path.join(ROOT, "include", "rcscene.h")]
 
 

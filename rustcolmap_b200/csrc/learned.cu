@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "rcmvs_internal.cuh"
+#include "tc.cuh"
 #include "learned.cuh"
 
 namespace rcmvs {
@@ -186,75 +187,11 @@ __device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
 constexpr int TILE_H = 8, TILE_W = 16;  // output pixels per block: 8 rows x 16 columns (4 warps x 2 rows)
 
 // ---- 5th-generation tensor cores (tcgen05): the forward/data convolution
-// Shared-memory matrix descriptor of a tcgen05.mma operand, no swizzle,
-// K-major: 8-row x 16-byte core matrices, `lbo` bytes between core matrices
-// adjacent in K, `sbo` bytes between core matrices adjacent in M/N (PTX ISA,
-// tcgen05 "Shared memory descriptor"; version 1 at bits 46-47).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
-
 // Instruction descriptor of tcgen05.mma.kind::f16: FP32 accumulator (bits
 // 4-5 = 1), BF16 A and B (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits
 // 17-22, M >> 4 at bits 24-28.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
-        :
-        : "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0), "r"(0), "r"(0), "r"(0));
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Waits for phase `parity` of the mbarrier at shared address `bar`; gives
-// up after `limit_ns` of wall time (returns false).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-    const uint64_t t0 = global_ns();
-    while (true) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P1;\n\t}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (global_ns() - t0 > limit_ns) return false;
-    }
-}
-
-template <int N>
-__device__ __forceinline__ void tmem_ld_32x32b(uint32_t taddr, uint32_t* v);
-template <>
-__device__ __forceinline__ void tmem_ld_32x32b<16>(uint32_t taddr, uint32_t* v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
-}
-template <>
-__device__ __forceinline__ void tmem_ld_32x32b<32>(uint32_t taddr, uint32_t* v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
 }
 
 // Set (never cleared by a kernel) when a tensor-core wait gave up; read and
@@ -266,7 +203,6 @@ constexpr int TC_SW = TC_TW + 2;              // staged halo tile width
 constexpr int TC_NPIX = (TC_TH + 2) * TC_SW;  // staged pixels
 constexpr int TC_GS = 2944;                   // bytes per channel group of a staged tile: 180 x 16, 128-aligned
 constexpr int TC_CTAS_PER_SM = 3;
-constexpr uint64_t TC_WAIT_NS = 2000000000ull;  // 2 s: far above a tile's few microseconds
 
 template <int CIN, int COUT, bool MASK>
 struct ConvSmem {
@@ -291,14 +227,6 @@ __device__ __forceinline__ void tma_load_4d(const void* tmap, uint32_t dst, uint
         :
         : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
         : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
 // y = conv3x3(x, w) + b, "same" zero padding; optional ReLU; optional f32
@@ -443,7 +371,7 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CU
                     const uint64_t a =
                         umma_desc(sx_a + (uint32_t)((2 * kc) * TC_GS + (ky * TC_SW + kx) * 16), TC_GS, TC_SW * 16);
                     const uint64_t b = umma_desc(sw_a + (uint32_t)((tap * KG + 2 * kc) * COUT * 16), COUT * 16, 128);
-                    umma_bf16(taddr, a, b, IDESC, (tap | kc) != 0 ? 1u : 0u);
+                    umma_f16(taddr, a, b, IDESC, (tap | kc) != 0 ? 1u : 0u);
                 }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_a)

@@ -5,9 +5,37 @@
 // of B by squared L2 distance, the same from B to A, Lowe's ratio test both
 // ways and the mutual-best check.
 //
-// The reference sums (a_k - b_k)^2 serially over k = 0..127 in f32.  A GEMM
-// (2 - 2 a.b) would round differently and move ratio-test and tie decisions,
-// so the distances are computed as written, on the FP32 pipes:
+// The reference sums (a_k - b_k)^2 serially over k = 0..127 in f32.  Its
+// result is only which descriptors pass the tests on the nearest and
+// second-nearest distance, so a tensor-core product with a proven error bound
+// decides every descriptor that is not within the bound of a test's edge,
+// and only the rest are summed as written:
+//
+//   pack_kernel   every frame as FP16 hi + lo (x = 2^-6 (hi + lo) to 2^-22) in
+//                 the tensor cores' operand order, blocks of 128 descriptors,
+//                 and squared norms
+//   nearest_kernel  one CTA per 128 descriptors of one frame (queries) against
+//                 all descriptors of the other, both directions of each pair:
+//                 |t|^2 - 2 q.t, the products as hi.hi + hi.lo + lo.hi on
+//                 tcgen05.mma with FP32 accumulation in tensor memory; one
+//                 thread keeps the two smallest of its query and half of the
+//                 targets
+//   outcome_kernel  per query: certainly refused, certainly accepted (then the
+//                 two targets of the smallest's column pair are summed
+//                 serially and the nearer is the answer), or listed
+//   rescan_kernel the listed queries against all targets, serially summed, and
+//                 the reference's tests
+//   mutual_kernel the reference's mutual check per row of A
+//
+// Error bound (u = 2^-24; |q|, |t| norms): operands to 2^-22 relative or 2^-31
+// absolute per component, lo.lo dropped (2^-22 |q||t|), 384 products summed in
+// FP32 (64 u), norms to 8 u, the reference's own serial sum 131 u d.  With S =
+// |q| + max |t|, an approximate distance is within
+// (2^-17 / 2 + 2^-20) S^2 + 2^-26 S of the exact one, and the reference's
+// within 7.9e-6 d of that.
+//
+// Frames with components past 1000 or not finite, and chunks in which many
+// queries are listed (repeated descriptors), run on the FP32 pipes instead:
 //
 //   dist_kernel   64x64 distances per block, 4x4 per thread; 32-wide k chunks
 //                 of both tiles staged k-major in shared memory (float4 reads,
@@ -23,7 +51,6 @@
 //                 the second smallest value, exactly what the reference's
 //                 sequential scan keeps (the merge is associative, so the
 //                 order of the tiles does not matter)
-//   decide_kernel the reference's tests per row of A
 //
 // Pairs run in chunks whose tile partials (the per-tile best/second entries
 // of every row and column, 12 bytes each; no distance matrix is written)
@@ -35,7 +62,10 @@
 #include <string>
 #include <vector>
 
+#include <cuda_fp16.h>
+
 #include "ctx_internal.cuh"
+#include "tc.cuh"
 
 namespace rcmvs {
 
@@ -51,6 +81,7 @@ struct PairJob {
     int64_t prow_off, pcol_off;  // tile partials: [column tile][na] rows, [row tile][nb] columns
     int32_t na, nb;
     int32_t row_off, col_off;  // into the chunk's forward / backward results
+    int32_t fa, fb;            // frames
 };
 
 struct Nearest {
@@ -207,6 +238,361 @@ __global__ void __launch_bounds__(256) cols_kernel(const PairJob* __restrict__ j
     bwd[J.col_off + ib] = m;
 }
 
+// ------------------------------------------------------ tensor-core search
+constexpr int QB = 128;                      // descriptors per packed block
+constexpr int QB_HALF = QB * DESC_LEN * 2;   // bytes of a block's hi (or lo) half
+constexpr int QB_BYTES = 2 * QB_HALF;
+constexpr float PACK_SCALE = 64.0f;          // keeps lo clear of FP16 subnormals for unit descriptors
+constexpr float PACK_LIMIT = 1000.0f;        // larger components overflow FP16 after scaling
+constexpr int RESCAN_MAX = 2048;             // listed queries a chunk may have
+
+struct Frame {
+    int64_t off;   // first descriptor
+    int64_t blk;   // first packed block (and 128 * blk: first norm)
+    int32_t n;
+};
+
+struct MatchStatus {
+    int wild;   // a component past PACK_LIMIT or not finite
+    int listed; // queries for rescan_kernel
+    int fault;  // a bounded wait gave up
+};
+
+// Block b of 128 descriptors: half (hi, lo) h, descriptor r, component k at
+// h * QB_HALF + (k / 8) * 2048 + r * 16 + (k % 8) * 2: [8-component group]
+// [descriptor][8], a canonical K-major operand.  Past the frame's end:
+// zeros with an infinite norm.
+__global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ desc, const Frame* __restrict__ frames,
+                                                   const int32_t* __restrict__ blk_start, int n_frames,
+                                                   unsigned char* __restrict__ packed, float* __restrict__ norms,
+                                                   int* __restrict__ max_norm, MatchStatus* __restrict__ st) {
+    __shared__ float part[2][QB];
+    int lo = 0, hi = n_frames - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (blk_start[mid] <= (int)blockIdx.x)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const Frame F = frames[lo];
+    const int r = threadIdx.x & (QB - 1), half = threadIdx.x >> 7;
+    const int row = ((int)blockIdx.x - blk_start[lo]) * QB + r;
+    const bool in = row < F.n;
+    const float* src = desc + (F.off + row) * DESC_LEN;
+    unsigned char* out = packed + (size_t)blockIdx.x * QB_BYTES + r * 16;
+    float sum = 0.0f;
+    bool wild = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int g = 2 * i + half;
+        float x[8] = {};
+        if (in) {
+            const float4 a = *reinterpret_cast<const float4*>(src + 8 * g), b = *reinterpret_cast<const float4*>(src + 8 * g + 4);
+            x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+        }
+        __half h[8], l[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            wild = wild || !(fabsf(x[c]) <= PACK_LIMIT);
+            sum = __fmaf_rn(x[c], x[c], sum);
+            const float v = x[c] * PACK_SCALE;
+            h[c] = __float2half_rn(v);
+            l[c] = __float2half_rn(v - __half2float(h[c]));
+        }
+        *reinterpret_cast<uint4*>(out + g * (QB * 16)) = *reinterpret_cast<const uint4*>(h);
+        *reinterpret_cast<uint4*>(out + QB_HALF + g * (QB * 16)) = *reinterpret_cast<const uint4*>(l);
+    }
+    part[half][r] = sum;
+    if (wild) st->wild = 1;
+    __syncthreads();
+    if (half == 0) {
+        const float n = part[0][r] + part[1][r];
+        norms[(size_t)blockIdx.x * QB + r] = in ? n : INFINITY;
+        float m = in ? n : 0.0f;
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(&max_norm[lo], __float_as_int(m));  // norms are not negative
+    }
+}
+
+struct Two {  // the two smallest values and the column pair (target / 2) of the smallest
+    float v0, v1;
+    int32_t pair;
+};
+
+// One direction of a pair: queries q against targets t; entry at `out`.
+__device__ __forceinline__ void direction(const PairJob& J, const Frame* frames, int dir, Frame& q, Frame& t, int& out) {
+    q = frames[dir ? J.fb : J.fa];
+    t = frames[dir ? J.fa : J.fb];
+    out = dir ? J.col_off : J.row_off;
+}
+
+// One CTA: up to two query blocks (256 queries) against every target block.
+// Shared memory holds the query blocks (128 KB) and a ring of three 32 KB
+// slots for the halves (hi, lo) of the target blocks; tensor memory two
+// accumulators per query block (128 columns each), one multiplying while the
+// other is read.  Warp 8's first thread loads and multiplies: step 2c is
+// block c's hi (queries lo, then hi), step 2c + 1 its lo (queries hi); the
+// load of step s + 2 starts when step s - 1's products are done, two steps
+// ahead of its use.  Warps 0-3 scan the first query block's values, 4-7 the
+// second's, one thread per query.  Bound by the tensor pipe (48 MMAs of
+// 128 x 128 x 16 per target block, 55% active) and the L2 reads of the target
+// blocks.  12 frames of 2048, 66 pairs (both directions): 429 us (FP32 pipes:
+// 4158); one query block per CTA and 64 KB target blocks in two buffers: 547
+// us (the load of a block had one scan's time to arrive); with the four
+// smallest kept in branches: 1040 us.
+constexpr int NSLOT = 3;
+constexpr int kNearestThreads = 288;
+constexpr int kNearestSmem = 2 * QB_BYTES + NSLOT * QB_HALF + 128;
+
+__global__ void __launch_bounds__(kNearestThreads, 1)
+    nearest_kernel(const PairJob* __restrict__ jobs, const Frame* __restrict__ frames,
+                   const unsigned char* __restrict__ packed, const float* __restrict__ norms, int blocks_per_cta,
+                   Two* __restrict__ fwd, Two* __restrict__ bwd, MatchStatus* __restrict__ st) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bars[1 + 2 * NSLOT + 4];  // queries; slot full, slot free; values full, values free
+    __shared__ uint32_t s_taddr;
+    const int dir = blockIdx.y & 1;
+    const PairJob J = jobs[blockIdx.y >> 1];
+    Frame q, t;
+    int out0;
+    direction(J, frames, dir, q, t, out0);
+    const int qb0 = blockIdx.x * blocks_per_cta;
+    const int nq = min(blocks_per_cta, (q.n + QB - 1) / QB - qb0);
+    const int n = (t.n + QB - 1) / QB;
+    if (nq <= 0 || n == 0) return;  // without targets the queries' entries are not read
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t sq = (smem_u32(smem) + 127u) & ~127u, ring = sq + 2 * QB_BYTES;
+    const uint32_t bar0 = smem_u32(bars);
+    auto full = [&](int k) { return bar0 + 8u + 8u * k; };
+    auto slot_free = [&](int k) { return bar0 + 8u + 8u * (NSLOT + k); };
+    auto acc_full = [&](int k) { return bar0 + 8u + 8u * (2 * NSLOT + k); };
+    auto acc_free = [&](int k) { return bar0 + 8u + 8u * (2 * NSLOT + 2 + k); };
+    if (warp == 8) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_taddr)),
+                     "r"(4 * QB));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < 1 + 2 * NSLOT + 2; ++k) mbar_init(bar0 + 8u * k, 1);
+        for (int k = 0; k < 2; ++k) mbar_init(acc_free(k), 4 * nq);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t taddr = s_taddr;
+    if (warp == 8) {
+        if (lane == 0) {
+            const int steps = 2 * n;
+            int loaded = 0, landed = 0, issued = 0, freed = 0;  // steps
+            auto load = [&](uint32_t dst, const unsigned char* src, uint32_t bytes, uint32_t bar) {
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                             "l"(src), "r"(bytes), "r"(bar)
+                             : "memory");
+            };
+            auto load_step = [&](int s) {
+                mbar_expect_tx(full(s % NSLOT), QB_HALF);
+                load(ring + (s % NSLOT) * QB_HALF, packed + (t.blk + (s >> 1)) * (int64_t)QB_BYTES + (s & 1) * QB_HALF,
+                     QB_HALF, full(s % NSLOT));
+                ++loaded;
+            };
+            mbar_expect_tx(bar0, nq * QB_BYTES);
+            load(sq, packed + (q.blk + qb0) * (int64_t)QB_BYTES, nq * QB_BYTES, bar0);
+            load_step(0);
+            load_step(1);
+            bool ok = mbar_wait(bar0, 0, TC_WAIT_NS);
+            const bool q_in = ok;
+            for (int s = 0; s < steps && ok; ++s) {
+                const int c = s >> 1, slot = s % NSLOT;
+                if (!(ok = mbar_wait(full(slot), (s / NSLOT) & 1, TC_WAIT_NS))) break;
+                ++landed;
+                if ((s & 1) == 0 && c >= 2 && !(ok = mbar_wait(acc_free(c & 1), ((c >> 1) - 1) & 1, TC_WAIT_NS))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                constexpr uint32_t IDESC = (1u << 4) | ((QB >> 3) << 17) | ((QB >> 4) << 24);  // F16 in, F32 out, 128 x 128
+                const uint32_t sb = ring + slot * QB_HALF;
+                for (int b = 0; b < nq; ++b) {
+                    const uint32_t d = taddr + (2 * b + (c & 1)) * QB;
+                    for (int term = (s & 1) ? 1 : 0; term < 2; ++term) {  // queries lo, then hi; only hi against lo
+                        const uint32_t a0 = sq + b * QB_BYTES + (term == 0 ? QB_HALF : 0);
+#pragma unroll
+                        for (int kc = 0; kc < DESC_LEN / 16; ++kc)
+                            umma_f16(d, umma_desc(a0 + kc * (2 * QB * 16), QB * 16, 128),
+                                     umma_desc(sb + kc * (2 * QB * 16), QB * 16, 128), IDESC,
+                                     ((s & 1) | term | kc) != 0 ? 1u : 0u);
+                    }
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(slot_free(slot))
+                             : "memory");
+                if (s & 1)
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(acc_full(c & 1))
+                                 : "memory");
+                ++issued;
+                if (s + 2 < steps) {
+                    if (s >= 1) {  // step s - 1's products have read the slot
+                        if (!(ok = mbar_wait(slot_free((s - 1) % NSLOT), ((s - 1) / NSLOT) & 1, TC_WAIT_NS))) break;
+                        freed = s;
+                    }
+                    load_step(s + 2);
+                }
+            }
+            // everything in flight ends before the memory is released
+            if (!ok) atomicExch(&st->fault, 1);
+            if (!q_in) mbar_wait(bar0, 0, TC_WAIT_NS);
+            for (; landed < loaded; ++landed) mbar_wait(full(landed % NSLOT), (landed / NSLOT) & 1, TC_WAIT_NS);
+            for (; freed < issued; ++freed) {
+                if (!mbar_wait(slot_free(freed % NSLOT), (freed / NSLOT) & 1, TC_WAIT_NS)) atomicExch(&st->fault, 1);
+            }
+        }
+        __syncwarp();
+    } else if ((warp >> 2) < nq) {
+        const int b = warp >> 2;
+        const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+        const float4* tn = reinterpret_cast<const float4*>(norms + t.blk * QB);
+        Two f{INFINITY, INFINITY, -1};
+        bool ok = true;
+        for (int c = 0; c < n; ++c) {
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(acc_full(c & 1), (c >> 1) & 1, TC_WAIT_NS)))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int part = 0; part < QB / 32; ++part) {
+                uint32_t v[32];
+                tmem_ld_32x32b<32>(taddr + lanes + (uint32_t)((2 * b + (c & 1)) * QB + 32 * part), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                constexpr float M2 = -2.0f / (PACK_SCALE * PACK_SCALE);
+                const int pair0 = (c * QB + 32 * part) / 2;
+#pragma unroll
+                for (int k = 0; k < 32; k += 4) {
+                    const float4 nb = __ldg(tn + (c * QB + 32 * part + k) / 4);
+                    auto scan = [&](float x, float y, int pair) {  // branch-free; column pairs halve the index work
+                        const float lo = fminf(x, y);
+                        f.v1 = fminf(fminf(f.v1, fmaxf(x, y)), fmaxf(f.v0, lo));
+                        f.pair = lo < f.v0 ? pair : f.pair;
+                        f.v0 = fminf(f.v0, lo);
+                    };
+                    scan(__fmaf_rn(M2, __uint_as_float(v[k]), nb.x), __fmaf_rn(M2, __uint_as_float(v[k + 1]), nb.y),
+                         pair0 + k / 2);
+                    scan(__fmaf_rn(M2, __uint_as_float(v[k + 2]), nb.z), __fmaf_rn(M2, __uint_as_float(v[k + 3]), nb.w),
+                         pair0 + k / 2 + 1);
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_free(c & 1)) : "memory");
+        }
+        if (!ok && lane == 0) atomicExch(&st->fault, 1);
+        const int row = (qb0 + b) * QB + 32 * (warp & 3) + lane;
+        if (ok && row < q.n) (dir ? bwd : fwd)[out0 + row] = f;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(4 * QB));
+}
+
+// The reference's distance (matching.rs:27-33).
+__device__ __forceinline__ float serial_dist(const float* __restrict__ a, const float* __restrict__ b) {
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < DESC_LEN / 4; ++k) {
+        const float4 x = *reinterpret_cast<const float4*>(a + 4 * k), y = *reinterpret_cast<const float4*>(b + 4 * k);
+        const float d0 = x.x - y.x, d1 = x.y - y.y, d2 = x.z - y.z, d3 = x.w - y.w;
+        s = s + d0 * d0;
+        s = s + d1 * d1;
+        s = s + d2 * d2;
+        s = s + d3 * d3;
+    }
+    return s;
+}
+
+// matching.rs:74-90 for one query: its answer, or UINT32_MAX.  The 0.9 cap is
+// the forward direction's.
+__device__ __forceinline__ uint32_t answer(uint32_t idx, float d1, float d2, float ratio, int dir) {
+    if (idx == UINT32_MAX || !isfinite(d2)) return UINT32_MAX;
+    if (dir == 0 && d1 > 0.9f) return UINT32_MAX;
+    return d1 > ratio * d2 ? UINT32_MAX : idx;
+}
+
+__global__ void __launch_bounds__(256) outcome_kernel(const PairJob* __restrict__ jobs, const Frame* __restrict__ frames,
+                                                      const float* __restrict__ desc, const float* __restrict__ norms,
+                                                      const int* __restrict__ max_norm, const Two* __restrict__ fwd2,
+                                                      const Two* __restrict__ bwd2, float ratio,
+                                                      uint32_t* __restrict__ fwd, uint32_t* __restrict__ bwd,
+                                                      int2* __restrict__ list, MatchStatus* __restrict__ st) {
+    const int dir = blockIdx.y & 1;
+    const PairJob J = jobs[blockIdx.y >> 1];
+    Frame q, t;
+    int out0;
+    direction(J, frames, dir, q, t, out0);
+    const int row = blockIdx.x * 256 + threadIdx.x;
+    if (row >= q.n) return;
+    uint32_t out = UINT32_MAX;
+    if (t.n > 1) {  // with fewer targets the second distance is infinite: refused
+        const Two f = (dir ? bwd2 : fwd2)[out0 + row];
+        const float qn = norms[q.blk * QB + row], tm = __int_as_float(max_norm[dir ? J.fa : J.fb]);
+        const float s = sqrtf(qn) + sqrtf(tm);
+        const float d1 = f.v0 + qn, d2 = f.v1 + qn;
+        // the bound at the larger of the two distances, 2% slack
+        const float e = 1.02f * ((3.82e-6f + 9.6e-7f) * s * s + 1.5e-8f * s + 8.0e-6f * fmaxf(d2, 0.0f));
+        const float r_lo = ratio * 0.9999995f, r_hi = ratio * 1.0000005f;
+        const bool refused = (dir == 0 && d1 - e > 0.9000002f) || d1 - e > r_hi * (d2 + e);
+        const bool accepted = (dir != 0 || d1 + e < 0.8999998f) && d1 + e < r_lo * (d2 - e) && d2 - d1 > 2.0f * e;
+        if (accepted) {
+            const int i = 2 * f.pair;
+            const float* a = desc + (q.off + row) * DESC_LEN;
+            const float* b = desc + (t.off + i) * DESC_LEN;
+            out = (uint32_t)i;
+            if (i + 1 < t.n && serial_dist(a, b + DESC_LEN) < serial_dist(a, b)) ++out;
+        } else if (!refused) {
+            const int at = atomicAdd(&st->listed, 1);
+            if (at < RESCAN_MAX) list[at] = make_int2((int)blockIdx.y, row);
+        }
+    }
+    (dir ? bwd : fwd)[out0 + row] = out;
+}
+
+// Listed queries against all targets; one block each.
+__global__ void __launch_bounds__(256) rescan_kernel(const PairJob* __restrict__ jobs, const Frame* __restrict__ frames,
+                                                     const float* __restrict__ desc, float ratio,
+                                                     uint32_t* __restrict__ fwd, uint32_t* __restrict__ bwd,
+                                                     const int2* __restrict__ list, const MatchStatus* __restrict__ st) {
+    __shared__ Nearest part[8];
+    const int n = st->listed;
+    if (n > RESCAN_MAX || st->wild) return;  // the chunk runs again on the FP32 pipes
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const int dir = list[e].x & 1, row = list[e].y;
+        Frame q, t;
+        int out0;
+        direction(jobs[list[e].x >> 1], frames, dir, q, t, out0);
+        float best = INFINITY, second = INFINITY;
+        uint32_t bi = UINT32_MAX;
+        for (int i = threadIdx.x; i < t.n; i += 256)
+            push(serial_dist(desc + (q.off + row) * DESC_LEN, desc + (t.off + i) * DESC_LEN), (uint32_t)i, best, bi, second);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            merge(best, bi, second, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, bi, o),
+                  __shfl_xor_sync(0xffffffffu, second, o));
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = Nearest{bi, best, second};
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < 8; ++k) merge(best, bi, second, part[k].d1, part[k].idx, part[k].d2);
+            (dir ? bwd : fwd)[out0 + row] = answer(bi, best, second, ratio, dir);
+        }
+        __syncthreads();
+    }
+}
+
+// matching.rs:90-94: mutual answers.
+__global__ void mutual_kernel(const PairJob* __restrict__ jobs, const uint32_t* __restrict__ fwd,
+                              const uint32_t* __restrict__ bwd, uint32_t* __restrict__ match_b) {
+    const PairJob J = jobs[blockIdx.y];
+    const int ia = blockIdx.x * 256 + threadIdx.x;
+    if (ia >= J.na) return;
+    const uint32_t f = fwd[J.row_off + ia];
+    match_b[J.row_off + ia] = f != UINT32_MAX && bwd[J.col_off + f] == (uint32_t)ia ? f : UINT32_MAX;
+}
+
 // matching.rs:74-94
 __global__ void decide_kernel(const PairJob* __restrict__ jobs, const Nearest* __restrict__ fwd,
                               const Nearest* __restrict__ bwd, float ratio, uint32_t* __restrict__ match_b) {
@@ -235,8 +621,14 @@ int mfail(rcmvs_ctx* ctx, int code, const std::string& msg) {
                          std::string(#x) + ": " + cudaGetErrorString(e_));                     \
     } while (0)
 
-// Context arena slots 160-167.
-enum { M_DESC = 160, M_JOBS, M_ROWP, M_FWD, M_BWD, M_MB, M_COLP };
+// Context arena slots 160-175.
+enum { M_DESC = 160, M_JOBS, M_ROWP, M_FWD, M_BWD, M_MB, M_COLP, M_FRAMES, M_PACK, M_NORM, M_MAXN, M_TWO, M_LIST, M_STATUS };
+
+// Chunks of fewer distances run on the FP32 pipes: there the tensor-core
+// search's extra launches cost more than its products save.  Whole calls,
+// FP32 / tensor: one pair of 512 122 / 145 us, of 1024 158 / 179, of 2048 290 /
+// 275; 10 pairs of up to 1100 385 / 301, 66 pairs of 2048 5350 / 1760.
+constexpr int64_t TENSOR_MIN = int64_t(1) << 22;
 
 }  // namespace
 }  // namespace rcmvs
@@ -293,18 +685,30 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
             MCK(cudaMemcpyAsync((float*)p_desc + foff[f] * DESC_LEN, desc[f], sizeof(float) * DESC_LEN * n_desc[f],
                                 cudaMemcpyHostToDevice, st));
     const float r32 = (float)ratio;
+    // the tensor-core search's packed frames (made with the first chunk that uses it)
+    std::vector<Frame> frames(n_frames);
+    std::vector<int32_t> blk(n_frames + 1, 0);
+    for (int f = 0; f < n_frames; ++f) {
+        frames[f] = Frame{foff[f], blk[f], n_desc[f]};
+        if (blk[f] > INT32_MAX / 2) return mfail(ctx, RCMVS_E_LIMIT, "too many descriptors");
+        blk[f + 1] = blk[f] + (n_desc[f] + QB - 1) / QB;
+    }
+    // tensor: no frame was found out of range (and a ratio the bound's tests take)
+    bool packed = false, tensor = r32 > 0.0f && r32 < 1e6f;
+    void *p_frames = nullptr, *p_blk = nullptr, *p_pack = nullptr, *p_norm = nullptr, *p_maxn = nullptr, *p_st = nullptr;
     int p = 0;
     while (p < n_pairs) {
         // a chunk of pairs whose distance matrices fit the budget (at least one)
         std::vector<PairJob> jobs;
-        int64_t prow = 0, pcol = 0, rows = 0, cols = 0;
+        int64_t prow = 0, pcol = 0, rows = 0, cols = 0, dists = 0;
         int max_na = 0, max_nb = 0;
-        while (p < n_pairs && jobs.size() < 65535) {
+        while (p < n_pairs && jobs.size() < 32767) {
             const int fa = pairs[2 * p], fb = pairs[2 * p + 1];
             const int na = n_desc[fa], nb = n_desc[fb];
             const int64_t pr = (int64_t)((nb + TILE - 1) / TILE) * na, pc = (int64_t)((na + TILE - 1) / TILE) * nb;
             if (!jobs.empty() && (size_t)(prow + pr + pcol + pc) * sizeof(Nearest) > P_BUDGET) break;
-            jobs.push_back(PairJob{foff[fa], foff[fb], prow, pcol, na, nb, (int32_t)rows, (int32_t)cols});
+            jobs.push_back(PairJob{foff[fa], foff[fb], prow, pcol, na, nb, (int32_t)rows, (int32_t)cols, fa, fb});
+            dists += (int64_t)na * nb;
             prow += pr;
             pcol += pc;
             rows += na;
@@ -318,33 +722,96 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
         if (max_na > 0 && max_nb > 0) {
             void *p_jobs, *p_rowp, *p_colp, *p_fwd, *p_bwd, *p_mb;
             MCK(A.get(M_JOBS, sizeof(PairJob) * jobs.size(), &p_jobs));
-            MCK(A.get(M_ROWP, sizeof(Nearest) * (size_t)std::max<int64_t>(prow, 1), &p_rowp));
-            MCK(A.get(M_COLP, sizeof(Nearest) * (size_t)std::max<int64_t>(pcol, 1), &p_colp));
             MCK(A.get(M_FWD, sizeof(Nearest) * (size_t)rows, &p_fwd));
             MCK(A.get(M_BWD, sizeof(Nearest) * (size_t)cols, &p_bwd));
             MCK(A.get(M_MB, sizeof(uint32_t) * (size_t)rows, &p_mb));
             MCK(cudaMemcpyAsync(p_jobs, jobs.data(), sizeof(PairJob) * jobs.size(), cudaMemcpyHostToDevice, st));
             const unsigned nj = (unsigned)jobs.size();
             const SpanHook& hook = ctx->hook();
-            hook.begin("match_dist");
-            dist_kernel<<<dim3((max_nb + TILE - 1) / TILE, (max_na + TILE - 1) / TILE, nj), 256, 0, st>>>(
-                (const float*)p_desc, (const PairJob*)p_jobs, (Nearest*)p_rowp, (Nearest*)p_colp);
-            MCK(cudaGetLastError());
-            hook.end("match_dist");
-            hook.begin("match_select");
-            rows_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>((const PairJob*)p_jobs,
-                                                                       (const Nearest*)p_rowp, (Nearest*)p_fwd);
-            MCK(cudaGetLastError());
-            cols_kernel<<<dim3((max_nb + 255) / 256, nj), 256, 0, st>>>((const PairJob*)p_jobs,
-                                                                       (const Nearest*)p_colp, (Nearest*)p_bwd);
-            MCK(cudaGetLastError());
-            decide_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>(
-                (const PairJob*)p_jobs, (const Nearest*)p_fwd, (const Nearest*)p_bwd, r32, (uint32_t*)p_mb);
-            MCK(cudaGetLastError());
-            hook.end("match_select");
             std::vector<uint32_t> mb((size_t)rows);
-            MCK(cudaMemcpyAsync(mb.data(), p_mb, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, st));
-            MCK(cudaStreamSynchronize(st));
+            bool on_tensor = tensor && dists >= TENSOR_MIN;
+            if (on_tensor) {
+                void *p_two, *p_list;
+                MCK(A.get(M_TWO, sizeof(Two) * (size_t)(rows + cols), &p_two));
+                MCK(A.get(M_LIST, sizeof(int2) * RESCAN_MAX, &p_list));
+                MCK(A.get(M_STATUS, sizeof(MatchStatus), &p_st));
+                Two *f2 = (Two*)p_two, *b2 = f2 + rows;
+                // the answers share the nearest entries' buffers (larger)
+                uint32_t *fo = (uint32_t*)p_fwd, *bo = (uint32_t*)p_bwd;
+                if (!packed) {
+                    const size_t nb = (size_t)std::max(blk[n_frames], 1);
+                    MCK(A.get(M_FRAMES, (sizeof(Frame) + sizeof(int32_t)) * n_frames, &p_frames));
+                    MCK(A.get(M_PACK, nb * QB_BYTES, &p_pack));
+                    MCK(A.get(M_NORM, nb * QB * sizeof(float), &p_norm));
+                    MCK(A.get(M_MAXN, sizeof(int) * n_frames, &p_maxn));
+                    p_blk = (Frame*)p_frames + n_frames;
+                    MCK(cudaMemcpyAsync(p_frames, frames.data(), sizeof(Frame) * n_frames, cudaMemcpyHostToDevice, st));
+                    MCK(cudaMemcpyAsync(p_blk, blk.data(), sizeof(int32_t) * n_frames, cudaMemcpyHostToDevice, st));
+                    MCK(cudaMemsetAsync(p_maxn, 0, sizeof(int) * n_frames, st));
+                    MCK(cudaFuncSetAttribute(nearest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNearestSmem));
+                }
+                MCK(cudaMemsetAsync(p_st, 0, sizeof(MatchStatus), st));
+                const PairJob* dj = (const PairJob*)p_jobs;
+                const Frame* df = (const Frame*)p_frames;
+                MatchStatus* ds = (MatchStatus*)p_st;
+                hook.begin("match_dist");
+                if (!packed) {
+                    pack_kernel<<<blk[n_frames], 256, 0, st>>>((const float*)p_desc, df, (const int32_t*)p_blk, n_frames,
+                                                               (unsigned char*)p_pack, (float*)p_norm, (int*)p_maxn, ds);
+                    MCK(cudaGetLastError());
+                    packed = true;
+                }
+                const int max_n = std::max(max_na, max_nb);
+                // two query blocks per CTA share each target block's load; one when
+                // that would leave SMs without a CTA
+                int64_t qblocks = 0;
+                for (const PairJob& j : jobs) qblocks += (j.na + QB - 1) / QB + (j.nb + QB - 1) / QB;
+                const int per = qblocks >= 2 * 148 ? 2 : 1;
+                const int max_blk = (max_n + QB - 1) / QB;
+                nearest_kernel<<<dim3((max_blk + per - 1) / per, 2 * nj), kNearestThreads, kNearestSmem, st>>>(
+                    dj, df, (const unsigned char*)p_pack, (const float*)p_norm, per, f2, b2, ds);
+                MCK(cudaGetLastError());
+                hook.end("match_dist");
+                hook.begin("match_select");
+                outcome_kernel<<<dim3((max_n + 255) / 256, 2 * nj), 256, 0, st>>>(
+                    dj, df, (const float*)p_desc, (const float*)p_norm, (const int*)p_maxn, f2, b2, r32, fo, bo,
+                    (int2*)p_list, ds);
+                MCK(cudaGetLastError());
+                rescan_kernel<<<296, 256, 0, st>>>(dj, df, (const float*)p_desc, r32, fo, bo, (const int2*)p_list, ds);
+                MCK(cudaGetLastError());
+                mutual_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>(dj, fo, bo, (uint32_t*)p_mb);
+                MCK(cudaGetLastError());
+                hook.end("match_select");
+                MatchStatus status{};
+                MCK(cudaMemcpyAsync(&status, p_st, sizeof(status), cudaMemcpyDeviceToHost, st));
+                MCK(cudaMemcpyAsync(mb.data(), p_mb, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, st));
+                MCK(cudaStreamSynchronize(st));
+                if (status.fault) return mfail(ctx, RCMVS_E_CUDA, "rcmvs_match_pairs: a tensor-core wait timed out");
+                if (status.wild) tensor = false;
+                on_tensor = !status.wild && status.listed <= RESCAN_MAX;
+            }
+            if (!on_tensor) {
+                MCK(A.get(M_ROWP, sizeof(Nearest) * (size_t)std::max<int64_t>(prow, 1), &p_rowp));
+                MCK(A.get(M_COLP, sizeof(Nearest) * (size_t)std::max<int64_t>(pcol, 1), &p_colp));
+                hook.begin("match_dist");
+                dist_kernel<<<dim3((max_nb + TILE - 1) / TILE, (max_na + TILE - 1) / TILE, nj), 256, 0, st>>>(
+                    (const float*)p_desc, (const PairJob*)p_jobs, (Nearest*)p_rowp, (Nearest*)p_colp);
+                MCK(cudaGetLastError());
+                hook.end("match_dist");
+                hook.begin("match_select");
+                rows_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>((const PairJob*)p_jobs,
+                                                                           (const Nearest*)p_rowp, (Nearest*)p_fwd);
+                MCK(cudaGetLastError());
+                cols_kernel<<<dim3((max_nb + 255) / 256, nj), 256, 0, st>>>((const PairJob*)p_jobs,
+                                                                           (const Nearest*)p_colp, (Nearest*)p_bwd);
+                MCK(cudaGetLastError());
+                decide_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>(
+                    (const PairJob*)p_jobs, (const Nearest*)p_fwd, (const Nearest*)p_bwd, r32, (uint32_t*)p_mb);
+                MCK(cudaGetLastError());
+                hook.end("match_select");
+                MCK(cudaMemcpyAsync(mb.data(), p_mb, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, st));
+                MCK(cudaStreamSynchronize(st));
+            }
             for (size_t c = 0; c < jobs.size(); ++c) {
                 for (int ia = 0; ia < jobs[c].na; ++ia) {
                     const uint32_t b = mb[(size_t)jobs[c].row_off + ia];
