@@ -8,8 +8,9 @@
 //   conv3x3_kernel      3x3 convolution as an implicit GEMM on the 5th-
 //                       generation tensor cores (tcgen05.mma, BF16 operands
 //                       in shared memory, FP32 accumulator in tensor memory)
-//   conv3x3_wgrad_kernel  weight gradient of the same convolution (mma.sync
-//                       m16n8k16, BF16 in, FP32 accumulate)
+//   conv3x3_wgrad_kernel  weight and bias gradients of the same convolution
+//                       (tcgen05.mma over the pixels, FP32 accumulator in
+//                       tensor memory)
 //   loss/Adam kernels   training
 // The patch-match init that consumes the predictions (confident pixels take
 // the predicted plane, the others fall back to the plane sweep) is
@@ -168,23 +169,9 @@ __global__ void __launch_bounds__(CV_TW * CV_TH)
 }
 
 // ------------------------------------------------------------ convolution
-// mma.sync.m16n8k16 BF16 -> FP32.  Fragment layout (PTX ISA, "Matrix
-// Fragments for mma.m16n8k16 with floating point type"): lane = 4*g + t;
-// A rows g and g+8, columns 2t..2t+1 and 2t+8..2t+9; B column g, rows
-// 2t..2t+1 and 2t+8..2t+9; C rows g and g+8, columns 2t..2t+1.
-__device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
 __device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
-
-constexpr int TILE_H = 8, TILE_W = 16;  // output pixels per block: 8 rows x 16 columns (4 warps x 2 rows)
 
 // ---- 5th-generation tensor cores (tcgen05): the forward/data convolution
 // Instruction descriptor of tcgen05.mma.kind::f16: FP32 accumulator (bits
@@ -202,12 +189,12 @@ constexpr int TC_TW = 8, TC_TH = 16;          // output tile: 16 rows x 8 column
 constexpr int TC_SW = TC_TW + 2;              // staged halo tile width
 constexpr int TC_NPIX = (TC_TH + 2) * TC_SW;  // staged pixels
 constexpr int TC_GS = 2944;                   // bytes per channel group of a staged tile: 180 x 16, 128-aligned
-constexpr int TC_CTAS_PER_SM = 3;
+constexpr int TC_CTAS_PER_SM = 5;  // conv3x3_kernel 32 -> 32 at 16 views of 240x180: 2 47 us, 3 45, 4 44, 5 40
 
-template <int CIN, int COUT, bool MASK>
+template <int CIN, int COUT>
 struct ConvSmem {
     static constexpr int KG = CIN / 8;                      // 16-byte channel groups
-    static constexpr int STAGES = MASK ? 1 : 2;             // TMA double buffer; thread staging single
+    static constexpr int STAGES = 2;                        // TMA double buffer
     static constexpr int W_BYTES = 9 * KG * COUT * 16;      // weights [tap][group][COUT][8]
     static constexpr int X_BYTES = KG * TC_GS;              // one staged tile [group][pixel][8]
     static constexpr int BYTES = 128 + W_BYTES + STAGES * X_BYTES;  // + alignment slack
@@ -230,8 +217,11 @@ __device__ __forceinline__ void tma_load_4d(const void* tmap, uint32_t dst, uint
 }
 
 // y = conv3x3(x, w) + b, "same" zero padding; optional ReLU; optional f32
-// output.  w: [9][COUT][CIN] BF16.  mask (optional): x is multiplied by
-// (mask > 0) on load (ReLU derivative of the layer that produced x).
+// output.  w: [9][COUT][CIN] BF16.  MASK: y is zeroed where mask (COUT
+// channels, BF16) is not positive (the backward pass: the ReLU derivative of
+// the layer whose output gradient y is, applied once where y is made instead
+// of in each of y's three readers: 16 views of 240x180, 32 -> 32 channels: 73
+// us with the input masked and staged by threads, 40 us).
 //
 // Implicit GEMM on the tensor cores: D[128 pixels][COUT] = sum over the 9
 // taps and CIN/16 channel chunks of A[128 pixels][16 channels] x
@@ -244,24 +234,21 @@ __device__ __forceinline__ void tma_load_4d(const void* tmap, uint32_t dst, uint
 // pixels x 16 bytes; the next 8 rows of A are the next staged row, 10 pixels
 // on; the next 8 channels are the next channel group), so no im2col copy is
 // made.  The weights are staged once per CTA as [tap][channel group][COUT][8
-// channels].  Persistent CTAs loop over the tiles.  Without a mask the tile
-// arrives by TMA (one box per channel group, zero fill at the borders) into
-// a double buffer: thread 0 starts the next tile's loads before the current
-// tile's MMAs, so they overlap the MMAs and the epilogue.  With a mask (the
-// backward pass) the threads stage the tile, masked, into one buffer.  The
-// accumulator (COUT f32 columns of 128 lanes) is read back by the four warps
+// channels].  Persistent CTAs loop over the tiles.  The tile arrives by TMA
+// (one box per channel group, zero fill at the borders) into a double
+// buffer: thread 0 starts the next tile's loads before the current tile's
+// MMAs, so they overlap the MMAs and the epilogue.  The accumulator (COUT f32 columns of 128 lanes) is read back by the four warps
 // with tcgen05.ld (warp w owns lanes 32w..32w+31).  Every wait is bounded:
 // on a time-out the CTA flags g_tc_fault, waits once more for what it has in
 // flight, frees its tensor memory and returns.
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CUtensorMap tmap,
-                                                      const bf16* __restrict__ x, const bf16* __restrict__ mask, int N,
-                                                      int H, int W, const bf16* __restrict__ wgt,
-                                                      const float* __restrict__ bias, void* __restrict__ y) {
+                                                      const bf16* __restrict__ mask, int N, int H, int W,
+                                                      const bf16* __restrict__ wgt, const float* __restrict__ bias,
+                                                      void* __restrict__ y) {
     static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "conv3x3 shape");
-    using L = ConvSmem<CIN, COUT, MASK>;
+    using L = ConvSmem<CIN, COUT>;
     constexpr int KG = L::KG;
-    constexpr bool TMA = !MASK;
     constexpr uint32_t IDESC = umma_idesc_bf16(128, COUT);
     constexpr uint32_t TILE_TX = (uint32_t)KG * TC_NPIX * 16;  // bytes one tile's boxes deliver
     extern __shared__ __align__(16) unsigned char smem[];
@@ -313,51 +300,29 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CU
     uint32_t issued0 = 0, issued1 = 0, landed0 = 0, landed1 = 0;
     uint32_t mma_issued = 0, mma_done = 0;
     bool ok = true;
-    if (TMA && (int)blockIdx.x < tiles) {
+    if ((int)blockIdx.x < tiles) {
         if (tid == 0) load_tile(blockIdx.x, 0);
         issued0 = 1;
     }
     int it = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
-        const int s = TMA ? (it & 1) : 0;
+        const int s = it & 1;
         const int n = t / per_img, r = t % per_img;
         const int y0 = (r / tiles_x) * TC_TH, x0 = (r % tiles_x) * TC_TW;
         const size_t img = (size_t)n * H * W;
-        if (TMA) {
-            // the other stage was read by the previous tile's MMAs, which completed
-            if (t + (int)gridDim.x < tiles) {
-                if (tid == 0) load_tile(t + gridDim.x, s ^ 1);
-                if (s) ++issued0; else ++issued1;
-            }
+        // the other stage was read by the previous tile's MMAs, which completed
+        if (t + (int)gridDim.x < tiles) {
+            if (tid == 0) load_tile(t + gridDim.x, s ^ 1);
+            if (s) ++issued0; else ++issued1;
+        }
+        {
             const bool got = mbar_wait(s ? full1 : full0, (s ? landed1 : landed0) & 1u, TC_WAIT_NS);
             if (!__syncthreads_and(got)) {
                 ok = false;
                 break;
             }
-            if (s) ++landed1; else ++landed0;
-        } else {
-            uint4* sx = reinterpret_cast<uint4*>(base + L::W_BYTES);
-            for (int i = tid; i < TC_NPIX * KG; i += 128) {
-                const int g = i % KG, p = i / KG;
-                const int gy = y0 - 1 + p / TC_SW, gx = x0 - 1 + p % TC_SW;
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
-                    const size_t gi = (img + (size_t)gy * W + gx) * CIN + g * 8;
-                    v = *reinterpret_cast<const uint4*>(x + gi);
-                    if (MASK) {
-                        const uint4 m = *reinterpret_cast<const uint4*>(mask + gi);
-                        const bf16* mv = reinterpret_cast<const bf16*>(&m);
-                        bf16* xv = reinterpret_cast<bf16*>(&v);
-#pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            if (!(__bfloat162float(mv[q]) > 0.0f)) xv[q] = __float2bfloat16(0.0f);
-                    }
-                }
-                sx[g * (TC_GS / 16) + p] = v;
-            }
-            // generic-proxy smem writes -> visible to the tensor core (async proxy)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
+        if (s) ++landed1; else ++landed0;
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -379,6 +344,13 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CU
         }
         ++mma_issued;
         __syncwarp();
+        const int m = 32 * warp + lane, oy = y0 + m / TC_TW, ox = x0 + m % TC_TW;
+        const size_t o = (img + (size_t)oy * W + ox) * COUT;
+        uint4 mk[MASK ? COUT / 8 : 1];
+        if (MASK && oy < H && ox < W) {  // in flight during the MMAs
+#pragma unroll
+            for (int c = 0; c < COUT / 8; ++c) mk[c] = __ldg(reinterpret_cast<const uint4*>(mask + o) + c);
+        }
         const bool got = mbar_wait(mma_a, mma_done & 1u, TC_WAIT_NS);
         if (!__syncthreads_and(got)) {
             ok = false;
@@ -389,14 +361,13 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CU
         uint32_t v[COUT];
         tmem_ld_32x32b<COUT>(taddr + ((uint32_t)(32 * warp) << 16), v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int m = 32 * warp + lane, oy = y0 + m / TC_TW, ox = x0 + m % TC_TW;
         if (oy < H && ox < W) {
-            const size_t o = (img + (size_t)oy * W + ox) * COUT;
             float f[COUT];
 #pragma unroll
             for (int c = 0; c < COUT; ++c) {
                 float sv = __uint_as_float(v[c]) + s_bias[c];
                 f[c] = RELU ? fmaxf(sv, 0.f) : sv;
+                if (MASK && !(__bfloat162float(reinterpret_cast<const bf16*>(mk)[c]) > 0.0f)) f[c] = 0.0f;
             }
             if (OUT_F32) {
                 float4* yo = reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + o);
@@ -426,137 +397,182 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CU
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(32));
 }
 
-// dW[tap][co][ci] += sum_p dy[p][co] * x[p + tap][ci] over the block's pixel
-// tiles; dy is masked by (mask > 0) when MASK.  Grid: (tile blocks, 9 taps).
-// Per warp: M = COUT rows (co), N = CIN columns (ci), K = 32 of the tile's
-// 128 pixels; partial sums are reduced in shared memory and added to dW.
-template <int CIN, int COUT, bool MASK>
-__global__ void __launch_bounds__(128) conv3x3_wgrad_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
-                                                            const bf16* __restrict__ mask, int N, int H, int W,
-                                                            float* __restrict__ dW) {
-    constexpr int SPX = CIN + 8;
-    constexpr int SPY = COUT + 8;
+template <int CIN>
+struct WgradSmem {
+    static constexpr int CB = (CIN + 31) / 32;    // blocks of 32 channels (zero-filled past CIN)
+    static constexpr int NX = 3 * CB;             // (column tap, block) boxes of x
+    static constexpr int NB = (NX + 3) / 4;       // fours of them: 128 rows of A
+    static constexpr int XB = (TC_TH + 2) * TC_TW * 64, Y_BYTES = TC_TH * TC_TW * 64;  // bytes of a box
+    static constexpr int X_BYTES = NX * XB;
+    // the last four's rows past NX read on into what follows: in bounds
+    static constexpr int READ = X_BYTES + 4 * NB * XB;
+    static constexpr int USED = 2 * (X_BYTES + Y_BYTES);
+    static constexpr int BYTES = 1024 + (READ > USED ? READ : USED);
+    static constexpr int COLS = NB * 3 * 32 <= 128 ? 128 : 256;
+};
+
+// dW[tap][co][ci] += sum_p dy[p][co] * x[p + tap][ci], db[co] += sum_p dy[p][co].
+//
+// On the tensor cores with the pixels as K: A = x^T, B = dy^T, both as TMA
+// lays NHWC tiles down -- 32 channels of a pixel are a 64-byte row, 8
+// consecutive pixels a 512-byte atom -- which is the M- / N-major 64-byte
+// swizzle layout (transpose bits of the instruction descriptor).  For M to
+// hold three taps, x is staged once per column tap kx, shifted by it (TMA
+// boxes of 18 rows x 8 columns x 32 channels): one MMA has the 3 CIN channels
+// (96 of 128 rows at CIN = 32; two fours of boxes at 48) as M, COUT (padded
+// to 32) as N and two tile rows (16 pixels) as K; the row tap ky moves A's
+// start by one row of the box.  The accumulators, one per (four, ky), stay in
+// tensor memory over all tiles of the persistent CTA and are added to dW
+// once.  The threads sum dy for the bias meanwhile.  16 views of 240x180, 32
+// -> 32 channels: mma.sync with a block per tap 365 us and the bias apart 239
+// us; boxes of 8 channels (16-byte pieces, four times as many) 106 us; 73 us
+// here.
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(128) conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap xmap,
+                                                            const __grid_constant__ CUtensorMap ymap, int N, int H, int W,
+                                                            float* __restrict__ dW, float* __restrict__ db) {
+    using L = WgradSmem<CIN>;
+    // F32 accumulator, BF16 operands, both MN-major, N >> 3, M >> 4
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                               ((32u >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ __align__(16) unsigned char smem[];
-    bf16* sx = reinterpret_cast<bf16*>(smem);
-    bf16* sy = sx + (TILE_H + 2) * (TILE_W + 2) * SPX;
-    float* red = reinterpret_cast<float*>(sy + TILE_H * TILE_W * SPY);
-    const int tap = blockIdx.y, ky = tap / 3, kx = tap % 3;
-    const int tiles_x = (W + TILE_W - 1) / TILE_W, tiles_y = (H + TILE_H - 1) / TILE_H;
-    const int n_tiles = N * tiles_x * tiles_y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    constexpr int MT = COUT / 16, NT = CIN / 8;
-    float acc[MT][NT][4];
+    __shared__ __align__(8) uint64_t bars[4];  // tile loaded (2 stages), MMAs done (2 stages)
+    __shared__ uint32_t s_taddr;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t raw_a = smem_u32(smem), base_a = (raw_a + 1023u) & ~1023u;
+    const unsigned char* base = smem + (base_a - raw_a);
+    const uint32_t bar0 = smem_u32(bars);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_taddr)),
+                     "r"(L::COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < 4; ++k) mbar_init(bar0 + 8u * k, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t taddr = s_taddr;
+    const int tiles_x = (W + TC_TW - 1) / TC_TW, tiles_y = (H + TC_TH - 1) / TC_TH;
+    const int per_img = tiles_x * tiles_y, tiles = per_img * N;
+    auto y_stage = [&](int s) { return (uint32_t)(2 * L::X_BYTES + s * L::Y_BYTES); };
+    auto load_tile = [&](int t, int s) {
+        const int n = t / per_img, r = t % per_img;
+        const int y0 = (r / tiles_x) * TC_TH, x0 = (r % tiles_x) * TC_TW;
+        const uint32_t bar = bar0 + 8u * s;
+        mbar_expect_tx(bar, L::X_BYTES + L::Y_BYTES);
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+        for (int kx = 0; kx < 3; ++kx)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.f;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int n = tile / (tiles_x * tiles_y), r = tile % (tiles_x * tiles_y);
-        const int x0 = (r % tiles_x) * TILE_W, y0 = (r / tiles_x) * TILE_H;
-        const size_t img = (size_t)n * H * W;
-        __syncthreads();
-        for (int i = threadIdx.x; i < (TILE_H + 2) * (TILE_W + 2) * (CIN / 8); i += 128) {
-            const int c8 = i % (CIN / 8), p = i / (CIN / 8);
-            const int gy = y0 - 1 + p / (TILE_W + 2), gx = x0 - 1 + p % (TILE_W + 2);
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (gy >= 0 && gy < H && gx >= 0 && gx < W)
-                v = *reinterpret_cast<const uint4*>(x + (img + (size_t)gy * W + gx) * CIN + c8 * 8);
-            *reinterpret_cast<uint4*>(sx + p * SPX + c8 * 8) = v;
-        }
-        for (int i = threadIdx.x; i < TILE_H * TILE_W * (COUT / 8); i += 128) {
-            const int c8 = i % (COUT / 8), p = i / (COUT / 8);
-            const int gy = y0 + p / TILE_W, gx = x0 + p % TILE_W;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (gy < H && gx < W) {
-                const size_t gi = (img + (size_t)gy * W + gx) * COUT + c8 * 8;
-                v = *reinterpret_cast<const uint4*>(dy + gi);
-                if (MASK) {
-                    const uint4 mm = *reinterpret_cast<const uint4*>(mask + gi);
-                    const bf16* mv = reinterpret_cast<const bf16*>(&mm);
-                    bf16* yv = reinterpret_cast<bf16*>(&v);
+            for (int c = 0; c < L::CB; ++c)
+                tma_load_4d(&xmap, base_a + s * L::X_BYTES + (kx * L::CB + c) * L::XB, bar, 32 * c, x0 - 1 + kx, y0 - 1, n);
+        tma_load_4d(&ymap, base_a + y_stage(s), bar, 0, x0, y0, n);
+    };
+    float bs[COUT];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (!(__bfloat162float(mv[q]) > 0.0f)) yv[q] = __float2bfloat16(0.0f);
+    for (int c = 0; c < COUT; ++c) bs[c] = 0.0f;
+    int loaded = 0, landed = 0, issued = 0, done = 0;  // tiles of this CTA (thread 0: done)
+    bool ok = true;
+    if ((int)blockIdx.x < tiles) {
+        if (tid == 0) load_tile(blockIdx.x, 0);
+        ++loaded;
+    }
+    int it = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
+        const int s = it & 1;
+        if (t + (int)gridDim.x < tiles) {
+            if (tid == 0) {
+                // the other stage's MMAs (the tile before) have read it
+                if (it > 0 && ok) {
+                    ok = mbar_wait(bar0 + 16u + 8u * (s ^ 1), ((it - 1) >> 1) & 1, TC_WAIT_NS);
+                    if (ok) done = it;
                 }
+                if (ok) load_tile(t + gridDim.x, s ^ 1);
             }
-            *reinterpret_cast<uint4*>(sy + p * SPY + c8 * 8) = v;
+            if (ok) ++loaded;
         }
-        __syncthreads();
-        // warp w: pixels k in [32w, 32w+32) of the tile = 2 k-steps of 16
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            const int kbase = warp * 32 + ks * 16;
-            const int pa = kbase + 2 * t, pb = pa + 8;  // pixel indices of this lane's k pairs
-            uint32_t a[MT][4];
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const int co = m * 16 + g;
-                a[m][0] = pack2(sy[pa * SPY + co], sy[(pa + 1) * SPY + co]);
-                a[m][1] = pack2(sy[pa * SPY + co + 8], sy[(pa + 1) * SPY + co + 8]);
-                a[m][2] = pack2(sy[pb * SPY + co], sy[(pb + 1) * SPY + co]);
-                a[m][3] = pack2(sy[pb * SPY + co + 8], sy[(pb + 1) * SPY + co + 8]);
-            }
-            // x at pixel p shifted by the tap: shared cell (p/16 + ky, p%16 + kx)
-            const int xa0 = ((pa / TILE_W) + ky) * (TILE_W + 2) + (pa % TILE_W) + kx;
-            const int xa1 = (((pa + 1) / TILE_W) + ky) * (TILE_W + 2) + ((pa + 1) % TILE_W) + kx;
-            const int xb0 = ((pb / TILE_W) + ky) * (TILE_W + 2) + (pb % TILE_W) + kx;
-            const int xb1 = (((pb + 1) / TILE_W) + ky) * (TILE_W + 2) + ((pb + 1) % TILE_W) + kx;
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                const int ci = nt * 8 + g;
-                const uint32_t b0 = pack2(sx[xa0 * SPX + ci], sx[xa1 * SPX + ci]);
-                const uint32_t b1 = pack2(sx[xb0 * SPX + ci], sx[xb1 * SPX + ci]);
-#pragma unroll
-                for (int m = 0; m < MT; ++m) mma_bf16(acc[m][nt], a[m], b0, b1);
-            }
+        __syncwarp();
+        const bool got = mbar_wait(bar0 + 8u * s, (it >> 1) & 1, TC_WAIT_NS);
+        if (!__syncthreads_and(got && ok)) {
+            ok = false;
+            break;
         }
+        ++landed;
+        if (tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t xs = base_a + s * L::X_BYTES, ys = base_a + y_stage(s);
+#pragma unroll
+            for (int b = 0; b < L::NB; ++b)
+#pragma unroll
+                for (int ky = 0; ky < 3; ++ky)
+#pragma unroll
+                    for (int k = 0; k < TC_TH / 2; ++k)
+                        umma_f16(taddr + (b * 3 + ky) * 32,
+                                 umma_desc_sw64_mn(xs + b * 4 * L::XB + (2 * k + ky) * (TC_TW * 64), L::XB, TC_TW * 64),
+                                 umma_desc_sw64_mn(ys + 2 * k * (TC_TW * 64), L::Y_BYTES, TC_TW * 64), IDESC,
+                                 (it | k) != 0 ? 1u : 0u);
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 16u + 8u * s)
+                         : "memory");
+        }
+        ++issued;
+#pragma unroll
+        for (int g = 0; g < COUT / 8; ++g) {  // pixel tid's chunk g
+            const uint4 v = *reinterpret_cast<const uint4*>(base + y_stage(s) + tid * 64 + ((g ^ (tid >> 1)) & 3) * 16);
+            const bf16* e = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) bs[8 * g + c] += __bfloat162float(e[c]);
+        }
+        __syncthreads();  // the stage's dy has been read
     }
-    // reduce the 4 warps: red[co][ci]
-    __syncthreads();
-    for (int i = threadIdx.x; i < COUT * CIN; i += 128) red[i] = 0.f;
-    __syncthreads();
+    // the MMAs still in flight (the last two tiles')
+    if (tid == 0) {
+        for (int k = done; k < issued; ++k) ok = mbar_wait(bar0 + 16u + 8u * (k & 1), (k >> 1) & 1, TC_WAIT_NS) && ok;
+        for (int k = landed; k < loaded; ++k) mbar_wait(bar0 + 8u * (k & 1), (k >> 1) & 1, TC_WAIT_NS);
+        if (!ok) atomicExch(&g_tc_fault, 1);
+    }
+    if (__syncthreads_and(ok) && it > 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+        for (int b = 0; b < L::NB; ++b) {
+            const int box = 4 * b + warp;  // row 32 warp + lane: its channel `lane`
+            const int kx = box / L::CB, ci = (box % L::CB) * 32 + lane;
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int co = m * 16 + g, ci = nt * 8 + 2 * t;
-            atomicAdd(&red[co * CIN + ci], acc[m][nt][0]);
-            atomicAdd(&red[co * CIN + ci + 1], acc[m][nt][1]);
-            atomicAdd(&red[(co + 8) * CIN + ci], acc[m][nt][2]);
-            atomicAdd(&red[(co + 8) * CIN + ci + 1], acc[m][nt][3]);
+            for (int ky = 0; ky < 3; ++ky) {
+                uint32_t v[32];
+                tmem_ld_32x32b<32>(taddr + ((uint32_t)(32 * warp) << 16) + (uint32_t)((b * 3 + ky) * 32), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (box < L::NX && ci < CIN)
+#pragma unroll
+                    for (int co = 0; co < COUT; ++co)
+                        atomicAdd(&dW[((size_t)(ky * 3 + kx) * COUT + co) * CIN + ci], __uint_as_float(v[co]));
+            }
         }
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) {
+            float v = bs[c];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) atomicAdd(&db[c], v);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < COUT * CIN; i += 128) atomicAdd(&dW[(size_t)tap * COUT * CIN + i], red[i]);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(L::COLS));
 }
 
-// db[c] += sum over pixels of dy[p][c] * (mask[p][c] > 0)
-template <int C, bool MASK>
-__global__ void bias_grad_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ mask, int64_t npx,
-                                 float* __restrict__ db) {
-    float s[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) s[c] = 0.f;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npx; p += (int64_t)gridDim.x * blockDim.x)
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            float v = __bfloat162float(dy[p * C + c]);
-            if (MASK && !(__bfloat162float(mask[p * C + c]) > 0.f)) v = 0.f;
-            s[c] += v;
-        }
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-        float v = s[c];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&db[c], v);
-    }
-}
-
-// backward-data weights: wt[tap][ci][co] = w[8 - tap][co][ci]
-__global__ void flip_weights_kernel(const bf16* __restrict__ w, int cout, int cin, bf16* __restrict__ wt) {
+// backward-data weights of layers 1 .. NET_LAYERS - 1: wt[tap][ci][co] =
+// w[8 - tap][co][ci], each layer at its offset (block row y: layer y + 1)
+struct FlipTable {
+    int off[NET_LAYERS - 1], cin[NET_LAYERS - 1], cout[NET_LAYERS - 1];
+};
+__global__ void flip_weights_kernel(const bf16* __restrict__ w, const __grid_constant__ FlipTable t,
+                                    bf16* __restrict__ wt) {
+    const int cin = t.cin[blockIdx.y], cout = t.cout[blockIdx.y], off = t.off[blockIdx.y];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 9 * cout * cin) return;
     const int ci = i % cin, co = (i / cin) % cout, tap = i / (cin * cout);
-    wt[((size_t)(8 - tap) * cin + ci) * cout + co] = w[i];
+    wt[off + ((8 - tap) * cin + ci) * cout + co] = w[off + i];
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ a, int64_t n, bf16* __restrict__ b) {
@@ -574,8 +590,12 @@ __global__ void loss_kernel(const float* __restrict__ out, const float* __restri
                             bf16* __restrict__ dout, float* __restrict__ acc) {
     float l = 0.f, cnt = 0.f;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npx; p += (int64_t)gridDim.x * blockDim.x) {
-        const float* o = out + p * NET_OUT_C;
-        const float* L = lab + p * 8;
+        // whole sectors at a time (t, normal | logit; t*, n* | n*z.., valid, tolerance)
+        const float4* o4 = reinterpret_cast<const float4*>(out + p * NET_OUT_C);
+        const float4* l4 = reinterpret_cast<const float4*>(lab + p * 8);
+        const float4 oa = o4[0], la = l4[0], lb = l4[1];
+        const float o[5] = {oa.x, oa.y, oa.z, oa.w, out[p * NET_OUT_C + 4]};
+        const float L[6] = {la.x, la.y, la.z, la.w, lb.x, lb.y};
         float g[NET_OUT_C];
 #pragma unroll
         for (int c = 0; c < NET_OUT_C; ++c) g[c] = 0.f;
@@ -594,8 +614,15 @@ __global__ void loss_kernel(const float* __restrict__ out, const float* __restri
             g[4] = LC * (pr - tgt);
             cnt += 1.f;
         }
+        uint4* d = reinterpret_cast<uint4*>(dout + p * NET_OUT_C);
 #pragma unroll
-        for (int c = 0; c < NET_OUT_C; ++c) dout[p * NET_OUT_C + c] = __float2bfloat16(g[c] * inv_n);
+        for (int c = 0; c < NET_OUT_C / 8; ++c) {
+            uint32_t v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                v[k] = pack2(__float2bfloat16(g[8 * c + 2 * k] * inv_n), __float2bfloat16(g[8 * c + 2 * k + 1] * inv_n));
+            d[c] = make_uint4(v[0], v[1], v[2], v[3]);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         l += __shfl_down_sync(0xffffffffu, l, o);
@@ -662,19 +689,29 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// The NHWC BF16 input as a 4-D tensor (C, W, H, N) for TMA, box (8, 10, 18,
-// 1): one channel group of a staged halo tile.
-cudaError_t input_tensor_map(const void* x, int cin, int N, int H, int W, CUtensorMap* out) {
+// An NHWC BF16 tensor as a 4-D one (C, W, H, N) for TMA, box (bc, bw, bh, 1):
+// a channel group of 8 of a staged tile, or 32 channels in the 64-byte swizzle.
+cudaError_t input_tensor_map(const void* x, int cin, int N, int H, int W, int bc, int bw, int bh, CUtensorMap* out) {
     auto enc = tensor_map_encoder();
     if (!enc) return cudaErrorNotSupported;
     const cuuint64_t dims[4] = {(cuuint64_t)cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
     const cuuint64_t strides[3] = {(cuuint64_t)cin * 2, (cuuint64_t)W * cin * 2, (cuuint64_t)H * W * cin * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)TC_SW, (cuuint32_t)(TC_TH + 2), 1};
+    const cuuint32_t box[4] = {(cuuint32_t)bc, (cuuint32_t)bw, (cuuint32_t)bh, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           bc == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// Persistent CTAs per SM of a tensor-core kernel: as many as its shared
+// memory (227 KB an SM, 1 KB each reserved) and tensor memory (512 columns)
+// hold, at most `most`.  (The occupancy calculator answers 1 for
+// kernels that allocate tensor memory.)
+static int tc_ctas(size_t smem, int columns, int most = TC_CTAS_PER_SM) {
+    const int n = std::min((int)(227 * 1024 / (smem + 1024)), 512 / columns);
+    return std::max(1, std::min(n, most));
 }
 
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
@@ -686,17 +723,16 @@ static cudaError_t conv_t(const void* x, const void* mask, int N, int H, int W, 
     CUtensorMap tmap;
     std::memset(&tmap, 0, sizeof(tmap));
     cudaError_t e;
-    if (!MASK && (e = input_tensor_map(x, CIN, N, H, W, &tmap))) return e;
-    const size_t sm = ConvSmem<CIN, COUT, MASK>::BYTES;
+    if ((e = input_tensor_map(x, CIN, N, H, W, 8, TC_SW, TC_TH + 2, &tmap))) return e;
+    const size_t sm = ConvSmem<CIN, COUT>::BYTES;
     auto k = conv3x3_kernel<CIN, COUT, RELU, OUT_F32, MASK>;
     if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm))) return e;
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return e;
     const long long tiles = (long long)((W + TC_TW - 1) / TC_TW) * ((H + TC_TH - 1) / TC_TH) * N;
     if (tiles > INT_MAX) return cudaErrorInvalidValue;
-    const int grid = (int)std::min<long long>(tiles, (long long)sms * TC_CTAS_PER_SM);
-    k<<<grid, 128, sm, st>>>(tmap, reinterpret_cast<const bf16*>(x), reinterpret_cast<const bf16*>(mask), N, H, W,
-                             reinterpret_cast<const bf16*>(w), b, y);
+    const int grid = (int)std::min<long long>(tiles, (long long)sms * tc_ctas(sm, 32));
+    k<<<grid, 128, sm, st>>>(tmap, reinterpret_cast<const bf16*>(mask), N, H, W, reinterpret_cast<const bf16*>(w), b, y);
     return cudaGetLastError();
 }
 
@@ -735,52 +771,58 @@ cudaError_t launch_conv3x3(int cin, int cout, bool relu, bool out_f32, const voi
     if (cin == 48 && cout == 32 && relu && !out_f32 && !m) return conv_t<48, 32, true, false, false>(x, mask, N, H, W, w, b, y, st);
     if (cin == 32 && cout == 32 && relu && !out_f32 && !m) return conv_t<32, 32, true, false, false>(x, mask, N, H, W, w, b, y, st);
     if (cin == 32 && cout == 16 && !relu && out_f32 && !m) return conv_t<32, 16, false, true, false>(x, mask, N, H, W, w, b, y, st);
-    // backward data: input = masked upstream gradient, no bias, no ReLU
-    if (cin == 16 && cout == 32 && !relu && !out_f32 && !m) return conv_t<16, 32, false, false, false>(x, mask, N, H, W, w, b, y, st);
+    // backward data: no bias, no ReLU, the result masked by the layer's output
+    if (cin == 16 && cout == 32 && !relu && !out_f32 && m) return conv_t<16, 32, false, false, true>(x, mask, N, H, W, w, b, y, st);
     if (cin == 32 && cout == 32 && !relu && !out_f32 && m) return conv_t<32, 32, false, false, true>(x, mask, N, H, W, w, b, y, st);
     return cudaErrorInvalidValue;
 }
 
-template <int CIN, int COUT, bool MASK>
-static cudaError_t wgrad_t(const void* x, const void* dy, const void* mask, int N, int H, int W, float* dW,
-                           cudaStream_t st) {
-    const size_t sm = sizeof(bf16) * ((TILE_H + 2) * (TILE_W + 2) * (CIN + 8) + TILE_H * TILE_W * (COUT + 8)) +
-                      sizeof(float) * COUT * CIN;
-    auto k = conv3x3_wgrad_kernel<CIN, COUT, MASK>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e) return e;
-    const int tiles = N * ((W + TILE_W - 1) / TILE_W) * ((H + TILE_H - 1) / TILE_H);
-    dim3 grid(std::min(tiles, 148 * 2), 9);
-    k<<<grid, 128, sm, st>>>(reinterpret_cast<const bf16*>(x), reinterpret_cast<const bf16*>(dy),
-                             reinterpret_cast<const bf16*>(mask), N, H, W, dW);
+template <int CIN, int COUT>
+static cudaError_t wgrad_t(const void* x, const void* dy, int N, int H, int W, float* dW, float* db, cudaStream_t st) {
+    if (N <= 0 || H <= 0 || W <= 0) return cudaSuccess;
+    if (((uintptr_t)x | (uintptr_t)dy) & 15) return cudaErrorMisalignedAddress;
+    using L = WgradSmem<CIN>;
+    CUtensorMap xmap, ymap;
+    cudaError_t e;
+    if ((e = input_tensor_map(x, CIN, N, H, W, 32, TC_TW, TC_TH + 2, &xmap)) ||
+        (e = input_tensor_map(dy, COUT, N, H, W, 32, TC_TW, TC_TH, &ymap)))
+        return e;
+    auto k = conv3x3_wgrad_kernel<CIN, COUT>;
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES))) return e;
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return e;
+    const long long tiles = (long long)((W + TC_TW - 1) / TC_TW) * ((H + TC_TH - 1) / TC_TH) * N;
+    if (tiles > INT_MAX) return cudaErrorInvalidValue;
+    // two: 73 us a layer of 32 channels; one 82; three 84 (each CTA adds 9 taps
+    // of sums to dW at its end)
+    const int grid = (int)std::min<long long>(tiles, (long long)sms * tc_ctas(L::BYTES, L::COLS, 2));
+    k<<<grid, 128, L::BYTES, st>>>(xmap, ymap, N, H, W, dW, db);
     return cudaGetLastError();
 }
 
-cudaError_t launch_conv3x3_wgrad(int cin, int cout, const void* x, const void* dy, const void* mask, int N, int H,
-                                 int W, float* dW, cudaStream_t st) {
-    const bool m = mask != nullptr;
-    if (cin == 48 && cout == 32 && m) return wgrad_t<48, 32, true>(x, dy, mask, N, H, W, dW, st);
-    if (cin == 32 && cout == 32 && m) return wgrad_t<32, 32, true>(x, dy, mask, N, H, W, dW, st);
-    if (cin == 32 && cout == 16 && !m) return wgrad_t<32, 16, false>(x, dy, mask, N, H, W, dW, st);
+cudaError_t launch_conv3x3_wgrad(int cin, int cout, const void* x, const void* dy, int N, int H, int W, float* dW,
+                                 float* db, cudaStream_t st) {
+    if (cin == 48 && cout == 32) return wgrad_t<48, 32>(x, dy, N, H, W, dW, db, st);
+    if (cin == 32 && cout == 32) return wgrad_t<32, 32>(x, dy, N, H, W, dW, db, st);
+    if (cin == 32 && cout == 16) return wgrad_t<32, 16>(x, dy, N, H, W, dW, db, st);
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_bias_grad(int c, const void* dy, const void* mask, int64_t npx, float* db, cudaStream_t st) {
-    const int blocks = (int)std::min<int64_t>((npx + 255) / 256, 148 * 4);
-    if (c == 32 && mask)
-        bias_grad_kernel<32, true><<<blocks, 256, 0, st>>>(reinterpret_cast<const bf16*>(dy),
-                                                           reinterpret_cast<const bf16*>(mask), npx, db);
-    else if (c == 16 && !mask)
-        bias_grad_kernel<16, false><<<blocks, 256, 0, st>>>(reinterpret_cast<const bf16*>(dy), nullptr, npx, db);
-    else
-        return cudaErrorInvalidValue;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_flip_weights(const void* w, int cout, int cin, void* wt, cudaStream_t st) {
-    const int n = 9 * cout * cin;
-    flip_weights_kernel<<<(n + 255) / 256, 256, 0, st>>>(reinterpret_cast<const bf16*>(w), cout, cin,
-                                                         reinterpret_cast<bf16*>(wt));
+cudaError_t launch_flip_weights(const void* w, void* wt, cudaStream_t st) {
+    FlipTable t;
+    int off = 0, most = 0;
+    for (int l = 0; l < NET_LAYERS; ++l) {
+        const int n = 9 * NET_CIN[l] * NET_COUT[l];
+        if (l > 0) {
+            t.off[l - 1] = off;
+            t.cin[l - 1] = NET_CIN[l];
+            t.cout[l - 1] = NET_COUT[l];
+            most = std::max(most, n);
+        }
+        off += n + NET_COUT[l];
+    }
+    flip_weights_kernel<<<dim3((most + 255) / 256, NET_LAYERS - 1), 256, 0, st>>>(reinterpret_cast<const bf16*>(w), t,
+                                                                                 reinterpret_cast<bf16*>(wt));
     return cudaGetLastError();
 }
 

@@ -33,10 +33,12 @@ int tc_fault_take();
 // One block waits limit_ns on an mbarrier that nothing arrives on and sets
 // the fault word when the wait gives up (rcmvs_diag_wait_timeout).
 cudaError_t launch_wait_probe(uint64_t limit_ns, cudaStream_t st);
-cudaError_t launch_conv3x3_wgrad(int cin, int cout, const void* x, const void* dy, const void* mask, int N, int H,
-                                 int W, float* dW, cudaStream_t st);
-cudaError_t launch_bias_grad(int c, const void* dy, const void* mask, int64_t npx, float* db, cudaStream_t st);
-cudaError_t launch_flip_weights(const void* w, int cout, int cin, void* wt, cudaStream_t st);
+// dW += and db += the convolution's weight and bias gradients.
+cudaError_t launch_conv3x3_wgrad(int cin, int cout, const void* x, const void* dy, int N, int H, int W, float* dW,
+                                 float* db, cudaStream_t st);
+// Backward-data weights of layers 1.. of the BF16 parameters w, each at its
+// own offset in wt (as large as w).
+cudaError_t launch_flip_weights(const void* w, void* wt, cudaStream_t st);
 cudaError_t launch_to_bf16(const float* a, int64_t n, void* b, cudaStream_t st);
 cudaError_t launch_loss(const float* out, const float* lab, int64_t npx, float inv_n, void* dout, float* acc,
                         cudaStream_t st);

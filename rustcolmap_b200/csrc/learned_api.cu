@@ -217,8 +217,11 @@ int rcmvs_net_train_step(rcmvs_ctx* ctx, rcmvs_net* net, const void* x_dev, cons
     LCK(cudaMemsetAsync(acc, 0, 16, st));
     LCK(launch_loss((const float*)out, labels_dev, npx, 1.0f, dout, (float*)acc, st));
     LCK(cudaMemsetAsync(net->g, 0, 4 * net->n, st));
-    // backward, last layer first.  dY of layer l is in `dcur` (its pre-ReLU
-    // gradient is dY * (Y > 0), applied on load through the mask).
+    void* flip;
+    LCK(net->arena.get(N_FLIP, 2 * net->n, &flip));
+    LCK(launch_flip_weights(net->pb, flip, st));
+    // backward, last layer first.  dcur: the pre-ReLU output gradient of
+    // layer l (the convolution that makes it applies the ReLU derivative)
     const void* dcur = dout;
     int flipbuf = 0;
     for (int l = NET_LAYERS - 1; l >= 0; --l) {
@@ -229,16 +232,12 @@ int rcmvs_net_train_step(rcmvs_ctx* ctx, rcmvs_net* net, const void* x_dev, cons
         } else {
             LCK(net->arena.get(N_ACT0 + l, 2 * npx * NET_COUT[l - 1], &xin));
         }
-        void* ymask = nullptr;  // this layer's ReLU output (none for the head)
-        if (l < NET_LAYERS - 1) LCK(net->arena.get(N_ACT0 + 1 + l, 2 * npx * y.cout, &ymask));
-        LCK(launch_conv3x3_wgrad(y.cin, y.cout, xin, dcur, ymask, n, h, w, net->g + y.w_off, st));
-        LCK(launch_bias_grad(y.cout, dcur, ymask, npx, net->g + y.b_off, st));
+        LCK(launch_conv3x3_wgrad(y.cin, y.cout, xin, dcur, n, h, w, net->g + y.w_off, net->g + y.b_off, st));
         if (l > 0) {
-            void *flip, *dnext;
-            LCK(net->arena.get(N_FLIP, 2 * 9 * y.cout * y.cin, &flip));
-            LCK(launch_flip_weights(wb(net, y), y.cout, y.cin, flip, st));
+            void* dnext;
             LCK(net->arena.get(N_DY0 + flipbuf, 2 * npx * y.cin, &dnext));
-            LCK(launch_conv3x3(y.cout, y.cin, false, false, dcur, ymask, n, h, w, flip, nullptr, dnext, st));
+            LCK(launch_conv3x3(y.cout, y.cin, false, false, dcur, xin, n, h, w, (const char*)flip + 2 * y.w_off, nullptr,
+                               dnext, st));
             dcur = dnext;
             flipbuf ^= 1;
         }

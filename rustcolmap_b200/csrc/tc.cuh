@@ -20,6 +20,14 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// The same for operands of 64-byte rows in the 64-byte swizzle (layout type 4
+// at bits 61-63: 16-byte chunk index XOR address bits 7-8, as TMA's
+// SWIZZLE_64B writes them).  M- / N-major: a row is 32 elements of M / N at
+// one k; `mn` bytes between blocks of 32, `k` bytes between groups of 8 k.
+__device__ __forceinline__ uint64_t umma_desc_sw64_mn(uint32_t saddr, uint32_t mn, uint32_t k) {
+    return umma_desc(saddr, mn, k) | (4ull << 61);
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
