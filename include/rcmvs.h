@@ -76,7 +76,7 @@ typedef struct rcmvs_options {
 
 /* The plane-sweep init evaluates each pixel's hypotheses one at a time, a
  * warp waiting at every hypothesis for its slowest lane, instead of the
- * default table sweep (RCMVS_FLAG_ROW_STEP_INIT).  Same results bit for
+ * default staged sweep (RCMVS_FLAG_ROW_STEP_INIT).  Same results bit for
  * bit; kept for comparison.  The Jacobi passes are chosen by
  * threads_per_pixel and RCMVS_FLAG_LOCKSTEP_PASSES. */
 #define RCMVS_FLAG_ONE_CANDIDATE 1u
@@ -126,12 +126,15 @@ typedef struct rcmvs_options {
  * pixel skips the sweep. */
 #define RCMVS_FLAG_SEED_AND_SWEEP 64u
 
-/* The plane sweep of the init by default walks the hypotheses block by
- * block: for each hypothesis and support view the window counts of a tile
- * and its halo are computed once into shared memory (on a fronto-parallel
- * plane a window cell's count does not depend on which pixel's window holds
- * it) and every pixel runs the reference's chain over them.  This flag
- * selects the row-step sweep instead (each lane streams its own hypotheses
+/* The plane sweep of the init by default is staged: per hypothesis the first
+ * support view's window counts of a 32x8 tile and its halo are computed once
+ * into shared memory (on a fronto-parallel plane a window cell's count does
+ * not depend on which pixel's window holds it), and only what survives that
+ * view goes through the others, packed.  With a tile shape chosen (tile_w /
+ * tile_h, RCMVS_FLAG_AUTOTUNE), RCMVS_FLAG_PERSISTENT, work counting,
+ * RCMVS_FLAG_NO_SKIP_DUPLICATES or RCMVS_FLAG_LOCKSTEP_PASSES the table sweep
+ * runs, which has such counts for every support view a pixel still needs.
+ * This flag selects the row-step sweep instead (each lane streams its own hypotheses
  * one window row at a time).  Same results bit for bit. */
 #define RCMVS_FLAG_ROW_STEP_INIT 128u
 

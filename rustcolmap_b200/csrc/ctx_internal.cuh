@@ -164,7 +164,7 @@ namespace rcmvs {
 // private to capi.cu 2-10, fuse.cu 16-37 and 70-74, learned_api.cu 40-47, depthvis.cu 50-55,
 // resize.cu 60-68, sift.cu 80-159 and match.cu 160-175).
 constexpr int kSlotJobs = 0, kSlotJobStart = 1, kSlotQueue = 11, kSlotTuneJobs = 12, kSlotTuneStart = 13,
-              kSlotStreamStart = 14, kSlotStreamScratch = 15;
+              kSlotStreamStart = 14, kSlotStreamScratch = 15, kSlotInitStart = 38;
 
 // resize.cu: argument and size checks of a resize, and the resize itself
 // on device buffers (d_gray mw*mh, d_rgb mw*mh*3), queued on the context's
@@ -195,6 +195,9 @@ struct StereoBatch {
     int tiled = TILED_NONE;
     std::vector<int32_t> sstart;
     LaunchGeom sgeom{};
+    // init_staged_kernel's, with the staged passes
+    std::vector<int32_t> istart;
+    LaunchGeom igeom{};
 };
 
 // The launch schedule of a batch: init -> n_passes Jacobi passes -> gate.

@@ -81,14 +81,14 @@ struct LaunchGeom {
     int tiles;
     unsigned int* queue;
     int tpp = 1;  // threads per pixel of the passes: 1, or 5 (pass_split_kernel)
-    bool radial = false;  // a support view of the batch has k != 0
+    bool radial = true;  // false: every reference and support camera of the launch has k = 0
     int tiled = 0;  // passes: the tiled kernels (TILED_*) over their own tiling (tiled_geom), 0 = one block per tile
     unsigned char* scratch = nullptr;  // tiled passes: per-block scratch (tiled_scratch_bytes)
     int scratch_blocks = 0;            // blocks the scratch holds (the launch uses at most this many)
 };
-// The pass kernels with a tiling of their own: pass_stream_kernel and
-// pass_staged_kernel's tile sizes.
-enum { TILED_NONE = 0, TILED_STREAM = 1, TILED_STAGED = 2 };
+// The kernels with a tiling of their own: pass_stream_kernel,
+// pass_staged_kernel and init_staged_kernel.
+enum { TILED_NONE = 0, TILED_STREAM = 1, TILED_STAGED = 2, TILED_INIT = 3 };
 // Tiled passes: tiles of a w x h view in the kernel's own tiling, and the
 // geometry of a launch over `tiles` of them.  The launch is always
 // persistent (g.queue set) over at most tiled_grid(g) blocks, each with its
@@ -125,6 +125,9 @@ int stereo_resident_grid(const LaunchGeom& g);
 cudaError_t launch_init(const DevJob* d_jobs, const int32_t* d_job_start, int n_jobs, const LaunchGeom& g, int nh,
                         const uint64_t* census, const float2* rays, PlaneBuf out, unsigned long long* d_work,
                         cudaStream_t st, int variant);
+// The same by init_staged_kernel over its own tiling (tiled_geom(TILED_INIT)).
+cudaError_t launch_init_staged(const DevJob* d_jobs, const int32_t* d_tile_start, int n_jobs, const LaunchGeom& g, int nh,
+                               const uint64_t* census, const float2* rays, PlaneBuf out, cudaStream_t st);
 // One Jacobi pass prev -> next (stereo.rs:271-371).
 cudaError_t launch_pass(const DevJob* d_jobs, const int32_t* d_job_start, int n_jobs, const LaunchGeom& g,
                         uint64_t pass, float sig_inv, float sig_n, const uint64_t* census, const float2* rays,

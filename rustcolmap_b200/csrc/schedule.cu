@@ -95,25 +95,25 @@ int assemble(rcmvs_ctx* ctx, rcmvs_scene* sc, const rcmvs_job* jobs, int n_jobs,
     if (tiles > INT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "too many tiles in one batch");
     b.start[n_jobs] = (int32_t)tiles;
     b.geom = LaunchGeom{nthr, smem, (int)tiles, nullptr};
+    b.geom.radial = false;
     for (const DevJob& J : b.jobs)
         for (int q = 0; q < J.nsrc; ++q) b.geom.radial = b.geom.radial || J.src[q].k != 0.0f;
     for (int j = 0; j < n_jobs; ++j) b.geom.radial = b.geom.radial || sc->cams[jobs[j].ref_idx].k != 0.0;
     return RCMVS_OK;
 }
 
-// The tiled passes' own tiling of b's jobs, in launch order.
-int assemble_tiled(rcmvs_ctx* ctx, int kind, StereoBatch& b) {
-    b.tiled = kind;
-    b.sstart.resize(b.jobs.size() + 1);
+// A tiled kernel's own tiling of b's jobs, in launch order.
+int assemble_tiled(rcmvs_ctx* ctx, int kind, const StereoBatch& b, std::vector<int32_t>& start, LaunchGeom& g) {
+    start.resize(b.jobs.size() + 1);
     int64_t tiles = 0;
     for (size_t p = 0; p < b.jobs.size(); ++p) {
-        b.sstart[p] = (int32_t)tiles;
+        start[p] = (int32_t)tiles;
         tiles += tiled_tiles(kind, b.jobs[p].w, b.jobs[p].h);
         if (tiles > INT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "too many tiles in one batch");
     }
-    b.sstart.back() = (int32_t)tiles;
-    b.sgeom = tiled_geom(kind, (int)tiles);
-    b.sgeom.radial = b.geom.radial;
+    start.back() = (int32_t)tiles;
+    g = tiled_geom(kind, (int)tiles);
+    g.radial = b.geom.radial;
     return RCMVS_OK;
 }
 
@@ -325,11 +325,14 @@ int build_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const rcmvs_job* jobs, int n_jo
     b.geom.tpp = tpp;
     // The staged passes evaluate candidates ahead of the reference's sequence;
     // work counts and its own call sequence come from the streamed ones.
-    if (rc == RCMVS_OK && tpp == 1 && !(opts->flags & RCMVS_FLAG_LOCKSTEP_PASSES))
-        rc = assemble_tiled(ctx,
-                            ctx->count_work || (opts->flags & RCMVS_FLAG_NO_SKIP_DUPLICATES) ? TILED_STREAM
-                                                                                             : TILED_STAGED,
-                            b);
+    if (rc == RCMVS_OK && tpp == 1 && !(opts->flags & RCMVS_FLAG_LOCKSTEP_PASSES)) {
+        b.tiled = ctx->count_work || (opts->flags & RCMVS_FLAG_NO_SKIP_DUPLICATES) ? TILED_STREAM : TILED_STAGED;
+        rc = assemble_tiled(ctx, b.tiled, b, b.sstart, b.sgeom);
+        // the staged sweep has one tiling; chosen tile shapes run the table sweep
+        if (rc == RCMVS_OK && b.tiled == TILED_STAGED && opts->tile_w == 0 && opts->tile_h == 0 &&
+            !(opts->flags & (RCMVS_FLAG_AUTOTUNE | RCMVS_FLAG_PERSISTENT)))
+            rc = assemble_tiled(ctx, TILED_INIT, b, b.istart, b.igeom);
+    }
     return rc;
 }
 
@@ -361,6 +364,21 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
         sgeom.scratch_blocks = std::min(tiled_grid(sgeom), sgeom.tiles);
         SCK(sc->arena.get(kSlotStreamScratch, tiled_scratch_bytes(b.tiled, sgeom.scratch_blocks), &pscr));
         sgeom.scratch = (unsigned char*)pscr;
+    }
+    // the default plane sweep, where the passes are staged too
+    const bool staged_init = s.init == Schedule::TABLE && !b.istart.empty() && !s.d_work && s.skip_duplicates;
+    LaunchGeom igeom = b.igeom;
+    void* pis = nullptr;
+    if (staged_init) {
+        igeom.scratch_blocks = std::min(tiled_grid(igeom), igeom.tiles);
+        SCK(sc->arena.get(kSlotInitStart, sizeof(int32_t) * (n_jobs + 1), &pis));
+        SCK(cudaMemcpyAsync(pis, b.istart.data(), sizeof(int32_t) * (n_jobs + 1), cudaMemcpyHostToDevice, st));
+        // one scratch: the init's launch ends before the first pass begins
+        SCK(sc->arena.get(kSlotStreamScratch,
+                          std::max(tiled_scratch_bytes(TILED_INIT, igeom.scratch_blocks),
+                                   tiled_scratch_bytes(b.tiled, sgeom.scratch_blocks)),
+                          &pscr));
+        igeom.scratch = sgeom.scratch = (unsigned char*)pscr;
     }
     const DevJob* dj = (const DevJob*)pj;
     const int32_t* dst = (const int32_t*)ps;
@@ -394,7 +412,11 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
         if (s.init == Schedule::LEARNED)
             e = launch_init_learned(dj, dst, n_jobs, g, s.nh, sc->census, sc->rays, A, s.pred, s.pred_off,
                                     s.logit_thr, s.n_local, s.span, s.sweep_seeded, s.d_learned, st);
-        else
+        else if (staged_init) {
+            LaunchGeom gi = igeom;
+            gi.queue = queue;
+            e = launch_init_staged(dj, (const int32_t*)pis, n_jobs, gi, s.nh, sc->census, sc->rays, A, st);
+        } else
             e = launch_init(dj, dst, n_jobs, g, s.nh, sc->census, sc->rays, A, s.d_work, st,
                             s.init == Schedule::ONE_CANDIDATE ? 1 : (s.init == Schedule::TABLE ? 2 : 0));
         hk.end(s.init == Schedule::LEARNED ? "learned_init" : "stereo_init");
@@ -430,6 +452,9 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
     append(key, b.geom.smem);
     append(key, b.geom.tpp);
     append(key, b.tiled);
+    append(key, staged_init);
+    append(key, b.istart.data(), sizeof(int32_t) * b.istart.size());
+    append(key, igeom.scratch_blocks);
     append(key, b.geom.radial);
     append(key, b.sstart.data(), sizeof(int32_t) * b.sstart.size());
     append(key, sgeom.scratch_blocks);
@@ -441,7 +466,7 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
     append(key, s.n_local);
     append(key, s.span);
     append(key, s.sweep_seeded);
-    const void* ptrs[] = {pj, ps, pss, pscr, pq, s.d_work, s.pred, s.pred_off, s.d_learned, sc->census, sc->rays,
+    const void* ptrs[] = {pj, ps, pss, pis, pscr, pq, s.d_work, s.pred, s.pred_off, s.d_learned, sc->census, sc->rays,
                           sc->plane_a, sc->plane_b, sc->pcost_a, sc->pcost_b, A0.d, B0.d, A0.flag, B0.flag,
                           sc->depth, sc->cost, sc->normal};
     append(key, ptrs, sizeof(ptrs));

@@ -2,7 +2,8 @@
 //
 // Restates mvs/src/stereo.rs:
 //   plane_cost      stereo.rs:158-228   (device function plane_cost)
-//   init sweep      stereo.rs:247-269   (init_kernel)
+//   init sweep      stereo.rs:247-269   (init_staged_kernel by default;
+//                   init_kernel is the plain form)
 //   Jacobi passes   stereo.rs:271-371   (pass_staged_kernel by default, one
 //                   launch per pass; pass_kernel is the plain form)
 //   texture gate    stereo.rs:373-393   (gate_kernel)
@@ -320,6 +321,38 @@ __device__ __forceinline__ float rcp_approx(float x) {  // relative error at mos
     return r;
 }
 
+// Maxima over a halo tile's rays into box (zeroed before; the block
+// synchronises after): |ray.x|, |ray.y|, and the largest change of either
+// component between horizontal / vertical neighbours, as float bits.
+__device__ __forceinline__ void ray_maxima(const float2* ray, int cells, int stw, int* box) {
+    float bx = 0.f, by = 0.f, sh = 0.f, sv = 0.f;
+    for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+        const float2 r = ray[i];
+        bx = fmaxf(bx, fabsf(r.x));
+        by = fmaxf(by, fabsf(r.y));
+        if (i % stw != stw - 1) {
+            const float2 e = ray[i + 1];
+            sh = fmaxf(sh, fmaxf(fabsf(e.x - r.x), fabsf(e.y - r.y)));
+        }
+        if (i + stw < cells) {
+            const float2 e = ray[i + stw];
+            sv = fmaxf(sv, fmaxf(fabsf(e.x - r.x), fabsf(e.y - r.y)));
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        bx = fmaxf(bx, __shfl_xor_sync(0xffffffffu, bx, o));
+        by = fmaxf(by, __shfl_xor_sync(0xffffffffu, by, o));
+        sh = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, o));
+        sv = fmaxf(sv, __shfl_xor_sync(0xffffffffu, sv, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&box[0], __float_as_int(bx));
+        atomicMax(&box[1], __float_as_int(by));
+        atomicMax(&box[2], __float_as_int(sh));
+        atomicMax(&box[3], __float_as_int(sv));
+    }
+}
+
 // What of the bound a plane does not change, per source: with ax = f |xn|,
 // E_x = (d wx + N tx + ax (d wz + N tz)) / zs' + c ax + bx.
 struct ProjConst {
@@ -419,32 +452,59 @@ __device__ __forceinline__ bool make_proj(const SrcRegs& s, const ProjConst& c, 
     return d > 0.0f && amin > 0.0501f && n < 10.0f && zmin > 0.002f * n && ex < 0.25f && ey < 0.25f;
 }
 
-// Where (M r)_xy = xy, (M r)_z = z lands: inside the source, and then at
-// census index off - (sw + 1).  Returns the coordinates' fractions - 0.5
-// (past P.lu / P.lv the reference's chain must decide).
+// The coordinates - 0.5 (their nearest integer is the pixel) of the point with
+// (x, y) = xy and 1 / z = q: f xy q + ch, distorted if RADIAL.
 template <bool RADIAL>
-__device__ __forceinline__ f32x2 proj_pixel(const Proj& P, f32x2 xy, float z, bool& in, unsigned& off) {
-    constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23: x + MAGIC holds round(x) in its low mantissa bits
-    const float q = rcp_approx(z);
-    f32x2 uv;  // coordinates - 0.5: their nearest integer is the pixel
-    if (RADIAL) {
-        float xs, ys;
-        unpack2(xy, xs, ys);
-        const float xn = xs * q, yn = ys * q;
-        const float g = P.f * __fmaf_rn(P.k, __fmaf_rn(xn, xn, yn * yn), 1.0f);
-        uv = fma2(pack2(xn, yn), pack2(g, g), P.ch);
-    } else {
-        uv = fma2(xy, pack2(q, q), P.ch);
+__device__ __forceinline__ f32x2 proj_uv(f32x2 xy, float q, float f, float k, f32x2 ch) {
+    if (!RADIAL) {
+        const float g = f * q;
+        return fma2(xy, pack2(g, g), ch);
     }
+    float xs, ys;
+    unpack2(xy, xs, ys);
+    const float xn = xs * q, yn = ys * q;
+    const float g = f * __fmaf_rn(k, __fmaf_rn(xn, xn, yn * yn), 1.0f);
+    return fma2(pack2(xn, yn), pack2(g, g), ch);
+}
+
+// The pixel of coordinates uv + 0.5: inside the source or not, and then at
+// census index off - (sw + 1); du, dv: the fractions - 0.5 (past the limits
+// the reference's chain must decide).
+__device__ __forceinline__ void proj_floor(f32x2 uv, unsigned sw, unsigned sh, bool& in, unsigned& off, float& du,
+                                           float& dv) {
+    constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23: x + MAGIC holds round(x) in its low mantissa bits
     const f32x2 fl = add2(uv, pack2(MAGIC, MAGIC));
     float fu, fv;
     unpack2(fl, fu, fv);
     // floor + 1, at least 1: inside when floor is in [-1, n) (trunc(-1 < x < 0) = 0)
     const unsigned tu = max((unsigned)__float_as_int(fu) - 0x4B3FFFFFu, 1u);
     const unsigned tv = max((unsigned)__float_as_int(fv) - 0x4B3FFFFFu, 1u);
-    in = tu <= P.sw && tv <= P.sh;
-    off = in ? tv * P.sw + tu : P.sw + 1u;
-    return fma2(add2(fl, pack2(-MAGIC, -MAGIC)), pack2(-1.0f, -1.0f), uv);
+    in = tu <= sw && tv <= sh;
+    off = in ? tv * sw + tu : sw + 1u;
+    unpack2(fma2(add2(fl, pack2(-MAGIC, -MAGIC)), pack2(-1.0f, -1.0f), uv), du, dv);
+}
+
+// The bound for fronto-parallel planes (n = (0, 0, 1), N = 1) at depth d, over
+// a whole tile: rc its middle ray, rb.step the largest distance of a ray from
+// it.  The coordinate is f (d R r + t)_xy / (d R r + t)_z in fused steps, one
+// rounding of f / z more than make_proj's.  Negative: no bound.
+template <bool RADIAL>
+__device__ __forceinline__ float2 fronto_limits(const SrcRegs& s, const ProjConst& c, float d, float2 rc,
+                                                const RayBox& rb) {
+    const float rx = s.rs0 * rc.x + s.rs1 * rc.y + s.rs2, ry = s.rs3 * rc.x + s.rs4 * rc.y + s.rs5;
+    const float rz = s.rs6 * rc.x + s.rs7 * rc.y + s.rs8;
+    const float zmin = d * (rz - (fabsf(s.rs6) + fabsf(s.rs7)) * rb.step) + s.ts2;
+    const float iz = rcp_approx(zmin);
+    const float ax = (fabsf(d * rx + s.ts0) + d * (fabsf(s.rs0) + fabsf(s.rs1)) * rb.step) * s.f * iz;
+    const float ay = (fabsf(d * ry + s.ts1) + d * (fabsf(s.rs3) + fabsf(s.rs4)) * rb.step) * s.f * iz;
+    const float ez = (d * c.wz + c.tz) * iz + (RADIAL ? 1.4e-6f : 8.6e-7f);  // 21 u, 13 u with slack
+    float ex = ax * ez + (d * c.wx + c.tx) * iz + c.bx, ey = ay * ez + (d * c.wy + c.ty) * iz + c.by;
+    if (RADIAL) {
+        const float xn = ax / s.f, yn = ay / s.f;
+        ex = ey = fmaxf(ex, ey) * (1.0f + 3.6f * fabsf(s.k) * (xn * xn + yn * yn));
+    }
+    const bool ok = d > 0.0f && zmin > 0.002f && ex < 0.25f && ey < 0.25f;
+    return ok ? make_float2(0.5f - ex, 0.5f - ey) : make_float2(-1.0f, -1.0f);
 }
 
 // The reference's chain for one term (stereo.rs:185-213): census index or -1.
@@ -1146,12 +1206,13 @@ __global__ void __launch_bounds__(STREAM_THREADS, RCMVS_STREAM_MINB)
 #define RCMVS_STAGED_THREADS 128
 #define RCMVS_STAGED_MINB 8
 #endif
-template <int TW_, int TH_, int THREADS_, int MINB_>
+template <int TW_, int TH_, int THREADS_, int MINB_, int RES_>
 struct StagedCfg {
     static constexpr int TW = TW_, TH = TH_, THREADS = THREADS_, MINB = MINB_;
     static constexpr int PX = TW * TH, STW = TW + 2 * HALO, CELLS = STW * (TH + 2 * HALO);
-    static constexpr int CAP = 7 * PX;  // list entries: at most 4 neighbours and 3 perturbations a pixel
-    static_assert(PX <= 1024 && THREADS % 32 == 0, "staged tile");
+    static constexpr int RES = RES_;      // candidates a pixel can have at a time
+    static constexpr int CAP = RES * PX;  // list entries
+    static_assert(PX <= 1024 && THREADS % 32 == 0 && RES <= 32, "staged tile");
 };
 
 template <class C>
@@ -1163,12 +1224,158 @@ struct StagedSmem {
     ProjConst pc[RCMVS_MAX_SOURCES];
     f32x2 colx[C::STW + 1];  // without distortion: the halo columns' ray.x, twice (ray.y depends on the row alone)
     float tab[64];
-    float pcost[C::PX];
+    float pcost[C::PX];      // the cost whose limits the evaluations run under
     uint32_t done[C::PX];    // completed candidates, one bit each
     uint16_t list[C::CAP];   // tile pixel | candidate << 10
     int box[4];              // float bits (non-negative): RayBox's maxima, horizontal and vertical ray steps
     int n, next, tile;
 };
+
+// A tile of job J for the staged kernels: support views (field-major), halo
+// tile, ray box and each source's part of the bound; an empty list.  The
+// block synchronises before it reads sm.pc and sm.colx.
+template <class C, bool RADIAL>
+__device__ __forceinline__ RayBox stage_tile(StagedSmem<C>& sm, const DevJob* J, int x0, int y0,
+                                             const uint64_t* __restrict__ census, const float2* __restrict__ rays) {
+    const int tid = threadIdx.x, w = J->w, h = J->h, nsrc = J->nsrc;
+    const size_t base = (size_t)J->off;
+    for (int i = tid; i < nsrc * SF_N; i += C::THREADS) {
+        const int s = i / SF_N, f = i - s * SF_N;
+        sm.sf[f * RCMVS_MAX_SOURCES + s] = src_field(J->src[s], f);
+    }
+    for (int s = tid; s < nsrc; s += C::THREADS) sm.scp[s] = census + J->src[s].off;
+    for (int i = tid; i < C::CELLS; i += C::THREADS) {
+        const int sx = i % C::STW, sy = i / C::STW;
+        const int gx = min(max(x0 - HALO + sx, 0), w - 1);
+        const int gy = min(max(y0 - HALO + sy, 0), h - 1);
+        const size_t g = base + (size_t)gy * w + gx;
+        sm.ray[i] = __ldg(rays + g);
+        sm.cen[i] = __ldg(census + g);
+    }
+    if (tid < 4) sm.box[tid] = 0;
+    if (tid == 0) sm.n = 0;
+    __syncthreads();
+    ray_maxima(sm.ray, C::CELLS, C::STW, sm.box);
+    __syncthreads();
+    const RayBox rb{__int_as_float(sm.box[0]), __int_as_float(sm.box[1]),
+                    2.001f * (__int_as_float(sm.box[2]) + __int_as_float(sm.box[3]))};
+    for (int s = tid; s < nsrc; s += C::THREADS) sm.pc[s] = proj_const<RADIAL>(J->src[s], rb);
+    if (!RADIAL)
+        for (int c = tid; c < C::STW; c += C::THREADS) sm.colx[c] = pack2(sm.ray[c].x, sm.ray[c].x);
+    return rb;
+}
+
+// The list's candidates through sources first .. nsrc - 1, one source per
+// stage (see above): completed ones in res (cost, largest mean) and sm.done.
+// lsum: (sum, largest mean) of the list's entries, read where first > 0 and
+// between stages.  plane(p, q, lx, ly): candidate q of tile pixel p.
+template <class C, bool RADIAL, class Plane>
+__device__ __forceinline__ void run_stages(StagedSmem<C>& sm, int first, int nsrc, float total, const RayBox& rb,
+                                           float2* __restrict__ lsum, float2* __restrict__ res, Plane plane) {
+    constexpr int stw = C::STW;
+    const int tid = threadIdx.x;
+    for (int si = first; si < nsrc; ++si) {
+        __syncthreads();  // the list, the sums and (first stage) the staging are complete
+        const int n = sm.n;
+        if (n == 0) break;
+        if (tid == 0) sm.next = 0;
+        const uint64_t* __restrict__ sc = sm.scp[si];
+        for (int b = 0; b < n; b += C::THREADS) {
+            const bool have = b + tid < n;
+            uint32_t e = 0;
+            float2 sv = make_float2(0.f, 0.f);
+            if (have) {
+                e = sm.list[b + tid];
+                if (si > 0) sv = lsum[b + tid];
+            }
+            __syncthreads();  // read before the survivors are appended over them
+            bool alive = have;
+            const int p = e & 1023, q = e >> 10;
+            const int lx = p % C::TW, ly = p / C::TW;
+            const int cell = ly * stw + lx;
+            float sum = sv.x, top = sv.y;
+            if (have) {
+                const float4 pl = plane(p, q, lx, ly);
+                const float best_c = sm.pcost[p];
+                const float thr = (best_c + 0.02f) + 0.12f;
+                const float rej = reject_bound(best_c, total);
+                Proj P;
+                const bool bound = make_proj<RADIAL>(load_src_fields(sm.sf, sc, si), sm.pc[si], pl.x, pl.y, pl.z,
+                                                     pl.w, sm.ray[cell + HALO * stw + HALO], rb, P);
+                if (!bound) P.lu = -1.0f;
+                const uint64_t* __restrict__ sc1 = sc - (P.sw + 1u);
+#pragma unroll 1
+                for (int dy = 0; dy < 5; ++dy) {
+                    const int row = cell + dy * stw;
+                    f32x2 by = 0;
+                    float bz = 0.0f;
+                    if (!RADIAL) {
+                        const float ry = sm.ray[row].y;
+                        by = fma2(P.m1, pack2(ry, ry), P.m2);
+                        bz = __fmaf_rn(P.z1, ry, P.z2);
+                    }
+                    unsigned near = 0;
+                    int hc[5];
+#pragma unroll
+                    for (int dx = 0; dx < 5; ++dx) {
+                        f32x2 xy;
+                        float z;
+                        if (RADIAL) {
+                            const float2 r = sm.ray[row + dx];
+                            xy = fma2(P.m0, pack2(r.x, r.x), fma2(P.m1, pack2(r.y, r.y), P.m2));
+                            z = __fmaf_rn(P.z0, r.x, __fmaf_rn(P.z1, r.y, P.z2));
+                        } else {
+                            const f32x2 rr = sm.colx[lx + dx];
+                            float rx, rx2;
+                            unpack2(rr, rx, rx2);
+                            xy = fma2(P.m0, rr, by);
+                            z = __fmaf_rn(P.z0, rx, bz);
+                        }
+                        bool in;
+                        unsigned off;
+                        float du, dv;
+                        const float q1 = rcp_approx(z);
+                        // the rows of a pinhole M hold f already
+                        const f32x2 uv = RADIAL ? proj_uv<true>(xy, q1, P.f, P.k, P.ch) : fma2(xy, pack2(q1, q1), P.ch);
+                        proj_floor(uv, P.sw, P.sh, in, off, du, dv);
+                        if (!(fabsf(du) <= P.lu && fabsf(dv) <= P.lv)) near |= 1u << dx;
+                        const int hv = __popcll(sm.cen[row + dx] ^ __ldg(sc1 + off));
+                        hc[dx] = in ? hv : 48;
+                    }
+                    while (near) {
+                        const int c = __ffs(near) - 1;
+                        near &= near - 1;
+                        const int v = exact_index(load_src_fields(sm.sf, sc, si), sm.ray[row + c], pl.x, pl.y,
+                                                  pl.z, pl.w);
+                        const int hv = v < 0 ? 48 : __popcll(sm.cen[row + c] ^ __ldg(sc + max(v, 0)));
+#pragma unroll
+                        for (int dx = 0; dx < 5; ++dx) hc[dx] = c == dx ? hv : hc[dx];
+                    }
+#pragma unroll
+                    for (int dx = 0; dx < 5; ++dx) sum += sm.tab[hc[dx]];
+                    const float den = abort_den(dy, si, nsrc, true);
+                    if (mean_above(sum, den, thr) || sum >= rej) {
+                        alive = false;
+                        break;
+                    }
+                    top = fmaxf(top, sum * rcp_approx(den));
+                }
+            }
+            if (alive) {
+                if (si == nsrc - 1) {
+                    res[p * C::RES + q] = make_float2(sum / total, top);
+                    atomicOr(&sm.done[p], 1u << q);
+                } else {
+                    const int at = atomicAdd(&sm.next, 1);
+                    sm.list[at] = (uint16_t)e;
+                    lsum[at] = make_float2(sum, top);
+                }
+            }
+        }
+        __syncthreads();
+        if (tid == 0) sm.n = sm.next;
+    }
+}
 
 // Bytes of a resident block's scratch: the random candidates' planes, the
 // list's (sum, largest mean), the completed candidates' (cost, largest mean).
@@ -1221,7 +1428,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     float2* const lsum = reinterpret_cast<float2*>(rnd + C::PX * 3);
     float2* const res = lsum + C::CAP;
     const uint8_t* __restrict__ pflag = prev.flag;
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     constexpr int stw = C::STW;
     for (int i = tid; i < 49; i += C::THREADS) sm.tab[i] = (float)i / 48.0f;
     for (int it = 0;; ++it) {
@@ -1237,58 +1444,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         const size_t base = (size_t)J->off;
         const size_t tb = base + (size_t)y0 * w + x0;  // the tile's first pixel
 
-        // ---- staging: support views (field-major), halo tile, ray box
-        for (int i = tid; i < nsrc * SF_N; i += C::THREADS) {
-            const int s = i / SF_N, f = i - s * SF_N;
-            sm.sf[f * RCMVS_MAX_SOURCES + s] = src_field(J->src[s], f);
-        }
-        for (int s = tid; s < nsrc; s += C::THREADS) sm.scp[s] = census + J->src[s].off;
-        for (int i = tid; i < C::CELLS; i += C::THREADS) {
-            const int sx = i % stw, sy = i / stw;
-            const int gx = min(max(x0 - HALO + sx, 0), w - 1);
-            const int gy = min(max(y0 - HALO + sy, 0), h - 1);
-            const size_t g = base + (size_t)gy * w + gx;
-            sm.ray[i] = __ldg(rays + g);
-            sm.cen[i] = __ldg(census + g);
-        }
-        if (tid < 4) sm.box[tid] = 0;
-        if (tid == 0) sm.n = 0;
-        __syncthreads();
-        {
-            float bx = 0.f, by = 0.f, sh = 0.f, sv = 0.f;
-            for (int i = tid; i < C::CELLS; i += C::THREADS) {
-                const float2 r = sm.ray[i];
-                bx = fmaxf(bx, fabsf(r.x));
-                by = fmaxf(by, fabsf(r.y));
-                if (i % stw != stw - 1) {
-                    const float2 e = sm.ray[i + 1];
-                    sh = fmaxf(sh, fmaxf(fabsf(e.x - r.x), fabsf(e.y - r.y)));
-                }
-                if (i + stw < C::CELLS) {
-                    const float2 e = sm.ray[i + stw];
-                    sv = fmaxf(sv, fmaxf(fabsf(e.x - r.x), fabsf(e.y - r.y)));
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                bx = fmaxf(bx, __shfl_xor_sync(0xffffffffu, bx, o));
-                by = fmaxf(by, __shfl_xor_sync(0xffffffffu, by, o));
-                sh = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, o));
-                sv = fmaxf(sv, __shfl_xor_sync(0xffffffffu, sv, o));
-            }
-            if (lane == 0) {
-                atomicMax(&sm.box[0], __float_as_int(bx));
-                atomicMax(&sm.box[1], __float_as_int(by));
-                atomicMax(&sm.box[2], __float_as_int(sh));
-                atomicMax(&sm.box[3], __float_as_int(sv));
-            }
-        }
-        __syncthreads();
-        const RayBox rb{__int_as_float(sm.box[0]), __int_as_float(sm.box[1]),
-                        2.001f * (__int_as_float(sm.box[2]) + __int_as_float(sm.box[3]))};
-        for (int s = tid; s < nsrc; s += C::THREADS) sm.pc[s] = proj_const<RADIAL>(J->src[s], rb);
-        if (!RADIAL)
-            for (int c = tid; c < stw; c += C::THREADS) sm.colx[c] = pack2(sm.ray[c].x, sm.ray[c].x);
-
+        const RayBox rb = stage_tile<C, RADIAL>(sm, J, x0, y0, census, rays);
         const float total = 5.0f * 5.0f * (float)nsrc;
         const float inv_min = J->inv_min, inv_max = J->inv_max;
         const float zlo = J->zmin * 0.5f, zhi = J->zmax * 2.0f;
@@ -1362,104 +1518,9 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         }
 
         // ---- 2. one source after the other
-        for (int si = 0; si < nsrc; ++si) {
-            __syncthreads();  // the list, the sums and (si = 0) the staging are complete
-            const int n = sm.n;
-            if (n == 0) break;
-            if (tid == 0) sm.next = 0;
-            const uint64_t* __restrict__ sc = sm.scp[si];
-            for (int b = 0; b < n; b += C::THREADS) {
-                const bool have = b + tid < n;
-                uint32_t e = 0;
-                float2 sv = make_float2(0.f, 0.f);
-                if (have) {
-                    e = sm.list[b + tid];
-                    if (si > 0) sv = lsum[b + tid];
-                }
-                __syncthreads();  // read before the survivors are appended over them
-                bool alive = have;
-                const int p = e & 1023, q = e >> 10;
-                const int lx = p % C::TW, ly = p / C::TW;
-                const int cell = ly * stw + lx;
-                float sum = sv.x, top = sv.y;
-                if (have) {
-                    const float4 pl = staged_plane(sm, prev.nz, tb, w, lx, ly, q, rnd, p);
-                    const float best_c = sm.pcost[p];
-                    const float thr = (best_c + 0.02f) + 0.12f;
-                    const float rej = reject_bound(best_c, total);
-                    Proj P;
-                    const bool bound = make_proj<RADIAL>(load_src_fields(sm.sf, sc, si), sm.pc[si], pl.x, pl.y, pl.z,
-                                                         pl.w, sm.ray[cell + HALO * stw + HALO], rb, P);
-                    if (!bound) P.lu = -1.0f;
-                    const uint64_t* __restrict__ sc1 = sc - (P.sw + 1u);
-#pragma unroll 1
-                    for (int dy = 0; dy < 5; ++dy) {
-                        const int row = cell + dy * stw;
-                        f32x2 by = 0;
-                        float bz = 0.0f;
-                        if (!RADIAL) {
-                            const float ry = sm.ray[row].y;
-                            by = fma2(P.m1, pack2(ry, ry), P.m2);
-                            bz = __fmaf_rn(P.z1, ry, P.z2);
-                        }
-                        unsigned near = 0;
-                        int hc[5];
-#pragma unroll
-                        for (int dx = 0; dx < 5; ++dx) {
-                            f32x2 xy;
-                            float z;
-                            if (RADIAL) {
-                                const float2 r = sm.ray[row + dx];
-                                xy = fma2(P.m0, pack2(r.x, r.x), fma2(P.m1, pack2(r.y, r.y), P.m2));
-                                z = __fmaf_rn(P.z0, r.x, __fmaf_rn(P.z1, r.y, P.z2));
-                            } else {
-                                const f32x2 rr = sm.colx[lx + dx];
-                                float rx, rx2;
-                                unpack2(rr, rx, rx2);
-                                xy = fma2(P.m0, rr, by);
-                                z = __fmaf_rn(P.z0, rx, bz);
-                            }
-                            bool in;
-                            unsigned off;
-                            float du, dv;
-                            unpack2(proj_pixel<RADIAL>(P, xy, z, in, off), du, dv);
-                            if (!(fabsf(du) <= P.lu && fabsf(dv) <= P.lv)) near |= 1u << dx;
-                            const int hv = __popcll(sm.cen[row + dx] ^ __ldg(sc1 + off));
-                            hc[dx] = in ? hv : 48;
-                        }
-                        while (near) {
-                            const int c = __ffs(near) - 1;
-                            near &= near - 1;
-                            const int v = exact_index(load_src_fields(sm.sf, sc, si), sm.ray[row + c], pl.x, pl.y,
-                                                      pl.z, pl.w);
-                            const int hv = v < 0 ? 48 : __popcll(sm.cen[row + c] ^ __ldg(sc + max(v, 0)));
-#pragma unroll
-                            for (int dx = 0; dx < 5; ++dx) hc[dx] = c == dx ? hv : hc[dx];
-                        }
-#pragma unroll
-                        for (int dx = 0; dx < 5; ++dx) sum += sm.tab[hc[dx]];
-                        const float den = abort_den(dy, si, nsrc, true);
-                        if (mean_above(sum, den, thr) || sum >= rej) {
-                            alive = false;
-                            break;
-                        }
-                        top = fmaxf(top, sum * rcp_approx(den));
-                    }
-                }
-                if (alive) {
-                    if (si == nsrc - 1) {
-                        res[p * 7 + q] = make_float2(sum / total, top);
-                        atomicOr(&sm.done[p], 1u << q);
-                    } else {
-                        const int at = atomicAdd(&sm.next, 1);
-                        sm.list[at] = (uint16_t)e;
-                        lsum[at] = make_float2(sum, top);
-                    }
-                }
-            }
-            __syncthreads();
-            if (tid == 0) sm.n = sm.next;
-        }
+        run_stages<C, RADIAL>(sm, 0, nsrc, total, rb, lsum, res, [&](int p, int q, int lx, int ly) {
+            return staged_plane(sm, prev.nz, tb, w, lx, ly, q, rnd, p);
+        });
         __syncthreads();
 
         // ---- 3. the completed candidates in order (stereo.rs:355-367)
@@ -1473,7 +1534,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             int best = -1;
             for (; m; m &= m - 1) {
                 const int q = __ffs(m) - 1;
-                const float2 r = res[p * 7 + q];
+                const float2 r = res[p * C::RES + q];
                 if (!(r.x < best_c)) continue;
                 if (best >= 0) {
                     const float thr = (best_c + 0.02f) + 0.12f;
@@ -1503,7 +1564,240 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     }
 }
 
-using StagedDefault = StagedCfg<RCMVS_STAGED_TW, RCMVS_STAGED_TH, RCMVS_STAGED_THREADS, RCMVS_STAGED_MINB>;
+using StagedDefault = StagedCfg<RCMVS_STAGED_TW, RCMVS_STAGED_TH, RCMVS_STAGED_THREADS, RCMVS_STAGED_MINB, 7>;
+__device__ __forceinline__ float hyp_depth(float inv_min, float inv_max, int hi, int nh) {
+    const float inv = inv_min + (inv_max - inv_min) * (float)hi / (float)(nh - 1);  // stereo.rs:259-260
+    return 1.0f / inv;
+}
+
+// ---------------------------------------------------------------- staged init
+// The default plane sweep.  Hypothesis 0, which nothing prunes, has the window
+// counts of every source in tables like init_table_kernel's.  The others go in
+// batches of 1, 2, 4, 8 and then 16 (a batch runs under the best cost at its
+// start): source 0's window counts of a tile
+// and its halo are computed once per hypothesis (on a fronto-parallel plane a
+// cell's count does not depend on the pixel whose window holds it), four
+// hypotheses between barriers, and every pixel adds its 25; what survives
+// source 0 -- few percent -- goes through the other sources as list entries
+// (run_stages) instead of a table of the whole tile for a few pixels.  The
+// batch runs under the pixel's best cost at its start and is resolved in the
+// hypotheses' order like the staged passes: every kept hypothesis and cost
+// is the reference's (stereo.rs:247-269).  Measured: 16 views 960x720, K = 8, 64
+// hypotheses: table sweep 19.9 ms, 15.4 here; 12 mixed views, K = 3, 48
+// hypotheses: 11.0, 8.7.  Bound by instruction issue and barriers.  Tiles of
+// 32x8 in blocks of 256 threads: 16x8 16.0 / 10.0, 16x16 16.2 / 9.0, 8x8 22.2 /
+// 15.8; hypothesis 0 through list entries like the others: 18.4 / 9.7.
+constexpr int INIT_BATCH = 16, INIT_TABLES = 4;
+#ifndef RCMVS_SINIT_TW
+#define RCMVS_SINIT_TW 32
+#define RCMVS_SINIT_TH 8
+#define RCMVS_SINIT_MINB 4
+#endif
+using StagedInit = StagedCfg<RCMVS_SINIT_TW, RCMVS_SINIT_TH, RCMVS_SINIT_TW * RCMVS_SINIT_TH, RCMVS_SINIT_MINB, INIT_BATCH>;
+
+template <class C>
+struct InitSmem : StagedSmem<C> {
+    float table[INIT_TABLES][C::CELLS];  // h / 48 of source 0's cells
+    float2 lim[RCMVS_MAX_SOURCES];       // fronto_limits: of source 0, a batch's hypotheses; of hypothesis 0, the sources
+    float depth[INIT_BATCH];
+};
+
+// One cell's h / 48 in source s at depth d: a, az = R r of the cell's ray.
+template <class C, bool RADIAL>
+__device__ __forceinline__ float fronto_cell(const InitSmem<C>& sm, const SrcRegs& s, float2 r, uint64_t cen, f32x2 a,
+                                             float az, float d, float2 lim) {
+    bool in;
+    unsigned off;
+    float du, dv;
+    const f32x2 xy = fma2(pack2(d, d), a, pack2(s.ts0, s.ts1));
+    proj_floor(proj_uv<RADIAL>(xy, rcp_approx(__fmaf_rn(d, az, s.ts2)), s.f, s.k, pack2(s.cx - 0.5f, s.cy - 0.5f)),
+               (unsigned)s.sw, (unsigned)s.sh, in, off, du, dv);
+    if (!(fabsf(du) <= lim.x && fabsf(dv) <= lim.y)) {
+        const int v = exact_index(s, r, 0.0f, 0.0f, 1.0f, d);
+        in = v >= 0;
+        off = (unsigned)max(v, 0) + (unsigned)s.sw + 1u;
+    }
+    const int hc = __popcll(cen ^ __ldg(s.sc - (s.sw + 1) + off));
+    return sm.tab[in ? hc : 48];
+}
+
+__device__ __forceinline__ f32x2 ray_xy(const SrcRegs& s, float2 r) {
+    return fma2(pack2(s.rs0, s.rs3), pack2(r.x, r.x), fma2(pack2(s.rs1, s.rs4), pack2(r.y, r.y), pack2(s.rs2, s.rs5)));
+}
+__device__ __forceinline__ float ray_z(const SrcRegs& s, float2 r) {
+    return __fmaf_rn(s.rs6, r.x, __fmaf_rn(s.rs7, r.y, s.rs8));
+}
+
+template <class C>
+__host__ __device__ constexpr size_t init_block_bytes() {
+    return C::CAP * 2 * sizeof(float2);
+}
+
+template <class C, bool RADIAL>
+__global__ void __launch_bounds__(C::THREADS, C::MINB)
+    init_staged_kernel(const DevJob* __restrict__ jobs, const int32_t* __restrict__ stile_start, int n_jobs, int tiles,
+                       unsigned int* queue, int nh, const uint64_t* __restrict__ census,
+                       const float2* __restrict__ rays, PlaneBuf out, unsigned char* __restrict__ scratch) {
+    static_assert(C::PX == C::THREADS, "one thread per pixel");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    InitSmem<C>& sm = *reinterpret_cast<InitSmem<C>*>(smem_raw);
+    float2* const lsum = reinterpret_cast<float2*>(scratch + (size_t)blockIdx.x * init_block_bytes<C>());
+    float2* const res = lsum + C::CAP;
+    const int tid = threadIdx.x;
+    constexpr int stw = C::STW, PER = (C::CELLS + C::THREADS - 1) / C::THREADS;
+    for (int i = tid; i < 49; i += C::THREADS) sm.tab[i] = (float)i / 48.0f;
+    for (int it = 0;; ++it) {
+        const int tile = next_tile(queue, tiles, it, &sm.tile);
+        if (tile < 0) break;
+        const int j = find_item(stile_start, n_jobs, tile);
+        const DevJob* J = jobs + j;
+        const int w = J->w, h = J->h, nsrc = J->nsrc;
+        const int t = tile - stile_start[j];
+        const int stx = (w + C::TW - 1) / C::TW;
+        const int x0 = (t % stx) * C::TW, y0 = (t / stx) * C::TH;
+        const RayBox rb = stage_tile<C, RADIAL>(sm, J, x0, y0, census, rays);
+        const float total = 5.0f * 5.0f * (float)nsrc;
+        const float inv_min = J->inv_min, inv_max = J->inv_max;
+        const int lx = tid % C::TW, ly = tid / C::TW, cell = ly * stw + lx;
+        const bool inside = x0 + lx < w && y0 + ly < h;
+        // a ray differs from the middle one's by at most half the tile's steps
+        const RayBox rt{rb.rx, rb.ry, 1.001f * ((stw / 2 + 1) * __int_as_float(sm.box[2]) +
+                                               ((C::TH + 2 * HALO) / 2 + 1) * __int_as_float(sm.box[3]))};
+        const float2 rc = sm.ray[(C::TH / 2 + HALO) * stw + stw / 2];
+        float best_c = INFINITY, best_d = 0.f;
+        // hypothesis 0: nothing to prune yet, so every source's table
+        {
+            __syncthreads();  // the staging
+            const float d = hyp_depth(inv_min, inv_max, 0, nh);
+            for (int s = tid; s < nsrc; s += C::THREADS)
+                sm.lim[s] = fronto_limits<RADIAL>(load_src_fields(sm.sf, sm.scp[s], s), sm.pc[s], d, rc, rt);
+            float sum = 0.f;
+            for (int s0 = 0; s0 < nsrc; s0 += INIT_TABLES) {
+                __syncthreads();  // the limits; the previous tables are no longer read
+                const int nt = min(INIT_TABLES, nsrc - s0);
+                for (int c = tid; c < C::CELLS; c += C::THREADS) {
+                    const float2 r = sm.ray[c];
+                    const uint64_t cen = sm.cen[c];
+#pragma unroll 2
+                    for (int k = 0; k < nt; ++k) {
+                        const SrcRegs s = load_src_fields(sm.sf, sm.scp[s0 + k], s0 + k);
+                        sm.table[k][c] = fronto_cell<C, RADIAL>(sm, s, r, cen, ray_xy(s, r), ray_z(s, r), d, sm.lim[s0 + k]);
+                    }
+                }
+                __syncthreads();
+                for (int k = 0; k < nt; ++k)
+#pragma unroll
+                    for (int dy = 0; dy < 5; ++dy)
+#pragma unroll
+                        for (int dx = 0; dx < 5; ++dx) sum += sm.table[k][cell + dy * stw + dx];
+            }
+            if (nsrc > 0) {  // without sources the cost is 0 / 0, never kept
+                best_c = sum / total;
+                best_d = d;
+            }
+        }
+        sm.pcost[tid] = best_c;
+        int h0 = 1, batch = 1;
+        while (h0 < nh && nsrc > 0) {
+            const int nb = min(batch, nh - h0);
+            __syncthreads();  // the previous batch's list, limits and tables
+            if (tid < nb) {
+                const float d = hyp_depth(inv_min, inv_max, h0 + tid, nh);
+                sm.depth[tid] = d;
+                sm.lim[tid] = fronto_limits<RADIAL>(load_src_fields(sm.sf, sm.scp[0], 0), sm.pc[0], d, rc, rt);
+            }
+            if (tid == 0) sm.n = 0;
+            sm.done[tid] = 0;
+            const float thr = (best_c + 0.02f) + 0.12f;
+            const float rej = reject_bound(best_c, total);
+            for (int b0 = 0; b0 < nb; b0 += INIT_TABLES) {
+                __syncthreads();  // depths and limits; the previous tables are no longer read
+                const int nt = min(INIT_TABLES, nb - b0);
+                {
+                    const SrcRegs s = load_src_fields(sm.sf, sm.scp[0], 0);
+#pragma unroll
+                    for (int e = 0; e < PER; ++e) {
+                        const int c = tid + e * C::THREADS;
+                        if (c >= C::CELLS) break;
+                        const float2 r = sm.ray[c];
+                        const uint64_t cen = sm.cen[c];
+                        const f32x2 a = ray_xy(s, r);  // once for the hypotheses
+                        const float az = ray_z(s, r);
+#pragma unroll
+                        for (int k = 0; k < INIT_TABLES; ++k) {
+                            if (k >= nt) break;
+                            sm.table[k][c] = fronto_cell<C, RADIAL>(sm, s, r, cen, a, az, sm.depth[b0 + k], sm.lim[b0 + k]);
+                        }
+                    }
+                }
+                __syncthreads();
+                if (inside) {
+#pragma unroll 1
+                    for (int k = 0; k < nt; ++k) {
+                        const float* tb = sm.table[k] + cell;
+                        float sum = 0.f, top = 0.f;
+                        bool alive = true;
+#pragma unroll
+                        for (int dy = 0; dy < 5; ++dy) {
+#pragma unroll
+                            for (int dx = 0; dx < 5; ++dx) sum += tb[dy * stw + dx];
+                            // rows 1-3 share row 4's divisor unless source 0 is the last: its test covers theirs
+                            if (dy == 0 || dy == 4 || nsrc == 1) {
+                                const float den = abort_den(dy, 0, nsrc, true);
+                                if (mean_above(sum, den, thr) || sum >= rej) {
+                                    alive = false;
+                                    break;
+                                }
+                                top = fmaxf(top, sum * rcp_approx(den));
+                            }
+                        }
+                        if (alive) {
+                            const int q = b0 + k;
+                            if (nsrc == 1) {
+                                res[tid * C::RES + q] = make_float2(sum / total, top);
+                                sm.done[tid] |= 1u << q;
+                            } else {
+                                const int at = atomicAdd(&sm.n, 1);
+                                sm.list[at] = (uint16_t)(tid | q << 10);
+                                lsum[at] = make_float2(sum, top);
+                            }
+                        }
+                    }
+                }
+            }
+            run_stages<C, RADIAL>(sm, 1, nsrc, total, rb, lsum, res, [&](int, int q, int, int) {
+                return make_float4(0.0f, 0.0f, 1.0f, sm.depth[q]);
+            });
+            __syncthreads();
+            for (unsigned m = sm.done[tid]; m; m &= m - 1) {  // the completed hypotheses in order
+                const int q = __ffs(m) - 1;
+                const float2 r = res[tid * C::RES + q];
+                if (!(r.x < best_c)) continue;
+                const float d = sm.depth[q];
+                if (best_c < sm.pcost[tid]) {  // improved within the batch: the tighter limits
+                    const float lim = (best_c + 0.02f) + 0.12f;
+                    if (r.y > lim * 1.000002f) continue;
+                    if (!(r.y < lim * 0.999998f) &&
+                        !staged_completes<C>(sm, cell, nsrc, make_float4(0.0f, 0.0f, 1.0f, d), lim,
+                                             reject_bound(best_c, total)))
+                        continue;
+                }
+                best_c = r.x;
+                best_d = d;
+            }
+            sm.pcost[tid] = best_c;
+            h0 += nb;
+            batch = min(h0, INIT_BATCH);
+        }
+        if (inside) {
+            const size_t i = (size_t)J->off + (size_t)(y0 + ly) * w + x0 + lx;
+            out.nz[i] = make_float4(0.0f, 0.0f, 1.0f, best_d);
+            out.cost[i] = fminf(best_c, 1.0f);
+            if (out.d) out.d[i] = best_d;  // n = (0,0,1): d = z
+        }
+    }
+}
+
 
 // ---------------------------------------------------------------- split passes
 // The same pass with five lanes per pixel (threads per pixel = 5, an
@@ -1725,11 +2019,6 @@ __global__ void __maxnreg__(80)
 // every lane of the warp has finished the current one.  Each candidate's
 // rows, abort tests, hint and best-cost bookkeeping happen in the
 // reference's order, so results are bit-identical to the kernels above.
-
-__device__ __forceinline__ float hyp_depth(float inv_min, float inv_max, int hi, int nh) {
-    const float inv = inv_min + (inv_max - inv_min) * (float)hi / (float)(nh - 1);  // stereo.rs:259-260
-    return 1.0f / inv;
-}
 
 template <bool COUNT, int MINB, bool PERSIST>
 __global__ void __launch_bounds__(256, MINB)
@@ -2261,8 +2550,8 @@ size_t stereo_smem_bytes(TileShape ts) { return smem_bytes(ts.tw, ts.th); }
 int split_threads(int px) { return 32 * ((px + SPLIT_PX - 1) / SPLIT_PX); }
 
 int tiled_tiles(int kind, int w, int h) {
-    const int tw = kind == TILED_STREAM ? STREAM_TW : StagedDefault::TW;
-    const int th = kind == TILED_STREAM ? STREAM_TH : StagedDefault::TH;
+    const int tw = kind == TILED_STREAM ? STREAM_TW : (kind == TILED_INIT ? StagedInit::TW : StagedDefault::TW);
+    const int th = kind == TILED_STREAM ? STREAM_TH : (kind == TILED_INIT ? StagedInit::TH : StagedDefault::TH);
     return ((w + tw - 1) / tw) * ((h + th - 1) / th);
 }
 
@@ -2271,14 +2560,19 @@ LaunchGeom tiled_geom(int kind, int tiles) {
     if (kind == TILED_STAGED) {
         g.nthr = StagedDefault::THREADS;
         g.smem = sizeof(StagedSmem<StagedDefault>);
+    } else if (kind == TILED_INIT) {
+        g.nthr = StagedInit::THREADS;
+        g.smem = sizeof(InitSmem<StagedInit>);
     }
     g.tiled = kind;
     return g;
 }
 
 size_t tiled_scratch_bytes(int kind, int blocks) {
-    return (kind == TILED_STREAM ? sizeof(float4) * STREAM_PX * 3 : staged_block_bytes<StagedDefault>()) *
-           (size_t)blocks;
+    const size_t b = kind == TILED_STREAM ? sizeof(float4) * STREAM_PX * 3
+                                          : (kind == TILED_INIT ? init_block_bytes<StagedInit>()
+                                                                : staged_block_bytes<StagedDefault>());
+    return b * (size_t)blocks;
 }
 
 namespace {
@@ -2307,6 +2601,9 @@ int tiled_grid(const LaunchGeom& g) {
     int n = 0;
     if (g.tiled == TILED_STREAM)
         n = launch_grid(pass_stream_kernel<false, true>, q);
+    else if (g.tiled == TILED_INIT)
+        n = g.radial ? launch_grid(init_staged_kernel<StagedInit, true>, q)
+                     : launch_grid(init_staged_kernel<StagedInit, false>, q);
     else if (g.radial)
         n = launch_grid(pass_staged_kernel<StagedDefault, true>, q);
     else
@@ -2382,6 +2679,22 @@ cudaError_t launch_init(const DevJob* d_jobs, const int32_t* d_job_start, int n_
         else
             init_as<false, false>(variant, d_jobs, d_job_start, n_jobs, g, nh, census, rays, out, nullptr, st);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_init_staged(const DevJob* d_jobs, const int32_t* d_tile_start, int n_jobs, const LaunchGeom& g, int nh,
+                               const uint64_t* census, const float2* rays, PlaneBuf out, cudaStream_t st) {
+    if (g.tiles <= 0) return cudaSuccess;
+    if (g.tiled != TILED_INIT || !g.queue || !g.scratch || g.scratch_blocks <= 0) return cudaErrorInvalidValue;
+    auto run = [&](auto kernel) {
+        const int grid = std::min(launch_grid(kernel, g), g.scratch_blocks);
+        kernel<<<grid, g.nthr, g.smem, st>>>(d_jobs, d_tile_start, n_jobs, g.tiles, g.queue, nh, census, rays, out,
+                                             g.scratch);
+    };
+    if (g.radial)
+        run(init_staged_kernel<StagedInit, true>);
+    else
+        run(init_staged_kernel<StagedInit, false>);
     return cudaGetLastError();
 }
 
