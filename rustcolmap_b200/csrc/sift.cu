@@ -3,37 +3,45 @@
 // Restates sfm-lite/src/sift.rs (extract_sift, :435-555) for one image:
 //
 //   resize      load-time resize to max_dim (resize.cu; `.max(1)` sides)
-//   pyramid     per octave six Gaussian levels (separable f32 blur with
+//   pyramid     the reference's per-octave levels (sift.rs:51-134) have sigma
+//               1.6 (1 << int(l / 3)): levels 1, 2 repeat level 0's and 4, 5
+//               level 3's, and the blur between equal sigmas (0.01) has the taps
+//               0, 1, 0 exactly, so those levels equal the one before bit for
+//               bit, every DoG but number 2 is zero, and no extremum can lie in
+//               a zero DoG.  Level 0 (blurred once, from the grey image), level
+//               3 and DoG 2 are all that is made (identity_taps checks it)
+//   octave      one kernel per octave: level 3 (separable f32 blur with
 //               clamped edges, f64 kernel weights cast to f32, taps summed in
-//               order: sift.rs:51-93), five DoGs, 2x2 box downsample of
-//               level 3 for the next octave (sift.rs:95-134)
-//   extrema     one thread per (DoG level 1-3, pixel): the 24-neighbour test,
-//               the quadratic fit (nalgebra's cofactor 3x3 inverse, f64), the
-//               contrast and curvature tests (sift.rs:176-262); flags are
-//               compacted stably, so keypoints keep the reference's
-//               (octave, level, y, x) order; each octave's count stays on the
-//               device and the next octave starts without waiting for it
-//   orientation one warp per keypoint (in response order, see output):
-//               lanes evaluate 32 window samples at a time (atan2, exp in
-//               f64), each lane owns histogram bins and
-//               adds the samples that fall in them in window order, so every
-//               bin is the reference's sequential f64 sum; lane 0 smooths and
-//               picks up to four peaks (sift.rs:274-334)
-//   descriptor  one warp per (keypoint, peak): the same split over the window
-//               (bilinear gradients, rotation, trilinear weights; up to 8
-//               histogram entries per sample).  Lane L owns the 4 bins of cell
-//               column L / 8 and orientation L % 8, so it finds its share of a
-//               sample from the sample's (row, column, orientation) base by
-//               arithmetic; L2 -> clip 0.2 -> L2 in f32 (sift.rs:340-431)
-//   output      the reference sorts its descriptors by response (stable) and
+//               order) and DoG 2 of a tile in shared memory, the 2x2 box
+//               downsample that is the next octave's level 0, and per pixel
+//               the 24-neighbour test, the quadratic fit (nalgebra's cofactor
+//               3x3 inverse, f64), the contrast and curvature tests
+//               (sift.rs:176-262); keypoints are appended with their place in
+//               the reference's (octave, level, y, x) order
+//   selection   the reference sorts its descriptors by response (stable) and
 //               keeps the first max_features (sift.rs:543-544).  A descriptor's
 //               response is its keypoint's, so that order is the keypoints of
-//               all octaves sorted stably by response (CUB radix sort) with
-//               each keypoint's peaks in turn; orientations, pairs and
-//               descriptors are produced in that order until max_features
-//               valid ones exist -- the same output without the orientations
-//               and descriptors the cap would discard (about 2k of 27k
-//               keypoints at 1600x1200)
+//               all octaves by (response descending, place) with each
+//               keypoint's peaks in turn.  A histogram of the responses picks a
+//               threshold for the first max_features and some, and those are
+//               ranked by counting
+//   orientation one warp per keypoint in that order: lanes evaluate 32 window
+//               samples at a time (atan2, exp in f64), each lane owns histogram
+//               bins and adds the samples that fall in them in window order, so
+//               every bin is the reference's sequential f64 sum; the lanes
+//               smooth and pick up to four peaks (sift.rs:274-334)
+//   descriptor  one block per (keypoint, peak): the threads evaluate the
+//               window's samples (bilinear gradients, rotation, trilinear
+//               parameters) into shared memory; then thread t owns bin t (cell
+//               row = its warp) and adds its share of the samples that touch
+//               the row, in window order; L2 -> clip 0.2 -> L2 in f32 with the
+//               reference's serial sums (sift.rs:340-431)
+//
+// All of it is queued without waiting: the counts stay on the device until
+// one read at the end.  Where that read shows that the first keypoints did not
+// fill max_features (or max_features is past QUICK_CAP), the general path
+// continues: all keypoints sorted by CUB, orientations and descriptors in
+// chunks until max_features valid ones exist.
 //
 // The library builds with --fmad=false: every f32/f64 product and sum rounds
 // as written, so the pyramid, the DoGs and the extrema with their fitted
@@ -44,6 +52,7 @@
 // differ.
 #include <thrust/iterator/counting_iterator.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -59,7 +68,6 @@ namespace {
 
 constexpr int NSPO = 3;
 constexpr int NLEV = NSPO + 3;  // blurred levels per octave
-constexpr int NDOG = NSPO + 2;
 constexpr int DESC_LEN = 128;
 constexpr int MAX_TAPS = 32;
 constexpr double SIGMA0 = 1.6;
@@ -73,90 +81,104 @@ struct BlurTaps {
     float k[MAX_TAPS];
 };
 
-struct KpArrays {  // raw keypoints in the reference's (octave, level, y, x) order
+struct KpArrays {  // raw keypoints, in no order
     double* x;       // octave coordinates
     double* y;
     double* resp;
-    int32_t* level;
+    uint32_t* place; // in the reference's (octave, level, y, x) order
     int32_t* oct;
 };
 
+constexpr int KP_LEVEL = 2;  // the DoG level every keypoint lies in
 constexpr int MAX_OCT = 8;
-struct OctTable {  // per octave: gradients of DoG levels 1..NSPO, size, scale
-    const float* gx[MAX_OCT];
-    const float* gy[MAX_OCT];
+struct OctTable {  // per octave: level 0 (= levels 1 and 2, whose gradients the keypoints use), size, scale
+    const float* img[MAX_OCT];
     int w[MAX_OCT], h[MAX_OCT];
     double scale[MAX_OCT];
+};
+
+struct Counts {  // on the device
+    uint32_t kp;     // raw keypoints
+    uint32_t kept;   // of them past the selection's threshold
+    uint32_t pairs;  // (keypoint, peak) pairs of the first keypoints
+    uint32_t valid;  // valid descriptors among the first max_features pairs
 };
 
 __device__ __host__ __forceinline__ double level_sigma(int l) {
     return SIGMA0 * (double)(1 << (int)((double)l / (double)NSPO));
 }
 
-__global__ void to_float_kernel(const uint8_t* __restrict__ g, int64_t n, float* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (float)g[i] / 255.0f;
-}
+// ---- separable blur of one tile (sift.rs:65-90): BX x BY outputs whose
+// first is at (x0, y0), the source clamped at the image's edges.  Each thread
+// makes eight neighbouring sums from one run of loads.  in: [BY + 2R][BX + 2R]
+// (pitch IN_P), mid: [BY + 2R][BX] (pitch MID_P).
+constexpr int BX = 64, BY = 32, BLUR_THREADS = 256;
+template <int R>
+struct BlurSmem {
+    static constexpr int IN_W = BX + 2 * R, IN_H = BY + 2 * R, IN_P = IN_W | 1, MID_P = BX + 1;
+    float in[IN_H * IN_P];
+    float mid[IN_H * MID_P];
+};
 
-// sift.rs:65-77 (horizontal) and :79-90 (vertical)
-template <bool VERT>
-__global__ void blur_kernel(const float* __restrict__ src, float* __restrict__ dst, int w, int h,
-                            const __grid_constant__ BlurTaps taps) {
-    const int64_t n = (int64_t)w * h;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
-        float acc = 0.0f;
-        for (int ki = 0; ki <= 2 * taps.radius; ++ki) {
-            if (VERT) {
-                const int yy = min(max(y + ki - taps.radius, 0), h - 1);
-                acc = acc + taps.k[ki] * src[(int64_t)yy * w + x];
-            } else {
-                const int xx = min(max(x + ki - taps.radius, 0), w - 1);
-                acc = acc + taps.k[ki] * src[(int64_t)y * w + xx];
-            }
-        }
-        dst[i] = acc;
+template <int R, class Load, class Store>
+__device__ __forceinline__ void blur_tile(BlurSmem<R>& sm, int x0, int y0, int w, int h, const BlurTaps& taps, Load load,
+                                          Store store) {
+    using S = BlurSmem<R>;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < S::IN_H * S::IN_W; i += BLUR_THREADS) {
+        const int ix = i % S::IN_W, iy = i / S::IN_W;
+        const int gx = min(max(x0 - R + ix, 0), w - 1), gy = min(max(y0 - R + iy, 0), h - 1);
+        sm.in[iy * S::IN_P + ix] = load((int64_t)gy * w + gx);
     }
-}
-
-__global__ void dog_kernel(const float* __restrict__ lev, float* __restrict__ dog, int64_t npx) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += (int64_t)gridDim.x * blockDim.x)
+    __syncthreads();
+    // horizontal: lanes on different rows (odd pitches: no bank conflicts)
+    for (int i = tid; i < 64 * (BX / 8); i += BLUR_THREADS) {
+        const int row = i & 63, g = i >> 6;
+        if (row >= S::IN_H) continue;
+        const float* src = sm.in + row * S::IN_P + 8 * g;
+        float v[8 + 2 * R];
 #pragma unroll
-        for (int d = 0; d < NDOG; ++d) dog[d * npx + i] = lev[(d + 1) * npx + i] - lev[d * npx + i];
-}
-
-// sift.rs:95-110
-__global__ void downsample_kernel(const float* __restrict__ src, int w, int h, float* __restrict__ dst, int nw,
-                                  int nh) {
-    const int64_t n = (int64_t)nw * nh;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int y = (int)(i / nw), x = (int)(i - (int64_t)y * nw);
-        const int x0 = min(2 * x, w - 1), y0 = min(2 * y, h - 1);
-        const int x1 = min(x0 + 1, w - 1), y1 = min(y0 + 1, h - 1);
-        const float s = src[(int64_t)y0 * w + x0] + src[(int64_t)y0 * w + x1] + src[(int64_t)y1 * w + x0] +
-                        src[(int64_t)y1 * w + x1];
-        dst[i] = 0.25f * s;
-    }
-}
-
-// sift.rs:137-149, for levels 1..NSPO
-__global__ void grad_kernel(const float* __restrict__ lev, int w, int h, float* __restrict__ gx,
-                            float* __restrict__ gy) {
-    const int64_t npx = (int64_t)w * h;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < NSPO * npx;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int l = (int)(t / npx);
-        const int64_t i = t - (int64_t)l * npx;
-        const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
-        const float* img = lev + (l + 1) * npx;
-        float a = 0.0f, b = 0.0f;
-        if (x >= 1 && y >= 1 && x + 1 < w && y + 1 < h) {
-            a = img[i + 1] - img[i - 1];
-            b = img[i + w] - img[i - w];
+        for (int k = 0; k < 8 + 2 * R; ++k) v[k] = src[k];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = 0; k <= 2 * R; ++k) acc = acc + taps.k[k] * v[o + k];
+            sm.mid[row * S::MID_P + 8 * g + o] = acc;
         }
-        gx[t] = a;
-        gy[t] = b;
     }
+    __syncthreads();
+    // vertical
+    {
+        const int col = tid & (BX - 1), g = tid / BX;
+        float v[8 + 2 * R];
+#pragma unroll
+        for (int k = 0; k < 8 + 2 * R; ++k) v[k] = sm.mid[(8 * g + k) * S::MID_P + col];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = 0; k <= 2 * R; ++k) acc = acc + taps.k[k] * v[o + k];
+            store(col, 8 * g + o, acc);
+        }
+    }
+}
+static_assert(BLUR_THREADS == BX * BY / 8 && BY + 2 * 9 <= 64, "blur tile");
+
+constexpr int R_BASE = 5, R_LEVEL = 9;  // radii of the base blur and of level 3's
+
+// Level 0 of the first octave from the grey image (sift.rs:446-457).
+__global__ void __launch_bounds__(BLUR_THREADS) base_kernel(const uint8_t* __restrict__ gray, int w, int h,
+                                                            const __grid_constant__ BlurTaps taps,
+                                                            float* __restrict__ out) {
+    __shared__ BlurSmem<R_BASE> sm;
+    const int tiles_x = (w + BX - 1) / BX;
+    const int x0 = (int)(blockIdx.x % tiles_x) * BX, y0 = (int)(blockIdx.x / tiles_x) * BY;
+    blur_tile<R_BASE>(
+        sm, x0, y0, w, h, taps, [&](int64_t i) { return (float)gray[i] / 255.0f; },
+        [&](int x, int y, float v) {
+            if (x0 + x < w && y0 + y < h) out[(int64_t)(y0 + y) * w + x0 + x] = v;
+        });
 }
 
 // nalgebra 0.32 Matrix3::try_inverse: cofactors over the determinant
@@ -180,85 +202,176 @@ __device__ __forceinline__ bool inverse3(const double m[9], double o[9]) {
     return true;
 }
 
-// sift.rs:176-262.  Thread t = (level - 1) * npx + pixel.
-__global__ void extrema_kernel(const float* __restrict__ dogs, int w, int h, double thr, uint8_t* __restrict__ flag,
-                               double* __restrict__ kx, double* __restrict__ ky, double* __restrict__ kresp) {
-    const int64_t npx = (int64_t)w * h;
+// One octave (see the file's head).  A block makes the DoG of BX x BY pixels
+// and answers for the inner (BX - 2) x (BY - 2): their extrema (sift.rs:176-262,
+// the DoGs above and below being zero) and their part of the next octave's
+// level 0 (sift.rs:95-110; next may be null).  1600x1200, six octaves: five blurs
+// each, DoGs, extrema over three levels, gradients and their selections took
+// 124 launches and 590 us; 150 us here with the base.
+__global__ void __launch_bounds__(BLUR_THREADS) octave_kernel(const float* __restrict__ lev0, int w, int h,
+                                                              const __grid_constant__ BlurTaps taps, double thr,
+                                                              float* __restrict__ next, int nw, int nh, int octave,
+                                                              uint32_t place0, KpArrays kp, Counts* __restrict__ counts) {
+    __shared__ BlurSmem<R_LEVEL> sm;
+    __shared__ float lev3[BY][BX];
+    __shared__ float dog[BY][BX + 1];
+    const int tiles_x = (w + BX - 3) / (BX - 2);
+    const int x0 = (int)(blockIdx.x % tiles_x) * (BX - 2);  // the first inner pixel
+    const int y0 = (int)(blockIdx.x / tiles_x) * (BY - 2);
+    blur_tile<R_LEVEL>(
+        sm, x0 - 1, y0 - 1, w, h, taps, [&](int64_t i) { return __ldg(lev0 + i); },
+        [&](int x, int y, float v) {
+            lev3[y][x] = v;
+            dog[y][x] = v - sm.in[(y + R_LEVEL) * BlurSmem<R_LEVEL>::IN_P + x + R_LEVEL];
+        });
+    __syncthreads();
     const double edge_lim = (EDGE_THR + 1.0) * (EDGE_THR + 1.0) / EDGE_THR;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < NSPO * npx;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int level = 1 + (int)(t / npx);
-        const int64_t i = t - (int64_t)(level - 1) * npx;
-        const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
-        uint8_t ok = 0;
-        if (x >= 1 && y >= 1 && x + 1 < w && y + 1 < h) {
-            const float* dog = dogs + level * npx;
-            const float* below = dogs + (level - 1) * npx;
-            const float* above = dogs + (level + 1) * npx;
-            const float v = dog[i];
-            if (!((double)fabsf(v) < thr)) {
-                bool is_max = true, is_min = true;
-                for (int dy = -1; dy <= 1; ++dy)
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        if (dy == 0 && dx == 0) continue;
-                        const int64_t j = i + (int64_t)dy * w + dx;
-                        const float n0 = dog[j], n1 = below[j], n2 = above[j];
-                        if (n0 >= v || n1 >= v || n2 >= v) is_max = false;
-                        if (n0 <= v || n1 <= v || n2 <= v) is_min = false;
-                    }
-                if (is_max || is_min) {
-                    const float fdx = 0.5f * (dog[i + 1] - dog[i - 1]);
-                    const float fdy = 0.5f * (dog[i + w] - dog[i - w]);
-                    const float fds = 0.5f * (above[i] - below[i]);
-                    const float dxx = dog[i + 1] + dog[i - 1] - 2.0f * v;
-                    const float dyy = dog[i + w] + dog[i - w] - 2.0f * v;
-                    const float dss = above[i] + below[i] - 2.0f * v;
-                    const float dxy = 0.25f * (dog[i + w + 1] + dog[i - w - 1] - dog[i + w - 1] - dog[i - w + 1]);
-                    const float dxs = 0.25f * (above[i + 1] + below[i - 1] - above[i - 1] - below[i + 1]);
-                    const float dys = 0.25f * (above[i + w] + below[i - w] - above[i - w] - below[i + w]);
-                    const double hm[9] = {dxx, dxy, dxs, dxy, dyy, dys, dxs, dys, dss};
-                    double hi[9];
-                    if (inverse3(hm, hi)) {
-                        const double g0 = -(double)fdx, g1 = -(double)fdy, g2 = -(double)fds;
-                        const double ox = hi[0] * g0 + hi[1] * g1 + hi[2] * g2;
-                        const double oy = hi[3] * g0 + hi[4] * g1 + hi[5] * g2;
-                        const double os = hi[6] * g0 + hi[7] * g1 + hi[8] * g2;
-                        if (!(fabs(ox) > 1.0 || fabs(oy) > 1.0 || fabs(os) > 1.0)) {
-                            const double contrast =
-                                (double)v + 0.5 * ((double)fdx * ox + (double)fdy * oy + (double)fds * os);
-                            const double tr = (double)(dxx + dyy);
-                            const double det = (double)(dxx * dyy - dxy * dxy);
-                            if (!(fabs(contrast) < thr) && !(det <= 0.0 || tr * tr / det > edge_lim)) {
-                                ok = 1;
-                                kx[t] = (double)x + ox;
-                                ky[t] = (double)y + oy;
-                                kresp[t] = fabs(contrast);
-                            }
-                        }
-                    }
-                }
+    for (int i = threadIdx.x; i < (BX - 2) * (BY - 2); i += BLUR_THREADS) {
+        const int cx = 1 + i % (BX - 2), cy = 1 + i / (BX - 2);
+        const int x = x0 + cx - 1, y = y0 + cy - 1;
+        if (x < 1 || y < 1 || x + 1 >= w || y + 1 >= h) continue;
+        const float v = dog[cy][cx];
+        if ((double)fabsf(v) < thr) continue;
+        // a neighbour of the zero DoGs is 0
+        bool is_max = !(0.0f >= v), is_min = !(0.0f <= v);
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+            for (int dx = -1; dx <= 1; ++dx) {
+                if (dy == 0 && dx == 0) continue;
+                const float n = dog[cy + dy][cx + dx];
+                if (n >= v) is_max = false;
+                if (n <= v) is_min = false;
             }
+        if (!is_max && !is_min) continue;
+        auto d = [&](int dx, int dy) { return dog[cy + dy][cx + dx]; };
+        const float zero = 0.0f;
+        const float fdx = 0.5f * (d(1, 0) - d(-1, 0));
+        const float fdy = 0.5f * (d(0, 1) - d(0, -1));
+        const float fds = 0.5f * (zero - zero);
+        const float dxx = d(1, 0) + d(-1, 0) - 2.0f * v;
+        const float dyy = d(0, 1) + d(0, -1) - 2.0f * v;
+        const float dss = zero + zero - 2.0f * v;
+        const float dxy = 0.25f * (d(1, 1) + d(-1, -1) - d(-1, 1) - d(1, -1));
+        const float dxs = 0.25f * (zero + zero - zero - zero);
+        const float dys = 0.25f * (zero + zero - zero - zero);
+        const double hm[9] = {dxx, dxy, dxs, dxy, dyy, dys, dxs, dys, dss};
+        double hi[9];
+        if (!inverse3(hm, hi)) continue;
+        const double g0 = -(double)fdx, g1 = -(double)fdy, g2 = -(double)fds;
+        const double ox = hi[0] * g0 + hi[1] * g1 + hi[2] * g2;
+        const double oy = hi[3] * g0 + hi[4] * g1 + hi[5] * g2;
+        const double os = hi[6] * g0 + hi[7] * g1 + hi[8] * g2;
+        if (fabs(ox) > 1.0 || fabs(oy) > 1.0 || fabs(os) > 1.0) continue;
+        const double contrast = (double)v + 0.5 * ((double)fdx * ox + (double)fdy * oy + (double)fds * os);
+        const double tr = (double)(dxx + dyy);
+        const double det = (double)(dxx * dyy - dxy * dxy);
+        if (fabs(contrast) < thr || det <= 0.0 || tr * tr / det > edge_lim) continue;
+        const uint32_t k = atomicAdd(&counts->kp, 1u);
+        kp.x[k] = (double)x + ox;
+        kp.y[k] = (double)y + oy;
+        kp.resp[k] = fabs(contrast);
+        kp.place[k] = place0 + (uint32_t)y * (uint32_t)w + (uint32_t)x;
+        kp.oct[k] = octave;
+    }
+    if (next) {
+        for (int i = threadIdx.x; i < (BX / 2 - 1) * (BY / 2 - 1); i += BLUR_THREADS) {
+            const int tx = i % (BX / 2 - 1), ty = i / (BX / 2 - 1);
+            const int x = x0 / 2 + tx, y = y0 / 2 + ty;
+            if (x >= nw || y >= nh) continue;
+            const int ax = 1 + 2 * tx, ay = 1 + 2 * ty;
+            const int bx = min(2 * x + 1, w - 1) - x0 + 1, by = min(2 * y + 1, h - 1) - y0 + 1;
+            const float sum = lev3[ay][ax] + lev3[ay][bx] + lev3[by][ax] + lev3[by][bx];
+            next[(int64_t)y * nw + x] = 0.25f * sum;
         }
-        flag[t] = ok;
     }
 }
 
-// Appends the compacted keypoints of one octave (sel: indices into its flag
-// space; counts[o]: each octave's count, on the device) after those of the
-// octaves before it.
-__global__ void gather_kp_kernel(const uint32_t* __restrict__ sel, const int* __restrict__ counts, int octave,
-                                 int64_t npx, const double* __restrict__ kx, const double* __restrict__ ky,
-                                 const double* __restrict__ kresp, KpArrays kp) {
-    int64_t base = 0;
-    for (int q = 0; q < octave; ++q) base += counts[q];
-    const int n = counts[octave];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t t = sel[k];
-        kp.x[base + k] = kx[t];
-        kp.y[base + k] = ky[t];
-        kp.resp[base + k] = kresp[t];
-        kp.level[base + k] = 1 + (int)((int64_t)t / npx);
-        kp.oct[base + k] = octave;
+// ---- selection of the first `want` keypoints by (response descending, place)
+constexpr int SEL_BINS = 2048, SEL_CAP = 16384;
+
+// A response's order: it is never negative, so its bits are ordered as it is.
+__device__ __forceinline__ long long resp_key(double r) { return __double_as_longlong(r); }
+
+// Monotone in the key: 256 bins per octave from 2^-9, clamped.
+__device__ __forceinline__ int resp_bin(double r) {
+    const int b = (__float_as_int((float)r) - 0x3B000000) >> 15;
+    return min(max(b, 0), SEL_BINS - 1);
+}
+
+__global__ void __launch_bounds__(256) hist_kernel(const double* __restrict__ resp, const Counts* __restrict__ counts,
+                                                   uint32_t* __restrict__ hist) {
+    __shared__ uint32_t s_hist[SEL_BINS];
+    for (int i = threadIdx.x; i < SEL_BINS; i += 256) s_hist[i] = 0;
+    __syncthreads();
+    const uint32_t n = counts->kp;
+    for (uint32_t k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256) atomicAdd(&s_hist[resp_bin(resp[k])], 1u);
+    __syncthreads();
+    for (int i = threadIdx.x; i < SEL_BINS; i += 256)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
+// The keypoints whose bin is at least the highest one with `want` keypoints
+// at or above it.
+__global__ void __launch_bounds__(256) keep_kernel(const double* __restrict__ resp, const uint32_t* __restrict__ hist,
+                                                   uint32_t want, Counts* __restrict__ counts, uint32_t* __restrict__ kept) {
+    __shared__ uint32_t s_sum[256];
+    __shared__ int s_bin;
+    constexpr int PER = SEL_BINS / 256;
+    // thread t: bins from the top, [t * PER, (t + 1) * PER)
+    uint32_t c[PER], sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        c[i] = hist[SEL_BINS - 1 - (threadIdx.x * PER + i)];
+        sum += c[i];
+    }
+    s_sum[threadIdx.x] = sum;
+    if (threadIdx.x == 0) s_bin = 0;
+    __syncthreads();
+    for (int o = 1; o < 256; o <<= 1) {
+        const uint32_t v = (int)threadIdx.x >= o ? s_sum[threadIdx.x - o] : 0;
+        __syncthreads();
+        s_sum[threadIdx.x] += v;
+        __syncthreads();
+    }
+    uint32_t above = s_sum[threadIdx.x] - sum;
+    if (above < want && s_sum[threadIdx.x] >= want) {
+        int bin = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (above < want) {
+                above += c[i];
+                bin = SEL_BINS - 1 - (threadIdx.x * PER + i);
+            }
+        s_bin = bin;
+    }
+    __syncthreads();
+    const int bin = s_bin;  // 0 with fewer than `want`
+    const uint32_t n = counts->kp;
+    for (uint32_t k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
+        if (resp_bin(resp[k]) >= bin) {
+            const uint32_t at = atomicAdd(&counts->kept, 1u);
+            if (at < SEL_CAP) kept[at] = k;
+        }
+}
+
+// Rank of each kept keypoint by counting; skp[rank] = keypoint.  One warp each.
+__global__ void __launch_bounds__(256) rank_kernel(const KpArrays kp, const uint32_t* __restrict__ kept,
+                                                   const Counts* __restrict__ counts, uint32_t* __restrict__ skp) {
+    const uint32_t n = counts->kept;
+    if (n > SEL_CAP) return;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i = (blockIdx.x * 256 + threadIdx.x) >> 5; i < n; i += gridDim.x * 8) {
+        const uint32_t k = kept[i], place = kp.place[k];
+        const long long r = resp_key(kp.resp[k]);
+        uint32_t before = 0;
+        for (uint32_t j = lane; j < n; j += 32) {
+            const uint32_t o = kept[j];
+            const long long q = resp_key(kp.resp[o]);
+            before += q > r || (q == r && kp.place[o] < place);
+        }
+        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (lane == 0) skp[before] = k;
     }
 }
 
@@ -268,23 +381,27 @@ __device__ __forceinline__ double rem_euclid(double a, double b) {
 }
 
 // sift.rs:274-334.  One warp per keypoint, for the keypoints at sorted
-// positions base .. base + n - 1 (skp[pos] = keypoint); theta[4 pos ..] and
-// cnt[pos] (0 when the keypoint is outside the 8-pixel margin of the image,
-// sift.rs:519-521).
+// positions base .. base + n - 1 (skp[pos] = keypoint), or with `counts` as many
+// of them as were kept; theta[4 pos ..] and cnt[pos] (0 when the keypoint is
+// outside the 8-pixel margin of the image, sift.rs:519-521, or there is none).
 __global__ void __launch_bounds__(32 * WARPS) orient_kernel(KpArrays kp, const uint32_t* __restrict__ skp,
-                                                           int64_t base, int n, const __grid_constant__ OctTable oct,
-                                                           int img_w, int img_h, double* __restrict__ theta,
-                                                           int32_t* __restrict__ cnt) {
+                                                           int64_t base, int n, const Counts* __restrict__ counts,
+                                                           const __grid_constant__ OctTable oct, int img_w, int img_h,
+                                                           double* __restrict__ theta, int32_t* __restrict__ cnt) {
     __shared__ int sbin[WARPS][32];
     __shared__ double sval[WARPS][32];
-    __shared__ double shist[WARPS][36];
+    __shared__ double shist[WARPS][2][36];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * WARPS + wid;
     if (i >= n) return;
     const int64_t k = base + i;  // output position
+    if (counts && (counts->kept > SEL_CAP || (uint32_t)i >= counts->kept)) {
+        if (lane == 0) cnt[k] = 0;
+        return;
+    }
     const uint32_t kk = skp[k];
     const double kx = kp.x[kk], ky = kp.y[kk];
-    const int level = kp.level[kk], o = kp.oct[kk];
+    const int o = kp.oct[kk];
     const double scale = oct.scale[o];
     const double x0 = kx * scale, y0 = ky * scale;
     if (x0 < 8.0 || y0 < 8.0 || x0 >= (double)img_w - 8.0 || y0 >= (double)img_h - 8.0) {
@@ -292,10 +409,8 @@ __global__ void __launch_bounds__(32 * WARPS) orient_kernel(KpArrays kp, const u
         return;
     }
     const int w = oct.w[o], h = oct.h[o];
-    const int64_t npx = (int64_t)w * h;
-    const float* gx = oct.gx[o] + (level - 1) * npx;
-    const float* gy = oct.gy[o] + (level - 1) * npx;
-    const double sigma = 1.5 * level_sigma(level);
+    const float* img = oct.img[o];
+    const double sigma = 1.5 * level_sigma(KP_LEVEL);
     const int radius = (int)fmax(ceil(3.0 * sigma), 1.0);
     const double s2 = 2.0 * sigma * sigma;
     const long long xr = (long long)round(kx), yr = (long long)round(ky);
@@ -311,7 +426,7 @@ __global__ void __launch_bounds__(32 * WARPS) orient_kernel(KpArrays kp, const u
             const long long sx = xr + dx, sy = yr + dy;
             if (!(sx < 1 || sy < 1 || sx >= w - 1 || sy >= h - 1)) {
                 const int64_t i = sy * w + sx;
-                const float a = gx[i], b = gy[i];
+                const float a = img[i + 1] - img[i - 1], b = img[i + w] - img[i - w];  // sift.rs:137-149
                 const double mag = sqrt((double)(a * a + b * b));
                 const double ang = atan2((double)b, (double)a);
                 const double wgt = exp((-((double)dx * (double)dx) - (double)dy * (double)dy) / s2);
@@ -333,38 +448,89 @@ __global__ void __launch_bounds__(32 * WARPS) orient_kernel(KpArrays kp, const u
         }
         __syncwarp();
     }
-    shist[wid][b0] = acc0;
-    if (b1 < 36) shist[wid][b1] = acc1;
+    // two smoothings (every lane its bins), then the peaks in bin order
+    shist[wid][0][b0] = acc0;
+    if (b1 < 36) shist[wid][0][b1] = acc1;
     __syncwarp();
-    if (lane == 0) {
-        double hist[36];
-        for (int b = 0; b < 36; ++b) hist[b] = shist[wid][b];
-        for (int it = 0; it < 2; ++it) {
-            double sm[36];
-            for (int b = 0; b < 36; ++b) sm[b] = (hist[(b + 35) % 36] + 2.0 * hist[b] + hist[(b + 1) % 36]) / 4.0;
-            for (int b = 0; b < 36; ++b) hist[b] = sm[b];
-        }
-        double maxv = 0.0;
-        for (int b = 0; b < 36; ++b) maxv = fmax(maxv, hist[b]);
-        int np = 0;
-        if (maxv < 1e-12) {
-            theta[4 * (int64_t)k] = 0.0;
-            np = 1;
-        } else {
-            const double thresh = 0.8 * maxv;
-            for (int b = 0; b < 36 && np < 4; ++b) {
-                const double prev = hist[(b + 35) % 36], next = hist[(b + 1) % 36];
-                if (hist[b] > prev && hist[b] > next && hist[b] >= thresh) {
-                    const double denom = hist[b] * 2.0 - prev - next;
-                    const double d = fabs(denom) > 1e-12 ? 0.5 * (prev - next) / denom : 0.0;
-                    const double th = ((double)b + d) / 36.0 * 2.0 * PI - PI;
-                    theta[4 * (int64_t)k + np++] = rem_euclid(th, 2.0 * PI);
-                }
-            }
-            if (np == 0) theta[4 * (int64_t)k + np++] = 0.0;
-        }
-        cnt[k] = np;
+    for (int it = 0; it < 2; ++it) {
+        const double* hist = shist[wid][it];
+        double* sm = shist[wid][it ^ 1];
+        for (int b = lane; b < 36; b += 32) sm[b] = (hist[(b + 35) % 36] + 2.0 * hist[b] + hist[(b + 1) % 36]) / 4.0;
+        __syncwarp();
     }
+    const double* hist = shist[wid][0];
+    double maxv = fmax(hist[b0], b1 < 36 ? hist[b1] : 0.0);
+    for (int o = 16; o > 0; o >>= 1) maxv = fmax(maxv, __shfl_xor_sync(0xffffffffu, maxv, o));
+    maxv = fmax(0.0, maxv);
+    if (maxv < 1e-12) {
+        if (lane == 0) {
+            theta[4 * k] = 0.0;
+            cnt[k] = 1;
+        }
+        return;
+    }
+    const double thresh = 0.8 * maxv;
+    auto peak = [&](int b, double& th) -> bool {
+        if (b >= 36) return false;
+        const double prev = hist[(b + 35) % 36], next = hist[(b + 1) % 36];
+        if (!(hist[b] > prev && hist[b] > next && hist[b] >= thresh)) return false;
+        const double denom = hist[b] * 2.0 - prev - next;
+        const double d = fabs(denom) > 1e-12 ? 0.5 * (prev - next) / denom : 0.0;
+        th = rem_euclid(((double)b + d) / 36.0 * 2.0 * PI - PI, 2.0 * PI);
+        return true;
+    };
+    double t0 = 0.0, t1 = 0.0;
+    const unsigned m0 = __ballot_sync(0xffffffffu, peak(b0, t0)), m1 = __ballot_sync(0xffffffffu, peak(b1, t1));
+    const int at0 = __popc(m0 & ((1u << lane) - 1u)), at1 = __popc(m0) + __popc(m1 & ((1u << lane) - 1u));
+    if (((m0 >> lane) & 1u) && at0 < 4) theta[4 * k + at0] = t0;
+    if (((m1 >> lane) & 1u) && at1 < 4) theta[4 * k + at1] = t1;
+    if (lane == 0) {
+        const int np = min(__popc(m0) + __popc(m1), 4);
+        if (np == 0) theta[4 * k] = 0.0;
+        cnt[k] = max(np, 1);
+    }
+}
+
+// The pairs of the first n positions in one block: offsets by a scan of cnt,
+// then pairs_kernel's entries; counts->pairs.
+__global__ void __launch_bounds__(1024) first_pairs_kernel(const uint32_t* __restrict__ skp, int n,
+                                                           const int32_t* __restrict__ cnt,
+                                                           const double* __restrict__ theta,
+                                                           int32_t* __restrict__ pair_kp,
+                                                           double* __restrict__ pair_theta, Counts* __restrict__ counts) {
+    __shared__ int warp_sum[32];
+    __shared__ int s_base;
+    if (threadIdx.x == 0) s_base = 0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int b = 0; b < n; b += 1024) {
+        const int pos = b + threadIdx.x;
+        const int c = pos < n ? cnt[pos] : 0;
+        int x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_sum[wid] = x;
+        __syncthreads();
+        if (wid == 0) {
+            int v = warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += y;
+            }
+            warp_sum[lane] = v;
+        }
+        __syncthreads();
+        const int at = s_base + (wid ? warp_sum[wid - 1] : 0) + x - c;
+        for (int p = 0; p < c; ++p) {
+            pair_kp[at + p] = (int32_t)skp[pos];
+            pair_theta[at + p] = theta[4 * (int64_t)pos + p];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_base += warp_sum[31];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) counts->pairs = (uint32_t)s_base;
 }
 
 // (keypoint, peak) pairs of the keypoints at sorted positions base ..
@@ -381,151 +547,173 @@ __global__ void pairs_kernel(const uint32_t* __restrict__ skp, int64_t base, int
     }
 }
 
+__global__ void gather_resp_kernel(const double* __restrict__ resp, const uint32_t* __restrict__ idx, int64_t n,
+                                   double* __restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = resp[idx[i]];
+}
+
 __global__ void iota_kernel(uint32_t* __restrict__ out, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = (uint32_t)i;
 }
 
-// sift.rs:151-166
-__device__ __forceinline__ float bilinear(const float* __restrict__ img, int w, int h, double x, double y) {
-    const long long x0 = (long long)floor(x), y0 = (long long)floor(y);
-    const float fx = (float)(x - (double)x0), fy = (float)(y - (double)y0);
-    const long long xm = w - 1, ym = h - 1;
-    const long long ax = min(max(x0, 0LL), xm), ay = min(max(y0, 0LL), ym);
-    const long long bx = min(max(x0 + 1, 0LL), xm), by = min(max(y0 + 1, 0LL), ym);
-    const float a = img[ay * w + ax] * (1.0f - fx) + img[ay * w + bx] * fx;
-    const float b = img[by * w + ax] * (1.0f - fx) + img[by * w + bx] * fx;
-    return a * (1.0f - fy) + b * fy;
-}
-
-// sift.rs:340-431.  One warp per (keypoint, peak) pair, for the pairs
-// base .. base + n_pairs - 1 (in output order); descriptor and validity
-// stored at the pair's index.
-__global__ void __launch_bounds__(32 * WARPS) desc_kernel(KpArrays kp, int64_t base, int n_pairs,
-                                                         const int32_t* __restrict__ pair_kp,
-                                                         const double* __restrict__ pair_theta,
-                                                         const __grid_constant__ OctTable oct,
-                                                         float* __restrict__ desc, uint8_t* __restrict__ valid) {
+// sift.rs:340-431.  One block per (keypoint, peak) pair, for the pairs
+// base .. base + gridDim.x - 1 (in output order), or with `counts` those of
+// them that exist; descriptor and validity stored at the pair's index.  Bound
+// by the samples' f64 functions: 2048 descriptors 187 us.
+constexpr int DESC_RADIUS_MAX = 15, DESC_SAMPLES = (2 * DESC_RADIUS_MAX + 1) * (2 * DESC_RADIUS_MAX + 1);
+__global__ void __launch_bounds__(DESC_LEN) desc_kernel(KpArrays kp, int64_t base, const int32_t* __restrict__ pair_kp,
+                                                       const double* __restrict__ pair_theta,
+                                                       const Counts* __restrict__ counts,
+                                                       const __grid_constant__ OctTable oct, float* __restrict__ desc,
+                                                       uint8_t* __restrict__ valid) {
     constexpr int D = 4, N = 8;
-    __shared__ int hdr[WARPS][32];  // per sample: packed (by0, bx0, ob0 mod 8), or -1
-    __shared__ double cv[WARPS][32 * 8];
-    __shared__ float sd[WARPS][DESC_LEN];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * WARPS + wid;
-    if (i >= n_pairs) return;
-    const int64_t pos = base + i;
+    __shared__ uint16_t hdr[DESC_SAMPLES + 31];  // packed (by0 + 2, bx0 + 2, ob0 mod 8), or 0xFFFF
+    __shared__ double s_w[DESC_SAMPLES], s_fx[DESC_SAMPLES], s_fy[DESC_SAMPLES], s_fo[DESC_SAMPLES];
+    __shared__ float sd[DESC_LEN];
+    __shared__ float s_norm;
+    const int64_t pos = base + blockIdx.x;
+    if (counts && pos >= (int64_t)counts->pairs) return;
     const int k = pair_kp[pos];
     const double x = kp.x[k], y = kp.y[k], th = pair_theta[pos];
-    const int level = kp.level[k], o = kp.oct[k];
+    const int o = kp.oct[k];
     const int w = oct.w[o], h = oct.h[o];
-    const int64_t npx = (int64_t)w * h;
-    const float* gxi = oct.gx[o] + (level - 1) * npx;
-    const float* gyi = oct.gy[o] + (level - 1) * npx;
-    const double sigma = level_sigma(level);
+    const float* img = oct.img[o];
+    const double sigma = level_sigma(KP_LEVEL);
     const double cell = 3.0 * sigma;
-    const int radius = (int)ceil(sqrt(1.5) * cell * ((double)D + 1.0) * 0.5);
+    const int radius = (int)ceil(sqrt(1.5) * cell * ((double)D + 1.0) * 0.5);  // DESC_RADIUS_MAX
     const double cos_t = cos(th), sin_t = sin(th);
     const double exp_scale = -1.0 / ((double)(D * D) * 0.5);
     const double half = (double)D * 0.5;
     const int side = 2 * radius + 1, total = side * side;
-    // Lane L owns the bins 32q + L (q = 0..3): cell row q, cell column L / 8,
-    // orientation L % 8.  A sample adds to such a bin at most once.
-    const int cx = lane >> 3, co = lane & 7;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int base = 0; base < total; base += 32) {
-        const int s = base + lane;
-        int hd = -1;
-        if (s < total) {
-            const int dy = s / side - radius, dx = s % side - radius;
-            const double sx = x + (double)dx, sy = y + (double)dy;
-            if (!(sx < 1.0 || sy < 1.0 || sx >= (double)w - 2.0 || sy >= (double)h - 2.0)) {
-                const double gx = (double)bilinear(gxi, w, h, sx, sy);
-                const double gy = (double)bilinear(gyi, w, h, sx, sy);
-                const double mag = sqrt(gx * gx + gy * gy);
-                if (!(mag < 1e-12)) {
-                    const double rx = cos_t * (double)dx + sin_t * (double)dy;
-                    const double ry = -sin_t * (double)dx + cos_t * (double)dy;
-                    const double bx = rx / cell + half - 0.5;
-                    const double by = ry / cell + half - 0.5;
-                    if (!(bx < -1.0 || by < -1.0 || bx > (double)D || by > (double)D)) {
-                        const double ang = atan2(gy, gx) - th;
-                        const double ob = rem_euclid(ang, 2.0 * PI) / (2.0 * PI) * (double)N;
-                        double wgt =
-                            ((bx - half + 0.5) * (bx - half + 0.5) + (by - half + 0.5) * (by - half + 0.5)) * exp_scale;
-                        wgt = exp(wgt) * mag;
-                        // bx, by in [-1, 4], ob in [0, 8]
-                        const int bx0 = (int)floor(bx), by0 = (int)floor(by), ob0 = (int)floor(ob);
-                        const double fx = bx - (double)bx0, fy = by - (double)by0, fo = ob - (double)ob0;
-#pragma unroll
-                        for (int iy = 0; iy < 2; ++iy)
-#pragma unroll
-                            for (int ix = 0; ix < 2; ++ix) {
-                                const double wy = iy == 0 ? 1.0 - fy : fy;
-                                const double wx = ix == 0 ? 1.0 - fx : fx;
-#pragma unroll
-                                for (int io = 0; io < 2; ++io) {
-                                    const double wo = io == 0 ? 1.0 - fo : fo;
-                                    cv[wid][lane * 8 + iy * 4 + ix * 2 + io] = wgt * wx * wy * wo;
-                                }
-                            }
-                        hd = ((by0 + 2) << 8) | ((bx0 + 2) << 4) | (ob0 & 7);
-                    }
-                }
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int s = tid; s < total + 31; s += DESC_LEN) {
+        int hd = 0xFFFF;
+        const int dy = s / side - radius, dx = s % side - radius;
+        const double sx = x + (double)dx, sy = y + (double)dy;
+        const double rx = cos_t * (double)dx + sin_t * (double)dy;
+        const double ry = -sin_t * (double)dx + cos_t * (double)dy;
+        const double bx = rx / cell + half - 0.5;
+        const double by = ry / cell + half - 0.5;
+        if (s < total && !(sx < 1.0 || sy < 1.0 || sx >= (double)w - 2.0 || sy >= (double)h - 2.0) &&
+            !(bx < -1.0 || by < -1.0 || bx > (double)D || by > (double)D)) {
+            // sift.rs:137-166: bilinear gradients; 1 <= x0, x0 + 1 <= w - 2, so no
+            // clamp applies and every gradient is a central difference
+            const int x0 = (int)floor(sx), y0 = (int)floor(sy);
+            const float fx = (float)(sx - (double)x0), fy = (float)(sy - (double)y0);
+            const float* p = img + (int64_t)y0 * w + x0;
+            const float a0 = p[-1], a1 = p[0], a2 = p[1], a3 = p[2];
+            const float b0 = p[w - 1], b1 = p[w], b2 = p[w + 1], b3 = p[w + 2];
+            const float u1 = p[-w], u2 = p[-w + 1], d1 = p[2 * w], d2 = p[2 * w + 1];
+            const float gxa = (a2 - a0) * (1.0f - fx) + (a3 - a1) * fx, gxb = (b2 - b0) * (1.0f - fx) + (b3 - b1) * fx;
+            const float gya = (b1 - u1) * (1.0f - fx) + (b2 - u2) * fx, gyb = (d1 - a1) * (1.0f - fx) + (d2 - a2) * fx;
+            const double gx = (double)(gxa * (1.0f - fy) + gxb * fy);
+            const double gy = (double)(gya * (1.0f - fy) + gyb * fy);
+            const double mag = sqrt(gx * gx + gy * gy);
+            if (!(mag < 1e-12)) {
+                const double ang = atan2(gy, gx) - th;
+                const double ob = rem_euclid(ang, 2.0 * PI) / (2.0 * PI) * (double)N;
+                double wgt = ((bx - half + 0.5) * (bx - half + 0.5) + (by - half + 0.5) * (by - half + 0.5)) * exp_scale;
+                wgt = exp(wgt) * mag;
+                // bx, by in [-1, 4], ob in [0, 8]
+                const int bx0 = (int)floor(bx), by0 = (int)floor(by), ob0 = (int)floor(ob);
+                s_w[s] = wgt;
+                s_fx[s] = bx - (double)bx0;
+                s_fy[s] = by - (double)by0;
+                s_fo[s] = ob - (double)ob0;
+                hd = ((by0 + 2) << 8) | ((bx0 + 2) << 4) | (ob0 & 7);
             }
         }
-        hdr[wid][lane] = hd;
-        __syncwarp();
-        const int m = min(32, total - base);
-        for (int t = 0; t < m; ++t) {
-            const int hv = hdr[wid][t];
-            if (hv < 0) continue;
+        hdr[s] = (uint16_t)hd;
+    }
+    __syncthreads();
+    // Thread t owns bin t: cell row q = its warp, cell column lane / 8,
+    // orientation lane % 8.  A sample adds to such a bin at most once; the warp
+    // visits only the samples that touch its row.
+    const int cx = lane >> 3, co = lane & 7, q = wid;
+    double acc = 0.0;
+    for (int b = 0; b < total; b += 32) {
+        const int mine = hdr[b + lane];
+        const int myrow = (mine >> 8) - 2;  // 0xFFFF: 253
+        unsigned todo = __ballot_sync(0xffffffffu, myrow == q || myrow == q - 1);
+        while (todo) {
+            const int t = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int hv = __shfl_sync(0xffffffffu, mine, t);
             const int ix = cx - (((hv >> 4) & 15) - 2);
             const int io = (co - (hv & 7)) & 7;
             if ((unsigned)ix > 1u || io > 1) continue;
-            const int by0 = (hv >> 8) - 2;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int iy = q - by0;
-                if (iy == 0 || iy == 1) acc[q] += cv[wid][t * 8 + iy * 4 + ix * 2 + io];
-            }
+            const int s = b + t;
+            const bool low = q == (hv >> 8) - 2;
+            const double wy = low ? 1.0 - s_fy[s] : s_fy[s];
+            const double wx = ix == 0 ? 1.0 - s_fx[s] : s_fx[s];
+            const double wo = io == 0 ? 1.0 - s_fo[s] : s_fo[s];
+            acc += s_w[s] * wx * wy * wo;
         }
-        __syncwarp();
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sd[wid][lane + 32 * q] = (float)acc[q];
-    __syncwarp();
-    if (lane == 0) {
-        float* d = sd[wid];
-        float ss = 0.0f;
-        for (int i = 0; i < DESC_LEN; ++i) ss = ss + d[i] * d[i];
-        const float norm = sqrtf(ss);
-        bool ok = !(norm < 1e-6f);
-        if (ok) {
-            for (int i = 0; i < DESC_LEN; ++i) d[i] = d[i] / norm;
-            for (int i = 0; i < DESC_LEN; ++i)
-                if (d[i] > 0.2f) d[i] = 0.2f;
-            float ss2 = 0.0f;
-            for (int i = 0; i < DESC_LEN; ++i) ss2 = ss2 + d[i] * d[i];
-            const float norm2 = sqrtf(ss2);
-            ok = !(norm2 < 1e-6f);
-            if (ok)
-                for (int i = 0; i < DESC_LEN; ++i) d[i] = d[i] / norm2;
+    // the serial f32 sums of the reference; the elementwise steps by all
+    float d = (float)acc;
+    auto norm = [&]() -> float {
+        sd[tid] = d * d;
+        __syncthreads();
+        if (tid == 0) {
+            float ss = 0.0f;
+#pragma unroll 16
+            for (int i = 0; i < DESC_LEN; ++i) ss = ss + sd[i];
+            s_norm = sqrtf(ss);
         }
-        valid[pos] = ok ? 1 : 0;
+        __syncthreads();
+        return s_norm;
+    };
+    float nm = norm();
+    bool ok = !(nm < 1e-6f);
+    if (ok) {
+        d = d / nm;
+        if (d > 0.2f) d = 0.2f;
+        nm = norm();  // s_norm and sd are read before the next writes: both sides synchronise
+        ok = !(nm < 1e-6f);
+        if (ok) d = d / nm;
     }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) desc[pos * DESC_LEN + lane + 32 * q] = sd[wid][lane + 32 * q];
+    desc[pos * DESC_LEN + tid] = d;
+    if (tid == 0) valid[pos] = ok ? 1 : 0;
 }
 
-// sift.rs:543-554: output i is the sorted position sel[i] (the i-th valid
-// descriptor in response order); clamped position, descriptor, colour.
-__global__ void final_kernel(const uint32_t* __restrict__ sel, int n, const int32_t* __restrict__ pair_kp, KpArrays kp,
-                             const __grid_constant__ OctTable oct,
+// The valid ones among the first min(counts->pairs, cap) pairs, in order, in
+// one block; counts->valid.
+__global__ void __launch_bounds__(1024) first_valid_kernel(const uint8_t* __restrict__ valid, int cap,
+                                                           uint32_t* __restrict__ sel, Counts* __restrict__ counts) {
+    __shared__ int warp_sum[32];
+    __shared__ int s_base;
+    if (threadIdx.x == 0) s_base = 0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n = (int)min(counts->pairs, (uint32_t)cap);
+    __syncthreads();
+    for (int b = 0; b < n; b += 1024) {
+        const int i = b + threadIdx.x;
+        const bool v = i < n && valid[i];
+        const unsigned m = __ballot_sync(0xffffffffu, v);
+        if (lane == 0) warp_sum[wid] = __popc(m);
+        __syncthreads();
+        int before = s_base;
+        for (int k = 0; k < wid; ++k) before += warp_sum[k];
+        if (v) sel[before + __popc(m & ((1u << lane) - 1u))] = (uint32_t)i;
+        __syncthreads();
+        if (threadIdx.x == 1023) s_base = before + __popc(m);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) counts->valid = (uint32_t)s_base;
+}
+
+// sift.rs:543-554: output i is the pair sel[i] (the i-th valid descriptor in
+// response order), of n or with `counts` of the valid ones; clamped position,
+// descriptor, colour.
+__global__ void final_kernel(const uint32_t* __restrict__ sel, int n, const Counts* __restrict__ counts,
+                             const int32_t* __restrict__ pair_kp, KpArrays kp, const __grid_constant__ OctTable oct,
                              const float* __restrict__ desc, const uint8_t* __restrict__ rgb, int w, int h,
                              double* __restrict__ pts, float* __restrict__ odesc, uint8_t* __restrict__ col) {
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (wid >= n) return;
+    if (wid >= n || (counts && (uint32_t)wid >= counts->valid)) return;
     const uint32_t pos = sel[wid];
     if (lane == 0) {
         const int k = pair_kp[pos];
@@ -565,6 +753,14 @@ bool blur_taps(double sigma, BlurTaps& t) {
     return true;
 }
 
+// Taps that return their input: exactly 0 but for a 1 in the middle (0 x + a
+// and 1 x are exact for finite x).
+bool identity_taps(const BlurTaps& t) {
+    for (int i = 0; i <= 2 * t.radius; ++i)
+        if (t.k[i] != (i == t.radius ? 1.0f : 0.0f)) return false;
+    return true;
+}
+
 int sfail(rcmvs_ctx* ctx, int code, const std::string& msg) {
     if (ctx) ctx->err = msg;
     return code;
@@ -578,12 +774,18 @@ int sfail(rcmvs_ctx* ctx, int code, const std::string& msg) {
                          std::string(#x) + ": " + cudaGetErrorString(e_));                     \
     } while (0)
 
+// max_features up to which the first keypoints are selected, oriented and
+// described without waiting for their counts, and how many keypoints that
+// takes beyond max_features (margins drop some, extra peaks add some).
+constexpr int64_t QUICK_CAP = 8192;
+int64_t quick_keypoints(int64_t cap) { return cap + cap / 8 + 64; }
+
 // Context arena slots 80-159.
 enum {
-    F_IN = 80, F_GRAY, F_RGB, F_BASE, F_LEV, F_TMP, F_DOG, F_FLAG, F_KX, F_KY, F_KRESP, F_SEL, F_NSEL, F_TEMP,
-    F_KPX, F_KPY, F_KPRESP, F_KPLEV, F_KPOCT, F_THETA, F_CNT, F_OFF, F_PKP, F_PTH, F_PIDX, F_SRESP, F_SIDX,
-    F_DESC, F_VALID, F_OSEL, F_PTS, F_FDESC, F_COL, F_NEXT, F_OCTCNT,
-    F_GRAD = 130  // 130 + 2 * octave: gx, + 1: gy (octaves 0..7)
+    F_IN = 80, F_GRAY, F_RGB, F_KPX, F_KPY, F_KPRESP, F_KPPLACE, F_KPOCT, F_TEMP, F_THETA, F_CNT, F_OFF, F_PKP, F_PTH,
+    F_PIDX, F_PLACE2, F_PIDX2, F_SRESP, F_SRESP2, F_SIDX, F_DESC, F_VALID, F_OSEL, F_PTS, F_FDESC, F_COL, F_COUNTS,
+    F_HIST, F_KEPT, F_NSEL,
+    F_LEV = 130  // + octave: its level 0 (octaves 0..7)
 };
 
 // Grows an arena slot to `need` bytes keeping its first `keep` bytes: a
@@ -654,20 +856,19 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
     cudaStream_t st = ctx->stream;
     DeviceArena& A = ctx->arena;
     const int64_t n_in = (int64_t)w0 * h0, npx0 = (int64_t)w * h;
-    void *p_in, *p_gray, *p_rgb, *p_base;
+    if (NSPO * npx0 > (int64_t)UINT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "sift: octave too large");
+    void *p_in, *p_gray, *p_rgb;
     SCK(A.get(F_IN, (size_t)n_in * channels, &p_in));
     SCK(A.get(F_GRAY, (size_t)npx0, &p_gray));
     SCK(A.get(F_RGB, 3 * (size_t)npx0, &p_rgb));
-    SCK(A.get(F_BASE, sizeof(float) * (size_t)npx0, &p_base));
     SCK(cudaMemcpyAsync(p_in, img, (size_t)n_in * channels, cudaMemcpyHostToDevice, st));
     const int* d_err = nullptr;
     rc = resize_device(ctx, (const uint8_t*)p_in, w0, h0, channels, w, h, (uint8_t*)p_gray, (uint8_t*)p_rgb, &d_err);
     if (rc) return rc;
-    to_float_kernel<<<grid_of(npx0), 256, 0, st>>>((const uint8_t*)p_gray, npx0, (float*)p_base);
-    SCK(cudaGetLastError());
 
     int n_oct = 1;  // sift.rs:458-461
     while ((std::max(w, h) >> n_oct) >= 40 && n_oct < 8) ++n_oct;
+    if (n_oct > MAX_OCT) return sfail(ctx, RCMVS_E_LIMIT, "sift: too many octaves");
     BlurTaps first{}, inc[NLEV];
     const double fs = std::sqrt(std::max(SIGMA0 * SIGMA0 - ASSUMED_BLUR * ASSUMED_BLUR, 1e-4));
     if (!blur_taps(fs, first)) return sfail(ctx, RCMVS_E_LIMIT, "sift: blur kernel too wide");
@@ -675,130 +876,133 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
         const double sp = level_sigma(l - 1), sc = level_sigma(l);
         if (!blur_taps(std::sqrt(std::max(sc * sc - sp * sp, 1e-4)), inc[l]))
             return sfail(ctx, RCMVS_E_LIMIT, "sift: blur kernel too wide");
+        if (l != NSPO && !identity_taps(inc[l])) return sfail(ctx, RCMVS_E_STATE, "sift: levels of one sigma differ");
     }
+    if (first.radius != R_BASE || inc[NSPO].radius != R_LEVEL) return sfail(ctx, RCMVS_E_STATE, "sift: blur radius");
 
     const SpanHook& hook = ctx->hook();
-    if (n_oct > MAX_OCT) return sfail(ctx, RCMVS_E_LIMIT, "sift: too many octaves");
+    const int64_t cap = (int64_t)opts->max_features;
+    // keypoint arrays sized for every pixel of every octave
     OctTable table{};
-    int ow = w, oh = h;
-    thrust::counting_iterator<uint32_t> it(0);
-    void *p_temp, *p_nsel, *p_octcnt;
-    SCK(A.get(F_NSEL, sizeof(int) * 4, &p_nsel));
-    SCK(A.get(F_OCTCNT, sizeof(int) * MAX_OCT, &p_octcnt));
-    int* d_oct = (int*)p_octcnt;
-    // keypoint arrays sized for every pixel of DoG levels 1-3 of every
-    // octave, so the octaves run back to back with their counts on the device
     int64_t kcap = 0;
-    for (int o = 0, tw = w, th = h; o < n_oct; ++o, tw = std::max(tw / 2, 1), th = std::max(th / 2, 1))
-        kcap += NSPO * (int64_t)tw * th;
+    for (int o = 0, tw = w, th = h; o < n_oct; ++o, tw = std::max(tw / 2, 1), th = std::max(th / 2, 1)) {
+        void* p;
+        SCK(A.get(F_LEV + o, sizeof(float) * (size_t)tw * th, &p));
+        table.img[o] = (const float*)p;
+        table.w[o] = tw;
+        table.h[o] = th;
+        table.scale[o] = std::pow(2.0, o);
+        kcap += (int64_t)tw * th;
+    }
     KpArrays kp{};
+    Counts* d_counts;
+    uint32_t* d_hist;
     {
-        void *p_x, *p_y, *p_r, *p_l, *p_o;
+        void *p_x, *p_y, *p_r, *p_l, *p_o, *p_c;
         SCK(A.get(F_KPX, 8 * (size_t)kcap, &p_x));
         SCK(A.get(F_KPY, 8 * (size_t)kcap, &p_y));
         SCK(A.get(F_KPRESP, 8 * (size_t)kcap, &p_r));
-        SCK(A.get(F_KPLEV, 4 * (size_t)kcap, &p_l));
+        SCK(A.get(F_KPPLACE, 4 * (size_t)kcap, &p_l));
         SCK(A.get(F_KPOCT, 4 * (size_t)kcap, &p_o));
-        kp = KpArrays{(double*)p_x, (double*)p_y, (double*)p_r, (int32_t*)p_l, (int32_t*)p_o};
+        kp = KpArrays{(double*)p_x, (double*)p_y, (double*)p_r, (uint32_t*)p_l, (int32_t*)p_o};
+        SCK(A.get(F_COUNTS, sizeof(Counts) + sizeof(uint32_t) * SEL_BINS, &p_c));
+        d_counts = (Counts*)p_c;
+        d_hist = (uint32_t*)(d_counts + 1);
     }
+    SCK(cudaMemsetAsync(d_counts, 0, sizeof(Counts) + sizeof(uint32_t) * SEL_BINS, st));
+    hook.begin("sift_pyramid");
+    base_kernel<<<((w + BX - 1) / BX) * ((h + BY - 1) / BY), BLUR_THREADS, 0, st>>>((const uint8_t*)p_gray, w, h, first,
+                                                                                   const_cast<float*>(table.img[0]));
+    SCK(cudaGetLastError());
+    hook.end("sift_pyramid");
+    hook.begin("sift_extrema");
+    int64_t place = 0;
     for (int o = 0; o < n_oct; ++o) {
-        const int64_t npx = (int64_t)ow * oh;
-        void *p_lev, *p_tmp, *p_dog, *p_flag, *p_kx, *p_ky, *p_kr, *p_sel;
-        SCK(A.get(F_LEV, sizeof(float) * NLEV * (size_t)npx, &p_lev));
-        SCK(A.get(F_TMP, sizeof(float) * (size_t)npx, &p_tmp));
-        SCK(A.get(F_DOG, sizeof(float) * NDOG * (size_t)npx, &p_dog));
-        float* lev = (float*)p_lev;
-        float* tmp = (float*)p_tmp;
-        // level 0: the base (blurred by the first sigma in octave 0)
-        const float* base = (const float*)p_base;
-        hook.begin("sift_pyramid");
-        if (o == 0) {
-            blur_kernel<false><<<grid_of(npx), 256, 0, st>>>(base, tmp, ow, oh, first);
-            blur_kernel<true><<<grid_of(npx), 256, 0, st>>>(tmp, lev, ow, oh, first);
-        } else {
-            SCK(cudaMemcpyAsync(lev, base, sizeof(float) * npx, cudaMemcpyDeviceToDevice, st));
-        }
-        for (int l = 1; l < NLEV; ++l) {
-            blur_kernel<false><<<grid_of(npx), 256, 0, st>>>(lev + (l - 1) * npx, tmp, ow, oh, inc[l]);
-            blur_kernel<true><<<grid_of(npx), 256, 0, st>>>(tmp, lev + l * npx, ow, oh, inc[l]);
-        }
+        const int ow = table.w[o], oh = table.h[o];
+        const bool more = o + 1 < n_oct;
+        octave_kernel<<<((ow + BX - 3) / (BX - 2)) * ((oh + BY - 3) / (BY - 2)), BLUR_THREADS, 0, st>>>(
+            table.img[o], ow, oh, inc[NSPO], opts->contrast_thr, more ? const_cast<float*>(table.img[o + 1]) : nullptr,
+            more ? table.w[o + 1] : 0, more ? table.h[o + 1] : 0, o, (uint32_t)place, kp, d_counts);
         SCK(cudaGetLastError());
-        dog_kernel<<<grid_of(npx), 256, 0, st>>>(lev, (float*)p_dog, npx);
+        place += (int64_t)ow * oh;
+    }
+    hook.end("sift_extrema");
+
+    int64_t n_valid = 0;
+    void *p_skp = nullptr, *p_th = nullptr, *p_cnt = nullptr, *p_pkp = nullptr, *p_pth = nullptr, *p_desc = nullptr,
+         *p_valid = nullptr, *p_osel = nullptr, *p_pts = nullptr, *p_fdesc = nullptr, *p_col = nullptr;
+    const bool quick = cap > 0 && cap <= QUICK_CAP;
+    const int64_t want = quick_keypoints(cap);
+    if (quick) {
+        void* p_kept;
+        SCK(A.get(F_KEPT, sizeof(uint32_t) * SEL_CAP, &p_kept));
+        SCK(A.get(F_SIDX, sizeof(uint32_t) * SEL_CAP, &p_skp));
+        SCK(A.get(F_THETA, sizeof(double) * 4 * (size_t)want, &p_th));
+        SCK(A.get(F_CNT, sizeof(int32_t) * (size_t)want, &p_cnt));
+        SCK(A.get(F_PKP, sizeof(int32_t) * 4 * (size_t)want, &p_pkp));
+        SCK(A.get(F_PTH, sizeof(double) * 4 * (size_t)want, &p_pth));
+        SCK(A.get(F_VALID, (size_t)cap, &p_valid));
+        SCK(A.get(F_OSEL, sizeof(uint32_t) * (size_t)cap, &p_osel));
+        if ((rc = grow_copy(ctx, F_DESC, sizeof(float) * DESC_LEN * (size_t)cap, 0, &p_desc))) return rc;
+        SCK(A.get(F_PTS, sizeof(double) * 2 * cap, &p_pts));
+        SCK(A.get(F_FDESC, sizeof(float) * DESC_LEN * cap, &p_fdesc));
+        SCK(A.get(F_COL, 3 * (size_t)cap, &p_col));
+        hist_kernel<<<64, 256, 0, st>>>(kp.resp, d_counts, d_hist);
         SCK(cudaGetLastError());
-        hook.end("sift_pyramid");
-        const int64_t nt = NSPO * npx;
-        if (nt > (int64_t)UINT32_MAX) return sfail(ctx, RCMVS_E_LIMIT, "sift: octave too large");
-        SCK(A.get(F_FLAG, (size_t)nt, &p_flag));
-        SCK(A.get(F_KX, sizeof(double) * (size_t)nt, &p_kx));
-        SCK(A.get(F_KY, sizeof(double) * (size_t)nt, &p_ky));
-        SCK(A.get(F_KRESP, sizeof(double) * (size_t)nt, &p_kr));
-        SCK(A.get(F_SEL, sizeof(uint32_t) * (size_t)nt, &p_sel));
-        hook.begin("sift_extrema");
-        extrema_kernel<<<grid_of(nt), 256, 0, st>>>((const float*)p_dog, ow, oh, opts->contrast_thr,
-                                                     (uint8_t*)p_flag, (double*)p_kx, (double*)p_ky, (double*)p_kr);
+        keep_kernel<<<64, 256, 0, st>>>(kp.resp, d_hist, (uint32_t)want, d_counts, (uint32_t*)p_kept);
         SCK(cudaGetLastError());
-        hook.end("sift_extrema");
-        size_t tb = 0;
-        SCK(cub::DeviceSelect::Flagged(nullptr, tb, it, (const uint8_t*)p_flag, (uint32_t*)p_sel, d_oct + o,
-                                       (int)nt, st));
-        SCK(A.get(F_TEMP, tb, &p_temp));
-        SCK(cub::DeviceSelect::Flagged(p_temp, tb, it, (const uint8_t*)p_flag, (uint32_t*)p_sel, d_oct + o,
-                                       (int)nt, st));
-        table.w[o] = ow;
-        table.h[o] = oh;
-        table.scale[o] = std::pow(2.0, o);
-        gather_kp_kernel<<<grid_of(nt), 256, 0, st>>>((const uint32_t*)p_sel, d_oct, o, npx, (const double*)p_kx,
-                                                       (const double*)p_ky, (const double*)p_kr, kp);
+        rank_kernel<<<148 * 2, 256, 0, st>>>(kp, (const uint32_t*)p_kept, d_counts, (uint32_t*)p_skp);
         SCK(cudaGetLastError());
-        void *p_gx, *p_gy;
-        SCK(A.get(F_GRAD + 2 * o, sizeof(float) * NSPO * (size_t)npx, &p_gx));
-        SCK(A.get(F_GRAD + 2 * o + 1, sizeof(float) * NSPO * (size_t)npx, &p_gy));
-        table.gx[o] = (const float*)p_gx;
-        table.gy[o] = (const float*)p_gy;
-        grad_kernel<<<grid_of(NSPO * npx), 256, 0, st>>>(lev, ow, oh, (float*)p_gx, (float*)p_gy);
+        hook.begin("sift_orient");
+        orient_kernel<<<(unsigned)((want + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
+            kp, (const uint32_t*)p_skp, 0, (int)want, d_counts, table, w, h, (double*)p_th, (int32_t*)p_cnt);
         SCK(cudaGetLastError());
-        // next octave's base: level NSPO downsampled 2x2 (sift.rs:488-492)
-        const int nw = std::max(ow / 2, 1), nh = std::max(oh / 2, 1);
-        if (o + 1 < n_oct) {
-            void* p_next;
-            SCK(A.get(F_NEXT, sizeof(float) * (size_t)nw * nh, &p_next));
-            downsample_kernel<<<grid_of((int64_t)nw * nh), 256, 0, st>>>(lev + NSPO * npx, ow, oh, (float*)p_next,
-                                                                         nw, nh);
-            SCK(cudaGetLastError());
-            SCK(A.get(F_BASE, sizeof(float) * (size_t)nw * nh, &p_base));
-            SCK(cudaMemcpyAsync(p_base, p_next, sizeof(float) * (size_t)nw * nh, cudaMemcpyDeviceToDevice, st));
-        }
-        ow = nw;
-        oh = nh;
+        hook.end("sift_orient");
+        first_pairs_kernel<<<1, 1024, 0, st>>>((const uint32_t*)p_skp, (int)want, (const int32_t*)p_cnt,
+                                               (const double*)p_th, (int32_t*)p_pkp, (double*)p_pth, d_counts);
+        SCK(cudaGetLastError());
+        hook.begin("sift_desc");
+        desc_kernel<<<(unsigned)cap, DESC_LEN, 0, st>>>(kp, 0, (const int32_t*)p_pkp, (const double*)p_pth, d_counts,
+                                                        table, (float*)p_desc, (uint8_t*)p_valid);
+        SCK(cudaGetLastError());
+        hook.end("sift_desc");
+        first_valid_kernel<<<1, 1024, 0, st>>>((const uint8_t*)p_valid, (int)cap, (uint32_t*)p_osel, d_counts);
+        SCK(cudaGetLastError());
+        final_kernel<<<(int)((cap + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
+            (const uint32_t*)p_osel, (int)cap, d_counts, (const int32_t*)p_pkp, kp, table, (const float*)p_desc,
+            (const uint8_t*)p_rgb, w, h, (double*)p_pts, (float*)p_fdesc, (uint8_t*)p_col);
+        SCK(cudaGetLastError());
     }
     int bad = 0;
-    int oc[MAX_OCT] = {0};
+    Counts hc{};
     if (d_err) SCK(cudaMemcpyAsync(&bad, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SCK(cudaMemcpyAsync(oc, d_oct, sizeof(int) * n_oct, cudaMemcpyDeviceToHost, st));
+    SCK(cudaMemcpyAsync(&hc, d_counts, sizeof(Counts), cudaMemcpyDeviceToHost, st));
     SCK(cudaStreamSynchronize(st));
     if (bad) return sfail(ctx, RCMVS_E_CUDA, "sift: resize tap table overflow");
-    int64_t nkp = 0;  // keypoints of all octaves
-    for (int o = 0; o < n_oct; ++o) nkp += oc[o];
+    const int64_t nkp = hc.kp;  // keypoints of all octaves
     const uint64_t n_raw = (uint64_t)nkp;
     if (nkp > INT32_MAX / 4) return sfail(ctx, RCMVS_E_LIMIT, "sift: too many keypoints");
-
-    // The reference computes every (keypoint, peak) descriptor in (octave,
-    // keypoint, peak) order, sorts them by their keypoint's response with a
-    // stable sort and keeps the first max_features (sift.rs:497-544).  The
-    // same order is the keypoints sorted stably by response with each one's
-    // peaks in turn, so keypoints are sorted first and orientations, pairs
-    // and descriptors are produced in that order until max_features valid
-    // descriptors exist (a descriptor that normalises to nothing is dropped,
-    // as in the reference).
-    const int64_t cap = (int64_t)opts->max_features;
-    int64_t kdone = 0, np = 0, done = 0, n_valid = 0;
-    void *p_kidx = nullptr, *p_sresp = nullptr, *p_skp = nullptr, *p_th = nullptr, *p_cnt = nullptr,
-         *p_off = nullptr, *p_pkp = nullptr, *p_pth = nullptr, *p_desc = nullptr, *p_valid = nullptr,
-         *p_osel = nullptr;
-    if (nkp > 0 && cap > 0) {
+    // the quick path's answer stands when it filled the cap, or when it took
+    // every keypoint and described every pair of them
+    const bool all_taken = hc.kept == hc.kp && nkp <= want && (int64_t)hc.pairs <= cap;
+    const bool done_quick = quick && hc.kept <= (uint32_t)SEL_CAP && ((int64_t)hc.valid == cap || all_taken);
+    if (done_quick) {
+        n_valid = hc.valid;
+    } else if (nkp > 0 && cap > 0) {
+        // The general path: all keypoints by (response descending, place), then
+        // orientations, pairs and descriptors in that order until max_features
+        // valid descriptors exist (a descriptor that normalises to nothing is
+        // dropped, as in the reference).
+        thrust::counting_iterator<uint32_t> it(0);
+        void *p_temp, *p_off, *p_kidx, *p_place2, *p_kidx2, *p_r1, *p_r2, *p_nsel;
+        int64_t kdone = 0, np = 0, done = 0;
+        SCK(A.get(F_NSEL, sizeof(int) * 4, &p_nsel));
         SCK(A.get(F_PIDX, sizeof(uint32_t) * (size_t)nkp, &p_kidx));
-        SCK(A.get(F_SRESP, sizeof(double) * (size_t)nkp, &p_sresp));
-        SCK(A.get(F_SIDX, sizeof(uint32_t) * (size_t)nkp, &p_skp));
+        SCK(A.get(F_PLACE2, sizeof(uint32_t) * (size_t)nkp, &p_place2));
+        SCK(A.get(F_PIDX2, sizeof(uint32_t) * (size_t)nkp, &p_kidx2));
+        SCK(A.get(F_SRESP, sizeof(double) * (size_t)nkp, &p_r1));
+        SCK(A.get(F_SRESP2, sizeof(double) * (size_t)nkp, &p_r2));
+        SCK(A.get(F_SIDX, sizeof(uint32_t) * (size_t)std::max<int64_t>(nkp, SEL_CAP), &p_skp));
         SCK(A.get(F_THETA, sizeof(double) * 4 * (size_t)nkp, &p_th));
         SCK(A.get(F_CNT, sizeof(int32_t) * (size_t)nkp, &p_cnt));
         SCK(A.get(F_OFF, sizeof(int32_t) * (size_t)nkp, &p_off));
@@ -808,66 +1012,67 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
         SCK(A.get(F_OSEL, sizeof(uint32_t) * 4 * (size_t)nkp, &p_osel));
         iota_kernel<<<grid_of(nkp), 256, 0, st>>>((uint32_t*)p_kidx, nkp);
         SCK(cudaGetLastError());
-        size_t tb = 0;
-        SCK(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, (const double*)kp.resp, (double*)p_sresp,
-                                                      (const uint32_t*)p_kidx, (uint32_t*)p_skp, (int)nkp, 0, 64,
-                                                      st));
-        SCK(A.get(F_TEMP, tb, &p_temp));
-        SCK(cub::DeviceRadixSort::SortPairsDescending(p_temp, tb, (const double*)kp.resp, (double*)p_sresp,
-                                                      (const uint32_t*)p_kidx, (uint32_t*)p_skp, (int)nkp, 0, 64,
-                                                      st));
-    }
-    while (n_valid < cap && (done < np || kdone < nkp)) {
-        if (done == np) {
-            // orientations of the next keypoints in response order, and their pairs
-            const int64_t ck = std::min<int64_t>(nkp - kdone, std::max<int64_t>(cap - n_valid, 64));
-            hook.begin("sift_orient");
-            orient_kernel<<<(unsigned)((ck + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
-                kp, (const uint32_t*)p_skp, kdone, (int)ck, table, w, h, (double*)p_th, (int32_t*)p_cnt);
-            SCK(cudaGetLastError());
-            hook.end("sift_orient");
-            size_t tb = 0;
-            SCK(cub::DeviceScan::ExclusiveSum(nullptr, tb, (const int32_t*)p_cnt + kdone, (int32_t*)p_off, (int)ck,
-                                              st));
-            SCK(A.get(F_TEMP, tb, &p_temp));
-            SCK(cub::DeviceScan::ExclusiveSum(p_temp, tb, (const int32_t*)p_cnt + kdone, (int32_t*)p_off, (int)ck,
-                                              st));
-            pairs_kernel<<<grid_of(ck), 256, 0, st>>>((const uint32_t*)p_skp, kdone, (int)ck, (const int32_t*)p_cnt,
-                                                      (const int32_t*)p_off, (const double*)p_th, np,
-                                                      (int32_t*)p_pkp, (double*)p_pth);
-            SCK(cudaGetLastError());
-            int last_off = 0, last_cnt = 0;
-            SCK(cudaMemcpyAsync(&last_off, (int32_t*)p_off + ck - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-            SCK(cudaMemcpyAsync(&last_cnt, (int32_t*)p_cnt + kdone + ck - 1, sizeof(int), cudaMemcpyDeviceToHost,
-                                st));
-            SCK(cudaStreamSynchronize(st));
-            kdone += ck;
-            np += (int64_t)last_off + last_cnt;
-            continue;
-        }
-        const int64_t chunk = std::min<int64_t>(np - done, std::max<int64_t>(cap - n_valid, 32));
-        void* p_d;
-        if ((rc = grow_copy(ctx, F_DESC, sizeof(float) * DESC_LEN * (size_t)(done + chunk),
-                            sizeof(float) * DESC_LEN * (size_t)done, &p_d)))
-            return rc;
-        p_desc = p_d;
-        hook.begin("sift_desc");
-        desc_kernel<<<(unsigned)((chunk + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
-            kp, done, (int)chunk, (const int32_t*)p_pkp, (const double*)p_pth, table, (float*)p_desc,
-            (uint8_t*)p_valid);
+        size_t tb1 = 0, tb2 = 0;
+        SCK(cub::DeviceRadixSort::SortPairs(nullptr, tb1, (const uint32_t*)kp.place, (uint32_t*)p_place2,
+                                            (const uint32_t*)p_kidx, (uint32_t*)p_kidx2, (int)nkp, 0, 32, st));
+        SCK(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb2, (const double*)p_r1, (double*)p_r2,
+                                                      (const uint32_t*)p_kidx2, (uint32_t*)p_skp, (int)nkp, 0, 64, st));
+        SCK(A.get(F_TEMP, std::max(tb1, tb2), &p_temp));
+        SCK(cub::DeviceRadixSort::SortPairs(p_temp, tb1, (const uint32_t*)kp.place, (uint32_t*)p_place2,
+                                            (const uint32_t*)p_kidx, (uint32_t*)p_kidx2, (int)nkp, 0, 32, st));
+        gather_resp_kernel<<<grid_of(nkp), 256, 0, st>>>(kp.resp, (const uint32_t*)p_kidx2, nkp, (double*)p_r1);
         SCK(cudaGetLastError());
-        hook.end("sift_desc");
-        done += chunk;
-        size_t tb = 0;
-        SCK(cub::DeviceSelect::Flagged(nullptr, tb, it, (const uint8_t*)p_valid, (uint32_t*)p_osel,
-                                       (int*)p_nsel + 1, (int)done, st));
-        SCK(A.get(F_TEMP, tb, &p_temp));
-        SCK(cub::DeviceSelect::Flagged(p_temp, tb, it, (const uint8_t*)p_valid, (uint32_t*)p_osel,
-                                       (int*)p_nsel + 1, (int)done, st));
-        int nv = 0;
-        SCK(cudaMemcpyAsync(&nv, (int*)p_nsel + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        SCK(cudaStreamSynchronize(st));
-        n_valid = nv;
+        SCK(cub::DeviceRadixSort::SortPairsDescending(p_temp, tb2, (const double*)p_r1, (double*)p_r2,
+                                                      (const uint32_t*)p_kidx2, (uint32_t*)p_skp, (int)nkp, 0, 64, st));
+        while (n_valid < cap && (done < np || kdone < nkp)) {
+            if (done == np) {
+                // orientations of the next keypoints in response order, and their pairs
+                const int64_t ck = std::min<int64_t>(nkp - kdone, std::max<int64_t>(cap - n_valid, 64));
+                hook.begin("sift_orient");
+                orient_kernel<<<(unsigned)((ck + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
+                    kp, (const uint32_t*)p_skp, kdone, (int)ck, nullptr, table, w, h, (double*)p_th, (int32_t*)p_cnt);
+                SCK(cudaGetLastError());
+                hook.end("sift_orient");
+                size_t tb = 0;
+                SCK(cub::DeviceScan::ExclusiveSum(nullptr, tb, (const int32_t*)p_cnt + kdone, (int32_t*)p_off, (int)ck,
+                                                  st));
+                SCK(A.get(F_TEMP, tb, &p_temp));
+                SCK(cub::DeviceScan::ExclusiveSum(p_temp, tb, (const int32_t*)p_cnt + kdone, (int32_t*)p_off, (int)ck,
+                                                  st));
+                pairs_kernel<<<grid_of(ck), 256, 0, st>>>((const uint32_t*)p_skp, kdone, (int)ck, (const int32_t*)p_cnt,
+                                                          (const int32_t*)p_off, (const double*)p_th, np,
+                                                          (int32_t*)p_pkp, (double*)p_pth);
+                SCK(cudaGetLastError());
+                int last_off = 0, last_cnt = 0;
+                SCK(cudaMemcpyAsync(&last_off, (int32_t*)p_off + ck - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+                SCK(cudaMemcpyAsync(&last_cnt, (int32_t*)p_cnt + kdone + ck - 1, sizeof(int), cudaMemcpyDeviceToHost,
+                                    st));
+                SCK(cudaStreamSynchronize(st));
+                kdone += ck;
+                np += (int64_t)last_off + last_cnt;
+                continue;
+            }
+            const int64_t chunk = std::min<int64_t>(np - done, std::max<int64_t>(cap - n_valid, 32));
+            if ((rc = grow_copy(ctx, F_DESC, sizeof(float) * DESC_LEN * (size_t)(done + chunk),
+                                sizeof(float) * DESC_LEN * (size_t)done, &p_desc)))
+                return rc;
+            hook.begin("sift_desc");
+            desc_kernel<<<(unsigned)chunk, DESC_LEN, 0, st>>>(kp, done, (const int32_t*)p_pkp, (const double*)p_pth,
+                                                              nullptr, table, (float*)p_desc, (uint8_t*)p_valid);
+            SCK(cudaGetLastError());
+            hook.end("sift_desc");
+            done += chunk;
+            size_t tb = 0;
+            SCK(cub::DeviceSelect::Flagged(nullptr, tb, it, (const uint8_t*)p_valid, (uint32_t*)p_osel, (int*)p_nsel,
+                                           (int)done, st));
+            SCK(A.get(F_TEMP, tb, &p_temp));
+            SCK(cub::DeviceSelect::Flagged(p_temp, tb, it, (const uint8_t*)p_valid, (uint32_t*)p_osel, (int*)p_nsel,
+                                           (int)done, st));
+            int nv = 0;
+            SCK(cudaMemcpyAsync(&nv, (int*)p_nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
+            SCK(cudaStreamSynchronize(st));
+            n_valid = nv;
+        }
     }
 
     // sift.rs:543-544: the first max_features
@@ -884,14 +1089,15 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
         return sfail(ctx, RCMVS_E_NOMEM, "sift: host allocation failed");
     }
     if (n_out == 0) return RCMVS_OK;
-    void *p_pts, *p_fdesc, *p_col;
-    SCK(A.get(F_PTS, sizeof(double) * 2 * n_out, &p_pts));
-    SCK(A.get(F_FDESC, sizeof(float) * DESC_LEN * n_out, &p_fdesc));
-    SCK(A.get(F_COL, 3 * (size_t)n_out, &p_col));
-    final_kernel<<<(int)((n_out + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
-        (const uint32_t*)p_osel, (int)n_out, (const int32_t*)p_pkp, kp, table,
-        (const float*)p_desc, (const uint8_t*)p_rgb, w, h, (double*)p_pts, (float*)p_fdesc, (uint8_t*)p_col);
-    SCK(cudaGetLastError());
+    if (!done_quick) {
+        SCK(A.get(F_PTS, sizeof(double) * 2 * n_out, &p_pts));
+        SCK(A.get(F_FDESC, sizeof(float) * DESC_LEN * n_out, &p_fdesc));
+        SCK(A.get(F_COL, 3 * (size_t)n_out, &p_col));
+        final_kernel<<<(int)((n_out + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
+            (const uint32_t*)p_osel, (int)n_out, nullptr, (const int32_t*)p_pkp, kp, table, (const float*)p_desc,
+            (const uint8_t*)p_rgb, w, h, (double*)p_pts, (float*)p_fdesc, (uint8_t*)p_col);
+        SCK(cudaGetLastError());
+    }
     SCK(cudaMemcpyAsync(out->pts, p_pts, sizeof(double) * 2 * n_out, cudaMemcpyDeviceToHost, st));
     SCK(cudaMemcpyAsync(out->desc, p_fdesc, sizeof(float) * DESC_LEN * n_out, cudaMemcpyDeviceToHost, st));
     SCK(cudaMemcpyAsync(out->colors, p_col, 3 * (size_t)n_out, cudaMemcpyDeviceToHost, st));
