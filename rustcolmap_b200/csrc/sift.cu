@@ -125,10 +125,21 @@ __device__ __forceinline__ void blur_tile(BlurSmem<R>& sm, int x0, int y0, int w
                                           Store store) {
     using S = BlurSmem<R>;
     const int tid = threadIdx.x;
-    for (int i = tid; i < S::IN_H * S::IN_W; i += BLUR_THREADS) {
-        const int ix = i % S::IN_W, iy = i / S::IN_W;
-        const int gx = min(max(x0 - R + ix, 0), w - 1), gy = min(max(y0 - R + iy, 0), h - 1);
-        sm.in[iy * S::IN_P + ix] = load((int64_t)gy * w + gx);
+    // a warp per row; all of a thread's loads are in flight together
+    {
+        constexpr int ROWS = (S::IN_H + BLUR_THREADS / 32 - 1) / (BLUR_THREADS / 32), COLS = (S::IN_W + 31) / 32;
+        const int lane = tid & 31;
+        int gx[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) gx[c] = min(max(x0 - R + lane + 32 * c, 0), w - 1);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const int iy = (tid >> 5) + r * (BLUR_THREADS / 32);
+            const int64_t row = (int64_t)min(max(y0 - R + iy, 0), h - 1) * w;
+#pragma unroll
+            for (int c = 0; c < COLS; ++c)
+                if (iy < S::IN_H && lane + 32 * c < S::IN_W) sm.in[iy * S::IN_P + lane + 32 * c] = load(row + gx[c]);
+        }
     }
     __syncthreads();
     // horizontal: lanes on different rows (odd pitches: no bank conflicts)
@@ -207,7 +218,8 @@ __device__ __forceinline__ bool inverse3(const double m[9], double o[9]) {
 // the DoGs above and below being zero) and their part of the next octave's
 // level 0 (sift.rs:95-110; next may be null).  1600x1200, six octaves: five blurs
 // each, DoGs, extrema over three levels, gradients and their selections took
-// 124 launches and 590 us; 150 us here with the base.
+// 124 launches and 590 us; 78 us here with the base (the fits in a second
+// pass over the tile's candidates; 150 us with them in the first).
 __global__ void __launch_bounds__(BLUR_THREADS) octave_kernel(const float* __restrict__ lev0, int w, int h,
                                                               const __grid_constant__ BlurTaps taps, double thr,
                                                               float* __restrict__ next, int nw, int nh, int octave,
@@ -215,6 +227,10 @@ __global__ void __launch_bounds__(BLUR_THREADS) octave_kernel(const float* __res
     __shared__ BlurSmem<R_LEVEL> sm;
     __shared__ float lev3[BY][BX];
     __shared__ float dog[BY][BX + 1];
+    // strict extrema: at most one maximum and one minimum in any 2 x 2 pixels
+    __shared__ uint16_t cand[2 * (BX / 2 - 1) * (BY / 2 - 1)];
+    __shared__ int n_cand;
+    if (threadIdx.x == 0) n_cand = 0;
     const int tiles_x = (w + BX - 3) / (BX - 2);
     const int x0 = (int)(blockIdx.x % tiles_x) * (BX - 2);  // the first inner pixel
     const int y0 = (int)(blockIdx.x / tiles_x) * (BY - 2);
@@ -243,7 +259,14 @@ __global__ void __launch_bounds__(BLUR_THREADS) octave_kernel(const float* __res
                 if (n >= v) is_max = false;
                 if (n <= v) is_min = false;
             }
-        if (!is_max && !is_min) continue;
+        if (is_max || is_min) cand[atomicAdd(&n_cand, 1)] = (uint16_t)(cy * BX + cx);
+    }
+    __syncthreads();
+    // the fits, of all candidates at once: one f64 chain per block, not per warp
+    for (int i = threadIdx.x; i < n_cand; i += BLUR_THREADS) {
+        const int cx = cand[i] % BX, cy = cand[i] / BX;
+        const int x = x0 + cx - 1, y = y0 + cy - 1;
+        const float v = dog[cy][cx];
         auto d = [&](int dx, int dy) { return dog[cy + dy][cx + dx]; };
         const float zero = 0.0f;
         const float fdx = 0.5f * (d(1, 0) - d(-1, 0));
@@ -289,6 +312,11 @@ __global__ void __launch_bounds__(BLUR_THREADS) octave_kernel(const float* __res
 
 // ---- selection of the first `want` keypoints by (response descending, place)
 constexpr int SEL_BINS = 2048, SEL_CAP = 16384;
+struct Kept {  // SEL_CAP entries each
+    long long* key;
+    uint32_t* place;
+    uint32_t* kp;
+};
 
 // A response's order: it is never negative, so its bits are ordered as it is.
 __device__ __forceinline__ long long resp_key(double r) { return __double_as_longlong(r); }
@@ -314,7 +342,8 @@ __global__ void __launch_bounds__(256) hist_kernel(const double* __restrict__ re
 // The keypoints whose bin is at least the highest one with `want` keypoints
 // at or above it.
 __global__ void __launch_bounds__(256) keep_kernel(const double* __restrict__ resp, const uint32_t* __restrict__ hist,
-                                                   uint32_t want, Counts* __restrict__ counts, uint32_t* __restrict__ kept) {
+                                                   const uint32_t* __restrict__ place, uint32_t want,
+                                                   Counts* __restrict__ counts, Kept kept) {
     __shared__ uint32_t s_sum[256];
     __shared__ int s_bin;
     constexpr int PER = SEL_BINS / 256;
@@ -351,52 +380,61 @@ __global__ void __launch_bounds__(256) keep_kernel(const double* __restrict__ re
     for (uint32_t k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
         if (resp_bin(resp[k]) >= bin) {
             const uint32_t at = atomicAdd(&counts->kept, 1u);
-            if (at < SEL_CAP) kept[at] = k;
+            if (at < SEL_CAP) {
+                kept.key[at] = resp_key(resp[k]);
+                kept.place[at] = place[k];
+                kept.kp[at] = k;
+            }
         }
 }
 
 // Rank of each kept keypoint by counting; skp[rank] = keypoint.  One warp each.
-__global__ void __launch_bounds__(256) rank_kernel(const KpArrays kp, const uint32_t* __restrict__ kept,
-                                                   const Counts* __restrict__ counts, uint32_t* __restrict__ skp) {
+__global__ void __launch_bounds__(256) rank_kernel(const Kept kept, const Counts* __restrict__ counts,
+                                                   uint32_t* __restrict__ skp) {
     const uint32_t n = counts->kept;
     if (n > SEL_CAP) return;
     const int lane = threadIdx.x & 31;
     for (uint32_t i = (blockIdx.x * 256 + threadIdx.x) >> 5; i < n; i += gridDim.x * 8) {
-        const uint32_t k = kept[i], place = kp.place[k];
-        const long long r = resp_key(kp.resp[k]);
+        const uint32_t place = kept.place[i];
+        const long long key = kept.key[i];
         uint32_t before = 0;
+#pragma unroll 8
         for (uint32_t j = lane; j < n; j += 32) {
-            const uint32_t o = kept[j];
-            const long long q = resp_key(kp.resp[o]);
-            before += q > r || (q == r && kp.place[o] < place);
+            const long long q = __ldg(kept.key + j);
+            const uint32_t qp = __ldg(kept.place + j);
+            before += q > key || (q == key && qp < place);
         }
         for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-        if (lane == 0) skp[before] = k;
+        if (lane == 0) skp[before] = kept.kp[i];
     }
 }
 
 __device__ __forceinline__ double rem_euclid(double a, double b) {
-    const double r = fmod(a, b);
+    // fmod(a, b), b > 0: below 2 b in magnitude the subtraction is exact
+    const double m = fabs(a);
+    const double r = m < b ? a : m < 2.0 * b ? copysign(m - b, a) : fmod(a, b);
     return r < 0.0 ? r + fabs(b) : r;
 }
 
-// sift.rs:274-334.  One warp per keypoint, for the keypoints at sorted
-// positions base .. base + n - 1 (skp[pos] = keypoint), or with `counts` as many
-// of them as were kept; theta[4 pos ..] and cnt[pos] (0 when the keypoint is
-// outside the 8-pixel margin of the image, sift.rs:519-521, or there is none).
-__global__ void __launch_bounds__(32 * WARPS) orient_kernel(KpArrays kp, const uint32_t* __restrict__ skp,
-                                                           int64_t base, int n, const Counts* __restrict__ counts,
-                                                           const __grid_constant__ OctTable oct, int img_w, int img_h,
-                                                           double* __restrict__ theta, int32_t* __restrict__ cnt) {
-    __shared__ int sbin[WARPS][32];
-    __shared__ double sval[WARPS][32];
-    __shared__ double shist[WARPS][2][36];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * WARPS + wid;
-    if (i >= n) return;
-    const int64_t k = base + i;  // output position
-    if (counts && (counts->kept > SEL_CAP || (uint32_t)i >= counts->kept)) {
-        if (lane == 0) cnt[k] = 0;
+// sift.rs:274-334.  One block per keypoint, for the keypoints at sorted
+// positions base .. base + gridDim.x - 1 (skp[pos] = keypoint), or with `counts`
+// as many of them as were kept; theta[4 pos ..] and cnt[pos] (0 when the keypoint
+// is outside the 8-pixel margin of the image, sift.rs:519-521, or there is none).
+// Bound by the latency of a sample's f64 chain (atan2, exp): five warps take
+// the window in two rounds where one warp took ten.  2432 keypoints: 37 -> 29 us.
+constexpr int ORI_BINS = 36, ORI_RADIUS = 8, ORI_SIDE = 2 * ORI_RADIUS + 1, ORI_SAMPLES = ORI_SIDE * ORI_SIDE;
+constexpr int ORI_THREADS = 160;
+__global__ void __launch_bounds__(ORI_THREADS) orient_kernel(KpArrays kp, const uint32_t* __restrict__ skp, int64_t base,
+                                                             const Counts* __restrict__ counts,
+                                                             const __grid_constant__ OctTable oct, int img_w, int img_h,
+                                                             double* __restrict__ theta, int32_t* __restrict__ cnt) {
+    __shared__ int sbin[ORI_SAMPLES];
+    __shared__ double sval[ORI_SAMPLES];
+    __shared__ double shist[2][ORI_BINS];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t k = base + blockIdx.x;  // output position
+    if (counts && (counts->kept > SEL_CAP || blockIdx.x >= counts->kept)) {
+        if (tid == 0) cnt[k] = 0;
         return;
     }
     const uint32_t kk = skp[k];
@@ -405,60 +443,54 @@ __global__ void __launch_bounds__(32 * WARPS) orient_kernel(KpArrays kp, const u
     const double scale = oct.scale[o];
     const double x0 = kx * scale, y0 = ky * scale;
     if (x0 < 8.0 || y0 < 8.0 || x0 >= (double)img_w - 8.0 || y0 >= (double)img_h - 8.0) {
-        if (lane == 0) cnt[k] = 0;
+        if (tid == 0) cnt[k] = 0;
         return;
     }
     const int w = oct.w[o], h = oct.h[o];
     const float* img = oct.img[o];
-    const double sigma = 1.5 * level_sigma(KP_LEVEL);
-    const int radius = (int)fmax(ceil(3.0 * sigma), 1.0);
+    const double sigma = 1.5 * level_sigma(KP_LEVEL);  // 2.4: a radius of ceil(3 sigma) = ORI_RADIUS
     const double s2 = 2.0 * sigma * sigma;
     const long long xr = (long long)round(kx), yr = (long long)round(ky);
-    const int side = 2 * radius + 1, total = side * side;
-    const int b0 = lane, b1 = lane + 32;
-    double acc0 = 0.0, acc1 = 0.0;
-    for (int base = 0; base < total; base += 32) {
-        const int s = base + lane;
+    for (int s = tid; s < ORI_SAMPLES; s += ORI_THREADS) {
         int bin = -1;
         double val = 0.0;
-        if (s < total) {
-            const int dy = s / side - radius, dx = s % side - radius;
-            const long long sx = xr + dx, sy = yr + dy;
-            if (!(sx < 1 || sy < 1 || sx >= w - 1 || sy >= h - 1)) {
-                const int64_t i = sy * w + sx;
-                const float a = img[i + 1] - img[i - 1], b = img[i + w] - img[i - w];  // sift.rs:137-149
-                const double mag = sqrt((double)(a * a + b * b));
-                const double ang = atan2((double)b, (double)a);
-                const double wgt = exp((-((double)dx * (double)dx) - (double)dy * (double)dy) / s2);
-                const double fb = floor((ang + PI) / (2.0 * PI) * 36.0);
-                bin = !(fb > 0.0) ? 0 : (int)((long long)fb % 36);
-                val = wgt * mag;
-            }
+        const int dy = s / ORI_SIDE - ORI_RADIUS, dx = s % ORI_SIDE - ORI_RADIUS;
+        const long long sx = xr + dx, sy = yr + dy;
+        if (!(sx < 1 || sy < 1 || sx >= w - 1 || sy >= h - 1)) {
+            const int64_t i = sy * w + sx;
+            const float a = img[i + 1] - img[i - 1], b = img[i + w] - img[i - w];  // sift.rs:137-149
+            const double mag = sqrt((double)(a * a + b * b));
+            const double ang = atan2((double)b, (double)a);
+            const double wgt = exp((-((double)dx * (double)dx) - (double)dy * (double)dy) / s2);
+            const double fb = floor((ang + PI) / (2.0 * PI) * 36.0);
+            bin = !(fb > 0.0) ? 0 : (int)((long long)fb % 36);
+            val = wgt * mag;
         }
-        sbin[wid][lane] = bin;
-        sval[wid][lane] = val;
-        __syncwarp();
-        const int m = min(32, total - base);
-        for (int t = 0; t < m; ++t) {
-            const int b = sbin[wid][t];
-            if (b == b0)
-                acc0 += sval[wid][t];
-            else if (b == b1)
-                acc1 += sval[wid][t];
-        }
-        __syncwarp();
+        sbin[s] = bin;
+        sval[s] = val;
     }
-    // two smoothings (every lane its bins), then the peaks in bin order
-    shist[wid][0][b0] = acc0;
-    if (b1 < 36) shist[wid][0][b1] = acc1;
-    __syncwarp();
+    __syncthreads();
+    // thread b's bin: its samples in window order
+    if (tid < ORI_BINS) {
+        double acc = 0.0;
+#pragma unroll 17
+        for (int t = 0; t < ORI_SAMPLES; ++t) {
+            const double v = sval[t];
+            if (sbin[t] == tid) acc += v;
+        }
+        shist[0][tid] = acc;
+    }
+    __syncthreads();
     for (int it = 0; it < 2; ++it) {
-        const double* hist = shist[wid][it];
-        double* sm = shist[wid][it ^ 1];
-        for (int b = lane; b < 36; b += 32) sm[b] = (hist[(b + 35) % 36] + 2.0 * hist[b] + hist[(b + 1) % 36]) / 4.0;
-        __syncwarp();
+        const double* from = shist[it];
+        if (tid < ORI_BINS)
+            shist[it ^ 1][tid] = (from[(tid + 35) % 36] + 2.0 * from[tid] + from[(tid + 1) % 36]) / 4.0;
+        __syncthreads();
     }
-    const double* hist = shist[wid][0];
+    if (tid >= 32) return;
+    // the peaks, in bin order
+    const int b0 = lane, b1 = lane + 32;
+    const double* hist = shist[0];
     double maxv = fmax(hist[b0], b1 < 36 ? hist[b1] : 0.0);
     for (int o = 16; o > 0; o >>= 1) maxv = fmax(maxv, __shfl_xor_sync(0xffffffffu, maxv, o));
     maxv = fmax(0.0, maxv);
@@ -561,18 +593,35 @@ __global__ void iota_kernel(uint32_t* __restrict__ out, int64_t n) {
 // sift.rs:340-431.  One block per (keypoint, peak) pair, for the pairs
 // base .. base + gridDim.x - 1 (in output order), or with `counts` those of
 // them that exist; descriptor and validity stored at the pair's index.  Bound
-// by the samples' f64 functions: 2048 descriptors 187 us.
-constexpr int DESC_RADIUS_MAX = 15, DESC_SAMPLES = (2 * DESC_RADIUS_MAX + 1) * (2 * DESC_RADIUS_MAX + 1);
-__global__ void __launch_bounds__(DESC_LEN) desc_kernel(KpArrays kp, int64_t base, const int32_t* __restrict__ pair_kp,
-                                                       const double* __restrict__ pair_theta,
-                                                       const Counts* __restrict__ counts,
-                                                       const __grid_constant__ OctTable oct, float* __restrict__ desc,
-                                                       uint8_t* __restrict__ valid) {
-    constexpr int D = 4, N = 8;
-    __shared__ uint16_t hdr[DESC_SAMPLES + 31];  // packed (by0 + 2, bx0 + 2, ob0 mod 8), or 0xFFFF
-    __shared__ double s_w[DESC_SAMPLES], s_fx[DESC_SAMPLES], s_fy[DESC_SAMPLES], s_fo[DESC_SAMPLES];
-    __shared__ float sd[DESC_LEN];
-    __shared__ float s_norm;
+// by the samples' f64 functions, so the samples of the rotated window (three
+// fifths of the square) are first packed, by an approximate test with a margin,
+// and each cell walks a list of its own samples (about 90).  2048 descriptors:
+// 187 us without the two, 73 us.
+//
+// Lattice points in a square of side s number at most (s + sqrt 2)^2 (their
+// unit squares are disjoint and lie within sqrt(1/2) of it): 645 in the window,
+// of 5 cells' side, and 121 that touch one cell, in 2 cells' side.
+constexpr int DESC_RADIUS = 15, DESC_SIDE = 2 * DESC_RADIUS + 1, DESC_SAMPLES = DESC_SIDE * DESC_SIDE;
+constexpr int DESC_HITS = 648, CELL_HITS = 124;
+struct DescSmem {
+    double w[DESC_HITS], fx[DESC_HITS], fy[DESC_HITS], fo[DESC_HITS];
+    uint16_t hdr[DESC_HITS + 32];  // (by0 + 2, bx0 + 2, ob0 mod 8) of 4 bits each, or 0xFFFF
+    union {
+        uint16_t cand[DESC_HITS];         // the samples of the window, in order
+        uint16_t cell[16][CELL_HITS];     // a cell's: index, ob0 << 10, upper column << 13, upper row << 14
+    };
+    float sq[DESC_LEN];
+    double cos_t, sin_t;
+    float norm;
+    int count[4];
+};
+__global__ void __launch_bounds__(DESC_LEN, 8) desc_kernel(KpArrays kp, int64_t base, const int32_t* __restrict__ pair_kp,
+                                                          const double* __restrict__ pair_theta,
+                                                          const Counts* __restrict__ counts,
+                                                          const __grid_constant__ OctTable oct, float* __restrict__ desc,
+                                                          uint8_t* __restrict__ valid) {
+    constexpr int D = 4, N = 8, ROUNDS = (DESC_SAMPLES + DESC_LEN - 1) / DESC_LEN;
+    __shared__ DescSmem sm;
     const int64_t pos = base + blockIdx.x;
     if (counts && pos >= (int64_t)counts->pairs) return;
     const int k = pair_kp[pos];
@@ -580,26 +629,56 @@ __global__ void __launch_bounds__(DESC_LEN) desc_kernel(KpArrays kp, int64_t bas
     const int o = kp.oct[k];
     const int w = oct.w[o], h = oct.h[o];
     const float* img = oct.img[o];
-    const double sigma = level_sigma(KP_LEVEL);
-    const double cell = 3.0 * sigma;
-    const int radius = (int)ceil(sqrt(1.5) * cell * ((double)D + 1.0) * 0.5);  // DESC_RADIUS_MAX
-    const double cos_t = cos(th), sin_t = sin(th);
-    const double exp_scale = -1.0 / ((double)(D * D) * 0.5);
+    // 4.8: a radius of ceil(sqrt(1.5) cell (D + 1) / 2) = DESC_RADIUS
+    const double cell = 3.0 * level_sigma(KP_LEVEL);
     const double half = (double)D * 0.5;
-    const int side = 2 * radius + 1, total = side * side;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int s = tid; s < total + 31; s += DESC_LEN) {
+    if (wid == 0) sm.cos_t = cos(th);
+    if (wid == 1) sm.sin_t = sin(th);
+    __syncthreads();
+    const double cos_t = sm.cos_t, sin_t = sm.sin_t;
+    {
+        // warp w: samples [32 ROUNDS w, 32 ROUNDS (w + 1))
+        const double inv = 1.0 / cell, lo = -1.0 - 1e-6, hi = (double)D + 1e-6;
+        unsigned m[ROUNDS];
+        int n = 0;
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const int s = (wid * ROUNDS + r) * 32 + lane;
+            const int dy = s / DESC_SIDE - DESC_RADIUS, dx = s % DESC_SIDE - DESC_RADIUS;
+            const double sx = x + (double)dx, sy = y + (double)dy;
+            const double bx = (cos_t * (double)dx + sin_t * (double)dy) * inv + half - 0.5;
+            const double by = (-sin_t * (double)dx + cos_t * (double)dy) * inv + half - 0.5;
+            m[r] = __ballot_sync(0xffffffffu, s < DESC_SAMPLES && !(sx < 1.0 || sy < 1.0 || sx >= (double)w - 2.0 ||
+                                                                   sy >= (double)h - 2.0) &&
+                                                  bx >= lo && by >= lo && bx <= hi && by <= hi);
+            n += __popc(m[r]);
+        }
+        if (lane == 0) sm.count[wid] = n;
+        __syncthreads();
+        int at = 0;
+        for (int i = 0; i < wid; ++i) at += sm.count[i];
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            if ((m[r] >> lane) & 1u) sm.cand[at + __popc(m[r] & ((1u << lane) - 1u))] = (uint16_t)((wid * ROUNDS + r) * 32 + lane);
+            at += __popc(m[r]);
+        }
+    }
+    const int n = sm.count[0] + sm.count[1] + sm.count[2] + sm.count[3];
+    __syncthreads();
+    const double exp_scale = -1.0 / ((double)(D * D) * 0.5);
+    for (int i = tid; i < n + 32; i += DESC_LEN) {
         int hd = 0xFFFF;
-        const int dy = s / side - radius, dx = s % side - radius;
-        const double sx = x + (double)dx, sy = y + (double)dy;
+        const int s = i < n ? sm.cand[i] : 0;
+        const int dy = s / DESC_SIDE - DESC_RADIUS, dx = s % DESC_SIDE - DESC_RADIUS;
         const double rx = cos_t * (double)dx + sin_t * (double)dy;
         const double ry = -sin_t * (double)dx + cos_t * (double)dy;
         const double bx = rx / cell + half - 0.5;
         const double by = ry / cell + half - 0.5;
-        if (s < total && !(sx < 1.0 || sy < 1.0 || sx >= (double)w - 2.0 || sy >= (double)h - 2.0) &&
-            !(bx < -1.0 || by < -1.0 || bx > (double)D || by > (double)D)) {
+        if (i < n && !(bx < -1.0 || by < -1.0 || bx > (double)D || by > (double)D)) {
             // sift.rs:137-166: bilinear gradients; 1 <= x0, x0 + 1 <= w - 2, so no
             // clamp applies and every gradient is a central difference
+            const double sx = x + (double)dx, sy = y + (double)dy;
             const int x0 = (int)floor(sx), y0 = (int)floor(sy);
             const float fx = (float)(sx - (double)x0), fy = (float)(sy - (double)y0);
             const float* p = img + (int64_t)y0 * w + x0;
@@ -618,60 +697,72 @@ __global__ void __launch_bounds__(DESC_LEN) desc_kernel(KpArrays kp, int64_t bas
                 wgt = exp(wgt) * mag;
                 // bx, by in [-1, 4], ob in [0, 8]
                 const int bx0 = (int)floor(bx), by0 = (int)floor(by), ob0 = (int)floor(ob);
-                s_w[s] = wgt;
-                s_fx[s] = bx - (double)bx0;
-                s_fy[s] = by - (double)by0;
-                s_fo[s] = ob - (double)ob0;
+                sm.w[i] = wgt;
+                sm.fx[i] = bx - (double)bx0;
+                sm.fy[i] = by - (double)by0;
+                sm.fo[i] = ob - (double)ob0;
                 hd = ((by0 + 2) << 8) | ((bx0 + 2) << 4) | (ob0 & 7);
             }
         }
-        hdr[s] = (uint16_t)hd;
+        sm.hdr[i] = (uint16_t)hd;
     }
     __syncthreads();
-    // Thread t owns bin t: cell row q = its warp, cell column lane / 8,
-    // orientation lane % 8.  A sample adds to such a bin at most once; the warp
-    // visits only the samples that touch its row.
+    // Warp q makes the lists of cell row q.
     const int cx = lane >> 3, co = lane & 7, q = wid;
+    int hits = 0;  // of this lane's cell
+    {
+        int at[4] = {0, 0, 0, 0};
+        for (int b = 0; b < n; b += 32) {
+            const int hv = sm.hdr[b + lane];
+            const int row = q + 2 - (hv >> 8), col = ((hv >> 4) & 15) - 2;  // row 0xFFFF: negative
+            const int e = (b + lane) | (hv & 7) << 10 | row << 14;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const bool mine = (unsigned)row <= 1u && (unsigned)(c - col) <= 1u;
+                const unsigned m = __ballot_sync(0xffffffffu, mine);
+                if (mine) sm.cell[4 * q + c][at[c] + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(e | (c - col) << 13);
+                at[c] += __popc(m);
+            }
+        }
+        hits = cx == 0 ? at[0] : cx == 1 ? at[1] : cx == 2 ? at[2] : at[3];
+    }
+    __syncwarp();
+    // Thread t owns bin t: cell row q, cell column lane / 8, orientation lane % 8.
+    // A sample adds to a bin at most once, in window order.
     double acc = 0.0;
-    for (int b = 0; b < total; b += 32) {
-        const int mine = hdr[b + lane];
-        const int myrow = (mine >> 8) - 2;  // 0xFFFF: 253
-        unsigned todo = __ballot_sync(0xffffffffu, myrow == q || myrow == q - 1);
-        while (todo) {
-            const int t = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int hv = __shfl_sync(0xffffffffu, mine, t);
-            const int ix = cx - (((hv >> 4) & 15) - 2);
-            const int io = (co - (hv & 7)) & 7;
-            if ((unsigned)ix > 1u || io > 1) continue;
-            const int s = b + t;
-            const bool low = q == (hv >> 8) - 2;
-            const double wy = low ? 1.0 - s_fy[s] : s_fy[s];
-            const double wx = ix == 0 ? 1.0 - s_fx[s] : s_fx[s];
-            const double wo = io == 0 ? 1.0 - s_fo[s] : s_fo[s];
-            acc += s_w[s] * wx * wy * wo;
+    const uint16_t* list = sm.cell[4 * q + cx];
+#pragma unroll 4
+    for (int j = 0; j < hits; ++j) {
+        const int e = list[j];
+        const int s = e & 1023, io = (co - (e >> 10)) & 7;
+        const double wgt = sm.w[s], fx = sm.fx[s], fy = sm.fy[s], fo = sm.fo[s];
+        if (io <= 1) {
+            const double wy = e & (1 << 14) ? fy : 1.0 - fy;
+            const double wx = e & (1 << 13) ? fx : 1.0 - fx;
+            const double wo = io ? fo : 1.0 - fo;
+            acc += wgt * wx * wy * wo;
         }
     }
     // the serial f32 sums of the reference; the elementwise steps by all
     float d = (float)acc;
     auto norm = [&]() -> float {
-        sd[tid] = d * d;
+        sm.sq[tid] = d * d;
         __syncthreads();
         if (tid == 0) {
             float ss = 0.0f;
 #pragma unroll 16
-            for (int i = 0; i < DESC_LEN; ++i) ss = ss + sd[i];
-            s_norm = sqrtf(ss);
+            for (int i = 0; i < DESC_LEN; ++i) ss = ss + sm.sq[i];
+            sm.norm = sqrtf(ss);
         }
         __syncthreads();
-        return s_norm;
+        return sm.norm;
     };
     float nm = norm();
     bool ok = !(nm < 1e-6f);
     if (ok) {
         d = d / nm;
         if (d > 0.2f) d = 0.2f;
-        nm = norm();  // s_norm and sd are read before the next writes: both sides synchronise
+        nm = norm();  // sm.norm and sm.sq are read before the next writes: both sides synchronise
         ok = !(nm < 1e-6f);
         if (ok) d = d / nm;
     }
@@ -935,7 +1026,7 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
     const int64_t want = quick_keypoints(cap);
     if (quick) {
         void* p_kept;
-        SCK(A.get(F_KEPT, sizeof(uint32_t) * SEL_CAP, &p_kept));
+        SCK(A.get(F_KEPT, 16 * (size_t)SEL_CAP, &p_kept));
         SCK(A.get(F_SIDX, sizeof(uint32_t) * SEL_CAP, &p_skp));
         SCK(A.get(F_THETA, sizeof(double) * 4 * (size_t)want, &p_th));
         SCK(A.get(F_CNT, sizeof(int32_t) * (size_t)want, &p_cnt));
@@ -949,13 +1040,15 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
         SCK(A.get(F_COL, 3 * (size_t)cap, &p_col));
         hist_kernel<<<64, 256, 0, st>>>(kp.resp, d_counts, d_hist);
         SCK(cudaGetLastError());
-        keep_kernel<<<64, 256, 0, st>>>(kp.resp, d_hist, (uint32_t)want, d_counts, (uint32_t*)p_kept);
+        const Kept kept{(long long*)p_kept, (uint32_t*)((long long*)p_kept + SEL_CAP),
+                        (uint32_t*)((long long*)p_kept + SEL_CAP) + SEL_CAP};
+        keep_kernel<<<64, 256, 0, st>>>(kp.resp, d_hist, kp.place, (uint32_t)want, d_counts, kept);
         SCK(cudaGetLastError());
-        rank_kernel<<<148 * 2, 256, 0, st>>>(kp, (const uint32_t*)p_kept, d_counts, (uint32_t*)p_skp);
+        rank_kernel<<<148 * 2, 256, 0, st>>>(kept, d_counts, (uint32_t*)p_skp);
         SCK(cudaGetLastError());
         hook.begin("sift_orient");
-        orient_kernel<<<(unsigned)((want + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
-            kp, (const uint32_t*)p_skp, 0, (int)want, d_counts, table, w, h, (double*)p_th, (int32_t*)p_cnt);
+        orient_kernel<<<(unsigned)want, ORI_THREADS, 0, st>>>(
+            kp, (const uint32_t*)p_skp, 0, d_counts, table, w, h, (double*)p_th, (int32_t*)p_cnt);
         SCK(cudaGetLastError());
         hook.end("sift_orient");
         first_pairs_kernel<<<1, 1024, 0, st>>>((const uint32_t*)p_skp, (int)want, (const int32_t*)p_cnt,
@@ -1029,8 +1122,8 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
                 // orientations of the next keypoints in response order, and their pairs
                 const int64_t ck = std::min<int64_t>(nkp - kdone, std::max<int64_t>(cap - n_valid, 64));
                 hook.begin("sift_orient");
-                orient_kernel<<<(unsigned)((ck + WARPS - 1) / WARPS), 32 * WARPS, 0, st>>>(
-                    kp, (const uint32_t*)p_skp, kdone, (int)ck, nullptr, table, w, h, (double*)p_th, (int32_t*)p_cnt);
+                orient_kernel<<<(unsigned)ck, ORI_THREADS, 0, st>>>(
+                    kp, (const uint32_t*)p_skp, kdone, nullptr, table, w, h, (double*)p_th, (int32_t*)p_cnt);
                 SCK(cudaGetLastError());
                 hook.end("sift_orient");
                 size_t tb = 0;
