@@ -625,6 +625,7 @@ int fuse_views(rcmvs_ctx* ctx, rcmvs_scene* sc, const int32_t* order_offsets, co
         F.order_end = order_offsets[v + 1];
         const HostCam& c = sc->cams[v];
         F.f = c.f;
+        F.rf = 1.0 / c.f;
         F.cx = c.cx;
         F.cy = c.cy;
         F.k = c.k;

@@ -17,6 +17,8 @@
 #include <thrust/iterator/counting_iterator.h>
 
 #include <climits>
+#include <cmath>
+#include <limits>
 #include <cub/cub.cuh>
 
 #include "rcmvs_internal.cuh"
@@ -26,7 +28,7 @@ namespace rcmvs {
 namespace {
 
 constexpr int FT = 256;  // threads per block for pixel kernels
-constexpr int RT = 64;   // threads per block of the voxel reduce: few voxels, spread over every SM
+constexpr int VPX = 4 * FT;  // pixels per block of valid_kernel
 
 __device__ __forceinline__ int find_item(const int32_t* start, int n, int b) {
     int lo = 0, hi = n - 1;
@@ -40,10 +42,34 @@ __device__ __forceinline__ int find_item(const int32_t* start, int n, int b) {
     return lo;
 }
 
+// Quotients by one divisor, correctly rounded as a / b is: with y the
+// correctly rounded 1 / b and q within one unit in the last place of a / b,
+// q + fma(-b, q, a) y rounds to RN(a / b) (P. Markstein, IBM J. Res. Dev. 34,
+// 1990, theorem on division).  The first correction brings a y within one
+// unit, the second one rounds.  Exponents are kept to where no step can
+// overflow or lose bits to the subnormals; zero and what lies outside is
+// divided.  Five operations where a division takes about thirty.
+struct Recip {
+    double b, y;
+    bool ok;
+};
+__device__ __forceinline__ bool exponent_in(double x, int lo, int hi) {
+    return (unsigned)(((__double2hiint(x) >> 20) & 0x7FF) - (1023 + lo)) < (unsigned)(hi - lo);
+}
+__device__ __forceinline__ Recip recip(double b) { return Recip{b, __drcp_rn(b), exponent_in(b, -100, 100)}; }
+__device__ __forceinline__ Recip recip(double b, double y) { return Recip{b, y, exponent_in(b, -100, 100)}; }
+__device__ __forceinline__ double quot(double a, const Recip& r) {
+    if (!(r.ok && exponent_in(a, -900, 900))) return a / r.b;
+    double q = a * r.y;
+    q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+    return __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+}
+
 // sfm-lite/src/geom.rs:28-42
 __device__ __forceinline__ void cam_normalize(const FuseView& v, double u, double w, double& xn, double& yn) {
-    xn = (u - v.cx) / v.f;
-    yn = (w - v.cy) / v.f;
+    const Recip f = recip(v.f, v.rf);
+    xn = quot(u - v.cx, f);
+    yn = quot(w - v.cy, f);
     // with k = 0 and a finite radius, d = 1 + 0 * r2 is exactly 1, f * d = f,
     // and both iterations give back xn, yn: skipped
     if (v.k == 0.0 && isfinite(xn * xn + yn * yn)) return;
@@ -51,9 +77,26 @@ __device__ __forceinline__ void cam_normalize(const FuseView& v, double u, doubl
         double r2 = xn * xn + yn * yn;
         double d = 1.0 + v.k * r2;
         if (fabs(d) < 1e-12) break;
-        xn = (u - v.cx) / (v.f * d);
-        yn = (w - v.cy) / (v.f * d);
+        const Recip fd = recip(v.f * d);
+        xn = quot(u - v.cx, fd);
+        yn = quot(w - v.cy, fd);
     }
+}
+
+struct Pose {
+    double R[9], t[3];
+};
+__device__ __forceinline__ Pose load_pose(const FuseView& v) {
+    Pose p;
+    const double2* s = reinterpret_cast<const double2*>(v.R);
+    double* d = p.R;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const double2 q = __ldg(s + i);
+        d[2 * i] = q.x;  // t follows R
+        d[2 * i + 1] = q.y;
+    }
+    return p;
 }
 
 // nalgebra 3x3 products, k ascending
@@ -64,37 +107,35 @@ __device__ __forceinline__ void matt_vec(const double* m, const double* x, doubl
     for (int i = 0; i < 3; ++i) o[i] = m[i] * x[0] + m[3 + i] * x[1] + m[6 + i] * x[2];
 }
 
-// sfm-lite/src/geom.rs:64-75
-__device__ __forceinline__ bool project(const FuseView& v, const double* x, double& u, double& w) {
-    double xc[3];
-    mat_vec(v.R, x, xc);
-    for (int i = 0; i < 3; ++i) xc[i] = xc[i] + v.t[i];
-    const double z = xc[2];
-    if (z <= 1e-9) return false;
-    const double xn = xc[0] / z, yn = xc[1] / z;
+// World -> camera (sfm-lite/src/geom.rs:64-66)
+__device__ __forceinline__ void to_cam(const Pose& p, const double* x, double* xc) {
+    mat_vec(p.R, x, xc);
+    for (int i = 0; i < 3; ++i) xc[i] = xc[i] + p.t[i];
+}
+
+// Camera -> pixel (sfm-lite/src/geom.rs:67-75); z is recip(xc[2])
+__device__ __forceinline__ void project(const FuseView& v, const double* xc, const Recip& z, double& u, double& w) {
+    const double xn = quot(xc[0], z), yn = quot(xc[1], z);
     const double r2 = xn * xn + yn * yn;
     const double d = 1.0 + v.k * r2;
     u = v.f * xn * d + v.cx;
     w = v.f * yn * d + v.cy;
-    return true;
 }
 
-// Rust `f64 as i32` (saturating, NaN -> 0): cvt.rzi.s32.f64
-__device__ __forceinline__ int f64_to_i32(double x) { return __double2int_rz(x); }
-
-// fuse.rs:32-62
+// fuse.rs:32-62.  The reference truncates floor(u) to an i32 and tests
+// 0 <= u0, u0 + 1 < w (a NaN counts as 0, and the weights it makes give 0):
+// the same tests on u itself need no conversion, and below 2^31 adding 1.5 2^52
+// rounded down leaves floor(u) in the low word.
 __device__ __forceinline__ double sample_depth(const float* __restrict__ dm, int w, int h, double u, double v) {
-    const int u0 = f64_to_i32(floor(u));
-    const int v0 = f64_to_i32(floor(v));
-    // The reference tests `u0 + 1 >= w`.  u0 saturates at INT_MAX for points
-    // barely in front of the camera, where `+ 1` would overflow (Rust wraps in
-    // release builds and then panics on the slice index); `u0 >= w - 1` is
-    // the same test without the overflow and treats such points as off-image.
-    if (u0 < 0 || v0 < 0 || u0 >= w - 1 || v0 >= h - 1) return 0.0;
-    const float fx = (float)(u - (double)u0);
-    const float fy = (float)(v - (double)v0);
-    const float d00 = __ldg(dm + (size_t)v0 * w + u0), d10 = __ldg(dm + (size_t)v0 * w + u0 + 1);
-    const float d01 = __ldg(dm + (size_t)(v0 + 1) * w + u0), d11 = __ldg(dm + (size_t)(v0 + 1) * w + u0 + 1);
+    if (!(u >= 0.0 && v >= 0.0 && u < (double)(w - 1) && v < (double)(h - 1))) return 0.0;
+    const double big = 6755399441055744.0;
+    const double ub = __dadd_rd(u, big), vb = __dadd_rd(v, big);
+    const int u0 = __double2loint(ub), v0 = __double2loint(vb);
+    const float fx = (float)(u - (ub - big));
+    const float fy = (float)(v - (vb - big));
+    const float* p = dm + (size_t)v0 * w + u0;
+    const float d00 = __ldg(p), d10 = __ldg(p + 1);
+    const float d01 = __ldg(p + w), d11 = __ldg(p + w + 1);
     const float ds[4] = {d00, d10, d01, d11};
     const float wt[4] = {(1.0f - fx) * (1.0f - fy), fx * (1.0f - fy), (1.0f - fx) * fy, fx * fy};
     float acc = 0.f, wsum = 0.f;
@@ -116,25 +157,32 @@ __global__ void __launch_bounds__(FT) valid_kernel(const FuseView* __restrict__ 
                                                    const float* __restrict__ depth, uint8_t* __restrict__ flag) {
     const int item = find_item(blk_start, n_items, blockIdx.x);
     const FuseView& v = views[blk_view[item]];
-    const int64_t local = (int64_t)(blockIdx.x - blk_start[item]) * FT + threadIdx.x;
-    if (local >= (int64_t)v.w * v.h) return;
+    const int64_t n = (int64_t)v.w * v.h;
+    const int64_t local = (int64_t)(blockIdx.x - blk_start[item]) * VPX + threadIdx.x;
     const size_t gi = (size_t)v.off + (size_t)local;
-    flag[gi] = depth[gi] > 0.0f ? 1 : 0;
+    float d[VPX / FT];
+#pragma unroll
+    for (int k = 0; k < VPX / FT; ++k) d[k] = local + k * FT < n ? __ldg(depth + gi + k * FT) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < VPX / FT; ++k)
+        if (local + k * FT < n) flag[gi + k * FT] = d[k] > 0.0f ? 1 : 0;
 }
 
 // fuse.rs:96-167 for one pixel with a depth: flag + averaged point.  One
 // thread per entry of the list of such pixels (global indices; view k of
-// the map-holding views starts at voff[k]).  Register cap 64 (four blocks
-// per SM): on 100 1080p views it runs in 50 ms against 56 ms at 80
-// registers, though it spills -- more resident warps hide the latency of
-// the depth gathers from other views.
+// the map-holding views starts at voff[k]).  Bound by issued instructions: the
+// f64 divisions of a check (two per projection, the relative difference, two
+// per back-projection) share reciprocals (quot), the reprojection distance is
+// compared under its square (reproj_sq: the largest double whose root is
+// within the limit), and poses are read 16 bytes at a time.  24 views of
+// 960 x 720, 8 sources, a third of the pixels with a depth: 1640 -> 1490 us.
 __global__ void __launch_bounds__(FT, 4) candidates_kernel(const FuseView* __restrict__ views,
                                                            const int64_t* __restrict__ voff,
                                                            const int32_t* __restrict__ vidx, int n_items,
                                                            const uint32_t* __restrict__ work, uint32_t n_work,
                                                            const int32_t* __restrict__ order,
                                                            const float* __restrict__ depth, uint32_t min_consistent,
-                                                           double depth_diff, double reproj_px,
+                                                           double depth_diff, bool gate, double reproj_sq,
                                                            uint8_t* __restrict__ flag, double* __restrict__ pts) {
     const uint32_t t = blockIdx.x * FT + threadIdx.x;
     if (t >= n_work) return;
@@ -156,44 +204,48 @@ __global__ void __launch_bounds__(FT, 4) candidates_kernel(const FuseView* __res
         double nx, ny;
         cam_normalize(v, (double)px, (double)py, nx, ny);
         const double xr[3] = {nx * zr, ny * zr, 1.0 * zr};
-        const double dd[3] = {xr[0] - v.t[0], xr[1] - v.t[1], xr[2] - v.t[2]};
+        const Pose ref = load_pose(v);
+        const double dd[3] = {xr[0] - ref.t[0], xr[1] - ref.t[1], xr[2] - ref.t[2]};
         double xw[3];
-        matt_vec(v.R, dd, xw);
+        matt_vec(ref.R, dd, xw);
         double acc[3] = {xw[0], xw[1], xw[2]};
         uint32_t n_cons = 0;
         for (int q = v.order_begin; q < v.order_end; ++q) {
             const FuseView& sv = views[order[q]];
+            const Pose sp = load_pose(sv);
             double xs[3];
-            mat_vec(sv.R, xw, xs);
-            for (int a = 0; a < 3; ++a) xs[a] = xs[a] + sv.t[a];
+            to_cam(sp, xw, xs);
             if (xs[2] <= 1e-6) continue;
+            const Recip z = recip(xs[2]);
             double us, vs;
-            if (!project(sv, xw, us, vs)) continue;
+            project(sv, xs, z, us, vs);
             const double zs = sample_depth(depth + sv.off, sv.w, sv.h, us, vs);
             if (zs <= 0.0) continue;
-            const double rel = fabs((xs[2] - zs) / xs[2]);
+            const double rel = fabs(quot(xs[2] - zs, z));
             if (rel < depth_diff) {
                 double sx, sy;
                 cam_normalize(sv, us, vs, sx, sy);
                 const double xs2[3] = {sx * zs, sy * zs, 1.0 * zs};
-                const double d2[3] = {xs2[0] - sv.t[0], xs2[1] - sv.t[1], xs2[2] - sv.t[2]};
+                const double d2[3] = {xs2[0] - sp.t[0], xs2[1] - sp.t[1], xs2[2] - sp.t[2]};
                 double xw2[3];
-                matt_vec(sv.R, d2, xw2);
-                if (reproj_px > 0.0) {  // extension: forward-backward reprojection gate
-                    double ru, rv;
-                    if (!project(v, xw2, ru, rv)) continue;
+                matt_vec(sp.R, d2, xw2);
+                if (gate) {  // extension: forward-backward reprojection gate
+                    double xc[3], ru, rv;
+                    to_cam(load_pose(v), xw2, xc);
+                    if (xc[2] <= 1e-9) continue;
+                    project(v, xc, recip(xc[2]), ru, rv);
                     const double ex = ru - (double)px, ey = rv - (double)py;
-                    if (!(sqrt(ex * ex + ey * ey) <= reproj_px)) continue;
+                    if (!(ex * ex + ey * ey <= reproj_sq)) continue;
                 }
                 for (int a = 0; a < 3; ++a) acc[a] += xw2[a];
                 ++n_cons;
             }
         }
         if (n_cons >= min_consistent) {
-            const double m = (double)(n_cons + 1);
-            pts[3 * gi] = acc[0] / m;
-            pts[3 * gi + 1] = acc[1] / m;
-            pts[3 * gi + 2] = acc[2] / m;
+            const Recip m = recip((double)(n_cons + 1));
+            pts[3 * gi] = quot(acc[0], m);
+            pts[3 * gi + 1] = quot(acc[1], m);
+            pts[3 * gi + 2] = quot(acc[2], m);
             ok = 1;
         }
     }
@@ -201,16 +253,17 @@ __global__ void __launch_bounds__(FT, 4) candidates_kernel(const FuseView* __res
 }
 
 // Rust `f64 as i64` (saturating, NaN -> 0): cvt.rzi.s64.f64
-__device__ __forceinline__ long long vkey(double p, double cell) { return __double2ll_rz(floor(p / cell)); }
+__device__ __forceinline__ long long vkey(double p, const Recip& cell) { return __double2ll_rz(floor(quot(p, cell))); }
 
 __global__ void keys_minmax_kernel(const uint32_t* __restrict__ cand, uint32_t n, const double* __restrict__ pts,
                                    double cell, long long* __restrict__ kmin, long long* __restrict__ kmax) {
     __shared__ long long smin[3][FT / 32], smax[3][FT / 32];
+    const Recip rc = recip(cell);
     long long lo[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, hi[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
     for (uint32_t c = blockIdx.x * FT + threadIdx.x; c < n; c += gridDim.x * FT) {
         const size_t g = cand[c];
         for (int a = 0; a < 3; ++a) {
-            long long k = vkey(pts[3 * g + a], cell);
+            long long k = vkey(pts[3 * g + a], rc);
             lo[a] = min(lo[a], k);
             hi[a] = max(hi[a], k);
         }
@@ -240,98 +293,91 @@ __global__ void keys_minmax_kernel(const uint32_t* __restrict__ cand, uint32_t n
 }
 
 __global__ void pack_keys_kernel(const uint32_t* __restrict__ cand, uint32_t n, const double* __restrict__ pts,
-                                 double cell, const long long* __restrict__ kmin, uint64_t* __restrict__ keys,
-                                 uint32_t* __restrict__ vals) {
+                                 double cell, const long long* __restrict__ kmin, int ybits, int zbits,
+                                 uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     const uint32_t c = blockIdx.x * FT + threadIdx.x;
     if (c >= n) return;
     const size_t g = cand[c];
+    const Recip rc = recip(cell);
     uint64_t key = 0;
     for (int a = 0; a < 3; ++a) {
-        const uint64_t k = (uint64_t)(vkey(pts[3 * g + a], cell) - kmin[a]);
-        key = (key << 21) | k;  // x in the high bits: lexicographic (x, y, z)
+        const uint64_t k = (uint64_t)(vkey(pts[3 * g + a], rc) - kmin[a]);
+        key = (key << (a == 0 ? 0 : a == 1 ? ybits : zbits)) | k;  // x in the high bits: lexicographic (x, y, z)
     }
     keys[c] = key;
     vals[c] = c;
 }
 
 // fuse.rs:194-213: in-order sums per voxel (u16 colour sums wrap), means,
-// and the 15-byte PLY vertex record of fuse.rs:232-237.
-__global__ void reduce_kernel(const uint32_t* __restrict__ run_off, const uint32_t* __restrict__ run_len,
-                              const uint32_t* __restrict__ n_runs_p, const uint32_t* __restrict__ sorted_vals,
-                              const uint32_t* __restrict__ cand, const double* __restrict__ pts,
-                              const uint8_t* __restrict__ rgb, double* __restrict__ out_xyz,
-                              uint8_t* __restrict__ out_rgb, uint8_t* __restrict__ ply) {
-    const uint32_t r = blockIdx.x * RT + threadIdx.x;
-    if (r >= *n_runs_p) return;
+// and the 15-byte PLY vertex record of fuse.rs:232-237.  G lanes per voxel
+// fetch G members at a time (sorted position -> candidate -> point, the next
+// ones before the last are added); lanes 0-2 add one coordinate each in member
+// order.  Bound by that chain: with a thread per voxel the voxel of most members
+// set the time.  24 views of 960 x 720: 350 us with a thread per voxel, 81 us
+// with a warp (G = 32).  G = 8 where the mean is under 8 members: 212 k voxels
+// of 3 members 26 us against 75 us.
+template <int G>
+__global__ void __launch_bounds__(FT) reduce_kernel(const uint32_t* __restrict__ run_off,
+                                                    const uint32_t* __restrict__ run_len, uint32_t n_runs,
+                                                    const uint32_t* __restrict__ sorted_vals,
+                                                    const uint32_t* __restrict__ cand, const double* __restrict__ pts,
+                                                    const uint8_t* __restrict__ rgb, double* __restrict__ out_xyz,
+                                                    uint8_t* __restrict__ out_rgb, uint8_t* __restrict__ ply) {
+    __shared__ double s_pt[FT / G][3][G];
+    const uint32_t r = blockIdx.x * (FT / G) + threadIdx.x / G;
+    const int lane = threadIdx.x % G;
+    const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) / G * G);
+    if (r >= n_runs) return;
     const uint32_t b = run_off[r], n = run_len[r];
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    uint16_t cr = 0, cg = 0, cb = 0;
-    // Members four at a time: the four chains of dependent loads (sorted
-    // position -> candidate -> point) are issued together, then added in
-    // member order, so the f64 sums are the sequential ones.
-    constexpr int U = 4;
-    uint32_t m = 0;
-    for (; m + U <= n; m += U) {
-        size_t g[U];
-#pragma unroll
-        for (int k = 0; k < U; ++k) g[k] = cand[sorted_vals[b + m + k]];
-        double px[U], py[U], pz[U];
-        uint8_t qr[U], qg[U], qb[U];
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            px[k] = pts[3 * g[k]];
-            py[k] = pts[3 * g[k] + 1];
-            pz[k] = pts[3 * g[k] + 2];
-            qr[k] = rgb[3 * g[k]];
-            qg[k] = rgb[3 * g[k] + 1];
-            qb[k] = rgb[3 * g[k] + 2];
-        }
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            sx += px[k];
-            sy += py[k];
-            sz += pz[k];
-            cr = (uint16_t)(cr + qr[k]);
-            cg = (uint16_t)(cg + qg[k]);
-            cb = (uint16_t)(cb + qb[k]);
-        }
-    }
-    for (; m < n; ++m) {
+    double(*pt)[G] = s_pt[threadIdx.x / G];
+    uint32_t cr = 0, cg = 0, cb = 0;
+    double x = 0.0, y = 0.0, z = 0.0, sum = 0.0;
+    auto fetch = [&](uint32_t m) {
+        if (m >= n) return;
         const size_t g = cand[sorted_vals[b + m]];
-        sx += pts[3 * g];
-        sy += pts[3 * g + 1];
-        sz += pts[3 * g + 2];
-        cr = (uint16_t)(cr + rgb[3 * g]);
-        cg = (uint16_t)(cg + rgb[3 * g + 1]);
-        cb = (uint16_t)(cb + rgb[3 * g + 2]);
-    }
-    const double nn = (double)n;
-    const double x = sx / nn, y = sy / nn, z = sz / nn;
-    out_xyz[3 * (size_t)r] = x;
-    out_xyz[3 * (size_t)r + 1] = y;
-    out_xyz[3 * (size_t)r + 2] = z;
-    uint8_t c3[3];
-    const uint16_t cs[3] = {cr, cg, cb};
-    for (int a = 0; a < 3; ++a) {
-        double q = round((double)cs[a] / nn);  // half away from zero, as f64::round
-        c3[a] = q <= 0.0 ? 0 : (q >= 255.0 ? 255 : (uint8_t)q);
-        out_rgb[3 * (size_t)r + a] = c3[a];
-    }
-    if (ply) {
-        const float fx = (float)x, fy = (float)y, fz = (float)z;
-        uint8_t* o = ply + 15 * (size_t)r;
-        const uint8_t* bx = reinterpret_cast<const uint8_t*>(&fx);
-        const uint8_t* by = reinterpret_cast<const uint8_t*>(&fy);
-        const uint8_t* bz = reinterpret_cast<const uint8_t*>(&fz);
-        for (int q = 0; q < 4; ++q) {
-            o[q] = bx[q];
-            o[4 + q] = by[q];
-            o[8 + q] = bz[q];
+        x = pts[3 * g];
+        y = pts[3 * g + 1];
+        z = pts[3 * g + 2];
+        cr += rgb[3 * g];
+        cg += rgb[3 * g + 1];
+        cb += rgb[3 * g + 2];
+    };
+    fetch(lane);
+    for (uint32_t base = 0; base < n; base += G) {
+        pt[0][lane] = x;
+        pt[1][lane] = y;
+        pt[2][lane] = z;
+        __syncwarp(mask);
+        fetch(base + G + lane);
+        if (lane < 3) {
+            const int m = (int)min((uint32_t)G, n - base);
+            if (m == G) {
+#pragma unroll
+                for (int t = 0; t < G; ++t) sum += pt[lane][t];
+            } else {
+                for (int t = 0; t < m; ++t) sum += pt[lane][t];
+            }
         }
-        o[12] = c3[0];
-        o[13] = c3[1];
-        o[14] = c3[2];
+        __syncwarp(mask);
     }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        cr += __shfl_xor_sync(mask, cr, o);
+        cg += __shfl_xor_sync(mask, cg, o);
+        cb += __shfl_xor_sync(mask, cb, o);
+    }
+    if (lane >= 3) return;
+    const double nn = (double)n;
+    const double mean = sum / nn;
+    out_xyz[3 * (size_t)r + lane] = mean;
+    const uint16_t cs = (uint16_t)(lane == 0 ? cr : lane == 1 ? cg : cb);
+    const double q = round((double)cs / nn);  // half away from zero, as f64::round
+    const uint8_t c = q <= 0.0 ? 0 : (q >= 255.0 ? 255 : (uint8_t)q);
+    out_rgb[3 * (size_t)r + lane] = c;
+    uint8_t* o = ply + 15 * (size_t)r;
+    const uint32_t bits = __float_as_uint((float)mean);
+    for (int i = 0; i < 4; ++i) o[4 * lane + i] = (uint8_t)(bits >> (8 * i));
+    o[12 + lane] = c;
 }
 
 __global__ void init_minmax_kernel(long long* kmin, long long* kmax) {
@@ -395,7 +441,7 @@ int fuse_candidates_device(DeviceArena& A, const FuseView* h_views, int n_views,
         if (!h_views[v].has_depth || !h_views[v].is_ref) continue;
         blk_start.push_back((int32_t)total_blocks);
         blk_view.push_back(v);
-        total_blocks += ((int64_t)h_views[v].w * h_views[v].h + FT - 1) / FT;
+        total_blocks += ((int64_t)h_views[v].w * h_views[v].h + VPX - 1) / VPX;
     }
     *n_cand_out = 0;
     *d_cand = nullptr;
@@ -444,11 +490,20 @@ int fuse_candidates_device(DeviceArena& A, const FuseView* h_views, int n_views,
     uint32_t n_work = 0;
     FCK(cudaMemcpyAsync(&n_work, (uint32_t*)p_nsel + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     FCK(cudaStreamSynchronize(st));
+    // sqrt rounds correctly and grows with its argument: sqrt(s) <= reproj_px
+    // exactly where s is at most the largest double with that
+    const bool gate = reproj_px > 0.0;
+    double reproj_sq = reproj_px * reproj_px;
+    if (gate && std::isfinite(reproj_px)) {
+        const double inf = std::numeric_limits<double>::infinity();
+        while (std::sqrt(reproj_sq) > reproj_px) reproj_sq = std::nextafter(reproj_sq, 0.0);
+        while (std::sqrt(std::nextafter(reproj_sq, inf)) <= reproj_px) reproj_sq = std::nextafter(reproj_sq, inf);
+    }
     if (n_work > 0)
         candidates_kernel<<<(n_work + FT - 1) / FT, FT, 0, st>>>(
             (const FuseView*)p_views, (const int64_t*)p_voff, (const int32_t*)p_blk + n_items + 1, n_items,
-            (const uint32_t*)p_work, n_work, (const int32_t*)p_order, depth, min_consistent, depth_diff, reproj_px,
-            flag, pts);
+            (const uint32_t*)p_work, n_work, (const int32_t*)p_order, depth, min_consistent, depth_diff, gate,
+            reproj_sq, flag, pts);
     FCK(cudaGetLastError());
     hook.end("fuse_candidates");
 
@@ -471,7 +526,7 @@ int fuse_reduce_device(DeviceArena& A, const uint32_t* d_cand, uint32_t n_cand, 
     const void* p_cand = d_cand;
     void* p_temp;
     size_t tb = 0;
-    // voxel keys, packed 21 bits per axis
+    // voxel keys, packed; at most 21 bits per axis
     void* p_kmin;
     FCK(A.get(S_KMIN, sizeof(long long) * 6, &p_kmin));
     long long* kmin = (long long*)p_kmin;
@@ -480,6 +535,7 @@ int fuse_reduce_device(DeviceArena& A, const uint32_t* d_cand, uint32_t n_cand, 
     const unsigned gb = (unsigned)std::min<uint32_t>((n_cand + FT - 1) / FT, 148u * 8u);
     keys_minmax_kernel<<<gb, FT, 0, st>>>((const uint32_t*)p_cand, n_cand, pts, cell, kmin, kmax);
     FCK(cudaGetLastError());
+    int bits[3];
     long long hk[6];
     FCK(cudaMemcpyAsync(hk, kmin, sizeof(hk), cudaMemcpyDeviceToHost, st));
     FCK(cudaStreamSynchronize(st));
@@ -489,22 +545,25 @@ int fuse_reduce_device(DeviceArena& A, const uint32_t* d_cand, uint32_t n_cand, 
             *err = "fusion: voxel index range exceeds 2^21 cells per axis (cell too small for the cloud)";
             return RCMVS_E_LIMIT;
         }
+        for (bits[a] = 0; (span >> bits[a]) != 0;) ++bits[a];
     }
+    // the sort's passes go by the bits that the ranges need
+    const int key_bits = std::max(1, bits[0] + bits[1] + bits[2]);
     void *p_keys, *p_vals, *p_keys2, *p_vals2;
     FCK(A.get(S_KEYS, sizeof(uint64_t) * n_cand, &p_keys));
     FCK(A.get(S_VALS, sizeof(uint32_t) * n_cand, &p_vals));
     FCK(A.get(S_KEYS2, sizeof(uint64_t) * n_cand, &p_keys2));
     FCK(A.get(S_VALS2, sizeof(uint32_t) * n_cand, &p_vals2));
     pack_keys_kernel<<<(n_cand + FT - 1) / FT, FT, 0, st>>>((const uint32_t*)p_cand, n_cand, pts, cell, kmin,
-                                                            (uint64_t*)p_keys, (uint32_t*)p_vals);
+                                                            bits[1], bits[2], (uint64_t*)p_keys, (uint32_t*)p_vals);
     FCK(cudaGetLastError());
-    // stable LSD radix sort over the 63 used bits
+    // stable LSD radix sort
     tb = 0;
     FCK(cub::DeviceRadixSort::SortPairs(nullptr, tb, (const uint64_t*)p_keys, (uint64_t*)p_keys2,
-                                        (const uint32_t*)p_vals, (uint32_t*)p_vals2, n_cand, 0, 63, st));
+                                        (const uint32_t*)p_vals, (uint32_t*)p_vals2, n_cand, 0, key_bits, st));
     FCK(A.get(S_TEMP, tb, &p_temp));
     FCK(cub::DeviceRadixSort::SortPairs(p_temp, tb, (const uint64_t*)p_keys, (uint64_t*)p_keys2,
-                                        (const uint32_t*)p_vals, (uint32_t*)p_vals2, n_cand, 0, 63, st));
+                                        (const uint32_t*)p_vals, (uint32_t*)p_vals2, n_cand, 0, key_bits, st));
     // runs of equal keys = voxels
     void *p_runkey, *p_runlen, *p_runoff, *p_nruns;
     FCK(A.get(S_RUNKEY, sizeof(uint64_t) * n_cand, &p_runkey));
@@ -528,10 +587,15 @@ int fuse_reduce_device(DeviceArena& A, const uint32_t* d_cand, uint32_t n_cand, 
     FCK(A.get(S_OUTRGB, 3 * (size_t)n_runs, &p_orgb));
     FCK(A.get(S_PLY, 15 * (size_t)n_runs, &p_ply));
     hook.begin("fuse_reduce");
-    reduce_kernel<<<(n_runs + RT - 1) / RT, RT, 0, st>>>((const uint32_t*)p_runoff, (const uint32_t*)p_runlen,
-                                                         (const uint32_t*)p_nruns, (const uint32_t*)p_vals2,
-                                                         (const uint32_t*)p_cand, pts, rgb, (double*)p_oxyz,
-                                                         (uint8_t*)p_orgb, (uint8_t*)p_ply);
+    auto reduce = [&](auto kernel, uint32_t per_block) {
+        kernel<<<(n_runs + per_block - 1) / per_block, FT, 0, st>>>(
+            (const uint32_t*)p_runoff, (const uint32_t*)p_runlen, n_runs, (const uint32_t*)p_vals2,
+            (const uint32_t*)p_cand, pts, rgb, (double*)p_oxyz, (uint8_t*)p_orgb, (uint8_t*)p_ply);
+    };
+    if (n_cand / 8 < n_runs)
+        reduce(reduce_kernel<8>, FT / 8);
+    else
+        reduce(reduce_kernel<32>, FT / 32);
     FCK(cudaGetLastError());
     hook.end("fuse_reduce");
     *d_xyz = (double*)p_oxyz;

@@ -148,15 +148,17 @@ cudaError_t launch_cost_field(const DevJob* d_job, const int32_t* d_job_start, c
 cudaError_t launch_f2i(const float* in, int n, int32_t* out, cudaStream_t st);
 
 // Fusion (fuse.cu).  View arrays hold per-view f64 cameras/poses.
-struct FuseView {
+struct alignas(16) FuseView {
     int32_t w, h;
     int64_t off;
     int32_t has_depth;
     int32_t order_begin, order_end;
     int32_t is_ref;  // its pixels are checked (else it only serves as a source)
     double f, cx, cy, k;
+    double rf;  // 1 / f
+    double pad;
     double R[9];
-    double t[3];
+    double t[3];  // follows R (six 16-byte loads)
 };
 
 struct FuseResult {
