@@ -151,3 +151,22 @@ def sparse_struct(xyz, track_offsets, track_views):
     s = Sparse(len(xyz), xyz.ctypes.data, off.ctypes.data, tv.ctypes.data)
     s._keep = (xyz, off, tv)
     return s
+
+
+class Owned:
+    """A result struct whose buffers the library allocated: the arrays taken
+    from it are views that keep it alive, and the last one frees it."""
+
+    def __init__(self, struct, free):
+        self.struct, self._free = struct, free
+
+    def array(self, address, ctype, shape):
+        n = int(np.prod(shape))
+        if n == 0:
+            return np.empty(shape, np.dtype(ctype))
+        buf = (ctype * n).from_address(address)
+        buf.owner = self
+        return np.ctypeslib.as_array(buf).reshape(shape)
+
+    def __del__(self):
+        self._free(C.byref(self.struct))

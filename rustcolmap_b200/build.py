@@ -28,12 +28,12 @@ FLAGS = ARCH + [
 
 LIBS = {
     "librcmvs.so": ["capi.cu", "census.cu", "stereo.cu", "fuse.cu", "noalloc.cu", "learned.cu", "learned_api.cu",
-                   "schedule.cu", "depthvis.cu", "resize.cu", "sift.cu", "match.cu"],
+                   "schedule.cu", "depthvis.cu", "resize.cu", "sift.cu", "match.cu", "hostcopy.cu"],
     "librcscene.so": ["scene.cu"],
 }
 LINK = {"librcmvs.so": ["-lz"]}  # zlib: the grey PNG writer
 HEADERS = [os.path.join(CSRC, "rcmvs_internal.cuh"), os.path.join(CSRC, "ctx_internal.cuh"),
-           os.path.join(CSRC, "learned.cuh"),
+           os.path.join(CSRC, "learned.cuh"), os.path.join(CSRC, "hostcopy.cuh"),
            os.path.join(CSRC, "tc.cuh"), os.path.join(ROOT, "include", "rcmvs.h"),
            os.path.join(ROOT, "include", "rcscene.h")]
 

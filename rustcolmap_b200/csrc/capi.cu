@@ -166,6 +166,7 @@ int rcmvs_ctx_create(int device, rcmvs_ctx** out) {
             return RCMVS_E_NOMEM;
         }
     }
+    rcmvs::host_copy_attach();
     *out = ctx;
     return RCMVS_OK;
 }
@@ -184,6 +185,7 @@ void rcmvs_ctx_destroy(rcmvs_ctx* ctx) {
         cudaStreamDestroy(ctx->upload);
     }
     cudaStreamDestroy(ctx->stream);
+    rcmvs::host_copy_detach();
     delete ctx;
 }
 
@@ -539,9 +541,9 @@ int rcmvs_scene_get_depth(rcmvs_ctx* ctx, rcmvs_scene* sc, int32_t view, float* 
     const DevView& V = sc->views[view];
     const size_t n = (size_t)V.w * V.h;
     cudaStream_t st = ctx->stream;
-    if (depth) CK(cudaMemcpyAsync(depth, sc->depth + V.off, 4 * n, cudaMemcpyDeviceToHost, st));
-    if (cost) CK(cudaMemcpyAsync(cost, sc->cost + V.off, 4 * n, cudaMemcpyDeviceToHost, st));
-    if (normal) CK(cudaMemcpyAsync(normal, sc->normal + 3 * V.off, 12 * n, cudaMemcpyDeviceToHost, st));
+    if (depth) CK(rcmvs::host_download(depth, sc->depth + V.off, 4 * n, st));
+    if (cost) CK(rcmvs::host_download(cost, sc->cost + V.off, 4 * n, st));
+    if (normal) CK(rcmvs::host_download(normal, sc->normal + 3 * V.off, 12 * n, st));
     CK(cudaStreamSynchronize(st));
     return RCMVS_OK;
 }
@@ -561,8 +563,11 @@ int rcmvs_scene_set_depth(rcmvs_ctx* ctx, rcmvs_scene* sc, int32_t view, const f
         return fail(ctx, RCMVS_E_ARG, "rcmvs_scene_set_depth: bad argument");
     CK(cudaSetDevice(ctx->device));
     const DevView& V = sc->views[view];
-    CK(cudaMemcpyAsync(sc->depth + V.off, depth, 4 * (size_t)V.w * V.h,
-                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
+    const size_t bytes = 4 * (size_t)V.w * V.h;
+    if (on_device)
+        CK(cudaMemcpyAsync(sc->depth + V.off, depth, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    else
+        CK(rcmvs::host_upload(sc->depth + V.off, depth, bytes, ctx->stream));
     if (!on_device) CK(cudaStreamSynchronize(ctx->stream));  // the host buffer may go away on return
     sc->has_depth[view] = 1;
     return RCMVS_OK;
@@ -573,7 +578,7 @@ int rcmvs_scene_get_census(rcmvs_ctx* ctx, rcmvs_scene* sc, int32_t view, uint64
         return fail(ctx, RCMVS_E_ARG, "rcmvs_scene_get_census: bad argument");
     CK(cudaSetDevice(ctx->device));
     const DevView& V = sc->views[view];
-    CK(cudaMemcpyAsync(census, sc->census + V.off, 8 * (size_t)V.w * V.h, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(rcmvs::host_download(census, sc->census + V.off, 8 * (size_t)V.w * V.h, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return RCMVS_OK;
 }
@@ -588,11 +593,13 @@ double voxel_cell(const double* xyz, uint64_t n, double voxel_rel) {
     for (int a = 0; a < 3; ++a) {
         std::vector<double> ax(n);
         for (uint64_t p = 0; p < n; ++p) ax[p] = xyz[3 * p + a];
-        std::sort(ax.begin(), ax.end());
         size_t len = ax.size();
         size_t lo = std::min((size_t)((double)len * 0.02), len - 1);
         size_t hi = std::min((size_t)((double)len * 0.98), len - 1);
-        ext[a] = ax[hi] - ax[lo];
+        std::nth_element(ax.begin(), ax.begin() + hi, ax.end());
+        const double top = ax[hi];
+        std::nth_element(ax.begin(), ax.begin() + lo, ax.begin() + hi + 1);
+        ext[a] = top - ax[lo];
     }
     double diag = std::sqrt(ext[0] * ext[0] + ext[1] * ext[1] + ext[2] * ext[2]);
     return std::fmax(diag * voxel_rel, 1e-9);
@@ -637,16 +644,16 @@ int fuse_views(rcmvs_ctx* ctx, rcmvs_scene* sc, const int32_t* order_offsets, co
 
 // Library-allocated host copy of n points (device xyz / rgb) into out.
 int take_points(rcmvs_ctx* ctx, const double* d_xyz, const uint8_t* d_rgb, uint64_t n, rcmvs_points* out) {
-    out->xyz = (double*)std::malloc(24 * std::max<uint64_t>(n, 1));
-    out->rgb = (uint8_t*)std::malloc(3 * std::max<uint64_t>(n, 1));
+    out->xyz = (double*)rcmvs::host_alloc(24 * n);
+    out->rgb = (uint8_t*)rcmvs::host_alloc(3 * n);
     if (!out->xyz || !out->rgb) {
         rcmvs_points_free(out);
         return fail(ctx, RCMVS_E_NOMEM, "host allocation of the point cloud failed");
     }
     out->n = n;
     if (n) {
-        CK(cudaMemcpyAsync(out->xyz, d_xyz, 24 * n, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaMemcpyAsync(out->rgb, d_rgb, 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(rcmvs::host_download(out->xyz, d_xyz, 24 * n, ctx->stream));
+        CK(rcmvs::host_download(out->rgb, d_rgb, 3 * n, ctx->stream));
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return RCMVS_OK;
@@ -839,9 +846,9 @@ int rcmvs_scene_get_points(rcmvs_ctx* ctx, rcmvs_scene* sc, double* xyz, uint8_t
     CK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const size_t n = sc->n_points;
-    if (xyz) CK(cudaMemcpyAsync(xyz, sc->d_pts_xyz, 24 * n, cudaMemcpyDeviceToHost, st));
-    if (rgb) CK(cudaMemcpyAsync(rgb, sc->d_pts_rgb, 3 * n, cudaMemcpyDeviceToHost, st));
-    if (ply_body) CK(cudaMemcpyAsync(ply_body, sc->d_ply, 15 * n, cudaMemcpyDeviceToHost, st));
+    if (xyz) CK(rcmvs::host_download(xyz, sc->d_pts_xyz, 24 * n, st));
+    if (rgb) CK(rcmvs::host_download(rgb, sc->d_pts_rgb, 3 * n, st));
+    if (ply_body) CK(rcmvs::host_download(ply_body, sc->d_ply, 15 * n, st));
     CK(cudaStreamSynchronize(st));
     return RCMVS_OK;
 }
@@ -997,14 +1004,14 @@ int rcmvs_fuse_depth_maps(rcmvs_ctx* ctx, const rcmvs_view* views, int32_t n_vie
         for (int v = 0; v < n_views; ++v) {
             if (!depth_maps[v]) continue;
             const DevView& V = sc->views[v];
-            CK(cudaMemcpyAsync(sc->depth + V.off, depth_maps[v], 4 * (size_t)V.w * V.h, cudaMemcpyHostToDevice, st));
+            CK(rcmvs::host_upload(sc->depth + V.off, depth_maps[v], 4 * (size_t)V.w * V.h, st));
             sc->has_depth[v] = 1;
         }
         uint64_t np = 0;
         int r = rcmvs_scene_fuse(ctx, sc, order_offsets, order, sparse_xyz, n_sparse, opts, &np);
         if (r) return r;
-        out->xyz = (double*)std::malloc(24 * std::max<uint64_t>(np, 1));
-        out->rgb = (uint8_t*)std::malloc(3 * std::max<uint64_t>(np, 1));
+        out->xyz = (double*)rcmvs::host_alloc(24 * np);
+        out->rgb = (uint8_t*)rcmvs::host_alloc(3 * np);
         if (!out->xyz || !out->rgb) {
             rcmvs_points_free(out);
             return fail(ctx, RCMVS_E_NOMEM, "host allocation of the point cloud failed");
@@ -1032,8 +1039,7 @@ int rcmvs_fuse_candidates(rcmvs_ctx* ctx, const rcmvs_view* views, int32_t n_vie
         for (int v = 0; v < n_views; ++v) {
             if (!depth_maps[v]) continue;
             const DevView& V = sc->views[v];
-            CK(cudaMemcpyAsync(sc->depth + V.off, depth_maps[v], 4 * (size_t)V.w * V.h, cudaMemcpyHostToDevice,
-                               ctx->stream));
+            CK(rcmvs::host_upload(sc->depth + V.off, depth_maps[v], 4 * (size_t)V.w * V.h, ctx->stream));
             sc->has_depth[v] = 1;
         }
         return rcmvs_scene_fuse_candidates(ctx, sc, order_offsets, order, ref_views, n_ref, opts, out, per_view);
@@ -1364,8 +1370,8 @@ static int run_mvs_impl(rcmvs_ctx* ctx, const rcmvs_view* views, int32_t n_views
         uint64_t np = 0;
         r = rcmvs_scene_fuse(ctx, sc, fo.data(), ff.data(), sparse->xyz, sparse->n_points, opts, &np);
         if (r) return r;
-        out->xyz = (double*)std::malloc(24 * std::max<uint64_t>(np, 1));
-        out->rgb = (uint8_t*)std::malloc(3 * std::max<uint64_t>(np, 1));
+        out->xyz = (double*)rcmvs::host_alloc(24 * np);
+        out->rgb = (uint8_t*)rcmvs::host_alloc(3 * np);
         if (!out->xyz || !out->rgb) {
             rcmvs_points_free(out);
             return fail(ctx, RCMVS_E_NOMEM, "host allocation of the point cloud failed");

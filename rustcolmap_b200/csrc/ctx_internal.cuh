@@ -5,6 +5,7 @@
 #include <string>
 #include <vector>
 
+#include "hostcopy.cuh"
 #include "rcmvs_internal.cuh"
 
 using rcmvs::DevView;

@@ -21,6 +21,7 @@
 #include <limits>
 #include <cub/cub.cuh>
 
+#include "hostcopy.cuh"
 #include "rcmvs_internal.cuh"
 
 namespace rcmvs {
@@ -618,8 +619,8 @@ int fuse_reduce_host(DeviceArena& A, const double* h_xyz, const uint8_t* h_rgb, 
     FCK(A.get(S_INXYZ, sizeof(double) * 3 * n, &p_xyz));
     FCK(A.get(S_INRGB, 3 * n, &p_rgb));
     FCK(A.get(S_IOTA, sizeof(uint32_t) * n, &p_iota));
-    FCK(cudaMemcpyAsync(p_xyz, h_xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-    FCK(cudaMemcpyAsync(p_rgb, h_rgb, 3 * n, cudaMemcpyHostToDevice, st));
+    FCK(host_upload(p_xyz, h_xyz, sizeof(double) * 3 * n, st));
+    FCK(host_upload(p_rgb, h_rgb, 3 * n, st));
     iota_kernel<<<fgrid((uint32_t)n), FT, 0, st>>>((uint32_t*)p_iota, (uint32_t)n);
     FCK(cudaGetLastError());
     return fuse_reduce_device(A, (const uint32_t*)p_iota, (uint32_t)n, (const double*)p_xyz, (const uint8_t*)p_rgb,

@@ -268,14 +268,14 @@ int rcmvs_resize_view(rcmvs_ctx* ctx, const uint8_t* img, int32_t w, int32_t h, 
     RCK(A.get(R_IN, (size_t)n_in * channels, &p_in));
     RCK(A.get(R_GRAY, (size_t)n_out, &p_gray));
     RCK(A.get(R_RGB, (size_t)n_out * 3, &p_rgb));
-    RCK(cudaMemcpyAsync(p_in, img, (size_t)n_in * channels, cudaMemcpyHostToDevice, st));
+    RCK(host_upload(p_in, img, (size_t)n_in * channels, st));
     const int* d_err = nullptr;
     rc = resize_device(ctx, (const uint8_t*)p_in, w, h, channels, mw, mh, (uint8_t*)p_gray, (uint8_t*)p_rgb, &d_err);
     if (rc) return rc;
     int bad = 0;
     if (d_err) RCK(cudaMemcpyAsync(&bad, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (gray_out) RCK(cudaMemcpyAsync(gray_out, p_gray, (size_t)n_out, cudaMemcpyDeviceToHost, st));
-    if (rgb_out) RCK(cudaMemcpyAsync(rgb_out, p_rgb, (size_t)n_out * 3, cudaMemcpyDeviceToHost, st));
+    if (gray_out) RCK(host_download(gray_out, p_gray, (size_t)n_out, st));
+    if (rgb_out) RCK(host_download(rgb_out, p_rgb, (size_t)n_out * 3, st));
     RCK(cudaStreamSynchronize(st));
     if (bad) return rfail(ctx, RCMVS_E_CUDA, "rcmvs_resize_view: tap table overflow");
     return RCMVS_OK;

@@ -952,7 +952,7 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
     SCK(A.get(F_IN, (size_t)n_in * channels, &p_in));
     SCK(A.get(F_GRAY, (size_t)npx0, &p_gray));
     SCK(A.get(F_RGB, 3 * (size_t)npx0, &p_rgb));
-    SCK(cudaMemcpyAsync(p_in, img, (size_t)n_in * channels, cudaMemcpyHostToDevice, st));
+    SCK(host_upload(p_in, img, (size_t)n_in * channels, st));
     const int* d_err = nullptr;
     rc = resize_device(ctx, (const uint8_t*)p_in, w0, h0, channels, w, h, (uint8_t*)p_gray, (uint8_t*)p_rgb, &d_err);
     if (rc) return rc;
@@ -1174,9 +1174,9 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
     out->height = h;
     out->n_raw = n_raw;
     out->n = (uint64_t)n_out;
-    out->pts = (double*)std::malloc(sizeof(double) * 2 * std::max<int64_t>(n_out, 1));
-    out->desc = (float*)std::malloc(sizeof(float) * DESC_LEN * std::max<int64_t>(n_out, 1));
-    out->colors = (uint8_t*)std::malloc(3 * std::max<int64_t>(n_out, 1));
+    out->pts = (double*)host_alloc(sizeof(double) * 2 * n_out);
+    out->desc = (float*)host_alloc(sizeof(float) * DESC_LEN * n_out);
+    out->colors = (uint8_t*)host_alloc(3 * n_out);
     if (!out->pts || !out->desc || !out->colors) {
         rcmvs_sift_frame_free(out);
         return sfail(ctx, RCMVS_E_NOMEM, "sift: host allocation failed");
@@ -1191,9 +1191,9 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
             (const uint8_t*)p_rgb, w, h, (double*)p_pts, (float*)p_fdesc, (uint8_t*)p_col);
         SCK(cudaGetLastError());
     }
-    SCK(cudaMemcpyAsync(out->pts, p_pts, sizeof(double) * 2 * n_out, cudaMemcpyDeviceToHost, st));
-    SCK(cudaMemcpyAsync(out->desc, p_fdesc, sizeof(float) * DESC_LEN * n_out, cudaMemcpyDeviceToHost, st));
-    SCK(cudaMemcpyAsync(out->colors, p_col, 3 * (size_t)n_out, cudaMemcpyDeviceToHost, st));
+    SCK(host_download(out->pts, p_pts, sizeof(double) * 2 * n_out, st));
+    SCK(host_download(out->desc, p_fdesc, sizeof(float) * DESC_LEN * n_out, st));
+    SCK(host_download(out->colors, p_col, 3 * (size_t)n_out, st));
     SCK(cudaStreamSynchronize(st));
     return RCMVS_OK;
 }

@@ -184,9 +184,9 @@ def _take_points(ctx, pts):
     if n == 0:
         ctx._L.rcmvs_points_free(C.byref(pts))
         return np.zeros((0, 3), np.float64), np.zeros((0, 3), np.uint8)
-    xyz = np.ctypeslib.as_array((C.c_double * (3 * n)).from_address(pts.xyz)).reshape(n, 3).copy()
-    rgb = np.ctypeslib.as_array((C.c_uint8 * (3 * n)).from_address(pts.rgb)).reshape(n, 3).copy()
-    ctx._L.rcmvs_points_free(C.byref(pts))
+    own = _abi.Owned(pts, ctx._L.rcmvs_points_free)
+    xyz = own.array(pts.xyz, C.c_double, (n, 3))
+    rgb = own.array(pts.rgb, C.c_uint8, (n, 3))
     return xyz, rgb
 
 

@@ -53,16 +53,10 @@ def extract_sift(img, name="", opts=None, ctx=None):
     o = opts.to_c()
     f = _abi.SiftFrame()
     ctx.check(ctx._L.rcmvs_extract_sift(ctx.ptr, a.ctypes.data, w, h, c, C.byref(o), C.byref(f)))
-    try:
-        n = f.n
-        k = max(n, 1)
-        pts = np.ctypeslib.as_array((C.c_double * (2 * k)).from_address(f.pts))[: 2 * n].reshape(n, 2).copy()
-        desc = np.ctypeslib.as_array((C.c_float * (DESC_LEN * k)).from_address(f.desc))[: DESC_LEN * n]
-        desc = desc.reshape(n, DESC_LEN).copy()
-        col = np.ctypeslib.as_array((C.c_uint8 * (3 * k)).from_address(f.colors))[: 3 * n].reshape(n, 3).copy()
-        return SiftFrame(name, f.width, f.height, pts, desc, col, int(f.n_raw))
-    finally:
-        ctx._L.rcmvs_sift_frame_free(C.byref(f))
+    own = _abi.Owned(f, ctx._L.rcmvs_sift_frame_free)
+    n = f.n
+    return SiftFrame(name, f.width, f.height, own.array(f.pts, C.c_double, (n, 2)),
+                     own.array(f.desc, C.c_float, (n, DESC_LEN)), own.array(f.colors, C.c_uint8, (n, 3)), int(f.n_raw))
 
 
 def extract_sift_many(images, names=None, opts=None, ctxs=None):
