@@ -88,7 +88,10 @@ struct LaunchGeom {
 };
 // The kernels with a tiling of their own: pass_stream_kernel,
 // pass_staged_kernel and init_staged_kernel.
-enum { TILED_NONE = 0, TILED_STREAM = 1, TILED_STAGED = 2, TILED_INIT = 3 };
+enum { TILED_NONE = 0, TILED_STREAM = 1, TILED_STAGED = 2, TILED_INIT = 3, TILED_STAGED_MID = 4, TILED_STAGED_SMALL = 5 };
+inline bool tiled_staged(int kind) { return kind == TILED_STAGED || kind == TILED_STAGED_MID || kind == TILED_STAGED_SMALL; }
+// The staged passes' tiling for a batch of `tiles` TILED_STAGED tiles.
+int staged_kind(int64_t tiles);
 // Tiled passes: tiles of a w x h view in the kernel's own tiling, and the
 // geometry of a launch over `tiles` of them.  The launch is always
 // persistent (g.queue set) over at most tiled_grid(g) blocks, each with its

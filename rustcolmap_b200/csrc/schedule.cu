@@ -326,10 +326,16 @@ int build_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const rcmvs_job* jobs, int n_jo
     // The staged passes evaluate candidates ahead of the reference's sequence;
     // work counts and its own call sequence come from the streamed ones.
     if (rc == RCMVS_OK && tpp == 1 && !(opts->flags & RCMVS_FLAG_LOCKSTEP_PASSES)) {
-        b.tiled = ctx->count_work || (opts->flags & RCMVS_FLAG_NO_SKIP_DUPLICATES) ? TILED_STREAM : TILED_STAGED;
+        if (ctx->count_work || (opts->flags & RCMVS_FLAG_NO_SKIP_DUPLICATES)) {
+            b.tiled = TILED_STREAM;
+        } else {
+            int64_t tiles = 0;
+            for (const DevJob& J : b.jobs) tiles += tiled_tiles(TILED_STAGED, J.w, J.h);
+            b.tiled = staged_kind(tiles);
+        }
         rc = assemble_tiled(ctx, b.tiled, b, b.sstart, b.sgeom);
         // the staged sweep has one tiling; chosen tile shapes run the table sweep
-        if (rc == RCMVS_OK && b.tiled == TILED_STAGED && opts->tile_w == 0 && opts->tile_h == 0 &&
+        if (rc == RCMVS_OK && tiled_staged(b.tiled) && opts->tile_w == 0 && opts->tile_h == 0 &&
             !(opts->flags & (RCMVS_FLAG_AUTOTUNE | RCMVS_FLAG_PERSISTENT)))
             rc = assemble_tiled(ctx, TILED_INIT, b, b.istart, b.igeom);
     }

@@ -1195,17 +1195,12 @@ __global__ void __launch_bounds__(STREAM_THREADS, RCMVS_STREAM_MINB)
 // 69.0 ms streamed, 37.4 staged; 4 passes after the learned init over 16 views
 // 1920x1080, K = 10: 164 -> 90 ms; 12 passes over 8 views 384x288, K = 4:
 // 11.3 -> 4.4 ms.  Of the 37.4 ms, 7.1 are the preparation, 19 source 0.
-// Tiles of 16x16 in blocks of 128 threads at 64 registers (8 blocks = 32
+// Three tilings, by the batch's 16x16 tiles (staged_kind).  Large batches:
+// tiles of 16x16 in blocks of 128 threads at 64 registers (8 blocks = 32
 // warps an SM): 16x16 / 64 threads 43.9, 32x16 / 128 42.2, 32x32 / 256 42.3,
 // 16x16 / 256 40.8, 16x8 / 128 39.6, 16x8 / 64 39.7, at 80 registers 40.5 (each
 // against 40.1 or 38.9 for this choice in the same build).  Unrolling the
 // rows: 48.0 (spills).
-#ifndef RCMVS_STAGED_TW
-#define RCMVS_STAGED_TW 16
-#define RCMVS_STAGED_TH 16
-#define RCMVS_STAGED_THREADS 128
-#define RCMVS_STAGED_MINB 8
-#endif
 template <int TW_, int TH_, int THREADS_, int MINB_, int RES_>
 struct StagedCfg {
     static constexpr int TW = TW_, TH = TH_, THREADS = THREADS_, MINB = MINB_;
@@ -1564,7 +1559,22 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     }
 }
 
-using StagedDefault = StagedCfg<RCMVS_STAGED_TW, RCMVS_STAGED_TH, RCMVS_STAGED_THREADS, RCMVS_STAGED_MINB, 7>;
+using StagedDefault = StagedCfg<16, 16, 128, 8, 7>;
+// Where the last of few waves would leave SMs idle, tiles of half the pixels;
+// where there is less than about a wave, a block's own time counts, and two
+// threads share a pixel.  One pass of K = 3, by 16x16 tiles (default / MID /
+// SMALL): 80: 89 / 55 / 37 us; 300: 130 / 80 / 60; 1200: 186 / 145 / 138; 2760:
+// 281 / 235 / 247; 8280: 607 / 588 / 695; 14400: 1090 / 1085; 21600: 1834 / 1859.
+using StagedMid = StagedCfg<16, 8, 128, 8, 7>;
+using StagedSmall = StagedCfg<16, 8, 256, 4, 7>;
+constexpr int64_t STAGED_SMALL_TILES = 2000, STAGED_MID_TILES = 18000;
+
+template <class F>
+auto with_staged(int kind, F f) {
+    if (kind == TILED_STAGED_MID) return f(StagedMid{});
+    if (kind == TILED_STAGED_SMALL) return f(StagedSmall{});
+    return f(StagedDefault{});
+}
 __device__ __forceinline__ float hyp_depth(float inv_min, float inv_max, int hi, int nh) {
     const float inv = inv_min + (inv_max - inv_min) * (float)hi / (float)(nh - 1);  // stereo.rs:259-260
     return 1.0f / inv;
@@ -2549,17 +2559,25 @@ size_t stereo_smem_bytes(TileShape ts) { return smem_bytes(ts.tw, ts.th); }
 // Threads of a split-pass block for tiles of up to `px` pixels.
 int split_threads(int px) { return 32 * ((px + SPLIT_PX - 1) / SPLIT_PX); }
 
+int staged_kind(int64_t tiles) {
+    return tiles < STAGED_SMALL_TILES ? TILED_STAGED_SMALL : tiles < STAGED_MID_TILES ? TILED_STAGED_MID : TILED_STAGED;
+}
+
 int tiled_tiles(int kind, int w, int h) {
-    const int tw = kind == TILED_STREAM ? STREAM_TW : (kind == TILED_INIT ? StagedInit::TW : StagedDefault::TW);
-    const int th = kind == TILED_STREAM ? STREAM_TH : (kind == TILED_INIT ? StagedInit::TH : StagedDefault::TH);
-    return ((w + tw - 1) / tw) * ((h + th - 1) / th);
+    auto count = [&](int tw, int th) { return ((w + tw - 1) / tw) * ((h + th - 1) / th); };
+    if (kind == TILED_STREAM) return count(STREAM_TW, STREAM_TH);
+    if (kind == TILED_INIT) return count(StagedInit::TW, StagedInit::TH);
+    return with_staged(kind, [&](auto c) { return count(c.TW, c.TH); });
 }
 
 LaunchGeom tiled_geom(int kind, int tiles) {
     LaunchGeom g{STREAM_THREADS, stream_smem_bytes(), tiles, nullptr};
-    if (kind == TILED_STAGED) {
-        g.nthr = StagedDefault::THREADS;
-        g.smem = sizeof(StagedSmem<StagedDefault>);
+    if (tiled_staged(kind)) {
+        with_staged(kind, [&](auto c) {
+            g.nthr = c.THREADS;
+            g.smem = sizeof(StagedSmem<decltype(c)>);
+            return 0;
+        });
     } else if (kind == TILED_INIT) {
         g.nthr = StagedInit::THREADS;
         g.smem = sizeof(InitSmem<StagedInit>);
@@ -2570,8 +2588,8 @@ LaunchGeom tiled_geom(int kind, int tiles) {
 
 size_t tiled_scratch_bytes(int kind, int blocks) {
     const size_t b = kind == TILED_STREAM ? sizeof(float4) * STREAM_PX * 3
-                                          : (kind == TILED_INIT ? init_block_bytes<StagedInit>()
-                                                                : staged_block_bytes<StagedDefault>());
+                     : kind == TILED_INIT ? init_block_bytes<StagedInit>()
+                                          : with_staged(kind, [](auto c) { return staged_block_bytes<decltype(c)>(); });
     return b * (size_t)blocks;
 }
 
@@ -2604,10 +2622,11 @@ int tiled_grid(const LaunchGeom& g) {
     else if (g.tiled == TILED_INIT)
         n = g.radial ? launch_grid(init_staged_kernel<StagedInit, true>, q)
                      : launch_grid(init_staged_kernel<StagedInit, false>, q);
-    else if (g.radial)
-        n = launch_grid(pass_staged_kernel<StagedDefault, true>, q);
     else
-        n = launch_grid(pass_staged_kernel<StagedDefault, false>, q);
+        n = with_staged(g.tiled, [&](auto c) {
+            using C = decltype(c);
+            return g.radial ? launch_grid(pass_staged_kernel<C, true>, q) : launch_grid(pass_staged_kernel<C, false>, q);
+        });
     return std::max(n, 1);
 }
 
@@ -2645,10 +2664,14 @@ void pass_as(const DevJob* d_jobs, const int32_t* d_job_start, int n_jobs, const
             kernel<<<grid, g.nthr, g.smem, st>>>(d_jobs, d_job_start, n_jobs, g.tiles, g.queue, pass, sig_inv, sig_n,
                                                  census, rays, prev, next, g.scratch);
         };
-        if (g.radial)
-            run(pass_staged_kernel<StagedDefault, true>);
-        else
-            run(pass_staged_kernel<StagedDefault, false>);
+        with_staged(g.tiled, [&](auto c) {
+            using C = decltype(c);
+            if (g.radial)
+                run(pass_staged_kernel<C, true>);
+            else
+                run(pass_staged_kernel<C, false>);
+            return 0;
+        });
         return;
     }
     if (g.tpp == SPLIT) {
@@ -2703,7 +2726,7 @@ cudaError_t launch_pass(const DevJob* d_jobs, const int32_t* d_job_start, int n_
                         PlaneBuf prev, PlaneBuf next, unsigned long long* d_work, cudaStream_t st) {
     if (g.tiles <= 0) return cudaSuccess;
     if (g.tiled && (!g.queue || !g.scratch || g.scratch_blocks <= 0)) return cudaErrorInvalidValue;
-    if (g.tiled == TILED_STAGED && (d_work || !prev.d || !next.d)) return cudaErrorInvalidValue;
+    if (tiled_staged(g.tiled) && (d_work || !prev.d || !next.d)) return cudaErrorInvalidValue;
     if (d_work) {
         if (g.queue)
             pass_as<true, true>(d_jobs, d_job_start, n_jobs, g, pass, sig_inv, sig_n, census, rays, prev, next, d_work,
