@@ -140,6 +140,11 @@ cudaError_t launch_init_learned(const DevJob* d_jobs, const int32_t* d_job_start
                                 int nh, const uint64_t* census, const float2* rays, PlaneBuf out, const float* pred,
                                 const int64_t* pred_off, float logit_thr, int n_local, float span, bool sweep_seeded,
                                 unsigned long long* d_learned, cudaStream_t st);
+// The same by init_learned_staged_kernel over its own tiling (tiled_geom(TILED_INIT)).
+cudaError_t launch_init_learned_staged(const DevJob* d_jobs, const int32_t* d_tile_start, int n_jobs, const LaunchGeom& g,
+                                       int nh, const uint64_t* census, const float2* rays, PlaneBuf out,
+                                       const float* pred, const int64_t* pred_off, float logit_thr, int n_local,
+                                       float span, bool sweep_seeded, unsigned long long* d_learned, cudaStream_t st);
 // Texture/cost/range gate (stereo.rs:373-393); never persistent.
 cudaError_t launch_gate(const DevJob* d_jobs, const int32_t* d_job_start, int n_jobs, const LaunchGeom& g,
                         float cost_thr, const uint64_t* census, PlaneBuf planes, float* depth, float* cost,

@@ -371,8 +371,9 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
         SCK(sc->arena.get(kSlotStreamScratch, tiled_scratch_bytes(b.tiled, sgeom.scratch_blocks), &pscr));
         sgeom.scratch = (unsigned char*)pscr;
     }
-    // the default plane sweep, where the passes are staged too
-    const bool staged_init = s.init == Schedule::TABLE && !b.istart.empty() && !s.d_work && s.skip_duplicates;
+    // the default plane sweep and learned init, where the passes are staged too
+    const bool staged_init = (s.init == Schedule::TABLE || s.init == Schedule::LEARNED) && !b.istart.empty() &&
+                             !s.d_work && s.skip_duplicates;
     LaunchGeom igeom = b.igeom;
     void* pis = nullptr;
     if (staged_init) {
@@ -415,14 +416,17 @@ int run_batch(rcmvs_ctx* ctx, rcmvs_scene* sc, const StereoBatch& b, const Sched
         PlaneBuf A = A0, B = B0;
         g.queue = s.persistent ? queue : nullptr;
         hk.begin(s.init == Schedule::LEARNED ? "learned_init" : "stereo_init");
-        if (s.init == Schedule::LEARNED)
+        LaunchGeom gi = igeom;
+        gi.queue = queue;
+        if (s.init == Schedule::LEARNED && staged_init)
+            e = launch_init_learned_staged(dj, (const int32_t*)pis, n_jobs, gi, s.nh, sc->census, sc->rays, A, s.pred,
+                                           s.pred_off, s.logit_thr, s.n_local, s.span, s.sweep_seeded, s.d_learned, st);
+        else if (s.init == Schedule::LEARNED)
             e = launch_init_learned(dj, dst, n_jobs, g, s.nh, sc->census, sc->rays, A, s.pred, s.pred_off,
                                     s.logit_thr, s.n_local, s.span, s.sweep_seeded, s.d_learned, st);
-        else if (staged_init) {
-            LaunchGeom gi = igeom;
-            gi.queue = queue;
+        else if (staged_init)
             e = launch_init_staged(dj, (const int32_t*)pis, n_jobs, gi, s.nh, sc->census, sc->rays, A, st);
-        } else
+        else
             e = launch_init(dj, dst, n_jobs, g, s.nh, sc->census, sc->rays, A, s.d_work, st,
                             s.init == Schedule::ONE_CANDIDATE ? 1 : (s.init == Schedule::TABLE ? 2 : 0));
         hk.end(s.init == Schedule::LEARNED ? "learned_init" : "stereo_init");

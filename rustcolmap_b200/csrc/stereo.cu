@@ -2496,6 +2496,282 @@ __global__ void __launch_bounds__(256, 4)
     }
 }
 
+// The default (init_learned_rows_kernel serves the flags and tile shapes that
+// keep the staged kernels off; the same results).
+//   seeds   a tile's 4x4 pixels of one quarter cell share the cell's plane, so
+//           a block of pixels shares its 8x8 window cells' counts: per source a
+//           table of 64 floats, by the bounded projection (a Proj per block and
+//           source, eight sources at a time), then every pixel adds its 25;
+//   sweep   the pixels without a seed -- few, scattered -- put all
+//           hypotheses of a batch (1, 1, 2, 4, 8, 16, 16 ...) into the list, and
+//           run_stages packs them: (pixel, hypothesis) pairs fill the lanes that
+//           pixels alone would not.
+// Learned init of 16 views 1920x1080, K = 10, 97% seeded: 21.6 ms by rows (13.0
+// the seeds, with three divides per count and a search per table entry), 10.9 ms
+// here (6.1 the seeds).  Bound by instruction issue in the seeds, by the
+// latency of stages of few entries in the sweep.
+template <class C>
+struct LearnedSmem : StagedSmem<C> {
+    static constexpr int BX = C::TW / 4, BLOCKS = C::PX / 16, GROUP = 8;
+    static constexpr int PITCH = 68;  // 64 counts; neighbouring blocks four banks apart
+    static_assert(C::TW % 4 == 0 && C::TH % 4 == 0 && C::THREADS == 16 * BLOCKS, "blocks of 4x4 pixels");
+    float table[BLOCKS][PITCH];
+    Proj proj[GROUP][BLOCKS];
+    float4 plane[BLOCKS];
+    int active[BLOCKS];  // (plane, source) + 1 that some pixel of the block still evaluates
+    float depth[INIT_BATCH];
+};
+
+template <class C, bool RADIAL>
+__global__ void __launch_bounds__(C::THREADS, C::MINB)
+    init_learned_staged_kernel(const DevJob* __restrict__ jobs, const int32_t* __restrict__ stile_start, int n_jobs,
+                               int tiles, unsigned int* queue, int nh, const uint64_t* __restrict__ census,
+                               const float2* __restrict__ rays, PlaneBuf out, unsigned char* __restrict__ scratch,
+                               const float* __restrict__ pred, const int64_t* __restrict__ pred_off, float logit_thr,
+                               int n_local, float span, int sweep_seeded, unsigned long long* d_learned) {
+    static_assert(C::PX == C::THREADS, "one thread per pixel");
+    using S = LearnedSmem<C>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    S& sm = *reinterpret_cast<S*>(smem_raw);
+    float2* const lsum = reinterpret_cast<float2*>(scratch + (size_t)blockIdx.x * init_block_bytes<C>());
+    float2* const res = lsum + C::CAP;
+    const int tid = threadIdx.x;
+    constexpr int stw = C::STW;
+    for (int i = tid; i < 49; i += C::THREADS) sm.tab[i] = (float)i / 48.0f;
+    for (int it = 0;; ++it) {
+        const int tile = next_tile(queue, tiles, it, &sm.tile);
+        if (tile < 0) break;
+        const int j = find_item(stile_start, n_jobs, tile);
+        const DevJob* J = jobs + j;
+        const int w = J->w, h = J->h, nsrc = J->nsrc;
+        const int t = tile - stile_start[j];
+        const int stx = (w + C::TW - 1) / C::TW;
+        const int x0 = (t % stx) * C::TW, y0 = (t / stx) * C::TH;
+        const RayBox rb = stage_tile<C, RADIAL>(sm, J, x0, y0, census, rays);
+        const float total = 5.0f * 5.0f * (float)nsrc;
+        const float inv_min = J->inv_min, inv_max = J->inv_max, span_inv = inv_max - inv_min;
+        const int lx = tid % C::TW, ly = tid / C::TW, cell = ly * stw + lx;
+        const int blk = (ly >> 2) * S::BX + (lx >> 2);
+        const int x = x0 + lx, y = y0 + ly;
+        const bool inside = x < w && y < h;
+        // a block's rays differ from its middle one's by at most four steps each way
+        const RayBox rk{rb.rx, rb.ry, 1.001f * (4.0f * __int_as_float(sm.box[2]) + 4.0f * __int_as_float(sm.box[3]))};
+        if (tid < S::BLOCKS) sm.active[tid] = 0;
+        bool any_local = false, learned = false;
+        float best_c = INFINITY;
+        {
+            // this pixel's prediction, as in init_learned_rows_kernel
+            const float zlo = J->zmin * 0.5f, zhi = J->zmax * 2.0f;
+            const float2 ri = sm.ray[cell + HALO * stw + HALO];
+            float pnx = 0.f, pny = 0.f, pnz = 1.f, pa = 1.f, pac = 1.f, t0 = 0.f;
+            const int wq = w >> 2, hq = h >> 2;
+            if (inside && wq > 0 && hq > 0) {
+                const int qx = min(x >> 2, wq - 1), qy = min(y >> 2, hq - 1);
+                const float* o = pred + (pred_off[j] + (int64_t)qy * wq + qx) * NET_OUT_C;
+                const float len = sqrtf(o[1] * o[1] + o[2] * o[2] + o[3] * o[3]);
+                if (o[4] >= logit_thr && len > 1e-6f) {
+                    pnx = o[1] / len;
+                    pny = o[2] / len;
+                    pnz = o[3] / len;
+                    pa = pnx * ri.x + pny * ri.y + pnz;
+                    t0 = o[0];
+                    learned = pa >= 0.1f;
+                    const float2 rc = __ldg(rays + (size_t)J->off + (size_t)(4 * qy + 1) * w + 4 * qx + 1);
+                    pac = pnx * rc.x + pny * rc.y + pnz;
+                    learned = learned && pac >= 0.1f;
+                }
+            }
+            float4 plane = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+            float plane_d = 0.f;
+            for (int k = 0; k < n_local; ++k) {
+                bool ev = false;
+                float zi = 0.f, dcell = 0.f;
+                __syncthreads();  // sm.active is cleared; the last plane is no longer read
+                if (learned) {
+                    const float tk = t0 + span * ((float)k / (float)max(n_local - 1, 1) - 0.5f);
+                    const float inv = inv_min + tk * span_inv;
+                    if (inv > 0.f) {
+                        const float z = 1.f / inv;
+                        dcell = z * pac;
+                        zi = dcell / pa;
+                        ev = zi >= zlo && zi <= zhi;
+                        sm.plane[blk] = make_float4(pnx, pny, pnz, dcell);  // the same from every pixel of the block
+                    }
+                }
+                any_local = any_local || ev;
+                const float thr = (best_c + 0.02f) + 0.12f;  // +inf for the first plane
+                const float rej = reject_bound(best_c, total);
+                bool alive = ev;
+                float sum = 0.f;
+                for (int si = 0; si < nsrc; ++si) {
+                    const int epoch = k * 64 + si + 1, g = si % S::GROUP;
+                    if (alive) sm.active[blk] = epoch;
+                    if (!__syncthreads_or(alive)) break;  // also: the previous table is no longer read
+                    if (g == 0) {
+                        const int ng = min(S::GROUP, nsrc - si);
+                        for (int i = tid; i < ng * S::BLOCKS; i += C::THREADS) {
+                            const int b = i % S::BLOCKS, s = si + i / S::BLOCKS;
+                            if (sm.active[b] != epoch) continue;
+                            const int mid = ((b / S::BX) * 4 + 4) * stw + (b % S::BX) * 4 + 4;
+                            const float4 pl = sm.plane[b];
+                            Proj P;
+                            if (!make_proj<RADIAL>(load_src_fields(sm.sf, sm.scp[s], s), sm.pc[s], pl.x, pl.y, pl.z,
+                                                   pl.w, sm.ray[mid], rk, P))
+                                P.lu = -1.0f;
+                            sm.proj[s - si][b] = P;
+                        }
+                        __syncthreads();
+                    }
+                    if (sm.active[tid >> 4] == epoch) {
+                        // four cells of a column of the block, every other row
+                        const int b = tid >> 4, col = (b % S::BX) * 4 + (tid & 7);
+                        const int c0 = ((b / S::BX) * 4 + ((tid >> 3) & 1)) * stw + col;
+                        const uint64_t* __restrict__ sc = sm.scp[si];
+                        const Proj& Q = sm.proj[g][b];
+                        const f32x2 m0 = Q.m0, m1 = Q.m1, m2 = Q.m2, ch = Q.ch;
+                        const float z0 = Q.z0, z1 = Q.z1, z2 = Q.z2, lu = Q.lu, lv = Q.lv;
+                        const unsigned sw = Q.sw, sh = Q.sh;
+                        const uint64_t* __restrict__ sc1 = sc - (sw + 1u);
+                        f32x2 bx = 0;
+                        float bz = 0.0f;
+                        if (!RADIAL) {  // ray.x depends on the column alone
+                            const f32x2 rr = sm.colx[col];
+                            float rx, rx2;
+                            unpack2(rr, rx, rx2);
+                            bx = fma2(m0, rr, m2);
+                            bz = __fmaf_rn(z0, rx, z2);
+                        }
+                        unsigned near = 0;
+                        int hc[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int c = c0 + 2 * i * stw;
+                            f32x2 xy;
+                            float z;
+                            if (RADIAL) {
+                                const float2 r = sm.ray[c];
+                                xy = fma2(m0, pack2(r.x, r.x), fma2(m1, pack2(r.y, r.y), m2));
+                                z = __fmaf_rn(z0, r.x, __fmaf_rn(z1, r.y, z2));
+                            } else {
+                                const float ry = sm.ray[c].y;
+                                xy = fma2(m1, pack2(ry, ry), bx);
+                                z = __fmaf_rn(z1, ry, bz);
+                            }
+                            const float q1 = rcp_approx(z);
+                            const f32x2 uv = RADIAL ? proj_uv<true>(xy, q1, Q.f, Q.k, ch) : fma2(xy, pack2(q1, q1), ch);
+                            bool in;
+                            unsigned off;
+                            float du, dv;
+                            proj_floor(uv, sw, sh, in, off, du, dv);
+                            if (!(fabsf(du) <= lu && fabsf(dv) <= lv)) near |= 1u << i;
+                            const int hv = __popcll(sm.cen[c] ^ __ldg(sc1 + off));
+                            hc[i] = in ? hv : 48;
+                        }
+                        while (near) {
+                            const int e = __ffs(near) - 1;
+                            near &= near - 1;
+                            const int c = c0 + 2 * e * stw;
+                            const float4 pl = sm.plane[b];
+                            const int v = exact_index(load_src_fields(sm.sf, sc, si), sm.ray[c], pl.x, pl.y, pl.z, pl.w);
+                            const int hv = v < 0 ? 48 : __popcll(sm.cen[c] ^ __ldg(sc + max(v, 0)));
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) hc[i] = i == e ? hv : hc[i];
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) sm.table[b][16 * i + (tid & 15)] = sm.tab[hc[i]];
+                    }
+                    __syncthreads();
+                    if (alive) {
+                        const float* tb = sm.table[blk] + (ly & 3) * 8 + (lx & 3);
+#pragma unroll
+                        for (int dy = 0; dy < 5; ++dy) {
+#pragma unroll
+                            for (int dx = 0; dx < 5; ++dx) sum += tb[dy * 8 + dx];
+                            // nothing ends the first plane
+                            if (k > 0 && (mean_above(sum, abort_den(dy, si, nsrc, true), thr) || sum >= rej)) {
+                                alive = false;
+                                break;
+                            }
+                        }
+                    }
+                }
+                if (ev) {
+                    const float c = alive ? sum / total : 1e9f;
+                    if (c < best_c) {
+                        best_c = c;
+                        plane = make_float4(pnx, pny, pnz, zi);
+                        plane_d = dcell;
+                    }
+                }
+            }
+            const bool seeded = inside && learned && any_local;
+            if (seeded) {
+                const size_t i = (size_t)J->off + (size_t)y * w + x;
+                out.nz[i] = plane;
+                out.cost[i] = fminf(best_c, 1.0f);
+                out.d[i] = plane_d;
+            } else {
+                best_c = INFINITY;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, seeded);
+            if ((tid & 31) == 0 && bal) atomicAdd(d_learned, (unsigned long long)__popc(bal));
+            any_local = seeded;
+        }
+        // the sweep; a seeded pixel (sweep_seeded) starts from its proposal's cost
+        const bool sweep = inside && (!any_local || sweep_seeded);
+        const float seed_c = best_c;
+        float best_d = 0.f;
+        const int n_sweep = __syncthreads_count(sweep);
+        if (n_sweep == 0) continue;
+        sm.pcost[tid] = best_c;
+        // few pixels: batches that fill the block (more of them is evaluated under
+        // the looser limits, by lanes that would idle)
+        const int fill = min(C::THREADS / n_sweep, INIT_BATCH);
+        int h0 = 0, batch = max(1, fill);
+        while (h0 < nh && nsrc > 0) {
+            const int nb = min(batch, nh - h0);
+            __syncthreads();  // the previous batch's list and depths
+            if (tid < nb) sm.depth[tid] = hyp_depth(inv_min, inv_max, h0 + tid, nh);
+            if (tid == 0) sm.n = 0;
+            sm.done[tid] = 0;
+            __syncthreads();
+            if (sweep) {
+                const int at = atomicAdd(&sm.n, nb);
+                for (int q = 0; q < nb; ++q) sm.list[at + q] = (uint16_t)(tid | q << 10);
+            }
+            run_stages<C, RADIAL>(sm, 0, nsrc, total, rb, lsum, res, [&](int, int q, int, int) {
+                return make_float4(0.0f, 0.0f, 1.0f, sm.depth[q]);
+            });
+            __syncthreads();
+            for (unsigned m = sm.done[tid]; m; m &= m - 1) {  // the completed hypotheses in order
+                const int q = __ffs(m) - 1;
+                const float2 r = res[tid * C::RES + q];
+                if (!(r.x < best_c)) continue;
+                const float d = sm.depth[q];
+                if (best_c < sm.pcost[tid]) {  // improved within the batch: the tighter limits
+                    const float lim = (best_c + 0.02f) + 0.12f;
+                    if (r.y > lim * 1.000002f) continue;
+                    if (!(r.y < lim * 0.999998f) &&
+                        !staged_completes<C>(sm, cell, nsrc, make_float4(0.0f, 0.0f, 1.0f, d), lim,
+                                             reject_bound(best_c, total)))
+                        continue;
+                }
+                best_c = r.x;
+                best_d = d;
+            }
+            sm.pcost[tid] = best_c;
+            h0 += nb;
+            batch = max(min(h0, INIT_BATCH), fill);
+        }
+        if (sweep && (best_c < seed_c || !(seed_c < INFINITY))) {
+            const size_t i = (size_t)J->off + (size_t)y * w + x;
+            out.nz[i] = make_float4(0.0f, 0.0f, 1.0f, best_d);
+            out.cost[i] = fminf(best_c, 1.0f);
+            out.d[i] = best_d;
+        }
+    }
+}
+
 // ---------------------------------------------------------------- gate
 // stereo.rs:373-393 (+ normals, an extension)
 __global__ void gate_kernel(const DevJob* __restrict__ jobs, const int32_t* __restrict__ job_start, int n_jobs,
@@ -2718,6 +2994,28 @@ cudaError_t launch_init_staged(const DevJob* d_jobs, const int32_t* d_tile_start
         run(init_staged_kernel<StagedInit, true>);
     else
         run(init_staged_kernel<StagedInit, false>);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_init_learned_staged(const DevJob* d_jobs, const int32_t* d_tile_start, int n_jobs, const LaunchGeom& g,
+                                       int nh, const uint64_t* census, const float2* rays, PlaneBuf out,
+                                       const float* pred, const int64_t* pred_off, float logit_thr, int n_local,
+                                       float span, bool sweep_seeded, unsigned long long* d_learned, cudaStream_t st) {
+    if (g.tiles <= 0) return cudaSuccess;
+    if (g.tiled != TILED_INIT || !g.queue || !g.scratch || g.scratch_blocks <= 0 || !out.d) return cudaErrorInvalidValue;
+    static_assert(sizeof(LearnedSmem<StagedInit>) <= 48 * 1024, "shared memory of a plain launch");
+    LaunchGeom gl = g;
+    gl.smem = sizeof(LearnedSmem<StagedInit>);
+    auto run = [&](auto kernel) {
+        const int grid = std::min(launch_grid(kernel, gl), g.scratch_blocks);
+        kernel<<<grid, gl.nthr, gl.smem, st>>>(d_jobs, d_tile_start, n_jobs, g.tiles, g.queue, nh, census, rays, out,
+                                               g.scratch, pred, pred_off, logit_thr, n_local, span, (int)sweep_seeded,
+                                               d_learned);
+    };
+    if (g.radial)
+        run(init_learned_staged_kernel<StagedInit, true>);
+    else
+        run(init_learned_staged_kernel<StagedInit, false>);
     return cudaGetLastError();
 }
 
