@@ -56,6 +56,7 @@
 // of every row and column, 12 bytes each; no distance matrix is written)
 // fit P_BUDGET; results come back as per-pair lists in the reference's order
 // (ascending index in A).
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -82,6 +83,7 @@ struct PairJob {
     int32_t na, nb;
     int32_t row_off, col_off;  // into the chunk's forward / backward results
     int32_t fa, fb;            // frames
+    int32_t pair;              // of the chunk
 };
 
 struct Nearest {
@@ -263,24 +265,25 @@ struct MatchStatus {
 // [descriptor][8], a canonical K-major operand.  Past the frame's end:
 // zeros with an infinite norm.
 __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ desc, const Frame* __restrict__ frames,
-                                                   const int32_t* __restrict__ blk_start, int n_frames,
+                                                   const int32_t* __restrict__ blk_start, int n_frames, int first,
                                                    unsigned char* __restrict__ packed, float* __restrict__ norms,
                                                    int* __restrict__ max_norm, MatchStatus* __restrict__ st) {
     __shared__ float part[2][QB];
+    const int block = first + (int)blockIdx.x;
     int lo = 0, hi = n_frames - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (blk_start[mid] <= (int)blockIdx.x)
+        if (blk_start[mid] <= block)
             lo = mid;
         else
             hi = mid - 1;
     }
     const Frame F = frames[lo];
     const int r = threadIdx.x & (QB - 1), half = threadIdx.x >> 7;
-    const int row = ((int)blockIdx.x - blk_start[lo]) * QB + r;
+    const int row = (block - blk_start[lo]) * QB + r;
     const bool in = row < F.n;
     const float* src = desc + (F.off + row) * DESC_LEN;
-    unsigned char* out = packed + (size_t)blockIdx.x * QB_BYTES + r * 16;
+    unsigned char* out = packed + (size_t)block * QB_BYTES + r * 16;
     float sum = 0.0f;
     bool wild = false;
 #pragma unroll
@@ -308,7 +311,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ des
     __syncthreads();
     if (half == 0) {
         const float n = part[0][r] + part[1][r];
-        norms[(size_t)blockIdx.x * QB + r] = in ? n : INFINITY;
+        norms[(size_t)block * QB + r] = in ? n : INFINITY;
         float m = in ? n : 0.0f;
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         if ((threadIdx.x & 31) == 0) atomicMax(&max_norm[lo], __float_as_int(m));  // norms are not negative
@@ -593,6 +596,69 @@ __global__ void mutual_kernel(const PairJob* __restrict__ jobs, const uint32_t* 
     match_b[J.row_off + ia] = f != UINT32_MAX && bwd[J.col_off + f] == (uint32_t)ia ? f : UINT32_MAX;
 }
 
+// The matches of a chunk packed in pair order: how many each pair has, where
+// they begin, and (second pass) the indices.  From COMPACT_MIN rows on: 135 k
+// rows of 66 pairs collected on the host from one entry per row took 400 us of
+// 1760.
+constexpr int64_t COMPACT_MIN = 16384;
+__device__ __forceinline__ int block_matches(const uint32_t* __restrict__ mb, int na, int base, uint32_t& b) {
+    const int ia = base + (int)threadIdx.x;
+    b = ia < na ? mb[ia] : UINT32_MAX;
+    return __syncthreads_count(b != UINT32_MAX);
+}
+__global__ void __launch_bounds__(256) count_kernel(const PairJob* __restrict__ jobs, const uint32_t* __restrict__ match_b,
+                                                    uint32_t* __restrict__ counts) {
+    const PairJob J = jobs[blockIdx.x];
+    int n = 0;
+    uint32_t b;
+    for (int base = 0; base < J.na; base += 256) n += block_matches(match_b + J.row_off, J.na, base, b);
+    if (threadIdx.x == 0) counts[J.pair] = (uint32_t)n;
+}
+__global__ void __launch_bounds__(1024) begin_kernel(const uint32_t* __restrict__ counts, int n, uint32_t* __restrict__ begin) {
+    __shared__ uint32_t s_sum[1024];
+    uint32_t before = 0;
+    for (int base = 0; base < n; base += 1024) {
+        const int i = base + (int)threadIdx.x;
+        const uint32_t c = i < n ? counts[i] : 0;
+        s_sum[threadIdx.x] = c;
+        __syncthreads();
+        for (int o = 1; o < 1024; o <<= 1) {
+            const uint32_t v = (int)threadIdx.x >= o ? s_sum[threadIdx.x - o] : 0;
+            __syncthreads();
+            s_sum[threadIdx.x] += v;
+            __syncthreads();
+        }
+        if (i < n) begin[i] = before + s_sum[threadIdx.x] - c;
+        before += s_sum[1023];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) begin[n] = before;
+}
+__global__ void __launch_bounds__(256) compact_kernel(const PairJob* __restrict__ jobs,
+                                                      const uint32_t* __restrict__ match_b,
+                                                      const uint32_t* __restrict__ begin, uint32_t* __restrict__ a,
+                                                      uint32_t* __restrict__ b) {
+    __shared__ int s_warp[8];
+    const PairJob J = jobs[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    size_t at = begin[J.pair];
+    for (int base = 0; base < J.na; base += 256) {
+        uint32_t v;
+        const int n = block_matches(match_b + J.row_off, J.na, base, v);
+        const unsigned m = __ballot_sync(0xffffffffu, v != UINT32_MAX);
+        if (lane == 0) s_warp[warp] = __popc(m);
+        __syncthreads();
+        int before = __popc(m & ((1u << lane) - 1u));
+        for (int k = 0; k < warp; ++k) before += s_warp[k];
+        if (v != UINT32_MAX) {
+            a[at + before] = (uint32_t)(base + (int)threadIdx.x);
+            b[at + before] = v;
+        }
+        at += n;
+        __syncthreads();
+    }
+}
+
 // matching.rs:74-94
 __global__ void decide_kernel(const PairJob* __restrict__ jobs, const Nearest* __restrict__ fwd,
                               const Nearest* __restrict__ bwd, float ratio, uint32_t* __restrict__ match_b) {
@@ -622,13 +688,24 @@ int mfail(rcmvs_ctx* ctx, int code, const std::string& msg) {
     } while (0)
 
 // Context arena slots 160-175.
-enum { M_DESC = 160, M_JOBS, M_ROWP, M_FWD, M_BWD, M_MB, M_COLP, M_FRAMES, M_PACK, M_NORM, M_MAXN, M_TWO, M_LIST, M_STATUS };
+enum { M_DESC = 160, M_JOBS, M_ROWP, M_FWD, M_BWD, M_MB, M_COLP, M_FRAMES, M_PACK, M_NORM, M_MAXN, M_TWO, M_LIST, M_STATUS, M_BEGIN, M_AB };
 
 // Chunks of fewer distances run on the FP32 pipes: there the tensor-core
 // search's extra launches cost more than its products save.  Whole calls,
 // FP32 / tensor: one pair of 512 122 / 145 us, of 1024 158 / 179, of 2048 290 /
-// 275; 10 pairs of up to 1100 385 / 301, 66 pairs of 2048 5350 / 1760.
+// 275; 10 pairs of up to 1100 385 / 301, 66 pairs of 2048 5350 / 1315.
 constexpr int64_t TENSOR_MIN = int64_t(1) << 22;
+constexpr int64_t GROUP_BYTES = 1 << 20;  // descriptors uploaded between two searches
+
+struct Event {  // no upload is left in flight when a call returns early
+    cudaEvent_t e = nullptr;
+    cudaStream_t stream = nullptr;
+    ~Event() {
+        if (!e) return;
+        cudaStreamSynchronize(stream);
+        cudaEventDestroy(e);
+    }
+};
 
 }  // namespace
 }  // namespace rcmvs
@@ -680,10 +757,11 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
     DeviceArena& A = ctx->arena;
     void* p_desc;
     MCK(A.get(M_DESC, sizeof(float) * DESC_LEN * (size_t)std::max<int64_t>(foff[n_frames], 1), &p_desc));
-    for (int f = 0; f < n_frames; ++f)
-        if (n_desc[f] > 0)
-            MCK(cudaMemcpyAsync((float*)p_desc + foff[f] * DESC_LEN, desc[f], sizeof(float) * DESC_LEN * n_desc[f],
-                                cudaMemcpyHostToDevice, st));
+    auto upload = [&](int f, cudaStream_t on) -> cudaError_t {
+        if (n_desc[f] == 0) return cudaSuccess;
+        return cudaMemcpyAsync((float*)p_desc + foff[f] * DESC_LEN, desc[f], sizeof(float) * DESC_LEN * n_desc[f],
+                               cudaMemcpyHostToDevice, on);
+    };
     const float r32 = (float)ratio;
     // the tensor-core search's packed frames (made with the first chunk that uses it)
     std::vector<Frame> frames(n_frames);
@@ -696,6 +774,31 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
     // tensor: no frame was found out of range (and a ratio the bound's tests take)
     bool packed = false, tensor = r32 > 0.0f && r32 < 1e6f;
     void *p_frames = nullptr, *p_blk = nullptr, *p_pack = nullptr, *p_norm = nullptr, *p_maxn = nullptr, *p_st = nullptr;
+    // Where all pairs make one chunk for the tensor-core search, the frames go
+    // up on the context's second stream in groups, and a group is packed and
+    // its pairs with the frames before it are searched while the next is
+    // copied.  66 pairs of 12 frames of 2048, with the packed matches: 1760 -> 1315 us.
+    bool overlap = false;
+    if (tensor && n_pairs <= 32767 && foff[n_frames] * (int64_t)sizeof(float) * DESC_LEN >= 2 * GROUP_BYTES) {
+        int64_t dists = 0, partials = 0, rows = 0, cols = 0;
+        for (int p = 0; p < n_pairs && rows <= INT32_MAX / 2 && cols <= INT32_MAX / 2; ++p) {
+            const int64_t na = n_desc[pairs[2 * p]], nb = n_desc[pairs[2 * p + 1]];
+            partials += (nb + TILE - 1) / TILE * na + (na + TILE - 1) / TILE * nb;
+            dists += na * nb;
+            rows += na;
+            cols += nb;
+        }
+        overlap = dists >= TENSOR_MIN && (size_t)partials * sizeof(Nearest) <= P_BUDGET && rows <= INT32_MAX / 2 &&
+                  cols <= INT32_MAX / 2;
+    }
+    Event uploaded;
+    if (overlap) {
+        if (!ctx->upload) MCK(cudaStreamCreateWithFlags(&ctx->upload, cudaStreamNonBlocking));
+        MCK(cudaEventCreateWithFlags(&uploaded.e, cudaEventDisableTiming));
+        uploaded.stream = ctx->upload;
+    } else {
+        for (int f = 0; f < n_frames; ++f) MCK(upload(f, st));
+    }
     int p = 0;
     while (p < n_pairs) {
         // a chunk of pairs whose distance matrices fit the budget (at least one)
@@ -707,7 +810,8 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
             const int na = n_desc[fa], nb = n_desc[fb];
             const int64_t pr = (int64_t)((nb + TILE - 1) / TILE) * na, pc = (int64_t)((na + TILE - 1) / TILE) * nb;
             if (!jobs.empty() && (size_t)(prow + pr + pcol + pc) * sizeof(Nearest) > P_BUDGET) break;
-            jobs.push_back(PairJob{foff[fa], foff[fb], prow, pcol, na, nb, (int32_t)rows, (int32_t)cols, fa, fb});
+            jobs.push_back(PairJob{foff[fa], foff[fb], prow, pcol, na, nb, (int32_t)rows, (int32_t)cols, fa, fb,
+                                   (int32_t)jobs.size()});
             dists += (int64_t)na * nb;
             prow += pr;
             pcol += pc;
@@ -725,10 +829,37 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
             MCK(A.get(M_FWD, sizeof(Nearest) * (size_t)rows, &p_fwd));
             MCK(A.get(M_BWD, sizeof(Nearest) * (size_t)cols, &p_bwd));
             MCK(A.get(M_MB, sizeof(uint32_t) * (size_t)rows, &p_mb));
-            MCK(cudaMemcpyAsync(p_jobs, jobs.data(), sizeof(PairJob) * jobs.size(), cudaMemcpyHostToDevice, st));
+            // on the device in the order in which their frames arrive
+            std::vector<PairJob> queue(jobs);
+            if (overlap)
+                std::stable_sort(queue.begin(), queue.end(), [](const PairJob& x, const PairJob& y) {
+                    return std::max(x.fa, x.fb) < std::max(y.fa, y.fb);
+                });
+            MCK(cudaMemcpyAsync(p_jobs, queue.data(), sizeof(PairJob) * jobs.size(), cudaMemcpyHostToDevice, st));
             const unsigned nj = (unsigned)jobs.size();
             const SpanHook& hook = ctx->hook();
-            std::vector<uint32_t> mb((size_t)rows);
+            const bool compact = rows >= COMPACT_MIN;
+            std::vector<uint32_t> mb(compact ? 0 : (size_t)rows), begin(compact ? jobs.size() + 1 : 0);
+            void *p_begin = nullptr, *p_ab = nullptr;
+            if (compact) {
+                MCK(A.get(M_BEGIN, sizeof(uint32_t) * (2 * jobs.size() + 1), &p_begin));
+                MCK(A.get(M_AB, sizeof(uint32_t) * 2 * (size_t)rows, &p_ab));
+            }
+            // the answers' counts, or the answers, to the host
+            auto collect = [&]() -> cudaError_t {
+                if (!compact)
+                    return cudaMemcpyAsync(mb.data(), p_mb, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, st);
+                uint32_t* d_begin = (uint32_t*)p_begin;
+                uint32_t* d_count = d_begin + jobs.size() + 1;
+                count_kernel<<<nj, 256, 0, st>>>((const PairJob*)p_jobs, (const uint32_t*)p_mb, d_count);
+                begin_kernel<<<1, 1024, 0, st>>>(d_count, (int)nj, d_begin);
+                compact_kernel<<<nj, 256, 0, st>>>((const PairJob*)p_jobs, (const uint32_t*)p_mb, d_begin, (uint32_t*)p_ab,
+                                                   (uint32_t*)p_ab + rows);
+                const cudaError_t e = cudaGetLastError();
+                return e != cudaSuccess ? e
+                                        : cudaMemcpyAsync(begin.data(), p_begin, sizeof(uint32_t) * begin.size(),
+                                                          cudaMemcpyDeviceToHost, st);
+            };
             bool on_tensor = tensor && dists >= TENSOR_MIN;
             if (on_tensor) {
                 void *p_two, *p_list;
@@ -755,22 +886,55 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                 const Frame* df = (const Frame*)p_frames;
                 MatchStatus* ds = (MatchStatus*)p_st;
                 hook.begin("match_dist");
-                if (!packed) {
-                    pack_kernel<<<blk[n_frames], 256, 0, st>>>((const float*)p_desc, df, (const int32_t*)p_blk, n_frames,
-                                                               (unsigned char*)p_pack, (float*)p_norm, (int*)p_maxn, ds);
-                    MCK(cudaGetLastError());
-                    packed = true;
-                }
+                auto pack = [&](int f0, int f1) -> cudaError_t {
+                    if (blk[f1] == blk[f0]) return cudaSuccess;
+                    pack_kernel<<<blk[f1] - blk[f0], 256, 0, st>>>((const float*)p_desc, df, (const int32_t*)p_blk,
+                                                                   n_frames, blk[f0], (unsigned char*)p_pack,
+                                                                   (float*)p_norm, (int*)p_maxn, ds);
+                    return cudaGetLastError();
+                };
+                auto nearest = [&](size_t j0, size_t j1) -> cudaError_t {
+                    // two query blocks per CTA share each target block's load; one when
+                    // that would leave SMs without a CTA
+                    int64_t qblocks = 0;
+                    int most = 0;
+                    for (size_t k = j0; k < j1; ++k) {
+                        const int qa = (queue[k].na + QB - 1) / QB, qb = (queue[k].nb + QB - 1) / QB;
+                        qblocks += qa + qb;
+                        most = std::max(most, std::max(qa, qb));
+                    }
+                    if (qblocks == 0) return cudaSuccess;
+                    const int per = qblocks >= 2 * 148 ? 2 : 1;
+                    nearest_kernel<<<dim3((most + per - 1) / per, 2 * (unsigned)(j1 - j0)), kNearestThreads, kNearestSmem,
+                                     st>>>(dj + j0, df, (const unsigned char*)p_pack, (const float*)p_norm, per, f2, b2,
+                                           ds);
+                    return cudaGetLastError();
+                };
                 const int max_n = std::max(max_na, max_nb);
-                // two query blocks per CTA share each target block's load; one when
-                // that would leave SMs without a CTA
-                int64_t qblocks = 0;
-                for (const PairJob& j : jobs) qblocks += (j.na + QB - 1) / QB + (j.nb + QB - 1) / QB;
-                const int per = qblocks >= 2 * 148 ? 2 : 1;
-                const int max_blk = (max_n + QB - 1) / QB;
-                nearest_kernel<<<dim3((max_blk + per - 1) / per, 2 * nj), kNearestThreads, kNearestSmem, st>>>(
-                    dj, df, (const unsigned char*)p_pack, (const float*)p_norm, per, f2, b2, ds);
-                MCK(cudaGetLastError());
+                if (overlap) {
+                    // earlier work on the descriptors' buffer ends before they are written
+                    MCK(cudaEventRecord(uploaded.e, st));
+                    MCK(cudaStreamWaitEvent(ctx->upload, uploaded.e, 0));
+                    size_t j0 = 0;
+                    for (int f0 = 0, f1; f0 < n_frames; f0 = f1) {
+                        int64_t bytes = 0;
+                        for (f1 = f0; f1 < n_frames && bytes < GROUP_BYTES; ++f1) {
+                            MCK(upload(f1, ctx->upload));
+                            bytes += (int64_t)sizeof(float) * DESC_LEN * n_desc[f1];
+                        }
+                        MCK(cudaEventRecord(uploaded.e, ctx->upload));
+                        MCK(cudaStreamWaitEvent(st, uploaded.e, 0));
+                        MCK(pack(f0, f1));
+                        size_t j1 = j0;
+                        while (j1 < queue.size() && std::max(queue[j1].fa, queue[j1].fb) < f1) ++j1;
+                        MCK(nearest(j0, j1));
+                        j0 = j1;
+                    }
+                } else {
+                    if (!packed) MCK(pack(0, n_frames));
+                    MCK(nearest(0, queue.size()));
+                }
+                packed = true;
                 hook.end("match_dist");
                 hook.begin("match_select");
                 outcome_kernel<<<dim3((max_n + 255) / 256, 2 * nj), 256, 0, st>>>(
@@ -784,7 +948,7 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                 hook.end("match_select");
                 MatchStatus status{};
                 MCK(cudaMemcpyAsync(&status, p_st, sizeof(status), cudaMemcpyDeviceToHost, st));
-                MCK(cudaMemcpyAsync(mb.data(), p_mb, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, st));
+                MCK(collect());
                 MCK(cudaStreamSynchronize(st));
                 if (status.fault) return mfail(ctx, RCMVS_E_CUDA, "rcmvs_match_pairs: a tensor-core wait timed out");
                 if (status.wild) tensor = false;
@@ -809,8 +973,21 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                     (const PairJob*)p_jobs, (const Nearest*)p_fwd, (const Nearest*)p_bwd, r32, (uint32_t*)p_mb);
                 MCK(cudaGetLastError());
                 hook.end("match_select");
-                MCK(cudaMemcpyAsync(mb.data(), p_mb, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, st));
+                MCK(collect());
                 MCK(cudaStreamSynchronize(st));
+            }
+            if (compact) {
+                const size_t had = ra.size(), n = begin.back();
+                ra.resize(had + n);
+                rb.resize(had + n);
+                if (n) {
+                    MCK(cudaMemcpyAsync(ra.data() + had, p_ab, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st));
+                    MCK(cudaMemcpyAsync(rb.data() + had, (uint32_t*)p_ab + rows, sizeof(uint32_t) * n,
+                                        cudaMemcpyDeviceToHost, st));
+                    MCK(cudaStreamSynchronize(st));
+                }
+                for (size_t c = 0; c < jobs.size(); ++c) out->offsets[first + c + 1] = had + begin[c + 1];
+                continue;
             }
             for (size_t c = 0; c < jobs.size(); ++c) {
                 for (int ia = 0; ia < jobs[c].na; ++ia) {
