@@ -92,25 +92,57 @@ __global__ void taps_kernel(int32_t n, int32_t m, int32_t maxt, int32_t* __restr
     count[o] = cnt;
 }
 
-// tmp[(y * w + x) * nc + c] for output row y, input column x, channel c < nc
-// of an input with `channels` bytes per pixel.
-__global__ void vert_kernel(const uint8_t* __restrict__ img, int32_t w, int32_t channels, int32_t nc, int32_t mh,
-                            const int32_t* __restrict__ first, const int32_t* __restrict__ count,
-                            const float* __restrict__ weight, int32_t maxt, float* __restrict__ tmp) {
-    const int64_t row = (int64_t)w * nc;
-    const int64_t total = row * mh;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int y = (int)(i / row);
-        const int64_t j = i - (int64_t)y * row;
-        const int x = (int)(j / nc), c = (int)(j - (int64_t)x * nc);
-        const int l = first[y], cnt = count[y];
-        const float* wy = weight + (size_t)y * maxt;
-        const uint8_t* src = img + ((int64_t)l * w + x) * channels + c;
-        const int64_t step = (int64_t)w * channels;
-        float t = 0.0f;
-        for (int k = 0; k < cnt; ++k) t = __fadd_rn(t, __fmul_rn((float)src[k * step], wy[k]));
-        tmp[i] = t;
+// tmp[(y * w + x) * NC + c] for output row y, input column x, channel c < NC
+// of an input with `channels` bytes per pixel.  A block takes RT_COLS elements of
+// a row, a thread four neighbours; VEC: the pixels are the NC channels and rows
+// start at multiples of four elements, so that four bytes load and four floats
+// store at once.  4000x3000 RGB to 1440 rows: 197 us with an element per thread
+// and its divisions, 44 us.
+constexpr int RT_THREADS = 128, RT_COLS = 4 * RT_THREADS;
+template <int NC, bool VEC>
+__global__ void __launch_bounds__(RT_THREADS) vert_kernel(const uint8_t* __restrict__ img, int32_t w, int32_t channels,
+                                                          int32_t chunks, const int32_t* __restrict__ first,
+                                                          const int32_t* __restrict__ count,
+                                                          const float* __restrict__ weight, int32_t maxt,
+                                                          float* __restrict__ tmp) {
+    const int y = (int)(blockIdx.x / (unsigned)chunks);
+    const int row = w * NC, step = w * channels;
+    const int j = ((int)(blockIdx.x - (unsigned)y * chunks) * RT_THREADS + (int)threadIdx.x) * 4;
+    if (j >= row) return;
+    const int l = first[y], cnt = count[y];
+    const float* wy = weight + (size_t)y * maxt;
+    const uint8_t* src = img + (int64_t)l * step;
+    float* out = tmp + (int64_t)y * row + j;
+    float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (VEC) {
+        src += j;
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) {
+            const uchar4 q = __ldg(reinterpret_cast<const uchar4*>(src + (int64_t)k * step));
+            const float wk = __ldg(wy + k);
+            t[0] = __fadd_rn(t[0], __fmul_rn((float)q.x, wk));
+            t[1] = __fadd_rn(t[1], __fmul_rn((float)q.y, wk));
+            t[2] = __fadd_rn(t[2], __fmul_rn((float)q.z, wk));
+            t[3] = __fadd_rn(t[3], __fmul_rn((float)q.w, wk));
+        }
+        *reinterpret_cast<float4*>(out) = make_float4(t[0], t[1], t[2], t[3]);
+    } else {
+        int at[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int x = min(j + e, row - 1) / NC;
+            at[e] = x * channels + min(j + e, row - 1) - x * NC;
+        }
+#pragma unroll 2
+        for (int k = 0; k < cnt; ++k) {
+            const float wk = __ldg(wy + k);
+            const uint8_t* s = src + (int64_t)k * step;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) t[e] = __fadd_rn(t[e], __fmul_rn((float)__ldg(s + at[e]), wk));
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (j + e < row) out[e] = t[e];
     }
 }
 
@@ -127,17 +159,20 @@ __global__ void horiz_kernel(const float* __restrict__ tmp, int32_t w, int32_t m
     const int64_t total = (int64_t)mw * mh;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int y = (int)(i / mw), x = (int)(i - (int64_t)y * mw);
+        const int y = (int)((uint32_t)i / (uint32_t)mw), x = (int)((uint32_t)i - (uint32_t)y * (uint32_t)mw);
         const int l = first[x], cnt = count[x];
         const float* wx = weight + (size_t)x * maxt;
         const float* src = tmp + ((int64_t)y * w + l) * NC;
+        float t[NC] = {};
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) {
+            const float wk = __ldg(wx + k);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) t[c] = __fadd_rn(t[c], __fmul_rn(__ldg(src + k * NC + c), wk));
+        }
         uint8_t v[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            float t = 0.0f;
-            for (int k = 0; k < cnt; ++k) t = __fadd_rn(t, __fmul_rn(src[k * NC + c], wx[k]));
-            v[c] = to_u8(t);
-        }
+        for (int c = 0; c < NC; ++c) v[c] = to_u8(t[c]);
         if constexpr (NC == 1) {
             gray[i] = v[0];
             rgb[3 * i] = rgb[3 * i + 1] = rgb[3 * i + 2] = v[0];
@@ -225,8 +260,16 @@ int resize_device(rcmvs_ctx* ctx, const uint8_t* d_in, int w, int h, int channel
     RCK(cudaGetLastError());
     taps_kernel<<<(mw + 127) / 128, 128, 0, st>>>(w, mw, th, hfirst, hfirst + mw, (float*)p_hw, (int*)p_err);
     RCK(cudaGetLastError());
-    vert_kernel<<<grid_for((int64_t)w * nc * mh), 256, 0, st>>>(d_in, w, channels, nc, mh, vfirst, vfirst + mh,
-                                                                 (const float*)p_vw, tv, (float*)p_tmp);
+    const int chunks = (w * nc + RT_COLS - 1) / RT_COLS;
+    auto vert = [&](auto kernel) {
+        kernel<<<(unsigned)chunks * (unsigned)mh, RT_THREADS, 0, st>>>(d_in, w, channels, chunks, vfirst, vfirst + mh,
+                                                                       (const float*)p_vw, tv, (float*)p_tmp);
+    };
+    const bool vec = channels == nc && (w * nc) % 4 == 0;
+    if (nc == 1)
+        vec ? vert(vert_kernel<1, true>) : vert(vert_kernel<1, false>);
+    else
+        vec ? vert(vert_kernel<3, true>) : vert(vert_kernel<3, false>);
     RCK(cudaGetLastError());
     if (nc == 1)
         horiz_kernel<1><<<grid_for(n_out), 256, 0, st>>>((const float*)p_tmp, w, mw, mh, hfirst, hfirst + mw,
