@@ -46,11 +46,10 @@ sys.path.insert(0, ROOT)
 
 FP32_NOMINAL_TOPS = 148 * 128 * 1.965e9 / 1e12  # SMs x FP32 lanes x max clock (ops/s, no FMA pairing)
 # DRAM bytes (read + write) per reference pixel of one pass launch, from an
-# ncu capture of the streamed pass kernel on 12 views at 1920x1080, K = 10
-# (learned arm, pass 2: 2.573 GB read + 1.300 GB written over 24.88 Mpx),
-# scaled to the measured workload's pixels for roofline.traffic.
-PASS_DRAM_BYTES_PER_PX = (2572771000 + 1299575000) / (12 * 1920 * 1080)
-
+# ncu capture of the staged pass kernel on 8 views at 960x720, K = 10 (learned
+# arm, mean of passes 0 and 1: 335.3 MB read + 172.3 MB written over 5.53
+# Mpx), scaled to the measured workload's pixels for roofline.traffic.
+PASS_DRAM_BYTES_PER_PX = (335305856 + 172263320) / (8 * 960 * 720)
 
 def configs():
     from rustcolmap_b200 import MvsOptions
@@ -436,7 +435,11 @@ def run_sfm(args):
         c.timing(False)
     frames, m = state["frames"], state["matches"]
     nfeat = [len(f.pts) for f in frames]
-    ops = sum(nfeat[i] * nfeat[j] for i, j in pairs) * 128 * 3  # sub, mul, add per component
+    # the search makes three FP16 products of 128 components per distance, in each direction
+    ops = sum(nfeat[i] * nfeat[j] for i, j in pairs) * 128 * 2 * 3 * 2
+    pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    peaks = json.load(open(pk)) if os.path.exists(pk) else {}
+    tensor_peak = peaks.get("bf16_tflops", 1590.0)
     dist_ms, dist_n = kt["match_dist"]
     dist_launch_ms = dist_ms / max(dist_n, 1)
     ops_per_launch = ops * args.steps / max(dist_n, 1)
@@ -451,9 +454,10 @@ def run_sfm(args):
                        "sift_workers": nw,
                        "features_mean": float(np.mean(nfeat)),
                        "matches_mean": float(np.mean([len(a) for a, _ in m]))},
-            "roofline": {"bound": "fp32_issue", "kernel": "match_dist", "achieved": achieved,
-                         "peak": FP32_NOMINAL_TOPS, "unit": "Top/s", "frac": achieved / FP32_NOMINAL_TOPS,
-                         "traffic": None, "peak_source": "nominal 148 SM x 128 FP32 lanes x 1.965 GHz",
+            "roofline": {"bound": "tensor", "kernel": "match_dist", "achieved": achieved,
+                         "peak": tensor_peak, "unit": "TFLOP/s", "frac": achieved / tensor_peak,
+                         "traffic": None,
+                         "peak_source": "MEASURED_PEAKS.json bf16_tflops" if peaks else "fallback 1590",
                          "ops_per_launch": ops_per_launch, "avg_launch_ms": dist_launch_ms},
             "kernel_ms_per_step": {k: v[0] / args.steps for k, v in kt.items()},
             "e2e": {"value": value, "unit": "images/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
@@ -781,8 +785,8 @@ def main():
             "roofline": {"bound": "hbm", "kernel": "stereo_pass", "achieved": achieved_gbs, "peak": hbm_peak,
                          "unit": "GB/s", "frac": achieved_gbs / hbm_peak,
                          "traffic": PASS_DRAM_BYTES_PER_PX * npx,
-                         "traffic_source": "ncu dram bytes per pixel of a 12-view 1920x1080 K=10 capture of "
-                                           "the streamed pass kernel (learned arm) x this launch's pixels",
+                         "traffic_source": "ncu dram bytes per pixel of an 8-view 960x720 K=10 capture of "
+                                           "the staged pass kernel (learned arm) x this launch's pixels",
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650",
                          "algorithmic_bytes_per_launch": bytes_per_launch, "avg_launch_ms": pass_avg_s * 1e3,
                          "note": "issue-bound kernel: see compute_roofline"},

@@ -133,7 +133,8 @@ typedef struct rcmvs_options {
  * view goes through the others, packed.  With a tile shape chosen (tile_w /
  * tile_h, RCMVS_FLAG_AUTOTUNE), RCMVS_FLAG_PERSISTENT, work counting,
  * RCMVS_FLAG_NO_SKIP_DUPLICATES or RCMVS_FLAG_LOCKSTEP_PASSES the table sweep
- * runs, which has such counts for every support view a pixel still needs.
+ * runs, which has such counts for every support view a pixel still needs;
+ * under the same conditions the learned init runs by rows instead of staged.
  * This flag selects the row-step sweep instead (each lane streams its own hypotheses
  * one window row at a time).  Same results bit for bit. */
 #define RCMVS_FLAG_ROW_STEP_INIT 128u
@@ -153,7 +154,7 @@ typedef struct rcmvs_options {
 /* The Jacobi passes run one thread per pixel in lockstep (tiles of
  * tile_w x tile_h): a warp runs each candidate slot for as long as its
  * slowest lane needs.  By default (threads_per_pixel 0 or 1) a pass is
- * staged: the candidates of a 16x16 tile go through the support views
+ * staged: the candidates of a 16x16 tile (16x8 in small batches) go through the support views
  * together, one view per stage, and the survivors are packed before the
  * next; a window term whose pixel a bounded projection is certain of skips
  * the reference's divide chain.  With RCMVS_COUNT set or
