@@ -168,5 +168,5 @@ class Owned:
         buf.owner = self
         return np.ctypeslib.as_array(buf).reshape(shape)
 
-    def __del__(self):
-        self._free(C.byref(self.struct))
+    def __del__(self, byref=C.byref):  # bound here: module globals go first at exit
+        self._free(byref(self.struct))

@@ -11,7 +11,7 @@
 // order.  Here candidates keep their global pixel index (views are
 // concatenated in order), are compacted stably, keyed by the packed voxel
 // index and radix-sorted stably, so each voxel's members stay in that order
-// and one thread per voxel reproduces the reference's f64 sums bit for bit.
+// and one lane per coordinate reproduces the reference's f64 sums bit for bit.
 // Output order is the sorted key order (the reference's HashMap order is
 // unspecified).
 #include <thrust/iterator/counting_iterator.h>

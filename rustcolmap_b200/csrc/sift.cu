@@ -25,16 +25,14 @@
 //               keypoint's peaks in turn.  A histogram of the responses picks a
 //               threshold for the first max_features and some, and those are
 //               ranked by counting
-//   orientation one warp per keypoint in that order: lanes evaluate 32 window
-//               samples at a time (atan2, exp in f64), each lane owns histogram
-//               bins and adds the samples that fall in them in window order, so
-//               every bin is the reference's sequential f64 sum; the lanes
-//               smooth and pick up to four peaks (sift.rs:274-334)
+//   orientation one block per keypoint in that order: its threads evaluate the
+//               window's samples (atan2, exp in f64), thread b adds bin b's in
+//               window order, so every bin is the reference's sequential f64 sum;
+//               a warp smooths and picks up to four peaks (sift.rs:274-334)
 //   descriptor  one block per (keypoint, peak): the threads evaluate the
 //               window's samples (bilinear gradients, rotation, trilinear
-//               parameters) into shared memory; then thread t owns bin t (cell
-//               row = its warp) and adds its share of the samples that touch
-//               the row, in window order; L2 -> clip 0.2 -> L2 in f32 with the
+//               parameters) into shared memory; then thread t owns bin t and
+//               walks the list of its cell's samples, in window order; L2 -> clip 0.2 -> L2 in f32 with the
 //               reference's serial sums (sift.rs:340-431)
 //
 // All of it is queued without waiting: the counts stay on the device until

@@ -62,9 +62,8 @@ def extract_sift(img, name="", opts=None, ctx=None):
 def extract_sift_many(images, names=None, opts=None, ctxs=None):
     """extract_sift of every image, spread over the contexts `ctxs` (one
     CUDA stream each) with one host thread per context: an extraction waits
-    on its stream a few times per image (keypoint counts, chunked
-    descriptors, results) and the library call releases the GIL, so the
-    images' round trips and kernels overlap.  Image i runs on context
+    on its stream for its counts and its results, and the library call
+    releases the GIL, so the images' round trips and kernels overlap.  Image i runs on context
     i % len(ctxs); each result is the single-context one (same kernels, same
     order of operations per image).  Returns the frames in image order."""
     from concurrent.futures import ThreadPoolExecutor
