@@ -251,14 +251,15 @@ const char* rcmvs_last_error(const rcmvs_ctx* ctx);
 void* rcmvs_ctx_stream(rcmvs_ctx* ctx);
 /* Blocks until the context's stream has drained.  Also returns
  * RCMVS_E_CUDA (message in rcmvs_last_error) if a tensor-core kernel
- * queued since the last call gave up one of its bounded waits for its MMAs
- * (the kernel then freed its tensor memory and returned early). */
+ * queued on the context gave up one of its bounded waits for its MMAs (the
+ * kernel then freed its tensor memory and returned early) and no call has
+ * reported it yet.  rcmvs_net_train_step reports it too, instead of a step. */
 int rcmvs_ctx_synchronize(rcmvs_ctx* ctx);
 /* Diagnostic of that path: one block waits, with a limit of `limit_ns`
  * (1 us .. 1 s), on an mbarrier nothing arrives on, as the tensor-core
- * kernels wait for their MMAs, and sets the same fault word when the limit
- * runs out; the next rcmvs_ctx_synchronize then reports it.  Queued on the
- * context's stream. */
+ * kernels wait for their MMAs, and sets the context's fault word when the
+ * limit runs out; the next rcmvs_ctx_synchronize (or rcmvs_net_train_step)
+ * then reports it.  Queued on the context's stream. */
 int rcmvs_diag_wait_timeout(rcmvs_ctx* ctx, uint64_t limit_ns);
 const char* rcmvs_version(void);
 
@@ -602,7 +603,8 @@ int rcmvs_net_forward(rcmvs_ctx* ctx, rcmvs_net* net, const void* x_dev, int32_t
  * n*y, n*z, valid, tolerance on t, 0, 0).  Loss per valid pixel:
  * |t - t*| + (1 - cos(n, n*)) + 0.1 BCE(sigmoid(logit), |t - t*| < tol).
  * apply != 0 takes an Adam step (lr); loss_out / grads_host (nullable)
- * receive the mean loss and its gradient (f32, parameter layout). */
+ * receive the mean loss and its gradient (f32, parameter layout).  After a
+ * tensor-core wait that gave up: RCMVS_E_CUDA, nothing written, no step. */
 int rcmvs_net_train_step(rcmvs_ctx* ctx, rcmvs_net* net, const void* x_dev,
                          const float* labels_dev, int32_t n, int32_t h, int32_t w, float lr,
                          int32_t apply, float* loss_out, float* grads_host);

@@ -113,6 +113,11 @@ int validate_jobs(rcmvs_ctx* ctx, int n_views, const rcmvs_job* jobs, int n_jobs
 }  // namespace
 
 // ================================================================ context
+int rcmvs::report_fault(rcmvs_ctx* ctx) {
+    CK(cudaMemsetAsync(ctx->d_fault, 0, sizeof(int), ctx->stream));
+    return fail(ctx, RCMVS_E_CUDA, "a tensor-core kernel timed out waiting for its MMAs");
+}
+
 extern "C" {
 
 const char* rcmvs_version(void) { return "rcmvs 0.1 (sm_100a)"; }
@@ -166,6 +171,14 @@ int rcmvs_ctx_create(int device, rcmvs_ctx** out) {
             return RCMVS_E_NOMEM;
         }
     }
+    if (cudaMalloc(&ctx->d_fault, sizeof(int)) != cudaSuccess ||
+        cudaMemsetAsync(ctx->d_fault, 0, sizeof(int), ctx->stream) != cudaSuccess) {
+        cudaFree(ctx->d_fault);
+        cudaFree(ctx->d_work);
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return RCMVS_E_NOMEM;
+    }
     rcmvs::host_copy_attach();
     *out = ctx;
     return RCMVS_OK;
@@ -180,6 +193,7 @@ void rcmvs_ctx_destroy(rcmvs_ctx* ctx) {
     for (rcmvs_scene* sc : ctx->live) sc->ctx = nullptr;
     ctx->clear_spans();
     if (ctx->d_work) cudaFree(ctx->d_work);
+    cudaFree(ctx->d_fault);
     if (ctx->upload) {
         cudaStreamSynchronize(ctx->upload);
         cudaStreamDestroy(ctx->upload);
@@ -197,18 +211,17 @@ int rcmvs_diag_wait_timeout(rcmvs_ctx* ctx, uint64_t limit_ns) {
     if (!ctx) return RCMVS_E_ARG;
     if (limit_ns < 1000 || limit_ns > 1000000000ull) return fail(ctx, RCMVS_E_ARG, "limit_ns must be 1 us .. 1 s");
     CK(cudaSetDevice(ctx->device));
-    CK(rcmvs::launch_wait_probe(limit_ns, ctx->stream));
+    CK(rcmvs::launch_wait_probe(limit_ns, ctx->d_fault, ctx->stream));
     return RCMVS_OK;
 }
 
 int rcmvs_ctx_synchronize(rcmvs_ctx* ctx) {
     if (!ctx) return RCMVS_E_ARG;
     CK(cudaSetDevice(ctx->device));
+    int fault = 0;
+    CK(cudaMemcpyAsync(&fault, ctx->d_fault, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    const int f = rcmvs::tc_fault_take();
-    if (f) return fail(ctx, RCMVS_E_CUDA, f > 0 ? "a tensor-core kernel timed out waiting for its MMAs"
-                                                 : "could not read the tensor-core fault word");
-    return RCMVS_OK;
+    return fault ? rcmvs::report_fault(ctx) : RCMVS_OK;
 }
 
 void rcmvs_points_free(rcmvs_points* p) {

@@ -26,6 +26,9 @@ struct rcmvs_ctx {
     DeviceArena arena;
     bool count_work = false;
     unsigned long long* d_work = nullptr;
+    // set by a tensor-core kernel whose bounded wait gave up, until the call
+    // that reports it (report_fault) clears it
+    int* d_fault = nullptr;
     uint64_t last_evals = 0, last_rows = 0;
     // autotuned tile shapes per resolution class, one thread count and one
     // threads-per-pixel of the passes for all
@@ -166,6 +169,9 @@ namespace rcmvs {
 // resize.cu 60-68, sift.cu 80-159 and match.cu 160-175).
 constexpr int kSlotJobs = 0, kSlotJobStart = 1, kSlotQueue = 11, kSlotTuneJobs = 12, kSlotTuneStart = 13,
               kSlotStreamStart = 14, kSlotStreamScratch = 15, kSlotInitStart = 38;
+
+// capi.cu: clears the context's fault word, which was read as set; its error.
+int report_fault(rcmvs_ctx* ctx);
 
 // resize.cu: argument and size checks of a resize, and the resize itself
 // on device buffers (d_gray mw*mh, d_rgb mw*mh*3), queued on the context's

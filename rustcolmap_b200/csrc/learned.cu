@@ -181,10 +181,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Set (never cleared by a kernel) when a tensor-core wait gave up; read and
-// cleared by tc_fault_take().
-__device__ int g_tc_fault = 0;
-
 constexpr int TC_TW = 8, TC_TH = 16;          // output tile: 16 rows x 8 columns = the 128 rows of M
 constexpr int TC_SW = TC_TW + 2;              // staged halo tile width
 constexpr int TC_NPIX = (TC_TH + 2) * TC_SW;  // staged pixels
@@ -239,13 +235,13 @@ __device__ __forceinline__ void tma_load_4d(const void* tmap, uint32_t dst, uint
 // buffer: thread 0 starts the next tile's loads before the current tile's
 // MMAs, so they overlap the MMAs and the epilogue.  The accumulator (COUT f32 columns of 128 lanes) is read back by the four warps
 // with tcgen05.ld (warp w owns lanes 32w..32w+31).  Every wait is bounded:
-// on a time-out the CTA flags g_tc_fault, waits once more for what it has in
+// on a time-out the CTA sets *fault, waits once more for what it has in
 // flight, frees its tensor memory and returns.
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CUtensorMap tmap,
                                                       const bf16* __restrict__ mask, int N, int H, int W,
                                                       const bf16* __restrict__ wgt, const float* __restrict__ bias,
-                                                      void* __restrict__ y) {
+                                                      void* __restrict__ y, int* fault) {
     static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "conv3x3 shape");
     using L = ConvSmem<CIN, COUT>;
     constexpr int KG = L::KG;
@@ -388,7 +384,7 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ CU
     if (!ok) {
         // wait once more for what is still in flight before the smem and the
         // tensor memory are released
-        if (tid == 0) atomicExch(&g_tc_fault, 1);
+        if (tid == 0) atomicExch(fault, 1);
         if (mma_issued > mma_done) mbar_wait(mma_a, mma_done & 1u, TC_WAIT_NS);
         for (uint32_t k = landed0; k < issued0; ++k) mbar_wait(full0, k & 1u, TC_WAIT_NS);
         for (uint32_t k = landed1; k < issued1; ++k) mbar_wait(full1, k & 1u, TC_WAIT_NS);
@@ -430,7 +426,8 @@ struct WgradSmem {
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap xmap,
                                                             const __grid_constant__ CUtensorMap ymap, int N, int H, int W,
-                                                            float* __restrict__ dW, float* __restrict__ db) {
+                                                            float* __restrict__ dW, float* __restrict__ db,
+                                                            int* fault) {
     using L = WgradSmem<CIN>;
     // F32 accumulator, BF16 operands, both MN-major, N >> 3, M >> 4
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
@@ -530,7 +527,7 @@ __global__ void __launch_bounds__(128) conv3x3_wgrad_kernel(const __grid_constan
     if (tid == 0) {
         for (int k = done; k < issued; ++k) ok = mbar_wait(bar0 + 16u + 8u * (k & 1), (k >> 1) & 1, TC_WAIT_NS) && ok;
         for (int k = landed; k < loaded; ++k) mbar_wait(bar0 + 8u * (k & 1), (k >> 1) & 1, TC_WAIT_NS);
-        if (!ok) atomicExch(&g_tc_fault, 1);
+        if (!ok) atomicExch(fault, 1);
     }
     if (__syncthreads_and(ok) && it > 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -716,7 +713,7 @@ static int tc_ctas(size_t smem, int columns, int most = TC_CTAS_PER_SM) {
 
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 static cudaError_t conv_t(const void* x, const void* mask, int N, int H, int W, const void* w, const float* b, void* y,
-                          cudaStream_t st) {
+                          int* fault, cudaStream_t st) {
     if (N <= 0 || H <= 0 || W <= 0) return cudaSuccess;
     // 16-byte operand loads and stores (and the TMA base address)
     if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (mask ? (uintptr_t)mask : 0)) & 15) return cudaErrorMisalignedAddress;
@@ -732,12 +729,13 @@ static cudaError_t conv_t(const void* x, const void* mask, int N, int H, int W, 
     const long long tiles = (long long)((W + TC_TW - 1) / TC_TW) * ((H + TC_TH - 1) / TC_TH) * N;
     if (tiles > INT_MAX) return cudaErrorInvalidValue;
     const int grid = (int)std::min<long long>(tiles, (long long)sms * tc_ctas(sm, 32));
-    k<<<grid, 128, sm, st>>>(tmap, reinterpret_cast<const bf16*>(mask), N, H, W, reinterpret_cast<const bf16*>(w), b, y);
+    k<<<grid, 128, sm, st>>>(tmap, reinterpret_cast<const bf16*>(mask), N, H, W, reinterpret_cast<const bf16*>(w), b, y,
+                             fault);
     return cudaGetLastError();
 }
 
 namespace {
-__global__ void wait_probe_kernel(uint64_t limit_ns) {
+__global__ void wait_probe_kernel(uint64_t limit_ns, int* fault) {
     __shared__ __align__(8) uint64_t bar;
     const uint32_t bar_a = smem_u32(&bar);
     if (threadIdx.x == 0) {
@@ -746,39 +744,30 @@ __global__ void wait_probe_kernel(uint64_t limit_ns) {
     }
     __syncthreads();
     const bool got = mbar_wait(bar_a, 0u, limit_ns);
-    if (!__syncthreads_and(got) && threadIdx.x == 0) atomicExch(&g_tc_fault, 1);
+    if (!__syncthreads_and(got) && threadIdx.x == 0) atomicExch(fault, 1);
 }
 }  // namespace
 
-cudaError_t launch_wait_probe(uint64_t limit_ns, cudaStream_t st) {
-    wait_probe_kernel<<<1, 32, 0, st>>>(limit_ns);
+cudaError_t launch_wait_probe(uint64_t limit_ns, int* fault, cudaStream_t st) {
+    wait_probe_kernel<<<1, 32, 0, st>>>(limit_ns, fault);
     return cudaGetLastError();
 }
 
-int tc_fault_take() {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tc_fault, sizeof(int)) != cudaSuccess) return -1;
-    if (v) {
-        const int z = 0;
-        if (cudaMemcpyToSymbol(g_tc_fault, &z, sizeof(int)) != cudaSuccess) return -1;
-    }
-    return v;
-}
-
 cudaError_t launch_conv3x3(int cin, int cout, bool relu, bool out_f32, const void* x, const void* mask, int N, int H,
-                           int W, const void* w, const float* b, void* y, cudaStream_t st) {
+                           int W, const void* w, const float* b, void* y, int* fault, cudaStream_t st) {
     const bool m = mask != nullptr;
-    if (cin == 48 && cout == 32 && relu && !out_f32 && !m) return conv_t<48, 32, true, false, false>(x, mask, N, H, W, w, b, y, st);
-    if (cin == 32 && cout == 32 && relu && !out_f32 && !m) return conv_t<32, 32, true, false, false>(x, mask, N, H, W, w, b, y, st);
-    if (cin == 32 && cout == 16 && !relu && out_f32 && !m) return conv_t<32, 16, false, true, false>(x, mask, N, H, W, w, b, y, st);
+    if (cin == 48 && cout == 32 && relu && !out_f32 && !m) return conv_t<48, 32, true, false, false>(x, mask, N, H, W, w, b, y, fault, st);
+    if (cin == 32 && cout == 32 && relu && !out_f32 && !m) return conv_t<32, 32, true, false, false>(x, mask, N, H, W, w, b, y, fault, st);
+    if (cin == 32 && cout == 16 && !relu && out_f32 && !m) return conv_t<32, 16, false, true, false>(x, mask, N, H, W, w, b, y, fault, st);
     // backward data: no bias, no ReLU, the result masked by the layer's output
-    if (cin == 16 && cout == 32 && !relu && !out_f32 && m) return conv_t<16, 32, false, false, true>(x, mask, N, H, W, w, b, y, st);
-    if (cin == 32 && cout == 32 && !relu && !out_f32 && m) return conv_t<32, 32, false, false, true>(x, mask, N, H, W, w, b, y, st);
+    if (cin == 16 && cout == 32 && !relu && !out_f32 && m) return conv_t<16, 32, false, false, true>(x, mask, N, H, W, w, b, y, fault, st);
+    if (cin == 32 && cout == 32 && !relu && !out_f32 && m) return conv_t<32, 32, false, false, true>(x, mask, N, H, W, w, b, y, fault, st);
     return cudaErrorInvalidValue;
 }
 
 template <int CIN, int COUT>
-static cudaError_t wgrad_t(const void* x, const void* dy, int N, int H, int W, float* dW, float* db, cudaStream_t st) {
+static cudaError_t wgrad_t(const void* x, const void* dy, int N, int H, int W, float* dW, float* db, int* fault,
+                           cudaStream_t st) {
     if (N <= 0 || H <= 0 || W <= 0) return cudaSuccess;
     if (((uintptr_t)x | (uintptr_t)dy) & 15) return cudaErrorMisalignedAddress;
     using L = WgradSmem<CIN>;
@@ -796,15 +785,15 @@ static cudaError_t wgrad_t(const void* x, const void* dy, int N, int H, int W, f
     // two: 73 us a layer of 32 channels; one 82; three 84 (each CTA adds 9 taps
     // of sums to dW at its end)
     const int grid = (int)std::min<long long>(tiles, (long long)sms * tc_ctas(L::BYTES, L::COLS, 2));
-    k<<<grid, 128, L::BYTES, st>>>(xmap, ymap, N, H, W, dW, db);
+    k<<<grid, 128, L::BYTES, st>>>(xmap, ymap, N, H, W, dW, db, fault);
     return cudaGetLastError();
 }
 
 cudaError_t launch_conv3x3_wgrad(int cin, int cout, const void* x, const void* dy, int N, int H, int W, float* dW,
-                                 float* db, cudaStream_t st) {
-    if (cin == 48 && cout == 32) return wgrad_t<48, 32>(x, dy, N, H, W, dW, db, st);
-    if (cin == 32 && cout == 32) return wgrad_t<32, 32>(x, dy, N, H, W, dW, db, st);
-    if (cin == 32 && cout == 16) return wgrad_t<32, 16>(x, dy, N, H, W, dW, db, st);
+                                 float* db, int* fault, cudaStream_t st) {
+    if (cin == 48 && cout == 32) return wgrad_t<48, 32>(x, dy, N, H, W, dW, db, fault, st);
+    if (cin == 32 && cout == 32) return wgrad_t<32, 32>(x, dy, N, H, W, dW, db, fault, st);
+    if (cin == 32 && cout == 16) return wgrad_t<32, 16>(x, dy, N, H, W, dW, db, fault, st);
     return cudaErrorInvalidValue;
 }
 

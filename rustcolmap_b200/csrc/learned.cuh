@@ -25,17 +25,16 @@ int costvol_tiles(int w, int h);
 cudaError_t launch_costvol(const DevJob* jobs, const int32_t* blk_start, int n_jobs, int total_blocks,
                            const int64_t* out_off, const uint64_t* census_q, const float2* rays_q,
                            const uint8_t* gray_q, void* out, cudaStream_t st);
+// fault: the context's fault word (rcmvs_ctx::d_fault), set when a bounded wait
+// gave up.
 cudaError_t launch_conv3x3(int cin, int cout, bool relu, bool out_f32, const void* x, const void* mask, int N, int H,
-                           int W, const void* w, const float* b, void* y, cudaStream_t st);
-// Reads and clears the device word the tensor-core kernels set when one of
-// their bounded waits gave up (1), 0 if none did, -1 if it could not be read.
-int tc_fault_take();
+                           int W, const void* w, const float* b, void* y, int* fault, cudaStream_t st);
 // One block waits limit_ns on an mbarrier that nothing arrives on and sets
-// the fault word when the wait gives up (rcmvs_diag_wait_timeout).
-cudaError_t launch_wait_probe(uint64_t limit_ns, cudaStream_t st);
+// *fault when the wait gives up (rcmvs_diag_wait_timeout).
+cudaError_t launch_wait_probe(uint64_t limit_ns, int* fault, cudaStream_t st);
 // dW += and db += the convolution's weight and bias gradients.
 cudaError_t launch_conv3x3_wgrad(int cin, int cout, const void* x, const void* dy, int N, int H, int W, float* dW,
-                                 float* db, cudaStream_t st);
+                                 float* db, int* fault, cudaStream_t st);
 // Backward-data weights of layers 1.. of the BF16 parameters w, each at its
 // own offset in wt (as large as w).
 cudaError_t launch_flip_weights(const void* w, void* wt, cudaStream_t st);

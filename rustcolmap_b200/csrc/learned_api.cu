@@ -174,11 +174,13 @@ int net_forward(rcmvs_ctx* ctx, rcmvs_net* net, const void* x, int N, int H, int
         const Layer& y = L[l];
         const float* b = net->p + y.b_off;
         if (l == NET_LAYERS - 1) {
-            LCK(launch_conv3x3(y.cin, y.cout, false, true, in, nullptr, N, H, W, wb(net, y), b, out, ctx->stream));
+            LCK(launch_conv3x3(y.cin, y.cout, false, true, in, nullptr, N, H, W, wb(net, y), b, out, ctx->d_fault,
+                               ctx->stream));
         } else {
             void* act;
             LCK(net->arena.get(N_ACT0 + 1 + l, 2 * npx * y.cout, &act));
-            LCK(launch_conv3x3(y.cin, y.cout, true, false, in, nullptr, N, H, W, wb(net, y), b, act, ctx->stream));
+            LCK(launch_conv3x3(y.cin, y.cout, true, false, in, nullptr, N, H, W, wb(net, y), b, act, ctx->d_fault,
+                               ctx->stream));
             in = act;
         }
     }
@@ -232,19 +234,24 @@ int rcmvs_net_train_step(rcmvs_ctx* ctx, rcmvs_net* net, const void* x_dev, cons
         } else {
             LCK(net->arena.get(N_ACT0 + l, 2 * npx * NET_COUT[l - 1], &xin));
         }
-        LCK(launch_conv3x3_wgrad(y.cin, y.cout, xin, dcur, n, h, w, net->g + y.w_off, net->g + y.b_off, st));
+        LCK(launch_conv3x3_wgrad(y.cin, y.cout, xin, dcur, n, h, w, net->g + y.w_off, net->g + y.b_off, ctx->d_fault,
+                                 st));
         if (l > 0) {
             void* dnext;
             LCK(net->arena.get(N_DY0 + flipbuf, 2 * npx * y.cin, &dnext));
             LCK(launch_conv3x3(y.cout, y.cin, false, false, dcur, xin, n, h, w, (const char*)flip + 2 * y.w_off, nullptr,
-                               dnext, st));
+                               dnext, ctx->d_fault, st));
             dcur = dnext;
             flipbuf ^= 1;
         }
     }
     float hacc[2];
+    int fault = 0;
     LCK(cudaMemcpyAsync(hacc, acc, 8, cudaMemcpyDeviceToHost, st));
+    LCK(cudaMemcpyAsync(&fault, ctx->d_fault, sizeof(int), cudaMemcpyDeviceToHost, st));
     LCK(cudaStreamSynchronize(st));
+    // a CTA that gave up left its part out of the sums: no loss, gradients or step
+    if (fault) return report_fault(ctx);
     const float cnt = hacc[1] > 0.f ? hacc[1] : 1.f;
     if (loss_out) *loss_out = hacc[0] / cnt;
     if (grads_host) {
