@@ -253,13 +253,14 @@ void* rcmvs_ctx_stream(rcmvs_ctx* ctx);
  * RCMVS_E_CUDA (message in rcmvs_last_error) if a tensor-core kernel
  * queued on the context gave up one of its bounded waits for its MMAs (the
  * kernel then freed its tensor memory and returned early) and no call has
- * reported it yet.  rcmvs_net_train_step reports it too, instead of a step. */
+ * reported it yet.  rcmvs_net_train_step and rcmvs_match_pairs report it too,
+ * instead of their results. */
 int rcmvs_ctx_synchronize(rcmvs_ctx* ctx);
 /* Diagnostic of that path: one block waits, with a limit of `limit_ns`
  * (1 us .. 1 s), on an mbarrier nothing arrives on, as the tensor-core
  * kernels wait for their MMAs, and sets the context's fault word when the
- * limit runs out; the next rcmvs_ctx_synchronize (or rcmvs_net_train_step)
- * then reports it.  Queued on the context's stream. */
+ * limit runs out; the next rcmvs_ctx_synchronize (or other call that
+ * reports the word) then does.  Queued on the context's stream. */
 int rcmvs_diag_wait_timeout(rcmvs_ctx* ctx, uint64_t limit_ns);
 const char* rcmvs_version(void);
 

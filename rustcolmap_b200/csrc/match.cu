@@ -257,7 +257,6 @@ struct Frame {
 struct MatchStatus {
     int wild;   // a component past PACK_LIMIT or not finite
     int listed; // queries for rescan_kernel
-    int fault;  // a bounded wait gave up
 };
 
 // Block b of 128 descriptors: half (hi, lo) h, descriptor r, component k at
@@ -351,7 +350,7 @@ constexpr int kNearestSmem = 2 * QB_BYTES + NSLOT * QB_HALF + 128;
 __global__ void __launch_bounds__(kNearestThreads, 1)
     nearest_kernel(const PairJob* __restrict__ jobs, const Frame* __restrict__ frames,
                    const unsigned char* __restrict__ packed, const float* __restrict__ norms, int blocks_per_cta,
-                   Two* __restrict__ fwd, Two* __restrict__ bwd, MatchStatus* __restrict__ st) {
+                   Two* __restrict__ fwd, Two* __restrict__ bwd, int* fault) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[1 + 2 * NSLOT + 4];  // queries; slot full, slot free; values full, values free
     __shared__ uint32_t s_taddr;
@@ -440,11 +439,11 @@ __global__ void __launch_bounds__(kNearestThreads, 1)
                 }
             }
             // everything in flight ends before the memory is released
-            if (!ok) atomicExch(&st->fault, 1);
+            if (!ok) atomicExch(fault, 1);
             if (!q_in) mbar_wait(bar0, 0, TC_WAIT_NS);
             for (; landed < loaded; ++landed) mbar_wait(full(landed % NSLOT), (landed / NSLOT) & 1, TC_WAIT_NS);
             for (; freed < issued; ++freed) {
-                if (!mbar_wait(slot_free(freed % NSLOT), (freed / NSLOT) & 1, TC_WAIT_NS)) atomicExch(&st->fault, 1);
+                if (!mbar_wait(slot_free(freed % NSLOT), (freed / NSLOT) & 1, TC_WAIT_NS)) atomicExch(fault, 1);
             }
         }
         __syncwarp();
@@ -484,7 +483,7 @@ __global__ void __launch_bounds__(kNearestThreads, 1)
             if (lane == 0)
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_free(c & 1)) : "memory");
         }
-        if (!ok && lane == 0) atomicExch(&st->fault, 1);
+        if (!ok && lane == 0) atomicExch(fault, 1);
         const int row = (qb0 + b) * QB + 32 * (warp & 3) + lane;
         if (ok && row < q.n) (dir ? bwd : fwd)[out0 + row] = f;
     }
@@ -517,12 +516,17 @@ __device__ __forceinline__ uint32_t answer(uint32_t idx, float d1, float d2, flo
     return d1 > ratio * d2 ? UINT32_MAX : idx;
 }
 
+// With *fault set (a wait of nearest_kernel gave up, so some of its entries were
+// not written) this kernel and the two after it read and answer nothing; the
+// host then reports the fault.
 __global__ void __launch_bounds__(256) outcome_kernel(const PairJob* __restrict__ jobs, const Frame* __restrict__ frames,
                                                       const float* __restrict__ desc, const float* __restrict__ norms,
                                                       const int* __restrict__ max_norm, const Two* __restrict__ fwd2,
                                                       const Two* __restrict__ bwd2, float ratio,
                                                       uint32_t* __restrict__ fwd, uint32_t* __restrict__ bwd,
-                                                      int2* __restrict__ list, MatchStatus* __restrict__ st) {
+                                                      int2* __restrict__ list, MatchStatus* __restrict__ st,
+                                                      const int* __restrict__ fault) {
+    if (*fault) return;
     const int dir = blockIdx.y & 1;
     const PairJob J = jobs[blockIdx.y >> 1];
     Frame q, t;
@@ -559,8 +563,10 @@ __global__ void __launch_bounds__(256) outcome_kernel(const PairJob* __restrict_
 __global__ void __launch_bounds__(256) rescan_kernel(const PairJob* __restrict__ jobs, const Frame* __restrict__ frames,
                                                      const float* __restrict__ desc, float ratio,
                                                      uint32_t* __restrict__ fwd, uint32_t* __restrict__ bwd,
-                                                     const int2* __restrict__ list, const MatchStatus* __restrict__ st) {
+                                                     const int2* __restrict__ list, const MatchStatus* __restrict__ st,
+                                                     const int* __restrict__ fault) {
     __shared__ Nearest part[8];
+    if (*fault) return;
     const int n = st->listed;
     if (n > RESCAN_MAX || st->wild) return;  // the chunk runs again on the FP32 pipes
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
@@ -588,7 +594,9 @@ __global__ void __launch_bounds__(256) rescan_kernel(const PairJob* __restrict__
 
 // matching.rs:90-94: mutual answers.
 __global__ void mutual_kernel(const PairJob* __restrict__ jobs, const uint32_t* __restrict__ fwd,
-                              const uint32_t* __restrict__ bwd, uint32_t* __restrict__ match_b) {
+                              const uint32_t* __restrict__ bwd, uint32_t* __restrict__ match_b,
+                              const int* __restrict__ fault) {
+    if (*fault) return;
     const PairJob J = jobs[blockIdx.y];
     const int ia = blockIdx.x * 256 + threadIdx.x;
     if (ia >= J.na) return;
@@ -907,7 +915,7 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                     const int per = qblocks >= 2 * 148 ? 2 : 1;
                     nearest_kernel<<<dim3((most + per - 1) / per, 2 * (unsigned)(j1 - j0)), kNearestThreads, kNearestSmem,
                                      st>>>(dj + j0, df, (const unsigned char*)p_pack, (const float*)p_norm, per, f2, b2,
-                                           ds);
+                                           ctx->d_fault);
                     return cudaGetLastError();
                 };
                 const int max_n = std::max(max_na, max_nb);
@@ -939,18 +947,21 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                 hook.begin("match_select");
                 outcome_kernel<<<dim3((max_n + 255) / 256, 2 * nj), 256, 0, st>>>(
                     dj, df, (const float*)p_desc, (const float*)p_norm, (const int*)p_maxn, f2, b2, r32, fo, bo,
-                    (int2*)p_list, ds);
+                    (int2*)p_list, ds, ctx->d_fault);
                 MCK(cudaGetLastError());
-                rescan_kernel<<<296, 256, 0, st>>>(dj, df, (const float*)p_desc, r32, fo, bo, (const int2*)p_list, ds);
+                rescan_kernel<<<296, 256, 0, st>>>(dj, df, (const float*)p_desc, r32, fo, bo, (const int2*)p_list, ds,
+                                                   ctx->d_fault);
                 MCK(cudaGetLastError());
-                mutual_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>(dj, fo, bo, (uint32_t*)p_mb);
+                mutual_kernel<<<dim3((max_na + 255) / 256, nj), 256, 0, st>>>(dj, fo, bo, (uint32_t*)p_mb, ctx->d_fault);
                 MCK(cudaGetLastError());
                 hook.end("match_select");
                 MatchStatus status{};
+                int fault = 0;
                 MCK(cudaMemcpyAsync(&status, p_st, sizeof(status), cudaMemcpyDeviceToHost, st));
+                MCK(cudaMemcpyAsync(&fault, ctx->d_fault, sizeof(int), cudaMemcpyDeviceToHost, st));
                 MCK(collect());
                 MCK(cudaStreamSynchronize(st));
-                if (status.fault) return mfail(ctx, RCMVS_E_CUDA, "rcmvs_match_pairs: a tensor-core wait timed out");
+                if (fault) return report_fault(ctx);
                 if (status.wild) tensor = false;
                 on_tensor = !status.wild && status.listed <= RESCAN_MAX;
             }

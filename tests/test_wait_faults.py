@@ -6,7 +6,8 @@ import contextlib
 import numpy as np
 import pytest
 
-from rustcolmap_b200 import learned, mvs
+from oracle import oracle
+from rustcolmap_b200 import learned, mvs, sift
 from rustcolmap_b200._lib import RcmvsError
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +40,23 @@ def test_train_step_takes_no_step():
         net.train_step(xd.data_ptr(), ld.data_ptr(), *shape, 1e-2)
         moved = np.abs(net.params() - p).max()
         assert 0 < moved <= 1.01e-2  # one first Adam step
+
+
+def test_matching_reads_no_unwritten_entry():
+    """The search's entries are kept in a buffer that earlier calls leave
+    larger indices in; with the fault set, no kernel follows them."""
+    def descs(n, seed):
+        d = np.random.default_rng(seed).random((n, 128), dtype=np.float32)
+        return np.ascontiguousarray(d / np.linalg.norm(d, axis=1, keepdims=True))
+
+    a, b = descs(2100, 1), descs(2050, 2)
+    b[:400] = a[1700:2100]
+    with contextlib.closing(mvs.Context(0)) as ctx:
+        sift.match_pairs([a, descs(9000, 3)], [(0, 1), (1, 0)], 1.0, ctx)
+        ctx.diag_wait_timeout(1_000_000)
+        with pytest.raises(RcmvsError, match="timed out"):
+            sift.match_pairs([a, b], [(0, 1)], 0.8, ctx)
+        ctx.synchronize()  # reported once
+        (ga, gb), = sift.match_pairs([a, b], [(0, 1)], 0.8, ctx)
+        oa, ob = oracle.match_pair(a, b, 0.8)
+        assert len(oa) >= 400 and np.array_equal(ga, oa) and np.array_equal(gb, ob)
