@@ -600,8 +600,9 @@ int rcmvs_net_get_params(rcmvs_net* net, float* out);
 /* Forward pass on device buffers: x_dev n*h*w*48 BF16 -> out_dev n*h*w*16 f32. */
 int rcmvs_net_forward(rcmvs_ctx* ctx, rcmvs_net* net, const void* x_dev, int32_t n, int32_t h,
                       int32_t w, float* out_dev);
-/* One training step on device buffers.  labels_dev: n*h*w*8 f32 = (t*, n*x,
- * n*y, n*z, valid, tolerance on t, 0, 0).  Loss per valid pixel:
+/* One training step on device buffers (x_dev aligned to 16 bytes, labels_dev
+ * to floats).  labels_dev: n*h*w*8 f32 = (t*, n*x, n*y, n*z, valid, tolerance
+ * on t, 0, 0).  Loss per valid pixel:
  * |t - t*| + (1 - cos(n, n*)) + 0.1 BCE(sigmoid(logit), |t - t*| < tol).
  * apply != 0 takes an Adam step (lr); loss_out / grads_host (nullable)
  * receive the mean loss and its gradient (f32, parameter layout).  After a

@@ -582,17 +582,26 @@ __global__ void to_bf16_kernel(const float* __restrict__ a, int64_t n, bf16* __r
 //   |t - t*| + LN (1 - cos(n, n*)) + LC BCE(sigmoid(c), |t - t*| < tol)
 // averaged over valid pixels; writes dL/dout (BF16, 16 channels) and adds the
 // summed loss and the valid count to acc[0..1].
+// VEC: the labels are 16-byte aligned and read as whole sectors; the caller's
+// may be aligned to floats only.
 constexpr float LN = 1.0f, LC = 0.1f;
+template <bool VEC>
 __global__ void loss_kernel(const float* __restrict__ out, const float* __restrict__ lab, int64_t npx, float inv_n,
                             bf16* __restrict__ dout, float* __restrict__ acc) {
     float l = 0.f, cnt = 0.f;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npx; p += (int64_t)gridDim.x * blockDim.x) {
-        // whole sectors at a time (t, normal | logit; t*, n* | n*z.., valid, tolerance)
-        const float4* o4 = reinterpret_cast<const float4*>(out + p * NET_OUT_C);
-        const float4* l4 = reinterpret_cast<const float4*>(lab + p * 8);
-        const float4 oa = o4[0], la = l4[0], lb = l4[1];
+        // t, normal | logit; t*, n*xyz | valid, tolerance
+        const float4 oa = *reinterpret_cast<const float4*>(out + p * NET_OUT_C);
         const float o[5] = {oa.x, oa.y, oa.z, oa.w, out[p * NET_OUT_C + 4]};
-        const float L[6] = {la.x, la.y, la.z, la.w, lb.x, lb.y};
+        float L[8];
+        if (VEC) {
+            const float4* l4 = reinterpret_cast<const float4*>(lab + p * 8);
+            const float4 la = l4[0], lb = l4[1];
+            L[0] = la.x, L[1] = la.y, L[2] = la.z, L[3] = la.w, L[4] = lb.x, L[5] = lb.y;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) L[c] = lab[p * 8 + c];
+        }
         float g[NET_OUT_C];
 #pragma unroll
         for (int c = 0; c < NET_OUT_C; ++c) g[c] = 0.f;
@@ -824,7 +833,11 @@ cudaError_t launch_to_bf16(const float* a, int64_t n, void* b, cudaStream_t st) 
 cudaError_t launch_loss(const float* out, const float* lab, int64_t npx, float inv_n, void* dout, float* acc,
                         cudaStream_t st) {
     const int blocks = (int)std::min<int64_t>((npx + 255) / 256, 148 * 4);
-    loss_kernel<<<blocks, 256, 0, st>>>(out, lab, npx, inv_n, reinterpret_cast<bf16*>(dout), acc);
+    auto run = [&](auto kernel) { kernel<<<blocks, 256, 0, st>>>(out, lab, npx, inv_n, reinterpret_cast<bf16*>(dout), acc); };
+    if (((uintptr_t)lab & 15) == 0)
+        run(loss_kernel<true>);
+    else
+        run(loss_kernel<false>);
     return cudaGetLastError();
 }
 
