@@ -649,8 +649,8 @@ int fuse_views(rcmvs_ctx* ctx, rcmvs_scene* sc, const int32_t* order_offsets, co
         F.cx = c.cx;
         F.cy = c.cy;
         F.k = c.k;
-        std::memcpy(F.R, c.R, sizeof(F.R));
-        std::memcpy(F.t, c.t, sizeof(F.t));
+        std::memcpy(F.pose, c.R, sizeof(c.R));
+        std::memcpy(F.pose + 9, c.t, sizeof(c.t));
     }
     return RCMVS_OK;
 }

@@ -85,17 +85,18 @@ __device__ __forceinline__ void cam_normalize(const FuseView& v, double u, doubl
 }
 
 struct Pose {
-    double R[9], t[3];
+    double m[12];  // R by rows, then t
+    __device__ __forceinline__ const double* R() const { return m; }
+    __device__ __forceinline__ double t(int i) const { return m[9 + i]; }
 };
 __device__ __forceinline__ Pose load_pose(const FuseView& v) {
     Pose p;
-    const double2* s = reinterpret_cast<const double2*>(v.R);
-    double* d = p.R;
+    const double2* s = reinterpret_cast<const double2*>(v.pose);
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         const double2 q = __ldg(s + i);
-        d[2 * i] = q.x;  // t follows R
-        d[2 * i + 1] = q.y;
+        p.m[2 * i] = q.x;
+        p.m[2 * i + 1] = q.y;
     }
     return p;
 }
@@ -110,8 +111,8 @@ __device__ __forceinline__ void matt_vec(const double* m, const double* x, doubl
 
 // World -> camera (sfm-lite/src/geom.rs:64-66)
 __device__ __forceinline__ void to_cam(const Pose& p, const double* x, double* xc) {
-    mat_vec(p.R, x, xc);
-    for (int i = 0; i < 3; ++i) xc[i] = xc[i] + p.t[i];
+    mat_vec(p.R(), x, xc);
+    for (int i = 0; i < 3; ++i) xc[i] = xc[i] + p.t(i);
 }
 
 // Camera -> pixel (sfm-lite/src/geom.rs:67-75); z is recip(xc[2])
@@ -206,9 +207,9 @@ __global__ void __launch_bounds__(FT, 4) candidates_kernel(const FuseView* __res
         cam_normalize(v, (double)px, (double)py, nx, ny);
         const double xr[3] = {nx * zr, ny * zr, 1.0 * zr};
         const Pose ref = load_pose(v);
-        const double dd[3] = {xr[0] - ref.t[0], xr[1] - ref.t[1], xr[2] - ref.t[2]};
+        const double dd[3] = {xr[0] - ref.t(0), xr[1] - ref.t(1), xr[2] - ref.t(2)};
         double xw[3];
-        matt_vec(ref.R, dd, xw);
+        matt_vec(ref.R(), dd, xw);
         double acc[3] = {xw[0], xw[1], xw[2]};
         uint32_t n_cons = 0;
         for (int q = v.order_begin; q < v.order_end; ++q) {
@@ -227,9 +228,9 @@ __global__ void __launch_bounds__(FT, 4) candidates_kernel(const FuseView* __res
                 double sx, sy;
                 cam_normalize(sv, us, vs, sx, sy);
                 const double xs2[3] = {sx * zs, sy * zs, 1.0 * zs};
-                const double d2[3] = {xs2[0] - sp.t[0], xs2[1] - sp.t[1], xs2[2] - sp.t[2]};
+                const double d2[3] = {xs2[0] - sp.t(0), xs2[1] - sp.t(1), xs2[2] - sp.t(2)};
                 double xw2[3];
-                matt_vec(sp.R, d2, xw2);
+                matt_vec(sp.R(), d2, xw2);
                 if (gate) {  // extension: forward-backward reprojection gate
                     double xc[3], ru, rv;
                     to_cam(load_pose(v), xw2, xc);

@@ -165,8 +165,7 @@ struct alignas(16) FuseView {
     double f, cx, cy, k;
     double rf;  // 1 / f
     double pad;
-    double R[9];
-    double t[3];  // follows R (six 16-byte loads)
+    double pose[12];  // R by rows, then t (six 16-byte loads)
 };
 
 struct FuseResult {
