@@ -223,7 +223,8 @@ typedef struct rcmvs_sparse {
 /* Fused point cloud: the `Vec<(f64,f64,f64,[u8;3])>` of
  * `fuse::fuse_depth_maps` (mvs/src/fuse.rs:64-71).  Points come out sorted
  * by voxel key (the reference's HashMap order is unspecified).  Arrays are
- * allocated by the library; release with rcmvs_points_free. */
+ * allocated by the library; release with rcmvs_points_free (unless the context
+ * has an allocator of the caller's, rcmvs_ctx_set_result_alloc). */
 typedef struct rcmvs_points {
     uint64_t n;
     double* xyz;             /* 3*n */
@@ -247,6 +248,19 @@ typedef struct rcmvs_ctx rcmvs_ctx;
 int rcmvs_ctx_create(int device, rcmvs_ctx** out);
 void rcmvs_ctx_destroy(rcmvs_ctx* ctx);
 const char* rcmvs_last_error(const rcmvs_ctx* ctx);
+/* Memory of the clouds and SIFT frames that calls on the context hand out.  By
+ * default the library allocates it (malloc) and rcmvs_points_free /
+ * rcmvs_sift_frame_free release it.  With an allocator set, each array comes
+ * from alloc(user, field, n), called on the calling thread for n points or
+ * features (NULL: RCMVS_E_NOMEM), and stays the caller's, also when the call
+ * then fails: it must not be given to those two.  NULL: the default again. */
+#define RCMVS_RESULT_XYZ 0    /* rcmvs_points: n * 3 double */
+#define RCMVS_RESULT_RGB 1    /* n * 3 uint8_t */
+#define RCMVS_RESULT_PTS 2    /* rcmvs_sift_frame: n * 2 double */
+#define RCMVS_RESULT_DESC 3   /* n * 128 float */
+#define RCMVS_RESULT_COLORS 4 /* n * 3 uint8_t */
+typedef void* (*rcmvs_result_alloc)(void* user, int32_t field, uint64_t n);
+int rcmvs_ctx_set_result_alloc(rcmvs_ctx* ctx, rcmvs_result_alloc alloc, void* user);
 /* The context's cudaStream_t, as an opaque pointer (for event timing). */
 void* rcmvs_ctx_stream(rcmvs_ctx* ctx);
 /* Blocks until the context's stream has drained.  Also returns
@@ -503,7 +517,8 @@ typedef struct rcmvs_sift_options {
 void rcmvs_sift_options_default(rcmvs_sift_options* opts);
 
 /* `sift::SiftFrame` (sfm-lite/src/sift.rs:34-41) without the name; arrays
- * are allocated by the library (rcmvs_sift_frame_free). */
+ * are allocated by the library (rcmvs_sift_frame_free, or the caller's with
+ * rcmvs_ctx_set_result_alloc). */
 typedef struct rcmvs_sift_frame {
     int32_t width, height;   /* working size the keypoints refer to */
     uint64_t n;              /* keypoints */

@@ -42,6 +42,11 @@ pub const RCMVS_FLAG_NO_REPEAT_SKIP: u32 = 256;
 pub const RCMVS_FLAG_LOCKSTEP_PASSES: u32 = 512;
 pub const RCMVS_MAX_PASSES: u32 = 4096;
 
+pub const RCMVS_RESULT_XYZ: i32 = 0;
+pub const RCMVS_RESULT_RGB: i32 = 1;
+pub const RCMVS_RESULT_PTS: i32 = 2;
+pub const RCMVS_RESULT_DESC: i32 = 3;
+pub const RCMVS_RESULT_COLORS: i32 = 4;
 pub const RCMVS_NOALLOC_MAX_PIXELS: u32 = 307200;
 pub const RCMVS_NOALLOC_MAX_SOURCES: u32 = 4;
 pub const RCMVS_NOALLOC_SCRATCH_BYTES: u64 = 38416384;
@@ -110,6 +115,9 @@ pub struct rcmvs_sparse {
     pub track_offsets: *const u64,
     pub track_views: *const i32,
 }
+
+/// Caller's allocator of result arrays: (user, RCMVS_RESULT_* field, elements).
+pub type rcmvs_result_alloc = Option<unsafe extern "C" fn(user: *mut c_void, field: i32, n: u64) -> *mut c_void>;
 
 /// Library-allocated cloud; release with [`rcmvs_points_free`].
 #[repr(C)]
@@ -205,6 +213,8 @@ pub fn rcmvs_options_default(opts: *mut rcmvs_options);
     pub fn rcmvs_ctx_create(device: c_int, out: *mut *mut rcmvs_ctx) -> c_int;
     pub fn rcmvs_ctx_destroy(ctx: *mut rcmvs_ctx);
     pub fn rcmvs_last_error(ctx: *const rcmvs_ctx) -> *const c_char;
+    /// Memory of clouds and SIFT frames from the caller's allocator (None: the library's).
+    pub fn rcmvs_ctx_set_result_alloc(ctx: *mut rcmvs_ctx, alloc: rcmvs_result_alloc, user: *mut c_void) -> c_int;
     pub fn rcmvs_ctx_stream(ctx: *mut rcmvs_ctx) -> *mut c_void;
     pub fn rcmvs_ctx_synchronize(ctx: *mut rcmvs_ctx) -> c_int;
     pub fn rcmvs_diag_wait_timeout(ctx: *mut rcmvs_ctx, limit_ns: u64) -> c_int;

@@ -3,6 +3,7 @@
 Only layouts live here; loading the CUDA library is rustcolmap_b200._lib's job.
 """
 import ctypes as C
+import threading
 
 import numpy as np
 
@@ -153,20 +154,31 @@ def sparse_struct(xyz, track_offsets, track_views):
     return s
 
 
-class Owned:
-    """A result struct whose buffers the library allocated: the arrays taken
-    from it are views that keep it alive, and the last one frees it."""
+# The arrays a call's results are written to: numpy allocates them when the
+# library asks, on the calling thread, so each owns its memory.
+RESULT_FIELDS = {0: (np.float64, 3), 1: (np.uint8, 3), 2: (np.float64, 2), 3: (np.float32, 128), 4: (np.uint8, 3)}
+XYZ, RGB, PTS, DESC, COLORS = RESULT_FIELDS
+ResultAlloc = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_int32, C.c_uint64)
+_results = threading.local()
 
-    def __init__(self, struct, free):
-        self.struct, self._free = struct, free
 
-    def array(self, address, ctype, shape):
-        n = int(np.prod(shape))
-        if n == 0:
-            return np.empty(shape, np.dtype(ctype))
-        buf = (ctype * n).from_address(address)
-        buf.owner = self
-        return np.ctypeslib.as_array(buf).reshape(shape)
+@ResultAlloc
+def result_alloc(user, field, n):
+    dtype, k = RESULT_FIELDS[field]
+    try:
+        a = np.empty((n, k), dtype)
+    except (MemoryError, ValueError):
+        return None
+    _results.__dict__[field] = a
+    return a.ctypes.data
 
-    def __del__(self, byref=C.byref):  # bound here: module globals go first at exit
-        self._free(byref(self.struct))
+
+def take_result(field):
+    """The array of the thread's last call (none was asked for: no rows)."""
+    dtype, k = RESULT_FIELDS[field]
+    a = _results.__dict__.pop(field, None)
+    return np.zeros((0, k), dtype) if a is None else a
+
+
+def drop_results():
+    _results.__dict__.clear()

@@ -38,6 +38,7 @@ def mvs():
         "rcmvs_ctx_create": ([C.c_int, vp], C.c_int),
         "rcmvs_ctx_destroy": ([vp], None),
         "rcmvs_last_error": ([vp], cp),
+        "rcmvs_ctx_set_result_alloc": ([vp, vp, vp], C.c_int),
         "rcmvs_ctx_stream": ([vp], vp),
         "rcmvs_ctx_synchronize": ([vp], C.c_int),
         "rcmvs_pass_count": ([vp], C.c_uint64),
@@ -128,7 +129,7 @@ def exported_symbols():
 
 _SIG_NAMES = [
     "rcmvs_options_default", "rcmvs_pass_count", "rcmvs_ctx_create", "rcmvs_ctx_destroy", "rcmvs_last_error",
-    "rcmvs_ctx_stream", "rcmvs_ctx_synchronize", "rcmvs_diag_wait_timeout", "rcmvs_version", "rcmvs_census",
+    "rcmvs_ctx_set_result_alloc", "rcmvs_ctx_stream", "rcmvs_ctx_synchronize", "rcmvs_diag_wait_timeout", "rcmvs_version", "rcmvs_census",
     "rcmvs_estimate_depth", "rcmvs_estimate_depth_batch", "rcmvs_fuse_depth_maps",
     "rcmvs_write_ply_binary", "rcmvs_write_dense_outputs", "rcmvs_plan", "rcmvs_run_mvs", "rcmvs_points_free",
     "rcmvs_scene_create", "rcmvs_scene_destroy", "rcmvs_scene_prepare",

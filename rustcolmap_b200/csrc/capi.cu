@@ -205,6 +205,13 @@ void rcmvs_ctx_destroy(rcmvs_ctx* ctx) {
 
 const char* rcmvs_last_error(const rcmvs_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
+int rcmvs_ctx_set_result_alloc(rcmvs_ctx* ctx, rcmvs_result_alloc alloc, void* user) {
+    if (!ctx) return RCMVS_E_ARG;
+    ctx->alloc = alloc;
+    ctx->alloc_user = user;
+    return RCMVS_OK;
+}
+
 void* rcmvs_ctx_stream(rcmvs_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 int rcmvs_diag_wait_timeout(rcmvs_ctx* ctx, uint64_t limit_ns) {
@@ -655,15 +662,22 @@ int fuse_views(rcmvs_ctx* ctx, rcmvs_scene* sc, const int32_t* order_offsets, co
     return RCMVS_OK;
 }
 
-// Library-allocated host copy of n points (device xyz / rgb) into out.
-int take_points(rcmvs_ctx* ctx, const double* d_xyz, const uint8_t* d_rgb, uint64_t n, rcmvs_points* out) {
-    out->xyz = (double*)rcmvs::host_alloc(24 * n);
-    out->rgb = (uint8_t*)rcmvs::host_alloc(3 * n);
+// Host memory for a cloud of n points.
+int alloc_points(rcmvs_ctx* ctx, uint64_t n, rcmvs_points* out) {
+    out->xyz = (double*)ctx->result(RCMVS_RESULT_XYZ, n, 24);
+    out->rgb = (uint8_t*)ctx->result(RCMVS_RESULT_RGB, n, 3);
     if (!out->xyz || !out->rgb) {
-        rcmvs_points_free(out);
+        ctx->drop(out);
         return fail(ctx, RCMVS_E_NOMEM, "host allocation of the point cloud failed");
     }
     out->n = n;
+    return RCMVS_OK;
+}
+
+// Host copy of n points (device xyz / rgb) into out.
+int take_points(rcmvs_ctx* ctx, const double* d_xyz, const uint8_t* d_rgb, uint64_t n, rcmvs_points* out) {
+    const int rc = alloc_points(ctx, n, out);
+    if (rc) return rc;
     if (n) {
         CK(rcmvs::host_download(out->xyz, d_xyz, 24 * n, ctx->stream));
         CK(rcmvs::host_download(out->rgb, d_rgb, 3 * n, ctx->stream));
@@ -1023,13 +1037,7 @@ int rcmvs_fuse_depth_maps(rcmvs_ctx* ctx, const rcmvs_view* views, int32_t n_vie
         uint64_t np = 0;
         int r = rcmvs_scene_fuse(ctx, sc, order_offsets, order, sparse_xyz, n_sparse, opts, &np);
         if (r) return r;
-        out->xyz = (double*)rcmvs::host_alloc(24 * np);
-        out->rgb = (uint8_t*)rcmvs::host_alloc(3 * np);
-        if (!out->xyz || !out->rgb) {
-            rcmvs_points_free(out);
-            return fail(ctx, RCMVS_E_NOMEM, "host allocation of the point cloud failed");
-        }
-        out->n = np;
+        if ((r = alloc_points(ctx, np, out))) return r;
         return rcmvs_scene_get_points(ctx, sc, out->xyz, out->rgb, nullptr);
     };
     rc = body();
@@ -1383,13 +1391,7 @@ static int run_mvs_impl(rcmvs_ctx* ctx, const rcmvs_view* views, int32_t n_views
         uint64_t np = 0;
         r = rcmvs_scene_fuse(ctx, sc, fo.data(), ff.data(), sparse->xyz, sparse->n_points, opts, &np);
         if (r) return r;
-        out->xyz = (double*)rcmvs::host_alloc(24 * np);
-        out->rgb = (uint8_t*)rcmvs::host_alloc(3 * np);
-        if (!out->xyz || !out->rgb) {
-            rcmvs_points_free(out);
-            return fail(ctx, RCMVS_E_NOMEM, "host allocation of the point cloud failed");
-        }
-        out->n = np;
+        if ((r = alloc_points(ctx, np, out))) return r;
         r = rcmvs_scene_get_points(ctx, sc, out->xyz, out->rgb, nullptr);
         if (r) return r;
         CK(cudaEventRecord(e3, ctx->stream));
@@ -1430,7 +1432,7 @@ static int run_mvs_impl(rcmvs_ctx* ctx, const rcmvs_view* views, int32_t n_views
     cudaEventDestroy(e1);
     cudaEventDestroy(e2);
     cudaEventDestroy(e3);
-    if (rc) rcmvs_points_free(out);
+    if (rc) ctx->drop(out);
     return rc;
 }
 

@@ -2,6 +2,8 @@
 // handles, shared by the translation units that implement the C ABI.
 #pragma once
 
+#include <algorithm>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -29,6 +31,21 @@ struct rcmvs_ctx {
     // set by a tensor-core kernel whose bounded wait gave up, until the call
     // that reports it (report_fault) clears it
     int* d_fault = nullptr;
+    rcmvs_result_alloc alloc = nullptr;  // rcmvs_ctx_set_result_alloc
+    void* alloc_user = nullptr;
+    // An array of a result: n elements (points, features), `each` bytes apiece.
+    void* result(int field, uint64_t n, size_t each) {
+        return alloc ? alloc(alloc_user, field, n) : std::malloc(std::max<size_t>(n * each, 1));
+    }
+    // What a failed call had allocated of its result.
+    void drop(rcmvs_points* p) {
+        if (alloc) *p = rcmvs_points{};
+        rcmvs_points_free(p);
+    }
+    void drop(rcmvs_sift_frame* f) {
+        if (alloc) f->pts = nullptr, f->desc = nullptr, f->colors = nullptr;
+        rcmvs_sift_frame_free(f);
+    }
     uint64_t last_evals = 0, last_rows = 0;
     // autotuned tile shapes per resolution class, one thread count and one
     // threads-per-pixel of the passes for all

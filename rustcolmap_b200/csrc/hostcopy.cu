@@ -14,7 +14,6 @@
 // goes the plain way).  The last context to close gives all of it back.
 #include "hostcopy.cuh"
 
-#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -297,19 +296,6 @@ cudaError_t host_upload(void* dev, const void* host, size_t n, cudaStream_t st) 
 }
 cudaError_t host_download(void* host, const void* dev, size_t n, cudaStream_t st) {
     return copy(const_cast<void*>(dev), host, n, st, false);
-}
-
-void* host_alloc(size_t n) {
-    void* p = std::malloc(std::max<size_t>(n, 1));
-    // large pages where they are offered on request: fewer faults on first touch
-    constexpr size_t BIG = 4 << 20;
-    if (p && n >= BIG) {
-        const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-        const uintptr_t a = ((uintptr_t)p + page - 1) & ~(uintptr_t)(page - 1);
-        const uintptr_t b = ((uintptr_t)p + n) & ~(uintptr_t)(page - 1);
-        if (b > a) (void)madvise((void*)a, b - a, MADV_HUGEPAGE);
-    }
-    return p;
 }
 
 void host_copy_attach() {

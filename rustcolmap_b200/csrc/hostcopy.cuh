@@ -13,9 +13,6 @@ cudaError_t host_upload(void* dev, const void* host, size_t n, cudaStream_t st);
 // The destination is filled on return, with all that was queued on st done.
 cudaError_t host_download(void* host, const void* dev, size_t n, cudaStream_t st);
 
-// malloc for a result of n bytes that a download will fill.
-void* host_alloc(size_t n);
-
 // Contexts that may copy; what the copies keep (threads, pinned buffers) is
 // given back with the last one.
 void host_copy_attach();

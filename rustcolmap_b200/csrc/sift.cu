@@ -1172,11 +1172,11 @@ int rcmvs_extract_sift(rcmvs_ctx* ctx, const uint8_t* img, int32_t w0, int32_t h
     out->height = h;
     out->n_raw = n_raw;
     out->n = (uint64_t)n_out;
-    out->pts = (double*)host_alloc(sizeof(double) * 2 * n_out);
-    out->desc = (float*)host_alloc(sizeof(float) * DESC_LEN * n_out);
-    out->colors = (uint8_t*)host_alloc(3 * n_out);
+    out->pts = (double*)ctx->result(RCMVS_RESULT_PTS, n_out, sizeof(double) * 2);
+    out->desc = (float*)ctx->result(RCMVS_RESULT_DESC, n_out, sizeof(float) * DESC_LEN);
+    out->colors = (uint8_t*)ctx->result(RCMVS_RESULT_COLORS, n_out, 3);
     if (!out->pts || !out->desc || !out->colors) {
-        rcmvs_sift_frame_free(out);
+        ctx->drop(out);
         return sfail(ctx, RCMVS_E_NOMEM, "sift: host allocation failed");
     }
     if (n_out == 0) return RCMVS_OK;

@@ -37,9 +37,11 @@ class Context:
                                  "(needs an sm_100 GPU)")
         self.ptr = p
         self.device = device
+        self.check(self._L.rcmvs_ctx_set_result_alloc(p, _abi.result_alloc, None))
 
     def check(self, rc):
         if rc != 0:
+            _abi.drop_results()
             raise RcmvsError(rc, self._L.rcmvs_last_error(self.ptr).decode())
 
     @property
@@ -176,18 +178,11 @@ def fuse_depth_maps(views, depth_maps, sources, sparse_xyz, opts, ctx=None):
     o = opts.to_c()
     ctx.check(ctx._L.rcmvs_fuse_depth_maps(ctx.ptr, va, len(views), dptr, off.ctypes.data, flat.ctypes.data,
                                            sp.ctypes.data, len(sp), C.byref(o), C.byref(pts)))
-    return _take_points(ctx, pts)
+    return _take_points()
 
 
-def _take_points(ctx, pts):
-    n = pts.n
-    if n == 0:
-        ctx._L.rcmvs_points_free(C.byref(pts))
-        return np.zeros((0, 3), np.float64), np.zeros((0, 3), np.uint8)
-    own = _abi.Owned(pts, ctx._L.rcmvs_points_free)
-    xyz = own.array(pts.xyz, C.c_double, (n, 3))
-    rgb = own.array(pts.rgb, C.c_uint8, (n, 3))
-    return xyz, rgb
+def _take_points():
+    return _abi.take_result(_abi.XYZ), _abi.take_result(_abi.RGB)
 
 
 def fuse_candidates(views, depth_maps, sources, ref_views, opts, ctx=None):
@@ -207,7 +202,7 @@ def fuse_candidates(views, depth_maps, sources, ref_views, opts, ctx=None):
     ctx.check(ctx._L.rcmvs_fuse_candidates(ctx.ptr, va, len(views), dptr, off.ctypes.data, flat.ctypes.data,
                                            refs.ctypes.data, len(ref_views), C.byref(o), C.byref(pts),
                                            per_view.ctypes.data))
-    xyz, rgb = _take_points(ctx, pts)
+    xyz, rgb = _take_points()
     return xyz, rgb, per_view
 
 
@@ -223,7 +218,7 @@ def fuse_reduce(xyz, rgb, sparse_xyz, opts, ctx=None):
     o = opts.to_c()
     ctx.check(ctx._L.rcmvs_fuse_reduce(ctx.ptr, xyz.ctypes.data, rgb.ctypes.data, len(xyz), sp.ctypes.data, len(sp),
                                        C.byref(o), C.byref(pts)))
-    return _take_points(ctx, pts)
+    return _take_points()
 
 
 def depth_vis(depth, ctx=None):
@@ -405,7 +400,7 @@ class DeviceScene:
         self.ctx.check(self.ctx._L.rcmvs_scene_fuse_candidates(self.ctx.ptr, self.ptr, off.ctypes.data,
                                                                flat.ctypes.data, refs.ctypes.data, len(ref_views),
                                                                C.byref(o), C.byref(pts), per_view.ctypes.data))
-        xyz, rgb = _take_points(self.ctx, pts)
+        xyz, rgb = _take_points()
         return xyz, rgb, per_view
 
     # device-to-device moves (one scene over several processes); ptr
@@ -547,7 +542,7 @@ def run_mvs(views, sparse, opts, out_dir=None, ctx=None, log=None, return_depth=
         ctx.check(ctx._L.rcmvs_run_mvs_learned(ctx.ptr, va, len(views), C.byref(sp), C.byref(o), net.ptr,
                                                float(conf_thr), int(n_local), float(span), douts, C.byref(pts),
                                                C.byref(st)))
-    xyz, rgb = _take_points(ctx, pts)
+    xyz, rgb = _take_points()
     if want_vis:
         srcs, _, _ = plan(sparse, views, opts)
         vis_dir = os.path.join(out_dir, "dense", "depth_vis")

@@ -53,10 +53,8 @@ def extract_sift(img, name="", opts=None, ctx=None):
     o = opts.to_c()
     f = _abi.SiftFrame()
     ctx.check(ctx._L.rcmvs_extract_sift(ctx.ptr, a.ctypes.data, w, h, c, C.byref(o), C.byref(f)))
-    own = _abi.Owned(f, ctx._L.rcmvs_sift_frame_free)
-    n = f.n
-    return SiftFrame(name, f.width, f.height, own.array(f.pts, C.c_double, (n, 2)),
-                     own.array(f.desc, C.c_float, (n, DESC_LEN)), own.array(f.colors, C.c_uint8, (n, 3)), int(f.n_raw))
+    pts, desc, colors = (_abi.take_result(k) for k in (_abi.PTS, _abi.DESC, _abi.COLORS))
+    return SiftFrame(name, f.width, f.height, pts, desc, colors, int(f.n_raw))
 
 
 def extract_sift_many(images, names=None, opts=None, ctxs=None):
