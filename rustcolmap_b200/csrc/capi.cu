@@ -172,14 +172,13 @@ int rcmvs_ctx_create(int device, rcmvs_ctx** out) {
         }
     }
     if (cudaMalloc(&ctx->d_fault, sizeof(int)) != cudaSuccess ||
-        cudaMemsetAsync(ctx->d_fault, 0, sizeof(int), ctx->stream) != cudaSuccess) {
+        cudaMemsetAsync(ctx->d_fault, 0, sizeof(int), ctx->stream) != cudaSuccess || !rcmvs::host_copy_attach()) {
         cudaFree(ctx->d_fault);
         cudaFree(ctx->d_work);
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return RCMVS_E_NOMEM;
     }
-    rcmvs::host_copy_attach();
     *out = ctx;
     return RCMVS_OK;
 }

@@ -19,12 +19,13 @@
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
-#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <exception>
+#include <memory>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -55,7 +56,7 @@ class Helpers {
         const unsigned n = std::min(THREADS, cores > 1 ? cores - 1 : 0u);
         try {
             while (threads_.size() < n) threads_.emplace_back([this] { loop(); });
-        } catch (const std::system_error&) {  // fewer, or none: the callers do the work
+        } catch (const std::exception&) {  // no thread or no memory: fewer, or none, and the callers do the work
         }
     }
     // Of this process: a forked child has the objects but not the threads.
@@ -129,12 +130,14 @@ struct Ring {
 };
 
 struct Service {
+    Service() { rings.reserve(LEASES); }
     std::mutex m;
     int users = 0;
     std::vector<Ring*> rings;
     Helpers helpers;
 };
-// never destroyed: threads may outlive static destruction at exit
+// never destroyed: threads may outlive static destruction at exit.  Made by the
+// first context; only that may throw.
 Service& service() {
     static Service* s = new Service;
     return *s;
@@ -173,7 +176,8 @@ Ring* take_ring() {
         free_ring(*it);
         s.rings.erase(it);
     }
-    Ring* r = new Ring;
+    Ring* r = new (std::nothrow) Ring;
+    if (!r) return nullptr;
     r->device = dev;
     bool ok = cudaHostAlloc((void**)&r->mem, SLOT * SLOTS, cudaHostAllocDefault) == cudaSuccess;
     for (int i = 0; i < SLOTS && ok; ++i) ok = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming) == cudaSuccess;
@@ -208,11 +212,10 @@ bool through_ring(const void* host, size_t n, cudaStream_t st, bool up) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-cudaError_t ring_copy(Ring* r, char* dev, char* host, size_t bytes, cudaStream_t st, bool up) {
+// done: one zero for each piece.
+cudaError_t ring_copy(Ring* r, char* dev, char* host, size_t bytes, std::atomic<int>* done, int n, cudaStream_t st,
+                      bool up) {
     Helpers& h = service().helpers;
-    const int n = (int)((bytes + SLOT - 1) / SLOT);
-    std::vector<std::atomic<int>> done(n);
-    for (auto& d : done) d.store(0, std::memory_order_relaxed);
     auto size = [&](int k) { return std::min(SLOT, bytes - SLOT * k); };
     auto slot = [&](int k) { return r->mem + SLOT * (k % SLOTS); };
     auto hand_over = [&](int k) {  // the host's part of piece k
@@ -273,20 +276,18 @@ cudaError_t ring_copy(Ring* r, char* dev, char* host, size_t bytes, cudaStream_t
 }
 
 cudaError_t copy(void* dev, void* host, size_t n, cudaStream_t st, bool up) {
-    Ring* r = through_ring(host, n, st, up) ? take_ring() : nullptr;
-    if (!r) {
-        const cudaError_t e = up ? cudaMemcpyAsync(dev, host, n, cudaMemcpyHostToDevice, st)
-                                 : cudaMemcpyAsync(host, dev, n, cudaMemcpyDeviceToHost, st);
-        return up || e != cudaSuccess ? e : cudaStreamSynchronize(st);
+    if (through_ring(host, n, st, up)) {
+        const int pieces = (int)((n + SLOT - 1) / SLOT);
+        std::unique_ptr<std::atomic<int>[]> done(new (std::nothrow) std::atomic<int>[pieces]());
+        if (Ring* r = done ? take_ring() : nullptr) {
+            const cudaError_t e = ring_copy(r, (char*)dev, (char*)host, n, done.get(), pieces, st, up);
+            give_ring(r);
+            return e;
+        }
     }
-    cudaError_t e;
-    try {
-        e = ring_copy(r, (char*)dev, (char*)host, n, st, up);
-    } catch (const std::bad_alloc&) {
-        e = cudaErrorMemoryAllocation;
-    }
-    give_ring(r);
-    return e;
+    const cudaError_t e = up ? cudaMemcpyAsync(dev, host, n, cudaMemcpyHostToDevice, st)
+                             : cudaMemcpyAsync(host, dev, n, cudaMemcpyDeviceToHost, st);
+    return up || e != cudaSuccess ? e : cudaStreamSynchronize(st);
 }
 
 }  // namespace
@@ -298,10 +299,15 @@ cudaError_t host_download(void* host, const void* dev, size_t n, cudaStream_t st
     return copy(const_cast<void*>(dev), host, n, st, false);
 }
 
-void host_copy_attach() {
-    Service& s = service();
-    std::lock_guard<std::mutex> l(s.m);
-    ++s.users;
+bool host_copy_attach() {
+    try {
+        Service& s = service();
+        std::lock_guard<std::mutex> l(s.m);
+        ++s.users;
+    } catch (const std::exception&) {
+        return false;
+    }
+    return true;
 }
 
 void host_copy_detach() {

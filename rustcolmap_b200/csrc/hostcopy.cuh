@@ -14,8 +14,8 @@ cudaError_t host_upload(void* dev, const void* host, size_t n, cudaStream_t st);
 cudaError_t host_download(void* host, const void* dev, size_t n, cudaStream_t st);
 
 // Contexts that may copy; what the copies keep (threads, pinned buffers) is
-// given back with the last one.
-void host_copy_attach();
+// given back with the last one.  false: no memory, nothing attached.
+bool host_copy_attach();
 void host_copy_detach();
 
 }  // namespace rcmvs
