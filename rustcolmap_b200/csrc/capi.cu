@@ -38,6 +38,12 @@ cudaError_t DeviceArena::get(int slot, size_t bytes, void** out) {
     return cudaSuccess;
 }
 
+void DeviceArena::drop(int slot) {
+    if ((int)slots.size() <= slot || !slots[slot].p) return;
+    cudaFree(slots[slot].p);
+    slots[slot] = Slot{};
+}
+
 void DeviceArena::release() {
     for (auto& s : slots)
         if (s.p) cudaFree(s.p);

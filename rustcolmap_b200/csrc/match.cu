@@ -257,6 +257,7 @@ struct Frame {
 struct MatchStatus {
     int wild;   // a component past PACK_LIMIT or not finite
     int listed; // queries for rescan_kernel
+    int fault;  // the context's fault word was set (outcome_kernel)
 };
 
 // Block b of 128 descriptors: half (hi, lo) h, descriptor r, component k at
@@ -526,7 +527,10 @@ __global__ void __launch_bounds__(256) outcome_kernel(const PairJob* __restrict_
                                                       uint32_t* __restrict__ fwd, uint32_t* __restrict__ bwd,
                                                       int2* __restrict__ list, MatchStatus* __restrict__ st,
                                                       const int* __restrict__ fault) {
-    if (*fault) return;
+    if (*fault) {
+        st->fault = 1;  // the host reads one block
+        return;
+    }
     const int dir = blockIdx.y & 1;
     const PairJob J = jobs[blockIdx.y >> 1];
     Frame q, t;
@@ -763,14 +767,33 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
     MCK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     DeviceArena& A = ctx->arena;
+    // tensor: no frame was found out of range (and a ratio the bound's tests
+    // take), and the search's buffers fit
+    const float r32 = (float)ratio;
+    bool packed = false, tensor = r32 > 0.0f && r32 < 1e6f;
+    // What the FP32 kernels need; the search's packed frames (as large as the
+    // descriptors), this call's or an earlier one's, go where they take its room.
+    auto need = [&](int slot, size_t bytes, void** p) -> cudaError_t {
+        cudaError_t e = A.get(slot, bytes, p);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        for (int s : {(int)M_PACK, (int)M_NORM, (int)M_TWO}) A.drop(s);
+        packed = tensor = false;
+        return A.get(slot, bytes, p);
+    };
+    // What they do without.
+    auto room = [&](int slot, size_t bytes, void** p) {
+        if (A.get(slot, bytes, p) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    };
     void* p_desc;
-    MCK(A.get(M_DESC, sizeof(float) * DESC_LEN * (size_t)std::max<int64_t>(foff[n_frames], 1), &p_desc));
+    MCK(need(M_DESC, sizeof(float) * DESC_LEN * (size_t)std::max<int64_t>(foff[n_frames], 1), &p_desc));
     auto upload = [&](int f, cudaStream_t on) -> cudaError_t {
         if (n_desc[f] == 0) return cudaSuccess;
         return cudaMemcpyAsync((float*)p_desc + foff[f] * DESC_LEN, desc[f], sizeof(float) * DESC_LEN * n_desc[f],
                                cudaMemcpyHostToDevice, on);
     };
-    const float r32 = (float)ratio;
     // the tensor-core search's packed frames (made with the first chunk that uses it)
     std::vector<Frame> frames(n_frames);
     std::vector<int32_t> blk(n_frames + 1, 0);
@@ -779,9 +802,26 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
         if (blk[f] > INT32_MAX / 2) return mfail(ctx, RCMVS_E_LIMIT, "too many descriptors");
         blk[f + 1] = blk[f] + (n_desc[f] + QB - 1) / QB;
     }
-    // tensor: no frame was found out of range (and a ratio the bound's tests take)
-    bool packed = false, tensor = r32 > 0.0f && r32 < 1e6f;
-    void *p_frames = nullptr, *p_blk = nullptr, *p_pack = nullptr, *p_norm = nullptr, *p_maxn = nullptr, *p_st = nullptr;
+    void *p_frames = nullptr, *p_blk = nullptr, *p_pack = nullptr, *p_norm = nullptr, *p_maxn = nullptr, *p_st = nullptr,
+         *p_two = nullptr, *p_list = nullptr;
+    void *p_jobs, *p_fwd, *p_bwd, *p_mb;
+    auto chunk_room = [&](size_t n_jobs, int64_t rows, int64_t cols) -> cudaError_t {
+        cudaError_t e = need(M_JOBS, sizeof(PairJob) * n_jobs, &p_jobs);
+        if (!e) e = need(M_FWD, sizeof(Nearest) * (size_t)rows, &p_fwd);
+        if (!e) e = need(M_BWD, sizeof(Nearest) * (size_t)cols, &p_bwd);
+        if (!e) e = need(M_MB, sizeof(uint32_t) * (size_t)rows, &p_mb);
+        return e;
+    };
+    auto tensor_room = [&](int64_t rows, int64_t cols) {
+        const size_t nb = (size_t)std::max(blk[n_frames], 1);
+        tensor = room(M_FRAMES, (sizeof(Frame) + sizeof(int32_t)) * n_frames, &p_frames) &&
+                 room(M_PACK, nb * QB_BYTES, &p_pack) && room(M_NORM, nb * QB * sizeof(float), &p_norm) &&
+                 room(M_MAXN, sizeof(int) * n_frames, &p_maxn) &&
+                 room(M_TWO, sizeof(Two) * (size_t)(rows + cols), &p_two) &&
+                 room(M_LIST, sizeof(int2) * RESCAN_MAX, &p_list) && room(M_STATUS, sizeof(MatchStatus), &p_st);
+        if (tensor) p_blk = (Frame*)p_frames + n_frames;
+        return tensor;
+    };
     // Where all pairs make one chunk for the tensor-core search, the frames go
     // up on the context's second stream in groups, and a group is packed and
     // its pairs with the frames before it are searched while the next is
@@ -797,7 +837,8 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
             cols += nb;
         }
         overlap = dists >= TENSOR_MIN && (size_t)partials * sizeof(Nearest) <= P_BUDGET && rows <= INT32_MAX / 2 &&
-                  cols <= INT32_MAX / 2;
+                  cols <= INT32_MAX / 2 && chunk_room((size_t)n_pairs, rows, cols) == cudaSuccess && tensor_room(rows, cols);
+        if (!overlap) cudaGetLastError();
     }
     Event uploaded;
     if (overlap) {
@@ -832,11 +873,8 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
         }
         const int first = p - (int)jobs.size();
         if (max_na > 0 && max_nb > 0) {
-            void *p_jobs, *p_rowp, *p_colp, *p_fwd, *p_bwd, *p_mb;
-            MCK(A.get(M_JOBS, sizeof(PairJob) * jobs.size(), &p_jobs));
-            MCK(A.get(M_FWD, sizeof(Nearest) * (size_t)rows, &p_fwd));
-            MCK(A.get(M_BWD, sizeof(Nearest) * (size_t)cols, &p_bwd));
-            MCK(A.get(M_MB, sizeof(uint32_t) * (size_t)rows, &p_mb));
+            void *p_rowp, *p_colp;
+            MCK(chunk_room(jobs.size(), rows, cols));
             // on the device in the order in which their frames arrive
             std::vector<PairJob> queue(jobs);
             if (overlap)
@@ -846,13 +884,10 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
             MCK(cudaMemcpyAsync(p_jobs, queue.data(), sizeof(PairJob) * jobs.size(), cudaMemcpyHostToDevice, st));
             const unsigned nj = (unsigned)jobs.size();
             const SpanHook& hook = ctx->hook();
-            const bool compact = rows >= COMPACT_MIN;
-            std::vector<uint32_t> mb(compact ? 0 : (size_t)rows), begin(compact ? jobs.size() + 1 : 0);
             void *p_begin = nullptr, *p_ab = nullptr;
-            if (compact) {
-                MCK(A.get(M_BEGIN, sizeof(uint32_t) * (2 * jobs.size() + 1), &p_begin));
-                MCK(A.get(M_AB, sizeof(uint32_t) * 2 * (size_t)rows, &p_ab));
-            }
+            const bool compact = rows >= COMPACT_MIN && room(M_BEGIN, sizeof(uint32_t) * (2 * jobs.size() + 1), &p_begin) &&
+                                 room(M_AB, sizeof(uint32_t) * 2 * (size_t)rows, &p_ab);
+            std::vector<uint32_t> mb(compact ? 0 : (size_t)rows), begin(compact ? jobs.size() + 1 : 0);
             // the answers' counts, or the answers, to the host
             auto collect = [&]() -> cudaError_t {
                 if (!compact)
@@ -868,22 +903,12 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                                         : cudaMemcpyAsync(begin.data(), p_begin, sizeof(uint32_t) * begin.size(),
                                                           cudaMemcpyDeviceToHost, st);
             };
-            bool on_tensor = tensor && dists >= TENSOR_MIN;
+            bool on_tensor = tensor && dists >= TENSOR_MIN && tensor_room(rows, cols);
             if (on_tensor) {
-                void *p_two, *p_list;
-                MCK(A.get(M_TWO, sizeof(Two) * (size_t)(rows + cols), &p_two));
-                MCK(A.get(M_LIST, sizeof(int2) * RESCAN_MAX, &p_list));
-                MCK(A.get(M_STATUS, sizeof(MatchStatus), &p_st));
                 Two *f2 = (Two*)p_two, *b2 = f2 + rows;
                 // the answers share the nearest entries' buffers (larger)
                 uint32_t *fo = (uint32_t*)p_fwd, *bo = (uint32_t*)p_bwd;
                 if (!packed) {
-                    const size_t nb = (size_t)std::max(blk[n_frames], 1);
-                    MCK(A.get(M_FRAMES, (sizeof(Frame) + sizeof(int32_t)) * n_frames, &p_frames));
-                    MCK(A.get(M_PACK, nb * QB_BYTES, &p_pack));
-                    MCK(A.get(M_NORM, nb * QB * sizeof(float), &p_norm));
-                    MCK(A.get(M_MAXN, sizeof(int) * n_frames, &p_maxn));
-                    p_blk = (Frame*)p_frames + n_frames;
                     MCK(cudaMemcpyAsync(p_frames, frames.data(), sizeof(Frame) * n_frames, cudaMemcpyHostToDevice, st));
                     MCK(cudaMemcpyAsync(p_blk, blk.data(), sizeof(int32_t) * n_frames, cudaMemcpyHostToDevice, st));
                     MCK(cudaMemsetAsync(p_maxn, 0, sizeof(int) * n_frames, st));
@@ -956,18 +981,16 @@ static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int3
                 MCK(cudaGetLastError());
                 hook.end("match_select");
                 MatchStatus status{};
-                int fault = 0;
                 MCK(cudaMemcpyAsync(&status, p_st, sizeof(status), cudaMemcpyDeviceToHost, st));
-                MCK(cudaMemcpyAsync(&fault, ctx->d_fault, sizeof(int), cudaMemcpyDeviceToHost, st));
                 MCK(collect());
                 MCK(cudaStreamSynchronize(st));
-                if (fault) return report_fault(ctx);
+                if (status.fault) return report_fault(ctx);
                 if (status.wild) tensor = false;
                 on_tensor = !status.wild && status.listed <= RESCAN_MAX;
             }
             if (!on_tensor) {
-                MCK(A.get(M_ROWP, sizeof(Nearest) * (size_t)std::max<int64_t>(prow, 1), &p_rowp));
-                MCK(A.get(M_COLP, sizeof(Nearest) * (size_t)std::max<int64_t>(pcol, 1), &p_colp));
+                MCK(need(M_ROWP, sizeof(Nearest) * (size_t)std::max<int64_t>(prow, 1), &p_rowp));
+                MCK(need(M_COLP, sizeof(Nearest) * (size_t)std::max<int64_t>(pcol, 1), &p_colp));
                 hook.begin("match_dist");
                 dist_kernel<<<dim3((max_nb + TILE - 1) / TILE, (max_na + TILE - 1) / TILE, nj), 256, 0, st>>>(
                     (const float*)p_desc, (const PairJob*)p_jobs, (Nearest*)p_rowp, (Nearest*)p_colp);

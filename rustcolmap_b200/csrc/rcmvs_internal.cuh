@@ -230,6 +230,7 @@ struct DeviceArena {
     };
     std::vector<Slot> slots;
     cudaError_t get(int slot, size_t bytes, void** out);
+    void drop(int slot);
     void release();
 };
 
