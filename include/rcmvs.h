@@ -557,6 +557,11 @@ typedef struct rcmvs_matches {
 int rcmvs_match_pairs(rcmvs_ctx* ctx, const float* const* desc, const int32_t* n_desc, int32_t n_frames,
                       const int32_t* pairs, int32_t n_pairs, double ratio, rcmvs_matches* out);
 void rcmvs_matches_free(rcmvs_matches* matches);
+/* Diagnostic of the tensor-core search behind rcmvs_match_pairs: the squared
+ * distance of each of n_q descriptors to its nearest of n_t as the search
+ * approximates it, and the bound within which it decides nothing by it. */
+int rcmvs_diag_match_distances(rcmvs_ctx* ctx, const float* q, int32_t n_q, const float* t, int32_t n_t,
+                               float* approx, float* bound);
 
 /* ---------------------------------------------------------- diagnostics */
 

@@ -309,6 +309,10 @@ pub fn rcmvs_options_default(opts: *mut rcmvs_options);
     pub fn rcmvs_match_pairs(ctx: *mut rcmvs_ctx, desc: *const *const f32, n_desc: *const i32, n_frames: i32,
                              pairs: *const i32, n_pairs: i32, ratio: f64, out: *mut rcmvs_matches) -> c_int;
     pub fn rcmvs_matches_free(matches: *mut rcmvs_matches);
+    /// Diagnostic: the tensor-core search's approximate nearest distances and their bounds.
+    pub fn rcmvs_diag_match_distances(
+        ctx: *mut rcmvs_ctx, q: *const f32, n_q: i32, t: *const f32, n_t: i32, approx: *mut f32, bound: *mut f32,
+    ) -> c_int;
     /// plane_cost (mvs/src/stereo.rs:158-228) at every pixel for a given plane field (diagnostic).
     pub fn rcmvs_plane_cost_field(ctx: *mut rcmvs_ctx, views: *const rcmvs_view, n_views: i32, ref_idx: i32,
                                   srcs: *const i32, n_src: i32, planes: *const f32, hints: *const f32,

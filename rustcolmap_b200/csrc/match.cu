@@ -7,7 +7,7 @@
 //
 // The reference sums (a_k - b_k)^2 serially over k = 0..127 in f32.  Its
 // result is only which descriptors pass the tests on the nearest and
-// second-nearest distance, so a tensor-core product with a proven error bound
+// second-nearest distance, so a tensor-core product with an error bound
 // decides every descriptor that is not within the bound of a test's edge,
 // and only the rest are summed as written:
 //
@@ -16,7 +16,7 @@
 //                 and squared norms
 //   nearest_kernel  one CTA per 128 descriptors of one frame (queries) against
 //                 all descriptors of the other, both directions of each pair:
-//                 |t|^2 - 2 q.t, the products as hi.hi + hi.lo + lo.hi on
+//                 |t|^2 - 2 q.t, the products as hi.lo + lo.hi + hi.hi on
 //                 tcgen05.mma with FP32 accumulation in tensor memory; one
 //                 thread keeps the two smallest of its query and half of the
 //                 targets
@@ -27,12 +27,22 @@
 //                 the reference's tests
 //   mutual_kernel the reference's mutual check per row of A
 //
-// Error bound (u = 2^-24; |q|, |t| norms): operands to 2^-22 relative or 2^-31
-// absolute per component, lo.lo dropped (2^-22 |q||t|), 384 products summed in
-// FP32 (64 u), norms to 8 u, the reference's own serial sum 131 u d.  With S =
-// |q| + max |t|, an approximate distance is within
-// (2^-17 / 2 + 2^-20) S^2 + 2^-26 S of the exact one, and the reference's
-// within 7.9e-6 d of that.
+// Error bound (u = 2^-24; |q|, |t| norms, S = |q| + max |t|, so |q||t| <= S^2 / 4).
+// In the distance, 2 q.t counts twice:
+//   operands to 2^-22 relative or 2^-31 absolute per component   4 u S^2 + 2^-26 S
+//   lo.lo dropped (2^-22 |q||t|)                                 2 u S^2
+//   sums of the products                                        42 u S^2
+//   norms (summed in f64), |t|^2 - 2 q.t and + |q|^2 rounded     4 u S^2
+// together 52 u S^2 + 2^-26 S; search_bound takes 80 u.  The sums' part rests on
+// a measurement, since PTX leaves the rounding of kind::f16 open: an MMA cuts its
+// 16 products and the accumulator toward zero to 2^-25 of the largest one's power
+// of two, adds them, and cuts the sum toward zero to FP32 (this model gave all of
+// 26389 products, magnitudes over 2^-28 .. 1 and both signs, bit for bit).  So an
+// MMA loses at most 17 u / 2 + 2 u of the largest term.  The products with a lo are
+// summed first, while all terms are below 2^-10 |q||t|; after them come 8 MMAs of
+// hi.hi: 84 u |q||t|.  (With hi.lo last there were 16 at full size: 168 u, of
+// which up to 95 u were measured.)  The reference's own serial sum is within
+// 131 u d < 7.9e-6 d of the exact distance.
 //
 // Frames with components past 1000 or not finite, and chunks in which many
 // queries are listed (repeated descriptors), run on the FP32 pipes instead:
@@ -268,7 +278,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ des
                                                    const int32_t* __restrict__ blk_start, int n_frames, int first,
                                                    unsigned char* __restrict__ packed, float* __restrict__ norms,
                                                    int* __restrict__ max_norm, MatchStatus* __restrict__ st) {
-    __shared__ float part[2][QB];
+    __shared__ double part[2][QB];
     const int block = first + (int)blockIdx.x;
     int lo = 0, hi = n_frames - 1;
     while (lo < hi) {
@@ -284,7 +294,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ des
     const bool in = row < F.n;
     const float* src = desc + (F.off + row) * DESC_LEN;
     unsigned char* out = packed + (size_t)block * QB_BYTES + r * 16;
-    float sum = 0.0f;
+    double sum = 0.0;
     bool wild = false;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -298,7 +308,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ des
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             wild = wild || !(fabsf(x[c]) <= PACK_LIMIT);
-            sum = __fmaf_rn(x[c], x[c], sum);
+            sum = __fma_rn((double)x[c], (double)x[c], sum);
             const float v = x[c] * PACK_SCALE;
             h[c] = __float2half_rn(v);
             l[c] = __float2half_rn(v - __half2float(h[c]));
@@ -310,7 +320,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ des
     if (wild) st->wild = 1;
     __syncthreads();
     if (half == 0) {
-        const float n = part[0][r] + part[1][r];
+        const float n = (float)(part[0][r] + part[1][r]);
         norms[(size_t)block * QB + r] = in ? n : INFINITY;
         float m = in ? n : 0.0f;
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -335,8 +345,8 @@ __device__ __forceinline__ void direction(const PairJob& J, const Frame* frames,
 // slots for the halves (hi, lo) of the target blocks; tensor memory two
 // accumulators per query block (128 columns each), one multiplying while the
 // other is read.  Warp 8's first thread loads and multiplies: step 2c is
-// block c's hi (queries lo, then hi), step 2c + 1 its lo (queries hi); the
-// load of step s + 2 starts when step s - 1's products are done, two steps
+// block c's lo (queries hi), step 2c + 1 its hi (queries lo, then hi: the small
+// terms first, for the error bound); the load of step s + 2 starts when step s - 1's products are done, two steps
 // ahead of its use.  Warps 0-3 scan the first query block's values, 4-7 the
 // second's, one thread per query.  Bound by the tensor pipe (48 MMAs of
 // 128 x 128 x 16 per target block, 55% active) and the L2 reads of the target
@@ -396,7 +406,7 @@ __global__ void __launch_bounds__(kNearestThreads, 1)
             };
             auto load_step = [&](int s) {
                 mbar_expect_tx(full(s % NSLOT), QB_HALF);
-                load(ring + (s % NSLOT) * QB_HALF, packed + (t.blk + (s >> 1)) * (int64_t)QB_BYTES + (s & 1) * QB_HALF,
+                load(ring + (s % NSLOT) * QB_HALF, packed + (t.blk + (s >> 1)) * (int64_t)QB_BYTES + ((s & 1) ^ 1) * QB_HALF,
                      QB_HALF, full(s % NSLOT));
                 ++loaded;
             };
@@ -416,13 +426,13 @@ __global__ void __launch_bounds__(kNearestThreads, 1)
                 const uint32_t sb = ring + slot * QB_HALF;
                 for (int b = 0; b < nq; ++b) {
                     const uint32_t d = taddr + (2 * b + (c & 1)) * QB;
-                    for (int term = (s & 1) ? 1 : 0; term < 2; ++term) {  // queries lo, then hi; only hi against lo
+                    for (int term = (s & 1) ? 0 : 1; term < 2; ++term) {  // queries lo, then hi; only hi against lo
                         const uint32_t a0 = sq + b * QB_BYTES + (term == 0 ? QB_HALF : 0);
 #pragma unroll
                         for (int kc = 0; kc < DESC_LEN / 16; ++kc)
                             umma_f16(d, umma_desc(a0 + kc * (2 * QB * 16), QB * 16, 128),
                                      umma_desc(sb + kc * (2 * QB * 16), QB * 16, 128), IDESC,
-                                     ((s & 1) | term | kc) != 0 ? 1u : 0u);
+                                     ((s & 1) | kc) != 0 ? 1u : 0u);
                     }
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(slot_free(slot))
@@ -494,6 +504,13 @@ __global__ void __launch_bounds__(kNearestThreads, 1)
     if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(4 * QB));
 }
 
+// What an approximate distance may be off (see the file's head), with 2% slack;
+// qn, tm: |q|^2 and the largest |t|^2.
+__device__ __forceinline__ float search_bound(float qn, float tm) {
+    const float s = sqrtf(qn) + sqrtf(tm);
+    return 1.02f * ((3.82e-6f + 9.6e-7f) * s * s + 1.5e-8f * s);
+}
+
 // The reference's distance (matching.rs:27-33).
 __device__ __forceinline__ float serial_dist(const float* __restrict__ a, const float* __restrict__ b) {
     float s = 0.0f;
@@ -542,10 +559,9 @@ __global__ void __launch_bounds__(256) outcome_kernel(const PairJob* __restrict_
     if (t.n > 1) {  // with fewer targets the second distance is infinite: refused
         const Two f = (dir ? bwd2 : fwd2)[out0 + row];
         const float qn = norms[q.blk * QB + row], tm = __int_as_float(max_norm[dir ? J.fa : J.fb]);
-        const float s = sqrtf(qn) + sqrtf(tm);
         const float d1 = f.v0 + qn, d2 = f.v1 + qn;
-        // the bound at the larger of the two distances, 2% slack
-        const float e = 1.02f * ((3.82e-6f + 9.6e-7f) * s * s + 1.5e-8f * s + 8.0e-6f * fmaxf(d2, 0.0f));
+        // the reference's own error at the larger of the two distances
+        const float e = search_bound(qn, tm) + 8.16e-6f * fmaxf(d2, 0.0f);
         const float r_lo = ratio * 0.9999995f, r_hi = ratio * 1.0000005f;
         const bool refused = (dir == 0 && d1 - e > 0.9000002f) || d1 - e > r_hi * (d2 + e);
         const bool accepted = (dir != 0 || d1 + e < 0.8999998f) && d1 + e < r_lo * (d2 - e) && d2 - d1 > 2.0f * e;
@@ -561,6 +577,17 @@ __global__ void __launch_bounds__(256) outcome_kernel(const PairJob* __restrict_
         }
     }
     (dir ? bwd : fwd)[out0 + row] = out;
+}
+
+// The smaller distance of each query of frame 0 (rcmvs_diag_match_distances) and
+// its bound.
+__global__ void distances_kernel(const Two* __restrict__ two, const float* __restrict__ norms,
+                                 const int* __restrict__ max_norm, int n, float* __restrict__ approx,
+                                 float* __restrict__ bound) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    approx[i] = two[i].v0 + norms[i];
+    bound[i] = search_bound(norms[i], __int_as_float(max_norm[1]));
 }
 
 // Listed queries against all targets; one block each.
@@ -734,6 +761,63 @@ void rcmvs_matches_free(rcmvs_matches* m) {
     m->offsets = nullptr;
     m->a = m->b = nullptr;
     m->n_pairs = 0;
+}
+
+int rcmvs_diag_match_distances(rcmvs_ctx* ctx, const float* q, int32_t n_q, const float* t, int32_t n_t, float* approx,
+                               float* bound) {
+    if (!ctx || !q || !t || n_q <= 0 || n_t <= 0 || n_q > (1 << 20) || n_t > (1 << 20) || !approx || !bound)
+        return mfail(ctx, RCMVS_E_ARG, "rcmvs_diag_match_distances: bad argument");
+    MCK(cudaSetDevice(ctx->device));
+    cudaStream_t st = ctx->stream;
+    DeviceArena& A = ctx->arena;
+    const int qb = (n_q + QB - 1) / QB, tb = (n_t + QB - 1) / QB;
+    const size_t n = (size_t)n_q + n_t, nb = (size_t)qb + tb, row = sizeof(float) * DESC_LEN;
+    const Frame frames[2] = {{0, 0, n_q}, {n_q, qb, n_t}};
+    const int32_t blk[3] = {0, qb, qb + tb};
+    PairJob job{};
+    job.na = n_q;
+    job.nb = n_t;
+    job.fb = 1;
+    void *p_desc, *p_frames, *p_pack, *p_norm, *p_maxn, *p_two, *p_st, *p_jobs, *p_out;
+    MCK(A.get(M_DESC, row * n, &p_desc));
+    MCK(A.get(M_FRAMES, sizeof(frames) + sizeof(blk), &p_frames));
+    MCK(A.get(M_PACK, nb * QB_BYTES, &p_pack));
+    MCK(A.get(M_NORM, nb * QB * sizeof(float), &p_norm));
+    MCK(A.get(M_MAXN, sizeof(int) * 2, &p_maxn));
+    MCK(A.get(M_TWO, sizeof(Two) * n, &p_two));
+    MCK(A.get(M_STATUS, sizeof(MatchStatus), &p_st));
+    MCK(A.get(M_JOBS, sizeof(PairJob), &p_jobs));
+    MCK(A.get(M_FWD, sizeof(float) * 2 * (size_t)n_q, &p_out));
+    Frame* df = (Frame*)p_frames;
+    const int32_t* d_blk = (const int32_t*)(df + 2);
+    MCK(cudaMemcpyAsync(p_desc, q, row * n_q, cudaMemcpyHostToDevice, st));
+    MCK(cudaMemcpyAsync((float*)p_desc + (size_t)n_q * DESC_LEN, t, row * n_t, cudaMemcpyHostToDevice, st));
+    MCK(cudaMemcpyAsync(df, frames, sizeof(frames), cudaMemcpyHostToDevice, st));
+    MCK(cudaMemcpyAsync(df + 2, blk, sizeof(blk), cudaMemcpyHostToDevice, st));
+    MCK(cudaMemcpyAsync(p_jobs, &job, sizeof(job), cudaMemcpyHostToDevice, st));
+    MCK(cudaMemsetAsync(p_maxn, 0, sizeof(int) * 2, st));
+    MCK(cudaMemsetAsync(p_st, 0, sizeof(MatchStatus), st));
+    MCK(cudaFuncSetAttribute(nearest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNearestSmem));
+    pack_kernel<<<(unsigned)nb, 256, 0, st>>>((const float*)p_desc, df, d_blk, 2, 0, (unsigned char*)p_pack,
+                                              (float*)p_norm, (int*)p_maxn, (MatchStatus*)p_st);
+    MCK(cudaGetLastError());
+    nearest_kernel<<<dim3(std::max(qb, tb), 2), kNearestThreads, kNearestSmem, st>>>(
+        (const PairJob*)p_jobs, df, (const unsigned char*)p_pack, (const float*)p_norm, 1, (Two*)p_two, (Two*)p_two + n_q,
+        ctx->d_fault);
+    MCK(cudaGetLastError());
+    distances_kernel<<<(n_q + 255) / 256, 256, 0, st>>>((const Two*)p_two, (const float*)p_norm, (const int*)p_maxn, n_q,
+                                                        (float*)p_out, (float*)p_out + n_q);
+    MCK(cudaGetLastError());
+    MatchStatus status{};
+    int fault = 0;
+    MCK(cudaMemcpyAsync(&status, p_st, sizeof(status), cudaMemcpyDeviceToHost, st));
+    MCK(cudaMemcpyAsync(&fault, ctx->d_fault, sizeof(int), cudaMemcpyDeviceToHost, st));
+    MCK(cudaMemcpyAsync(approx, p_out, sizeof(float) * n_q, cudaMemcpyDeviceToHost, st));
+    MCK(cudaMemcpyAsync(bound, (float*)p_out + n_q, sizeof(float) * n_q, cudaMemcpyDeviceToHost, st));
+    MCK(cudaStreamSynchronize(st));
+    if (fault) return report_fault(ctx);
+    if (status.wild) return mfail(ctx, RCMVS_E_LIMIT, "rcmvs_diag_match_distances: a component past the packed range");
+    return RCMVS_OK;
 }
 
 static int match_pairs_impl(rcmvs_ctx* ctx, const float* const* desc, const int32_t* n_desc, int32_t n_frames,
