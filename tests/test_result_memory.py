@@ -24,6 +24,7 @@ def test_allocator_hands_out_owned_arrays():
         at = _abi.result_alloc(None, field, 5)
         a = _abi.take_result(field)
         assert a.ctypes.data == at and a.shape == (5, k) and a.dtype == dtype
+        a[:] = 7  # unwritten memory may hold NaN
         _ordinary(a)
         assert _abi.take_result(field).shape == (0, k)  # taken once
         assert _abi.result_alloc(None, field, 2**62) is None  # too large: no memory
