@@ -46,10 +46,22 @@ sys.path.insert(0, ROOT)
 
 FP32_NOMINAL_TOPS = 148 * 128 * 1.965e9 / 1e12  # SMs x FP32 lanes x max clock (ops/s, no FMA pairing)
 # DRAM bytes (read + write) per reference pixel of one pass launch, from an
-# ncu capture of the staged pass kernel on 8 views at 960x720, K = 10 (learned
-# arm, mean of passes 0 and 1: 335.3 MB read + 172.3 MB written over 5.53
-# Mpx), scaled to the measured workload's pixels for roofline.traffic.
-PASS_DRAM_BYTES_PER_PX = (335305856 + 172263320) / (8 * 960 * 720)
+# ncu capture of the staged pass kernel on 8 views at 1920x1080, K = 10 (learned
+# arm, mean of its 4 passes: 1073.1 MB read + 546.3 MB written over 16.6 Mpx),
+# scaled to the measured workload's pixels for roofline.traffic.
+PASS_DRAM_BYTES_PER_PX = (1073147008 + 546319232) / (8 * 1920 * 1080)
+
+
+def plain_kernels(o):
+    """The init and passes that options o run (include/rcmvs.h, RCMVS_FLAG_*)."""
+    one_thread = o.threads_per_pixel in (0, 1)
+    staged = one_thread and not o.flags & (16 | 512)  # reference call sequence, lockstep
+    init = ("one-candidate init" if o.flags & 1 else "row-step init" if o.flags & 128 else
+            "staged init" if staged and not (o.tile_w or o.tile_h or o.flags & (2 | 8)) else "table-sweep init")
+    passes = ("staged passes" if staged else "five-lane passes" if not one_thread else
+              "lockstep passes" if o.flags & 512 else "streamed passes")
+    return f"{init}, {passes}"
+
 
 def configs():
     from rustcolmap_b200 import MvsOptions
@@ -435,8 +447,10 @@ def run_sfm(args):
         c.timing(False)
     frames, m = state["frames"], state["matches"]
     nfeat = [len(f.pts) for f in frames]
-    # the search makes three FP16 products of 128 components per distance, in each direction
-    ops = sum(nfeat[i] * nfeat[j] for i, j in pairs) * 128 * 2 * 3 * 2
+    # the work: one 128-component distance per descriptor pair; the search issues three FP16
+    # products for it, in each direction
+    ops = sum(nfeat[i] * nfeat[j] for i, j in pairs) * 128 * 2
+    issued_per_op = 3 * 2
     pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peaks = json.load(open(pk)) if os.path.exists(pk) else {}
     tensor_peak = peaks.get("bf16_tflops", 1590.0)
@@ -458,7 +472,10 @@ def run_sfm(args):
                          "peak": tensor_peak, "unit": "TFLOP/s", "frac": achieved / tensor_peak,
                          "traffic": None,
                          "peak_source": "MEASURED_PEAKS.json bf16_tflops" if peaks else "fallback 1590",
-                         "ops_per_launch": ops_per_launch, "avg_launch_ms": dist_launch_ms},
+                         "ops_per_launch": ops_per_launch, "avg_launch_ms": dist_launch_ms,
+                         "issued": achieved * issued_per_op, "issued_frac": achieved * issued_per_op / tensor_peak,
+                         "note": "achieved counts one product of 128 components per descriptor pair; issued "
+                                 "what the search gives the tensor pipe (FP16 hi.hi, hi.lo, lo.hi, both directions)"},
             "kernel_ms_per_step": {k: v[0] / args.steps for k, v in kt.items()},
             "e2e": {"value": value, "unit": "images/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "note": "value itself is measured through the host-buffer API (rcmvs_extract_sift, "
@@ -785,7 +802,7 @@ def main():
             "roofline": {"bound": "hbm", "kernel": "stereo_pass", "achieved": achieved_gbs, "peak": hbm_peak,
                          "unit": "GB/s", "frac": achieved_gbs / hbm_peak,
                          "traffic": PASS_DRAM_BYTES_PER_PX * npx,
-                         "traffic_source": "ncu dram bytes per pixel of an 8-view 960x720 K=10 capture of "
+                         "traffic_source": "ncu dram bytes per pixel of an 8-view 1920x1080 K=10 capture of "
                                            "the staged pass kernel (learned arm) x this launch's pixels",
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650",
                          "algorithmic_bytes_per_launch": bytes_per_launch, "avg_launch_ms": pass_avg_s * 1e3,
@@ -795,15 +812,19 @@ def main():
                                  "frac": achieved_tops / FP32_NOMINAL_TOPS if achieved_tops else None,
                                  "ops_per_term": fp32_ops_per_term,
                                  "peak_source": "nominal 148 SM x 128 FP32 lanes x 1.965 GHz",
-                                 "note": "achieved counts the terms evaluated; reference_equivalent counts the "
-                                         "terms the reference's call sequence evaluates for the same step "
-                                         "(duplicate skip off), over the same time",
+                                 "note": "work per time, not issue rate: achieved counts the terms that the "
+                                         "candidate-by-candidate kernels (streamed passes, table sweep) evaluate "
+                                         "for this step, over the time of the kernels that ran; the staged ones "
+                                         "evaluate others (looser limits, hypotheses ahead).  "
+                                         "reference_equivalent counts the terms of the reference's call sequence "
+                                         "(duplicate skip off) over the same time",
                                  "reference_equivalent": ref_tops,
                                  "reference_equivalent_frac": ref_tops / FP32_NOMINAL_TOPS if ref_tops else None},
             "gpu_launches": args.steps * per_step,
             "clocks": clocks,
             "e2e": e2e,
             "cpu_baseline": cpu,
+            # as compute_roofline: the candidate-by-candidate kernels' evaluations over this arm's time
             "gcost_evals_per_s_plain": evals * args.steps / (plain_ms / 1e3) / 1e9 if evals else None,
             "gcost_evals_per_s_plain_reference_equivalent":
                 ref_evals * args.steps / (plain_ms / 1e3) / 1e9 if ref_evals else None,
@@ -817,8 +838,7 @@ def main():
             "kernel_ms_per_step": {k: v[0] / args.steps for k, v in head_kt.items() if v[1]},
             "fused_points": head_pts,
             "setup_s": setup_s,
-            "kernels": ("one-candidate init" if opts.flags & 1 else
-                        "row-step init" if opts.flags & 128 else "table-sweep init"),
+            "kernels": plain_kernels(opts),
             "schedule": {"tile": f"{opts.tile_w}x{opts.tile_h}" if opts.tile_w else "8x8 (library default)",
                          "threads_per_pixel": max(opts.threads_per_pixel, 1), "flags": opts.flags,
                          "persistent_queue": bool(opts.flags & 2), "cuda_graph": bool(opts.flags & 4),
