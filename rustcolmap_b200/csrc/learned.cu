@@ -14,7 +14,8 @@
 //   loss/Adam kernels   training
 // The patch-match init that consumes the predictions (confident pixels take
 // the predicted plane, the others fall back to the plane sweep) is
-// init_learned_rows_kernel in stereo.cu.
+// init_learned_staged_kernel in stereo.cu (init_learned_rows_kernel with the
+// flags and tile shapes that keep the staged kernels off).
 //
 // Tensors are NHWC, BF16, channels padded to a multiple of 16.
 #include <cuda.h>

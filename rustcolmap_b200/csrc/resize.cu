@@ -24,9 +24,10 @@
 //
 //   taps_kernel    one thread per output coordinate of an axis: its first
 //                  tap, tap count and normalised weights (a table of m rows)
-//   vert_kernel    one thread per (output row, input column, channel): the
-//                  f32 image of mh rows; a warp reads consecutive bytes of
-//                  one input row per tap and shares its weight row
+//   vert_kernel    one thread per four neighbouring (column, channel)
+//                  elements of an output row: the f32 image of mh rows; a
+//                  warp reads consecutive bytes of one input row per tap and
+//                  shares its weight row
 //   horiz_kernel   one thread per output pixel: its channels, rounded, with
 //                  grey and RGB written together
 //   convert_kernel no resize: to_luma8 / to_rgb8 of the input

@@ -304,11 +304,14 @@ __device__ __forceinline__ float cost_row(const Smem& sm, int row, const SrcRegs
 // 10% slack for second-order terms; a term whose coordinate lies within E of
 // an integer (image borders are integers) is "near" and is evaluated by the
 // reference's chain, every other has the reference's pixel.  Typical E at
-// f = 2208: 0.001 px in x, 0.0005 px in y, so about 0.3% of the terms are
-// near (one bound for both axes and the whole image made it 1%, and the near
-// terms 39% of the pass).  Planes and sources that leave no bound (window
-// cells whose n.ray or depth in the source is close to the reference's gates)
-// take the reference's chain for every term.
+// f = 2208: 0.001 px in x, 0.0005 px in y, so few terms are near: 0.31% (8 views
+// of 1920x1080, K = 10, after the learned init), 0.19% (960x720, K = 8), 0.30%
+// (the same with k = -0.02), 0.08% (384x288, K = 4); one bound for both axes and
+// the whole image made it 1%, and the near terms 39% of the pass.  Over 97 million
+// random planes, sources and rays with a bound, distorted or not, the two values
+// lay at most 0.59 E apart.  Planes and sources that leave no bound (window cells
+// whose n.ray or depth in the source is close to the reference's gates) take the
+// reference's chain for every term.
 // RADIAL: some camera has k != 0; the distortion multiplies the bound of both
 // axes by 1 + 3.5 |k| r^2 and adds 8 f |xn| u.
 struct RayBox {
@@ -1190,8 +1193,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, RCMVS_STREAM_MINB)
 // running maximum of the means decides (to 2e-6; the rare closer call is
 // evaluated again row by row).
 //
-// What bounds it: instruction issue (78% of the slots, 24 of 32 lanes) and,
-// behind it, the census gathers.  12 passes over 16 views 960x720, K = 8:
+// What bounds it: instruction issue (67% of the slots, 23 to 24 of 32 lanes),
+// barriers between the stages and the census gathers.  12 passes over 16 views 960x720, K = 8:
 // 69.0 ms streamed, 37.4 staged; 4 passes after the learned init over 16 views
 // 1920x1080, K = 10: 164 -> 90 ms; 12 passes over 8 views 384x288, K = 4:
 // 11.3 -> 4.4 ms.  Of the 37.4 ms, 7.1 are the preparation, 19 source 0.  The rows'
@@ -2409,7 +2412,7 @@ __global__ void __launch_bounds__(256, 4)
                 }
                 __syncthreads();
                 if (alive) {
-                                const int bw = s_bx1[slot] - s_bx0[slot] + 1;
+                    const int bw = s_bx1[slot] - s_bx0[slot] + 1;
                     const int base = s_off[slot] + (ly - s_by0[slot]) * bw + (lx - s_bx0[slot]);
 #pragma unroll
                     for (int dy = 0; dy < 5; ++dy) {

@@ -24,6 +24,8 @@ FLAG_SEED_AND_SWEEP = 64  # learned init: seeded pixels also run the plane sweep
 FLAG_ROW_STEP_INIT = 128  # row-step plane sweep instead of the default staged sweep
 FLAG_NO_REPEAT_SKIP = 256  # evaluate unchanged neighbours' planes again (the repeat skip off)
 FLAG_LOCKSTEP_PASSES = 512  # passes one thread per pixel in lockstep (not staged)
+# The batched-schedule extensions together (their tilings run the table sweep;
+# the default flags' staged init is the faster one).
 FLAGS_BATCHED = FLAG_PERSISTENT | FLAG_CUDA_GRAPH | FLAG_AUTOTUNE
 
 
