@@ -346,13 +346,14 @@ __device__ __forceinline__ void direction(const PairJob& J, const Frame* frames,
 // accumulators per query block (128 columns each), one multiplying while the
 // other is read.  Warp 8's first thread loads and multiplies: step 2c is
 // block c's lo (queries hi), step 2c + 1 its hi (queries lo, then hi: the small
-// terms first, for the error bound); the load of step s + 2 starts when step s - 1's products are done, two steps
-// ahead of its use.  Warps 0-3 scan the first query block's values, 4-7 the
-// second's, one thread per query.  Bound by the tensor pipe (48 MMAs of
-// 128 x 128 x 16 per target block; 56% active over 170 pairs of 2048, 41% with one
-// query block per CTA) and the L2 reads of the target blocks.  12 frames of 2048, 66 pairs (both directions): 429 us (FP32 pipes:
-// 4158); one query block per CTA and 64 KB target blocks in two buffers: 547
-// us (the load of a block had one scan's time to arrive); with the four
+// terms first, for the error bound); the load of step s + 2 starts when step
+// s - 1's products are done, two steps ahead of its use.  Warps 0-3 scan the
+// first query block's values, 4-7 the second's, one thread per query.  Bound by
+// the tensor pipe (48 MMAs of 128 x 128 x 16 per target block; 56% active over
+// 170 pairs of 2048, 41% with one query block per CTA) and the L2 reads of the
+// target blocks.  12 frames of 2048, 66 pairs (both directions): 429 us (FP32
+// pipes: 4158); one query block per CTA and 64 KB target blocks in two buffers:
+// 547 us (the load of a block had one scan's time to arrive); with the four
 // smallest kept in branches: 1040 us.
 constexpr int NSLOT = 3;
 constexpr int kNearestThreads = 288;
